@@ -17,14 +17,19 @@
 // each of the 18 loads and stores of a warp is a contiguous row segment.  All
 // arithmetic is FP64 in the reference's expression order and this file is
 // compiled without FMA contraction (device and host), so every value rounds
-// as the reference's statement does.  check() sums on the host in the
-// reference's (j, i) loop order for the same reason.
+// as the reference's statement does; the collision and the two quotients of
+// macro are d2q9.cuh's, which give those bits with about 150 FP64 instructions
+// a node.  The FP64 pipe bounds the step: 1024^2 takes 331 us (3.17 GLUPS)
+// against 404 us with the statements written out (about 190 instructions).
+// check() sums on the host in the reference's (j, i) loop order for the same
+// reason.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
 
 #include "mglc.h"
+#include "d2q9.cuh"
 #include "lid2d.cuh"
 
 namespace mglc {
@@ -35,56 +40,18 @@ __device__ __constant__ int l2_ex[9] = {0, 1, 0, -1, 0, 1, -1, -1, 1};
 __device__ __constant__ int l2_ey[9] = {0, 0, 1, 0, -1, 1, 1, -1, -1};
 __device__ __constant__ int l2_op[9] = {0, 3, 4, 1, 2, 7, 8, 5, 6};
 
-// Quotients by the collision's constant divisors d = 6, 9, 12, 18, 36, rounded
-// exactly as IEEE division rounds them, from one multiply and one fused
-// multiply-add: x/d = RN(x*h + RN(x*l)) with h = 1/d rounded down and
-// l = 1/d - h rounded to nearest (a two-term reciprocal; Brisebarre, Muller and
-// Raina, "Accelerating correctly rounded floating-point division when the
-// divisor is known in advance", IEEE Trans. Computers 53(8), 2004).  Why the
-// rounding is the division's: d = 3*2^k or 9*2^k, so for normal x the exact
-// x/d lies at least ulp(x/d)/18 from every rounding midpoint (d times a
-// midpoint is an odd multiple of 2^(e-53), x an even one), while h + l is 1/d
-// to about 2^-106 relative, putting x*h + RN(x*l) within ~2^-104 relative of
-// x/d: no midpoint between them.  Zeros and infinities keep their signs
-// because l > 0, NaN stays NaN.  Inputs below 2^-900 in magnitude (x*l could
-// lose bits to underflow) take the true division: a node whose divided
-// values are not all normal-or-zero runs the division variant.
+// The two-term reciprocals of the collision's divisors (div_const, d2q9.cuh):
+// h = 1/d rounded down, l = 1/d - h rounded to nearest.  x/12 and x/18 need no
+// pair of their own: they are (x/6)/2 and 2 (x/36).
 constexpr double RH6 = 0x1.5555555555555p-3, RL6 = 0x1.5555555555555p-57;
 constexpr double RH9 = 0x1.c71c71c71c71cp-4, RL9 = 0x1.c71c71c71c71cp-58;
 constexpr double RH12 = 0x1.5555555555555p-4, RL12 = 0x1.5555555555555p-58;
 constexpr double RH18 = 0x1.c71c71c71c71cp-5, RL18 = 0x1.c71c71c71c71cp-59;
 constexpr double RH36 = 0x1.c71c71c71c71cp-6, RL36 = 0x1.c71c71c71c71cp-60;
-
-template <bool FAST>
-__device__ __forceinline__ double dv(double x, double d, double h, double l) {
-    return FAST ? __fma_rn(x, h, __dmul_rn(x, l)) : x / d;
-}
-
-// |x| >= 2^-900 (infinities and NaN included) or x == +-0
-__device__ __forceinline__ bool rcp_ok(double x) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    return ((b >> 52) & 0x7ff) >= 123 || (b << 1) == 0;
-}
-
-// f_post from m_post, evolution.f90:55-68, each quotient as its own rounded value
-template <bool FAST>
-__device__ __forceinline__ void l2_post(const double* mp, double* fp) {
-    const double q0 = dv<FAST>(mp[0], 9.0, RH9, RL9), q1a = dv<FAST>(mp[1], 36.0, RH36, RL36),
-                 q1b = dv<FAST>(mp[1], 18.0, RH18, RL18), q2a = dv<FAST>(mp[2], 18.0, RH18, RL18),
-                 q2b = dv<FAST>(mp[2], 36.0, RH36, RL36), q3 = dv<FAST>(mp[3], 6.0, RH6, RL6),
-                 q4 = dv<FAST>(mp[4], 6.0, RH6, RL6), q4b = dv<FAST>(mp[4], 12.0, RH12, RL12),
-                 q5 = dv<FAST>(mp[5], 6.0, RH6, RL6), q6 = dv<FAST>(mp[6], 6.0, RH6, RL6),
-                 q6b = dv<FAST>(mp[6], 12.0, RH12, RL12), q7 = mp[7] * 0.25, q8 = mp[8] * 0.25;
-    fp[0] = dv<FAST>(mp[0] - mp[1] + mp[2], 9.0, RH9, RL9);
-    fp[1] = q0 - q1a - q2a + q3 - q4 + q7;
-    fp[2] = q0 - q1a - q2a + q5 - q6 - q7;
-    fp[3] = q0 - q1a - q2a - q3 + q4 + q7;
-    fp[4] = q0 - q1a - q2a - q5 + q6 - q7;
-    fp[5] = q0 + q1b + q2b + q3 + q4b + q5 + q6b + q8;
-    fp[6] = q0 + q1b + q2b - q3 - q4b + q5 + q6b - q8;
-    fp[7] = q0 + q1b + q2b - q3 - q4b - q5 - q6b + q8;
-    fp[8] = q0 + q1b + q2b + q3 + q4b - q5 - q6b - q8;
-}
+static_assert(INV6_H == RH6 && INV6_L == RL6 && INV9_H == RH9 && INV9_L == RL9 &&
+                  INV18_H == RH18 && INV18_L == RL18 && INV36_H == RH36 && INV36_L == RL36 &&
+                  2 * RH12 == RH6 && 2 * RL12 == RL6 && RH18 == 2 * RH36 && RL18 == 2 * RL36,
+              "the collision's reciprocal pairs");
 
 struct L2K {
     const double* __restrict__ fin;
@@ -128,49 +95,11 @@ __global__ void __launch_bounds__(128) k_l2_step(L2K k) {
         r = k.rho[c];
         u = k.u[c];
         v = k.v[c];
-    } else {  // macro, evolution.f90:103-107
-        r = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8];
-        u = (f[1] - f[3] + f[5] - f[6] - f[7] + f[8]) / r;
-        v = (f[2] - f[4] + f[5] + f[6] - f[7] - f[8]) / r;
+    } else {
+        d2q9_macro(f, r, u, v);
     }
-    // collision, evolution.f90:16-68
-    double m[9], meq[9], s[9], mp[9], fp[9];
-    m[0] = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8];
-    m[1] = -4.0 * f[0] - f[1] - f[2] - f[3] - f[4] + 2.0 * (f[5] + f[6] + f[7] + f[8]);
-    m[2] = 4.0 * f[0] - 2.0 * (f[1] + f[2] + f[3] + f[4]) + f[5] + f[6] + f[7] + f[8];
-    m[3] = f[1] - f[3] + f[5] - f[6] - f[7] + f[8];
-    m[4] = -2.0 * f[1] + 2.0 * f[3] + f[5] - f[6] - f[7] + f[8];
-    m[5] = f[2] - f[4] + f[5] + f[6] - f[7] - f[8];
-    m[6] = -2.0 * f[2] + 2.0 * f[4] + f[5] + f[6] - f[7] - f[8];
-    m[7] = f[1] - f[2] + f[3] - f[4];
-    m[8] = f[5] - f[6] + f[7] - f[8];
-    meq[0] = r;
-    meq[1] = r * (-2.0 + 3.0 * (u * u + v * v));
-    meq[2] = r * (1.0 - 3.0 * (u * u + v * v));
-    meq[3] = r * u;
-    meq[4] = -r * u;
-    meq[5] = r * v;
-    meq[6] = -r * v;
-    meq[7] = r * (u * u - v * v);
-    meq[8] = r * (u * v);
-    s[0] = 0.0;
-    s[1] = k.snu;
-    s[2] = k.snu;
-    s[3] = 0.0;
-    s[4] = k.sq;
-    s[5] = 0.0;
-    s[6] = k.sq;
-    s[7] = k.snu;
-    s[8] = k.snu;
-#pragma unroll
-    for (int a = 0; a < 9; a++) mp[a] = m[a] - s[a] * (m[a] - meq[a]);
-    const bool fast = rcp_ok(mp[0]) && rcp_ok(mp[1]) && rcp_ok(mp[2]) && rcp_ok(mp[3]) &&
-                      rcp_ok(mp[4]) && rcp_ok(mp[5]) && rcp_ok(mp[6]) &&
-                      rcp_ok(mp[0] - mp[1] + mp[2]);
-    if (fast)
-        l2_post<true>(mp, fp);
-    else
-        l2_post<false>(mp, fp);
+    double fp[9];
+    d2q9_collide<true>(f, r, u, v, k.snu, k.sq, fp);
     // streaming + bounceback, evolution.f90:81-90 and bounceback.f90:6-42
 #pragma unroll
     for (int a = 0; a < 9; a++) {
