@@ -38,12 +38,13 @@ extern "C" {
 #define MGLC_ERR_PARTICLE 7    /* particle overlap or wall penetration */
 
 /* Storage / arithmetic form of the populations.
- *  FP64: FP64 storage and FP64 arithmetic -- the drop-in for the reference.
+ *  FP64: FP64 storage -- the drop-in for the reference.  The cavities' collisions
+ *  run in FP64 or, where the populations are in range, on 64-bit integers of
+ *  finer resolution (each result is closer to the exact collision).
  *  FP32/FP16/BF16: populations stored as deviations f_i - w_i*rho0 in that
  *  type, FP32 arithmetic; FP64 kept for reductions (residual, totals).
- *  FX64 (lid-driven and heated cavities): FP64 storage; the collisions run in
- *  64-bit fixed point with 55 fractional bits (exact moment transforms, one
- *  rounding to FP64 per stored value), everything else as FP64.
+ *  FX64 (lid-driven and heated cavities): as FP64, and a cell outside the range
+ *  box |f| < 1, 1/4 <= rho < 2, |u| < 1/2 writes NaN.
  *  FP16S/BF16S: FP16/BF16 deviation storage written with stochastic rounding
  *  (unbiased; the storage error stays at its one-step level instead of
  *  accumulating over a transient).  The stored state then fluctuates at the

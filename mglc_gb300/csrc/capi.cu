@@ -36,7 +36,7 @@ struct Range {
 
 struct mglc_ctx {
     int kind = 0, form = FORM_FP64;
-    bool fx64 = false;  // MGLC_FX64: FP64 storage (form FP64), Q55 fixed-point lid collision
+    bool fx64 = false;  // MGLC_FX64: FP64 (form FP64) with a range box
     P2Ctx* p2d = nullptr;  // MGLC_KIND_PARTICLE2D: the D2Q9 case4 state
     L2Ctx* l2d = nullptr;  // MGLC_KIND_LID2D: the D2Q9 lid-driven cavity
     bool sr = false;       // MGLC_FP16S / MGLC_BF16S: stochastic rounding of the 16-bit stores

@@ -132,125 +132,6 @@ __device__ __forceinline__ long long fx_recip(long long rho) {
     return x;
 }
 
-// Lid MRT collision (collision.f90:20-189, meq(12) without rho) on Q55
-// populations, in place.  FIRST: rho and u come from the stored macroscopic
-// fields; otherwise from the populations (rho u = j exactly).  Returns false
-// when rho or u leaves the range box.
-template <bool FIRST>
-__device__ __forceinline__ bool mrt_collide_fx(long long* f, long long rho_in, long long ux_in,
-                                               long long uy_in, long long uz_in,
-                                               const FxCoef& c, long long& rho_out) {
-    using ll = long long;
-    ll s1 = f[1] + f[2], d1 = f[1] - f[2];
-    ll s2 = f[3] + f[4], d2 = f[3] - f[4];
-    ll s3 = f[5] + f[6], d3 = f[5] - f[6];
-    ll s4 = f[7] + f[10], d4 = f[7] - f[10];
-    ll s5 = f[9] + f[8], d5 = f[9] - f[8];
-    ll s6 = f[11] + f[14], d6 = f[11] - f[14];
-    ll s7 = f[13] + f[12], d7 = f[13] - f[12];
-    ll s8 = f[15] + f[18], d8 = f[15] - f[18];
-    ll s9 = f[17] + f[16], d9 = f[17] - f[16];
-    const ll sa = s1 + s2 + s3;
-    const ll sxy = s4 + s5, sxz = s6 + s7, syz = s8 + s9;
-    const ll se = sxy + sxz + syz;
-    const ll ex_ = (d4 + d5) + (d6 + d7);
-    const ll ey_ = (d4 - d5) + (d8 + d9);
-    const ll ez_ = (d6 - d7) + (d8 - d9);
-    ll rho, ux, uy, uz, rux, ruy, ruz;
-    if (FIRST) {
-        rho = rho_in;
-        ux = ux_in;
-        uy = uy_in;
-        uz = uz_in;
-        rux = qmul(rho, ux);
-        ruy = qmul(rho, uy);
-        ruz = qmul(rho, uz);
-    } else {
-        rho = f[0] + sa + se;
-        rux = d1 + ex_;
-        ruy = d2 + ey_;
-        ruz = d3 + ez_;
-        const ll inv = fx_recip(rho);
-        ux = qmul(rux, inv);
-        uy = qmul(ruy, inv);
-        uz = qmul(ruz, inv);
-    }
-    rho_out = rho;
-    const ll uh = FX_ONE / 2;
-    const bool ok = rho >= FX_ONE / 4 && rho < 2 * FX_ONE && ux > -uh && ux < uh && uy > -uh &&
-                    uy < uh && uz > -uh && uz < uh;
-    const ll m1 = -30 * f[0] - 11 * sa + 8 * se;
-    const ll m2 = 12 * f[0] - 4 * sa + se;
-    const ll m4 = -4 * d1 + ex_;
-    const ll m6 = -4 * d2 + ey_;
-    const ll m8 = -4 * d3 + ez_;
-    const ll m9 = 2 * s1 - (s2 + s3) + (sxy + sxz) - 2 * syz;
-    const ll m10 = -4 * s1 + 2 * (s2 + s3) + (sxy + sxz) - 2 * syz;
-    const ll m11 = (s2 - s3) + (sxy - sxz);
-    const ll m12 = -2 * (s2 - s3) + (sxy - sxz);
-    const ll m13 = s4 - s5;
-    const ll m14 = s8 - s9;
-    const ll m15 = s6 - s7;
-    const ll m16 = (d4 + d5) - (d6 + d7);
-    const ll m17 = (d5 - d4) + (d8 + d9);
-    const ll m18 = (d6 - d7) - (d8 - d9);
-    // equilibrium parts
-    const ll ux2 = qmul(ux, ux), uy2 = qmul(uy, uy), uz2 = qmul(uz, uz);
-    const ll rusq = qmul(rho, ux2 + uy2 + uz2);
-    const ll p9 = 2 * ux2 - uy2 - uz2;
-    const ll p11 = uy2 - uz2;
-    const ll rp9 = qmul(rho, p9);
-    const ll n1 = m1 - (-11 * rho + 19 * rusq);
-    const ll n2 = m2 - (3 * rho - ((11 * rusq) >> 1));
-    const ll n4 = m4 + qmulc(2 * rux, FX_THIRD);
-    const ll n6 = m6 + qmulc(2 * ruy, FX_THIRD);
-    const ll n8 = m8 + qmulc(2 * ruz, FX_THIRD);
-    const ll n9 = m9 - rp9;
-    const ll n10 = m10 + (rp9 >> 1);
-    const ll n11 = m11 - qmul(rho, p11);
-    const ll n12 = m12 + (p11 >> 1);
-    const ll n13 = m13 - qmul(rux, uy);
-    const ll n14 = m14 - qmul(ruy, uz);
-    const ll n15 = m15 - qmul(rux, uz);
-    // r_k = c_k n_k
-    const ll r1 = qmulc(n1, c.c1), r2 = qmulc(n2, c.c2);
-    const ll r4 = qmulc(n4, c.c4), r6 = qmulc(n6, c.c4), r8 = qmulc(n8, c.c4);
-    const ll r9 = qmulc(n9, c.c9), r10 = qmulc(n10, c.c10), r11 = qmulc(n11, c.c11);
-    const ll r12 = qmulc(n12, c.c12);
-    const ll r13 = qmulc(n13, c.c13), r14 = qmulc(n14, c.c13), r15 = qmulc(n15, c.c13);
-    const ll r16 = qmulc(m16, c.c16), r17 = qmulc(m17, c.c16), r18 = qmulc(m18, c.c16);
-    // inverse transform M^T r by pairs (r3 = r5 = r7 = 0: conserved momentum)
-    const ll bax = -11 * r1 - 4 * r2;
-    const ll bed = 8 * r1 + r2;
-    f[0] -= -30 * r1 + 12 * r2;
-    const ll A9 = -r9 + 2 * r10, B11 = r11 - 2 * r12;
-    const ll S910 = r9 + r10, S1112 = r11 + r12;
-    const ll X = r4, Y = r6, Z = r8;
-    ll E, O;
-    E = bax + (2 * r9 - 4 * r10); O = -4 * r4;
-    f[1] -= E + O; f[2] -= E - O;
-    E = bax + A9 + B11; O = -4 * r6;
-    f[3] -= E + O; f[4] -= E - O;
-    E = bax + A9 - B11; O = -4 * r8;
-    f[5] -= E + O; f[6] -= E - O;
-    const ll be = bed + S910;
-    E = be + S1112 + r13; O = X + Y + (r16 - r17);
-    f[7] -= E + O; f[10] -= E - O;
-    E = be + S1112 - r13; O = X - Y + (r16 + r17);
-    f[9] -= E + O; f[8] -= E - O;
-    E = be - S1112 + r15; O = X + Z + (r18 - r16);
-    f[11] -= E + O; f[14] -= E - O;
-    E = be - S1112 - r15; O = X - Z - (r16 + r18);
-    f[13] -= E + O; f[12] -= E - O;
-    const ll bz = bed - 2 * S910;
-    E = bz + r14; O = Y + Z + (r17 - r18);
-    f[15] -= E + O; f[18] -= E - O;
-    E = bz - r14; O = Y - Z + (r17 + r18);
-    f[17] -= E + O; f[16] -= E - O;
-    return ok;
-}
-
-
 // ------------------------------------------------------------ heated cavity --
 // Constants of the forced D3Q19 MRT and of the D3Q7 MRT (bouyancy3d_mpi.F90:
 // 641-864, 1014-1070) for the Q55 form.  Factors below 1/2 are round(c 2^64)

@@ -29,16 +29,6 @@ __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
                                 K.seed);
 }
 
-template <bool FIRST, typename IDX>
-__global__ void __launch_bounds__(128)
-    k_lid_step_fx(const double* __restrict__ fin, double* __restrict__ fout, FxK K, IDX P,
-                  const double* __restrict__ mrho, const double* __restrict__ mu,
-                  const double* __restrict__ mv, const double* __restrict__ mw) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K.nx) return;
-    lid_cell_fx<FIRST, IDX>(i, blockIdx.y, blockIdx.z, fin, fout, K, P, mrho, mu, mv, mw);
-}
-
 // 4 blocks of 128 per SM (128 registers): measured faster than the 168-register
 // allocation at 3 blocks and than 5 blocks with spills
 template <bool FIRST, bool ROT, typename IDX>
@@ -80,9 +70,10 @@ static dim3 step_grid(const Geom& g, dim3 b) {
 
 template <typename S>
 static cudaError_t lid_go(bool first, const void* fin, void* fout, const LidStepArgs& a,
-                          cudaStream_t s) {
+                          cudaStream_t s, bool box = false) {
     using C = typename St<S>::C;
     StepK<C> K = make_k<C>(a.g, a.cd, a.u0, a.rho0, a.scale, a.inv_scale);
+    set_box(K.pk, box);
     K.seed = a.seed;
     K.sr = a.sr;
     dim3 b = step_block(a.g.nx), gr = step_grid(a.g, b);
@@ -105,30 +96,10 @@ static cudaError_t lid_go(bool first, const void* fin, void* fout, const LidStep
     return cudaGetLastError();
 }
 
-static cudaError_t lid_go_fx(bool first, const void* fin, void* fout, const LidStepArgs& a,
-                             cudaStream_t s) {
-    FxK K;
-    K.nx = a.g.nx; K.ny = a.g.ny; K.nz = a.g.nz;
-    K.c = make_fx_coef(a.cd, a.u0);
-    dim3 b = step_block(a.g.nx), gr = step_grid(a.g, b);
-    const bool small = (long long)Q19 * a.g.plane < (1ll << 31);
-    const double* fi = (const double*)fin;
-    double* fo = (double*)fout;
-#define FX_LAUNCH(FI, IT) \
-    k_lid_step_fx<FI, IT><<<gr, b, 0, s>>>(fi, fo, K, (IT)a.g.plane, a.rho, a.u, a.v, a.w)
-    if (small) {
-        if (first) FX_LAUNCH(true, unsigned); else FX_LAUNCH(false, unsigned);
-    } else {
-        if (first) FX_LAUNCH(true, long long); else FX_LAUNCH(false, long long);
-    }
-#undef FX_LAUNCH
-    return cudaGetLastError();
-}
-
 cudaError_t launch_lid_step(int form, bool first, const void* fin, void* fout,
                             const LidStepArgs& a, cudaStream_t s) {
     switch (form) {
-        case FORM_FX64: return lid_go_fx(first, fin, fout, a, s);
+        case FORM_FX64: return lid_go<double>(first, fin, fout, a, s, true);
         case FORM_FP64: return lid_go<double>(first, fin, fout, a, s);
         case FORM_FP32: return lid_go<float>(first, fin, fout, a, s);
         case FORM_FP16: return lid_go<__half>(first, fin, fout, a, s);
@@ -149,6 +120,7 @@ static cudaError_t th_go(bool first, const void* fin, void* fout, const void* gi
     K.chot = (C)((6.0 + a.para_a) / 21.0 * a.t_hot);
     K.ccold = (C)((6.0 + a.para_a) / 21.0 * a.t_cold);
     K.bc_y = a.bc_y; K.bc_z = a.bc_z;
+    pair_k_heat(K.pk, a.para_a, a.qd, a.qnu);
     dim3 b = step_block(a.g.nx), gr = step_grid(a.g, b);
     const bool rot = a.omega_rot != 0.0;
     const bool small = (long long)Q19 * a.g.plane < (1ll << 31);

@@ -25,17 +25,6 @@ __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
     lid_cell_from<S, FIRST, IDX, SR, !ODD>(i, j, k, raw, f, K, P, mrho, mu, mv, mw, K.seed);
 }
 
-// FX64 lid cavity in place (FP64 storage, Q55 collision)
-template <bool FIRST, typename IDX, bool ODD>
-__global__ void __launch_bounds__(128, 4)
-    k_lid_step_fx_aa(double* f, FxK K, IDX P, const double* __restrict__ mrho,
-                     const double* __restrict__ mu, const double* __restrict__ mv,
-                     const double* __restrict__ mw) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K.nx) return;
-    lid_cell_fx<FIRST, IDX, ODD ? 2 : 1>(i, blockIdx.y, blockIdx.z, f, f, K, P, mrho, mu, mv, mw);
-}
-
 // FX64 heated cavity in place (4 blocks of 128 per SM, as the two-buffer kernel)
 template <bool FIRST, bool ROT, typename IDX, bool ODD>
 __global__ void __launch_bounds__(128, 4)
@@ -105,9 +94,11 @@ dim3 aa_block(int nx) {
 }
 
 template <typename S>
-cudaError_t lid_go_aa(bool first, bool odd, void* f, const LidStepArgs& a, cudaStream_t s) {
+cudaError_t lid_go_aa(bool first, bool odd, void* f, const LidStepArgs& a, cudaStream_t s,
+                      bool box = false) {
     using C = typename St<S>::C;
     StepK<C> K = make_k<C>(a.g, a.cd, a.u0, a.rho0, a.scale, a.inv_scale);
+    set_box(K.pk, box);
     K.seed = a.seed;
     K.sr = a.sr;
     const dim3 b = aa_block(a.g.nx), gr((a.g.nx + b.x - 1) / b.x, a.g.ny, a.g.nz);
@@ -138,28 +129,6 @@ cudaError_t lid_go_aa(bool first, bool odd, void* f, const LidStepArgs& a, cudaS
     return cudaGetLastError();
 }
 
-cudaError_t lid_go_fx_aa(bool first, bool odd, void* f, const LidStepArgs& a, cudaStream_t s) {
-    FxK K;
-    K.nx = a.g.nx; K.ny = a.g.ny; K.nz = a.g.nz;
-    K.c = make_fx_coef(a.cd, a.u0);
-    const dim3 b = aa_block(a.g.nx), gr((a.g.nx + b.x - 1) / b.x, a.g.ny, a.g.nz);
-    double* fp = (double*)f;
-    const bool small = (long long)Q19 * a.g.plane < (1ll << 31);
-#define FA_LAUNCH(FI, IT, OD) \
-    k_lid_step_fx_aa<FI, IT, OD><<<gr, b, 0, s>>>(fp, K, (IT)a.g.plane, a.rho, a.u, a.v, a.w)
-    if (small) {
-        if (odd) FA_LAUNCH(false, unsigned, true);
-        else if (first) FA_LAUNCH(true, unsigned, false);
-        else FA_LAUNCH(false, unsigned, false);
-    } else {
-        if (odd) FA_LAUNCH(false, long long, true);
-        else if (first) FA_LAUNCH(true, long long, false);
-        else FA_LAUNCH(false, long long, false);
-    }
-#undef FA_LAUNCH
-    return cudaGetLastError();
-}
-
 template <typename S, int Q>
 cudaError_t swap_go(const Geom& g, void* f, cudaStream_t s) {
     const dim3 b = aa_block(g.nx), gr((g.nx + b.x - 1) / b.x, g.ny, g.nz);
@@ -182,6 +151,7 @@ cudaError_t th_go_aa(bool first, bool odd, void* f, void* g, void* F, const Ther
     K.chot = (C)((6.0 + a.para_a) / 21.0 * a.t_hot);
     K.ccold = (C)((6.0 + a.para_a) / 21.0 * a.t_cold);
     K.bc_y = a.bc_y; K.bc_z = a.bc_z;
+    pair_k_heat(K.pk, a.para_a, a.qd, a.qnu);
     const dim3 b = aa_block(a.g.nx), gr((a.g.nx + b.x - 1) / b.x, a.g.ny, a.g.nz);
     const bool rot = a.omega_rot != 0.0;
     const bool small = (long long)Q19 * a.g.plane < (1ll << 31);
@@ -221,7 +191,7 @@ cudaError_t launch_lid_step_aa(int form, bool first, bool odd, void* f, const Li
                                cudaStream_t s) {
     if (first && odd) return cudaErrorInvalidValue;
     switch (form) {
-        case FORM_FX64: return lid_go_fx_aa(first, odd, f, a, s);
+        case FORM_FX64: return lid_go_aa<double>(first, odd, f, a, s, true);
         case FORM_FP64: return lid_go_aa<double>(first, odd, f, a, s);
         case FORM_FP32: return lid_go_aa<float>(first, odd, f, a, s);
         case FORM_FP16: return lid_go_aa<__half>(first, odd, f, a, s);

@@ -18,6 +18,7 @@
 //    each opposite pair, about 3/4 of the moment form's operations.
 // Results differ from the literal form only by rounding (a few ulp per step).
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -445,6 +446,218 @@ __device__ __forceinline__ void trt_collide_t(T* g, T temp, T ux, T uy, T uz, T 
     pair(1, 2, temp * ux);
     pair(3, 4, temp * uy);
     pair(5, 6, temp * uz);
+}
+
+// ------------------------------------------- FP64: the pair form, regrouped --
+// The FP64 kernels are bound by the FP64 pipe, so they take the pair form with
+// the rates folded into the equilibrium.  With t = f_a + f_b, d = f_a - f_b (sums
+// that the density and momentum need anyway),
+//     f_a' = p + m,  f_b' = p - m,   p = (1 - Snu)/2 t + Snu/2 E,
+//                                    m = (1 - Sq)/2 d + Sq/2 O,
+// and with k = Snu/8 rho u (heated: Snu/8 V) the even equilibria come from the
+// six products X = k_x u_x, ..., c_xy = k_x u_y, ...: per unit of Snu/2,
+//     rest and base  b = Snu/36 rho - (X + Y + Z)/3,
+//     axis           2 b + 2 X,
+//     edges          b + X + Y +- 2 c_xy,
+// the odd ones from the momentum itself (rho u = j).  134 FP64 instructions a
+// lid cell with the moments against 149 for trt_collide_lid; the roundings are
+// other ones of the same size (measured against the reference's statements in
+// 64 bits: tests/test_lid_gpu.py and the host test of the formulas).
+// Reciprocal of a density, FP64: Newton-Raphson refinement r <- r + r(1 - x r)
+// of a single-precision seed; two steps take the 2^-23 seed error below 2^-52
+// with four FP64 FMAs, about half the FP64 work of an IEEE division.
+__device__ __forceinline__ double recip64(double x) {
+    double r = (double)__frcp_rn((float)x);
+    double e = fma(-x, r, 1.0);
+    r = fma(r, e, r);
+    e = fma(-x, r, 1.0);
+    return fma(r, e, r);
+}
+
+// coefficient |c| < 1/2 as two signed digits: C = c * 2^64 = h * 2^32 + l
+struct FixC {
+    int h, l;
+};
+inline FixC fix_coef(long long C) {
+    FixC k;
+    k.l = (int)(unsigned)((unsigned long long)C & 0xFFFFFFFFull);
+    k.h = (int)((C - (long long)k.l) >> 32);
+    return k;
+}
+// x / d * 2^64, rounded to nearest, for 0 <= x < 2 and d >= 4 (exact integers: a
+// double quotient's own rounding would be larger than 2^-64)
+inline long long fix_ratio(double x, int d) {
+    int e = 0;
+    const long long m = (long long)std::ldexp(std::frexp(x, &e), 53);  // x = m 2^(e - 53)
+    const int s = e + 11;
+    __int128 v = s >= 0 ? (__int128)m << s : (s > -63 ? (__int128)m >> -s : 0);
+    return (long long)((v * 2 / d + 1) / 2);
+}
+// coefficients of the collision on the integer pipe (fix61.cuh)
+struct FixK {
+    FixC c1, c2, l18, l0, l8, l6;  // (1-Snu)/2, (1-Sq)/2, Snu/36, Snu/6, Snu/4, Sq/12
+    FixC l19, l10, third, sixth;   // Snu/19, Sq/10, -1/3, 1/6
+    int on;                        // the rates are in range
+};
+inline FixK make_fix_k(double snu, double sq) {
+    FixK k;
+    // rates of a viscosity in use; others take the FP64 form
+    auto in = [](double s) { return s >= 0x1p-20 && s <= 2.0 - 0x1p-20; };
+    k.on = in(snu) && in(sq);
+    if (!k.on) return FixK{};
+    const long long half = 1LL << 62;  // 1/4
+    // (1 - s)/2 = 2 (1/4 - s/4), in halves of a unit
+    k.c1 = fix_coef(2 * (half - fix_ratio(snu, 4)));
+    k.c2 = fix_coef(2 * (half - fix_ratio(sq, 4)));
+    k.l18 = fix_coef(fix_ratio(snu, 36));
+    k.l0 = fix_coef(fix_ratio(snu, 6));
+    k.l8 = fix_coef(fix_ratio(snu, 4));
+    k.l6 = fix_coef(fix_ratio(sq, 12));
+    k.l19 = fix_coef(fix_ratio(snu, 19));
+    k.l10 = fix_coef(fix_ratio(sq, 10));
+    k.third = fix_coef(-6148914691236517205LL);
+    k.sixth = fix_coef(3074457345618258603LL);
+    return k;
+}
+// Coefficients, converted once on the host; empty for the other types.
+template <typename T>
+struct PairK {};
+template <>
+struct PairK<double> {
+    double c1, c2, om;             // (1 - Snu)/2, (1 - Sq)/2, 1 - Snu
+    double le4, le18;              // Snu/8, Snu/36
+    double lo3, lo6;               // Sq/6, Sq/12
+    double kv, kw6, lo10;          // forced: (1 - Snu/2)/4, (1 - Sq/2)/12, Sq/20
+    FixK fix;                         // the collision on integers (fix61.cuh)
+    int box;                          // FX64: a cell outside its range box writes NaN
+    double g1, g2, gom, ge0, gE, gd;  // D3Q7: (1-qnu)/2, (1-qd)/2, 1-qnu, its equilibria, qd/2
+};
+template <typename T>
+inline PairK<T> make_pair_k(double, double) { return PairK<T>{}; }
+template <>
+inline PairK<double> make_pair_k<double>(double snu, double sq) {
+    PairK<double> k{};
+    const double le = 0.5 * snu, lo = 0.5 * sq;
+    k.c1 = 0.5 - le; k.c2 = 0.5 - lo; k.om = 1.0 - snu;
+    k.le4 = 0.25 * le; k.le18 = le / 18.0;
+    k.lo3 = lo / 3.0; k.lo6 = lo / 6.0;
+    // le/4 * (1 - le)/le and lo/6 * (1 - lo)/(2 lo)... the relaxed source's shares
+    k.kv = 0.25 * (1.0 - le);
+    k.kw6 = (1.0 - lo) / 12.0;
+    k.lo10 = lo / 10.0;
+    k.fix = make_fix_k(snu, sq);
+    return k;
+}
+// D3Q7 part: g' = g - qnu (g - geq)^+ - qd (g - geq)^-, geq as trt_collide_t
+inline void pair_k_heat(PairK<double>& k, double para_a, double qd, double qnu) {
+    k.g1 = 0.5 - 0.5 * qnu; k.g2 = 0.5 - 0.5 * qd; k.gom = 1.0 - qnu;
+    k.ge0 = qnu * (1.0 - para_a) / 7.0;
+    k.gE = 0.5 * qnu * (6.0 + para_a) / 21.0;
+    k.gd = 0.5 * qd;
+}
+template <typename T>
+inline void pair_k_heat(PairK<T>&, double, double, double) {}
+inline void set_box(PairK<double>& k, bool on) { k.box = on ? 1 : 0; }
+template <typename T>
+inline void set_box(PairK<T>&, bool) {}
+
+// one pair: p from t and its even equilibrium, m from d and its odd one
+__device__ __forceinline__ void pair_out(double* f, int a, int b, double c1, double c2, double E,
+                                         double O) {
+    const double p = c1 * (f[a] + f[b]) + E, m = c2 * (f[a] - f[b]) + O;
+    f[a] = p + m;
+    f[b] = p - m;
+}
+
+// the lid collision (trt_collide_lid) of a cell whose rho, j and u = j inv,
+// inv = 1/rho, come from f
+__device__ __forceinline__ void pair_collide_lid(double* f, double rho, double jx, double jy,
+                                                 double jz, double inv, double ux, double uy,
+                                                 double uz, const PairK<double>& k) {
+    const double ke = rho * k.le4;
+    const double kx = ke * ux, ky = ke * uy, kz = ke * uz;
+    const double X = kx * ux, Y = ky * uy, Z = kz * uz;
+    const double cxy = kx * uy, cxz = kx * uz, cyz = ky * uz;
+    const double sxy = X + Y, sxz = X + Z, syz = Y + Z;
+    const double b = rho * k.le18 - (1.0 / 3.0) * (sxy + Z);
+    // meq(12) without rho: le D/3 with D = (rho - 1)(uy^2 - uz^2)/2 (trt_collide_lid)
+    const double q = (Y - Z) * (1.0 / 3.0 - (1.0 / 3.0) * inv);
+    const double b2 = b + b;
+    const double bxy = (b + 0.5 * q) + sxy, bxz = (b - 0.5 * q) + sxz, byz = b + syz;
+    const double gx = jx * k.lo6, gy = jy * k.lo6, gz = jz * k.lo6;
+    f[0] = k.om * f[0] + 12.0 * b;
+    pair_out(f, 1, 2, k.c1, k.c2, b2 + 2.0 * X, jx * k.lo3);
+    pair_out(f, 3, 4, k.c1, k.c2, (b2 - q) + 2.0 * Y, jy * k.lo3);
+    pair_out(f, 5, 6, k.c1, k.c2, (b2 + q) + 2.0 * Z, jz * k.lo3);
+    pair_out(f, 7, 10, k.c1, k.c2, bxy + 2.0 * cxy, gx + gy);
+    pair_out(f, 9, 8, k.c1, k.c2, bxy - 2.0 * cxy, gx - gy);
+    pair_out(f, 11, 14, k.c1, k.c2, bxz + 2.0 * cxz, gx + gz);
+    pair_out(f, 13, 12, k.c1, k.c2, bxz - 2.0 * cxz, gx - gz);
+    pair_out(f, 15, 18, k.c1, k.c2, byz + 2.0 * cyz, gy + gz);
+    pair_out(f, 17, 16, k.c1, k.c2, byz - 2.0 * cyz, gy - gz);
+}
+
+// the forced collision (trt_collide_forced): J = rho u = j + Fp/2, F this
+// step's force, dF = F - Fp (DF: not zero); ROT: F_x, F_y are not zero
+template <bool ROT, bool DF>
+__device__ __forceinline__ void pair_collide_forced(double* f, double rho, double Jx, double Jy,
+                                                    double Jz, double ux, double uy, double uz,
+                                                    double fx, double fy, double fz, double dfx,
+                                                    double dfy, double dfz,
+                                                    const PairK<double>& k) {
+    // Snu/8 V, V = rho u + (1 - le)/le F
+    const double vx = ROT ? Jx * k.le4 + k.kv * fx : Jx * k.le4;
+    const double vy = ROT ? Jy * k.le4 + k.kv * fy : Jy * k.le4;
+    const double vz = Jz * k.le4 + k.kv * fz;
+    const double X = ux * vx, Y = uy * vy, Z = uz * vz;
+    // half the sums of cross products: e.u e.V on the edges
+    const double cxy = ROT ? 0.5 * (ux * vy + uy * vx) : ux * vy;
+    const double cxz = 0.5 * (ux * vz + uz * vx), cyz = 0.5 * (uy * vz + uz * vy);
+    const double sxy = X + Y, sxz = X + Z, syz = Y + Z;
+    const double b = rho * k.le18 - (1.0 / 3.0) * (sxy + Z);
+    const double b2 = b + b, bxy = b + sxy, bxz = b + sxz, byz = b + syz;
+    // Sq/12 W, W = rho u + (1 - lo)/(2 lo) F, and Sq/20 dF
+    double wx = Jx * k.lo6, wy = Jy * k.lo6, ax, ay;
+    if (ROT) {
+        wx = wx + k.kw6 * fx;
+        wy = wy + k.kw6 * fy;
+    }
+    double wz = Jz * k.lo6 + k.kw6 * fz, az;
+    if (DF && ROT) {
+        ax = 2.0 * wx + k.lo10 * dfx;
+        ay = 2.0 * wy + k.lo10 * dfy;
+        wx = wx + k.lo10 * dfx;
+        wy = wy + k.lo10 * dfy;
+    } else {
+        ax = 2.0 * wx;
+        ay = 2.0 * wy;
+    }
+    if (DF) {
+        az = 2.0 * wz + k.lo10 * dfz;
+        wz = wz + k.lo10 * dfz;
+    } else {
+        az = 2.0 * wz;
+    }
+    f[0] = k.om * f[0] + 12.0 * b;
+    pair_out(f, 1, 2, k.c1, k.c2, b2 + 2.0 * X, ax);
+    pair_out(f, 3, 4, k.c1, k.c2, b2 + 2.0 * Y, ay);
+    pair_out(f, 5, 6, k.c1, k.c2, b2 + 2.0 * Z, az);
+    pair_out(f, 7, 10, k.c1, k.c2, bxy + 2.0 * cxy, wx + wy);
+    pair_out(f, 9, 8, k.c1, k.c2, bxy - 2.0 * cxy, wx - wy);
+    pair_out(f, 11, 14, k.c1, k.c2, bxz + 2.0 * cxz, wx + wz);
+    pair_out(f, 13, 12, k.c1, k.c2, bxz - 2.0 * cxz, wx - wz);
+    pair_out(f, 15, 18, k.c1, k.c2, byz + 2.0 * cyz, wy + wz);
+    pair_out(f, 17, 16, k.c1, k.c2, byz - 2.0 * cyz, wy - wz);
+}
+
+// D3Q7 (trt_collide_t): temp = sum g
+__device__ __forceinline__ void pair_collide_t(double* g, double temp, double ux, double uy,
+                                               double uz, const PairK<double>& k) {
+    const double E = temp * k.gE, h = temp * k.gd;
+    g[0] = k.gom * g[0] + temp * k.ge0;
+    pair_out(g, 1, 2, k.g1, k.g2, E, h * ux);
+    pair_out(g, 3, 4, k.g1, k.g2, E, h * uy);
+    pair_out(g, 5, 6, k.g1, k.g2, E, h * uz);
 }
 
 }  // namespace mglc

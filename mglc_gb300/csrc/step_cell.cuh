@@ -7,6 +7,7 @@
 
 #include <type_traits>
 
+#include "fix61.cuh"
 #include "fixed64.cuh"
 #include "kernels.cuh"
 
@@ -153,28 +154,18 @@ __device__ __forceinline__ void st_chk(T* p, IDX idx, IDX limit, V v) {
 }
 
 // Reciprocal of the density (rho is within a few percent of 1 in every
-// cavity flow).  FP32: the hardware reciprocal.  FP64: Newton-Raphson
-// refinement r <- r + r(1 - x r) of a single-precision seed; two steps take
-// the 2^-23 seed error below 2^-52 with four FP64 FMAs, about half the FP64
-// work of an IEEE division.
+// cavity flow).  FP32: the hardware reciprocal; FP64: recip64.
 __device__ __forceinline__ float recip(float x) { return __frcp_rn(x); }
-__device__ __forceinline__ double recip(double x) {
-    double r = (double)__frcp_rn((float)x);
-    double e = fma(-x, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-x, r, 1.0);
-    return fma(r, e, r);
-}
+__device__ __forceinline__ double recip(double x) { return recip64(x); }
 
-// Minimum resident blocks of 128 threads per SM for the lid step kernels: the
-// FP64 kernels are bound by the FP64 pipe, and 8 blocks (64 registers, a few
-// spilled values) measured 5% faster at 384^3 than the compiler's own 80
-// registers and 6 blocks (7 blocks: 4%); the other forms keep the compiler's
-// choice (0: no bound; a bound of 12 or 16 blocks slowed the 16-bit kernels by
-// 7-30%).
+// Minimum resident blocks of 128 threads per SM for the lid step kernels.  The
+// FP64 kernels, on the integer pipe, ran best at 5 (100 registers): 384^3 in
+// 3309 us a step, 3348 at 6 and 3557 at 4 (most populations converted back on
+// the FP64 unit); the other forms keep the compiler's choice (0: no bound; a
+// bound of 12 or 16 blocks slowed the 16-bit kernels by 7-30%).
 template <typename S>
 struct LidMinBlocks {
-    static constexpr int value = std::is_same<S, double>::value ? 8 : 0;
+    static constexpr int value = std::is_same<S, double>::value ? 5 : 0;
 };
 
 // Scalar constants converted once on the host to the arithmetic type.
@@ -189,6 +180,7 @@ struct StepK {
     // thermal
     C gbeta, omega_rot, t_ref, para_a, qd, qnu, chot, ccold;
     int bc_y, bc_z;
+    PairK<C> pk;  // FP64 only
 };
 
 template <typename C>
@@ -199,7 +191,19 @@ inline StepK<C> make_k(const Geom& g, const MrtCoef<double>& cd, double u0, doub
     k.u0 = (C)u0; k.rho0 = (C)rho0;
     k.scale = scale; k.inv_scale = inv_scale;
     k.c = cast_coef<C>(cd);
+    k.pk = make_pair_k<C>(cd.snu, 2.0 * cd.lo);
     return k;
+}
+
+// The range box of FX64: |f| < 1, 1/4 <= rho < 2, |u| < 1/2; a cell outside it,
+// or holding a NaN or an infinity, writes NaN.
+__device__ __forceinline__ bool out_of_box(double rho, double ux, double uy, double uz) {
+    return !(rho >= 0.25 && rho < 2.0 && fabs(ux) < 0.5 && fabs(uy) < 0.5 && fabs(uz) < 0.5);
+}
+template <int N>
+__device__ __forceinline__ void set_nan(double (&f)[N]) {
+#pragma unroll
+    for (int q = 0; q < N; q++) f[q] = __longlong_as_double(0x7ff8000000000000LL);
 }
 
 // Face mask of a cell: bit 0/1 = low/high x face, 2/3 = y, 4/5 = z.
@@ -290,41 +294,82 @@ __device__ __forceinline__ void lid_cell_from(int i, int j, int k, const S (&raw
     C f[Q19];
 #pragma unroll
     for (int q = 0; q < Q19; q++) f[q] = St<S>::cvt_s(raw[q]);
-    C rho_m, rho, ux, uy, uz;
-    if (FIRST) {
-        rho = (C)mrho[cell];
-        ux = (C)mu[cell];
-        uy = (C)mv[cell];
-        uz = (C)mw[cell];
-        rho_m = St<S>::SHIFT ? (rho - K.rho0) * sc : rho;
+    C rho, rhos;
+    if constexpr (std::is_same<S, double>::value) {
+        // in range: on the integer pipe (fix61.cuh); else the FP64 pair form
+        bool ok = K.pk.fix.on && fix61_ok(f);
+        if (ok) {
+            long long F[Q19], r = 0;
+#pragma unroll
+            for (int q = 0; q < Q19; q++) F[q] = fix61_load(f[q]);
+            if (FIRST)
+                ok = fix61_collide_lid<true>(F, K.pk.fix, r, mrho[cell], mu[cell], mv[cell], mw[cell]);
+            else
+                ok = fix61_collide_lid<false>(F, K.pk.fix, r);
+            rho = (double)r * (1.0 / FIX_ONE);
+            fix61_store_all(F, f);  // (out of range after all: the same values back)
+            if (K.pk.box && rho >= 2.0) set_nan(f);
+        }
+        if (!ok) {
+            C jx, jy, jz, ux, uy, uz;
+            bool bad = false;
+#pragma unroll
+            for (int q = 0; q < Q19; q++) bad |= !(fabs(f[q]) < 1.0);
+            moments0(f, rho, jx, jy, jz);
+            if (FIRST) {
+                const double rf = rho;
+                rho = mrho[cell];
+                ux = mu[cell];
+                uy = mv[cell];
+                uz = mw[cell];
+                trt_collide_lid<C, true>(f, rho, rho, ux, uy, uz, K.c, C(1), rf - rho,
+                                         jx - rho * ux, jy - rho * uy, jz - rho * uz);
+            } else {
+                const C inv = recip(rho);
+                ux = jx * inv;
+                uy = jy * inv;
+                uz = jz * inv;
+                pair_collide_lid(f, rho, jx, jy, jz, inv, ux, uy, uz, K.pk);
+            }
+            if (K.pk.box && (bad || out_of_box(rho, ux, uy, uz))) set_nan(f);
+        }
+        rhos = rho;
     } else {
-        C jx, jy, jz;
-        moments0(f, rho_m, jx, jy, jz);
-        rho = St<S>::SHIFT ? K.rho0 + (St<S>::SCALED ? rho_m * (C)K.inv_scale : rho_m) : rho_m;
-        const C inv = St<S>::SCALED ? recip(rho) * (C)K.inv_scale : recip(rho);
-        ux = jx * inv;
-        uy = jy * inv;
-        uz = jz * inv;
-    }
-    const C rhos = St<S>::SCALED ? rho * sc : rho;
-    // The pair form rounds the equilibrium itself (error ~ eps |feq|, where
-    // the moment form rounds only m - meq), and that rounding leaks into the
-    // conserved density and momentum step after step.  In FP64 the leak is
-    // ~1e-15 relative and in the 16-bit forms far below the storage error,
-    // but FP32 storage keeps 1e-7 of the FP64 result only with the moment
-    // form (64^3, Re = 400, 2000 steps: velocity 4e-6 with the pair form).
-    // The first step after initial or load takes rho and u from the macro
-    // arrays, so the pair form adds back what its relaxation would take from
-    // the conserved sums of f (zero when the arrays agree with f).
-    if (std::is_same<S, float>::value) {
-        mrt_collide<C, false, true>(f, rho_m, rhos, ux, uy, uz, C(0), C(0), C(0), K.c, sc);
-    } else if (FIRST) {
-        C rf, jx, jy, jz;
-        moments0(f, rf, jx, jy, jz);
-        trt_collide_lid<C, true>(f, rho_m, rhos, ux, uy, uz, K.c, sc, rf - rho_m,
-                                 jx - rhos * ux, jy - rhos * uy, jz - rhos * uz);
-    } else {
-        trt_collide_lid<C>(f, rho_m, rhos, ux, uy, uz, K.c, sc);
+        C rho_m, ux, uy, uz, jx, jy, jz, inv;
+        if (FIRST) {
+            rho = (C)mrho[cell];
+            ux = (C)mu[cell];
+            uy = (C)mv[cell];
+            uz = (C)mw[cell];
+            rho_m = St<S>::SHIFT ? (rho - K.rho0) * sc : rho;
+        } else {
+            moments0(f, rho_m, jx, jy, jz);
+            rho = St<S>::SHIFT ? K.rho0 + (St<S>::SCALED ? rho_m * (C)K.inv_scale : rho_m) : rho_m;
+            inv = St<S>::SCALED ? recip(rho) * (C)K.inv_scale : recip(rho);
+            ux = jx * inv;
+            uy = jy * inv;
+            uz = jz * inv;
+        }
+        rhos = St<S>::SCALED ? rho * sc : rho;
+        // The pair form rounds the equilibrium itself (error ~ eps |feq|, where
+        // the moment form rounds only m - meq), and that rounding leaks into the
+        // conserved density and momentum step after step.  In FP64 the leak is
+        // ~1e-15 relative and in the 16-bit forms far below the storage error,
+        // but FP32 storage keeps 1e-7 of the FP64 result only with the moment
+        // form (64^3, Re = 400, 2000 steps: velocity 4e-6 with the pair form).
+        // The first step after initial or load takes rho and u from the macro
+        // arrays, so the pair form adds back what its relaxation would take from
+        // the conserved sums of f (zero when the arrays agree with f).
+        if constexpr (std::is_same<S, float>::value) {
+            mrt_collide<C, false, true>(f, rho_m, rhos, ux, uy, uz, C(0), C(0), C(0), K.c, sc);
+        } else if constexpr (FIRST) {
+            C rf;
+            moments0(f, rf, jx, jy, jz);
+            trt_collide_lid<C, true>(f, rho_m, rhos, ux, uy, uz, K.c, sc, rf - rho_m,
+                                     jx - rhos * ux, jy - rhos * uy, jz - rhos * uz);
+        } else {
+            trt_collide_lid<C>(f, rho_m, rhos, ux, uy, uz, K.c, sc);
+        }
     }
     // moving lid: f(14) = f_post(11) - rho/6*U0, f(13) = f_post(12) + rho/6*U0
     // (bounce_back.f90:77-78).  On the top layer populations 11 and 12 always
@@ -425,13 +470,6 @@ __device__ __forceinline__ void lid_cell(int i, int j, int k, const S* __restric
     lid_cell_from<S, FIRST, IDX, SR>(i, j, k, raw, fout, K, P, mrho, mu, mv, mw, seed);
 }
 
-// ------------------------------------------------------ lid kernel, FX64 --
-// FP64 storage, Q55 fixed-point collision (fixed64.cuh); the same streaming,
-// halfway bounce-back and lid term as lid_cell.
-struct FxK {
-    int nx, ny, nz;
-    FxCoef c;
-};
 // populations converted on the FP64 unit (the rest with integer bit
 // operations), balancing that unit against the integer pipe
 #ifndef FX_CVT_IN
@@ -440,86 +478,6 @@ struct FxK {
 #ifndef FX_CVT_OUT
 #define FX_CVT_OUT 17
 #endif
-
-// AAM: 0 push (fin -> fout), 1 in-place even step, 2 in-place odd step (fin ==
-// fout; plain loads; see lid_cell_from for the pattern)
-template <bool FIRST, typename IDX, int AAM = 0>
-__device__ __forceinline__ void lid_cell_fx(int i, int j, int k, const double* fin,
-                                            double* fout, const FxK& K, IDX P,
-                                            const double* __restrict__ mrho,
-                                            const double* __restrict__ mu,
-                                            const double* __restrict__ mv,
-                                            const double* __restrict__ mw) {
-    const int nx = K.nx, ny = K.ny, nz = K.nz;
-    const IDX cell = (IDX)i + (IDX)nx * ((IDX)j + (IDX)ny * (IDX)k);
-    long long f[Q19];
-    {
-        // all loads issued before any conversion
-        double raw[Q19];
-        if (AAM == 0) {
-#pragma unroll
-            for (int q = 0; q < Q19; q++) raw[q] = oob((IDX)q * P + cell, (IDX)Q19 * P) ? 0.0 : __ldg(fin + ((IDX)q * P + cell));
-        } else {
-            lid_load_aa<double, IDX, AAM == 2>(i, j, k, fin, nx, ny, nz, P, raw);
-        }
-#pragma unroll
-        for (int q = 0; q < Q19; q++) f[q] = __double_as_longlong(raw[q]);
-    }
-    bool bad = false;
-#pragma unroll
-    for (int q = 0; q < Q19; q++) {
-        bad |= fx_bad(__longlong_as_double(f[q]));
-        f[q] = q < FX_CVT_IN ? d2q_cvt(__longlong_as_double(f[q])) : d2q(__longlong_as_double(f[q]));
-    }
-    long long rin = 0, uin = 0, vin = 0, win = 0;
-    if (FIRST) {
-        const double r = mrho[cell], a = mu[cell], b = mv[cell], c = mw[cell];
-        bad |= ((unsigned)(__double_as_longlong(r) >> 52) & 0x7FFu) >= 1024u;  // rho >= 2
-        bad |= fx_bad(a) || fx_bad(b) || fx_bad(c);
-        rin = d2q(r);
-        uin = d2q(a);
-        vin = d2q(b);
-        win = d2q(c);
-    }
-    long long rho;
-    bad |= !mrt_collide_fx<FIRST>(f, rin, uin, vin, win, K.c, rho);
-    // moving lid: f(14) = f_post(11) - rho/6*U0, f(13) = f_post(12) + rho/6*U0
-    // (bounce_back.f90:77-78); on the top layer populations 11 and 12 always
-    // leave through the lid, so the term is applied to them before rounding
-    if (k == nz - 1) {
-        const long long lid = qmulc(rho, K.c.u0_6);
-        f[11] -= lid;
-        f[12] += lid;
-    }
-    // one rounding per population; the store pattern below moves doubles only
-    double o[Q19];
-    const double nan = __longlong_as_double(0x7ff8000000000000LL);
-#pragma unroll
-    for (int q = 0; q < Q19; q++) o[q] = bad ? nan : (q < FX_CVT_OUT ? q2d_cvt(f[q]) : q2d(f[q]));
-    const IDX sy = (IDX)nx, sz = (IDX)nx * (IDX)ny;
-    const unsigned bm = face_mask(i, j, k, nx, ny, nz);
-    if (AAM == 1) {  // in-place even step: own cell, slot opp(q) (lid term already in o)
-#pragma unroll
-        for (int q = 0; q < Q19; q++) st_chk(fout, (IDX)opp19(q) * P + cell, (IDX)Q19 * P, o[q]);
-        return;
-    }
-    if (bm == 0) {
-#pragma unroll
-        for (int q = 0; q < Q19; q++) {
-            const int dx = ex19(q), dy = ey19(q), dz = ez19(q);
-            st_chk(fout, (IDX)((IDX)q * P + cell + (IDX)(dx + dy * (int)sy) + (IDX)dz * sz), (IDX)Q19 * P, o[q]);
-        }
-        return;
-    }
-#pragma unroll
-    for (int q = 0; q < Q19; q++) {
-        const int dx = ex19(q), dy = ey19(q), dz = ez19(q);
-        if ((bm & leave_bits(dx, dy, dz)) == 0)
-            st_chk(fout, (IDX)((IDX)q * P + cell + (IDX)(dx + dy * (int)sy) + (IDX)dz * sz), (IDX)Q19 * P, o[q]);
-        else
-            st_chk(fout, (IDX)((IDX)opp19(q) * P + cell), (IDX)Q19 * P, o[q]);
-    }
-}
 
 // -------------------------------------------------------- thermal kernel --
 // Temperature populations are kept in the arithmetic type (FP64, or FP32 for
@@ -560,7 +518,7 @@ __device__ __forceinline__ void thermal_cell_from(
     // storage scale sc (1 unless SCALED); rho, u, T and the carried force are
     // unscaled
     const C sc = St<S>::SCALED ? (C)K.scale : C(1);
-    C rho_m, rho, ux, uy, uz, temp;
+    C rho_m, rho, ux, uy, uz, temp, jx, jy, jz;  // j: rho u
     const C fxp = fp[0], fyp = fp[1], fzp = fp[2];  // carried from the previous step
     if (FIRST) {
         rho = (C)mrho[cell];
@@ -570,7 +528,6 @@ __device__ __forceinline__ void thermal_cell_from(
         temp = (C)mT[cell];
         rho_m = St<S>::SHIFT ? (rho - K.rho0) * sc : rho;
     } else {
-        C jx, jy, jz;
         moments0(f, rho_m, jx, jy, jz);
         if (St<S>::SCALED) {
             jx = jx * (C)K.inv_scale;
@@ -580,9 +537,12 @@ __device__ __forceinline__ void thermal_cell_from(
         rho = St<S>::SHIFT ? K.rho0 + (St<S>::SCALED ? rho_m * (C)K.inv_scale : rho_m) : rho_m;
         const C inv = recip(rho);
         // u^n = (sum f e + F^n/2)/rho^n with the force carried from the previous step
-        ux = (jx + C(0.5) * fxp) * inv;
-        uy = (jy + C(0.5) * fyp) * inv;
-        uz = (jz + C(0.5) * fzp) * inv;
+        jx = jx + C(0.5) * fxp;
+        jy = jy + C(0.5) * fyp;
+        jz = jz + C(0.5) * fzp;
+        ux = jx * inv;
+        uy = jy * inv;
+        uz = jz * inv;
         temp = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
     }
     // body force from (rho,u,T) of the previous macro (bouyancy3d_mpi.F90:743-745)
@@ -599,35 +559,35 @@ __device__ __forceinline__ void thermal_cell_from(
     if (!oob(fz_off + cell, fz_off + P)) F[fz_off + cell] = fz;
     // the pair form where its equilibrium rounding stays below the storage
     // error (FP64 and the 16-bit forms; see lid_cell_from)
-    if (std::is_same<S, float>::value) {
+    if constexpr (std::is_same<S, float>::value) {
         mrt_collide<C, true, false>(f, rho_m, rho, ux, uy, uz, fx, fy, fz, K.c);
-    } else if (FIRST) {
+    } else if constexpr (std::is_same<S, double>::value && !FIRST) {
+        pair_collide_forced<ROT, true>(f, rho, jx, jy, jz, ux, uy, uz, fx, fy, fz, fx - fxp,
+                                       fy - fyp, fz - fzp, K.pk);
+    } else if constexpr (FIRST) {
         // rho, u from the macro arrays: the odd term is e.(2 (j - rho u) + F)/10
         // and the density projection goes back in (trt_collide_forced)
-        C rf, jx, jy, jz;
+        C rf;
         moments0(f, rf, jx, jy, jz);
         const C rhos = rho * sc;
         trt_collide_forced<C, ROT, true>(
             f, rho_m, rhos, ux, uy, uz, fx * sc, fy * sc, fz * sc,
             fx * sc + C(2) * (jx - rhos * ux), fy * sc + C(2) * (jy - rhos * uy),
             fz * sc + C(2) * (jz - rhos * uz), K.c, rf - rho_m);
-    } else if (St<S>::SCALED) {
+    } else {
         trt_collide_forced<C, ROT>(f, rho_m, rho * sc, ux, uy, uz, fx * sc, fy * sc, fz * sc,
                                    (fx - fxp) * sc, (fy - fyp) * sc, (fz - fzp) * sc, K.c);
-    } else {
-        trt_collide_forced<C, ROT>(f, rho_m, rho, ux, uy, uz, fx, fy, fz, fx - fxp, fy - fyp,
-                                   fz - fzp, K.c);
     }
     // D3Q7: the pair form in FP64; the FP32 temperature populations of the
     // reduced forms keep the moment form (its rounding does not leak into
     // the conserved sum of g; see lid_cell_from for the FP32 measurement)
-    if (!std::is_same<C, double>::value) {
+    if constexpr (!std::is_same<C, double>::value) {
         mrt_collide_t<C>(g, temp, ux, uy, uz, K.para_a, K.qd, K.qnu);
-    } else if (FIRST) {
+    } else if constexpr (FIRST) {
         const C sg = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
         trt_collide_t<C, true>(g, temp, ux, uy, uz, K.para_a, K.qd, K.qnu, sg - temp);
     } else {
-        trt_collide_t<C>(g, temp, ux, uy, uz, K.para_a, K.qd, K.qnu);
+        pair_collide_t(g, temp, ux, uy, uz, K.pk);
     }
 
     const IDX sy = (IDX)nx, sz = (IDX)nx * (IDX)ny;
