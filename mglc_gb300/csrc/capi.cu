@@ -291,7 +291,7 @@ int natural_layout(mglc_ctx* c) {
 }
 
 // bring rho,u,v,w(,T) up to date with the current populations
-int refresh_macros(mglc_ctx* c) {
+int refresh_macros(mglc_ctx* c, bool ordered = false) {
     if (c->macros_valid) return MGLC_OK;
     int rc0 = natural_layout(c);
     if (rc0) return rc0;
@@ -303,7 +303,7 @@ int refresh_macros(mglc_ctx* c) {
         return MGLC_OK;
     }
     CK(launch_macro(c->form, thermal(c), c->geom, c->f[c->cur], thermal(c) ? c->g[c->cur] : nullptr,
-                    c->F, c->rho0, c->inv_scale, c->rho, c->u, c->v, c->w, c->T, c->stream),
+                    c->F, c->rho0, c->inv_scale, c->rho, c->u, c->v, c->w, c->T, ordered, c->stream),
        "macro");
     c->macros_valid = true;
     return MGLC_OK;
@@ -591,7 +591,7 @@ int mglc_load_state(mglc_ctx* c, const double* f, const double* g, const double*
         }
         c->cur = 0;
         c->macros_valid = false;
-        if ((rc = refresh_macros(c))) return rc;
+        if ((rc = refresh_macros(c, true))) return rc;
     }
     CK(cudaMemsetAsync(c->up, 0, b, c->stream), "zero up");
     CK(cudaMemsetAsync(c->vp, 0, b, c->stream), "zero vp");

@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "kernels.cuh"
+#include "macro64.cuh"
 
 namespace mglc {
 
@@ -35,46 +36,45 @@ __device__ __forceinline__ __nv_bfloat16 from_d<__nv_bfloat16>(double v) {
     return __float2bfloat16_rn((float)v);
 }
 
-// stored value -> absolute population (FP64)
-template <typename S>
-__device__ __forceinline__ double pop_abs(const S* p, long long idx, int q, double rho0,
-                                          double inv_scale, bool shifted) {
-    double v = to_d<S>(p[idx]);
-    if (shifted) v = v * inv_scale + w19(q) * rho0;
-    return v;
-}
-
 // ------------------------------------------------------------- macro() --
 // Reference order: rho = sum over alpha from 0..18 sequentially, momentum in
 // the order of the alpha loop (macro.f90:6-25 / bouyancy3d_mpi.F90:986-1010),
-// with the thermal half-force shift.  Uses IEEE-rounded adds, multiplies and
-// divisions so that for FP64 storage the fields equal the reference's.
+// with the thermal half-force shift; every operation rounds as IEEE FP64 does,
+// so that for FP64 storage the fields equal the reference's.
 // storage type of the temperature populations for a given f storage type
 template <typename S> struct GType { using T = float; };
 template <> struct GType<double> { using T = double; };
 
-template <typename S, bool THERMAL>
-__global__ void k_macro(const S* __restrict__ f, const typename GType<S>::T* __restrict__ gt,
-                        const void* Fv,
+// stored population of a reduced form, in its arithmetic type
+__device__ __forceinline__ float to_f(float v) { return v; }
+__device__ __forceinline__ float to_f(__half v) { return __half2float(v); }
+__device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+// macro64.cuh: 384^3 FP64 in about 3.5 ms (its traffic is 1.5 ms of HBM), 11 ms
+// with every addition on the FP64 pipe; 256^3 FP16 1.7 ms against 4.0
+// ORDERED (reduced forms): every addition in FP64 and in the reference's order,
+// for the fields that the first step after a load starts from (another rounding
+// of them, however small, and the 16-bit stores round otherwise from there on)
+template <typename S, bool THERMAL, bool ORDERED>
+__global__ void __launch_bounds__(256) k_macro(const S* __restrict__ f,
+                        const typename GType<S>::T* __restrict__ gt, const void* Fv,
                         Geom g, double rho0, double inv_scale, double* rho, double* u, double* v,
                         double* w, double* T) {
     const long long n = g.plane;
-    const bool shifted = !std::is_same<S, double>::value;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
          c += (long long)gridDim.x * blockDim.x) {
-        double fq[Q19];
+        double r, jx, jy, jz;
+        if constexpr (std::is_same<S, double>::value) {
+            double fq[Q19];
 #pragma unroll
-        for (int q = 0; q < Q19; q++) fq[q] = pop_abs<S>(f, q * n + c, q, rho0, inv_scale, shifted);
-        double r = fq[0];
+            for (int q = 0; q < Q19; q++) fq[q] = f[q * n + c];
+            macro_sums(fq, r, jx, jy, jz);
+        } else {
+            float fq[Q19];
 #pragma unroll
-        for (int q = 1; q < Q19; q++) r = __dadd_rn(r, fq[q]);
-        double jx = 0.0, jy = 0.0, jz = 0.0;
-        bool fx_ = false, fy_ = false, fz_ = false;
-#pragma unroll
-        for (int q = 1; q < Q19; q++) {
-            if (ex19(q)) { jx = fx_ ? __dadd_rn(jx, ex19(q) * fq[q]) : ex19(q) * fq[q]; fx_ = true; }
-            if (ey19(q)) { jy = fy_ ? __dadd_rn(jy, ey19(q) * fq[q]) : ey19(q) * fq[q]; fy_ = true; }
-            if (ez19(q)) { jz = fz_ ? __dadd_rn(jz, ez19(q) * fq[q]) : ez19(q) * fq[q]; fz_ = true; }
+            for (int q = 0; q < Q19; q++) fq[q] = to_f(f[q * n + c]);
+            if (ORDERED) macro_sums_ordered(fq, inv_scale, rho0, r, jx, jy, jz);
+            else macro_sums(fq, (float)inv_scale, rho0, r, jx, jy, jz);
         }
         if (THERMAL) {
             double Fx, Fy, Fz;
@@ -94,9 +94,11 @@ __global__ void k_macro(const S* __restrict__ f, const typename GType<S>::T* __r
             T[c] = t;
         }
         rho[c] = r;
-        u[c] = __ddiv_rn(jx, r);
-        v[c] = __ddiv_rn(jy, r);
-        w[c] = __ddiv_rn(jz, r);
+        double uu, vv, ww;
+        div_by(jx, jy, jz, r, uu, vv, ww);
+        u[c] = uu;
+        v[c] = vv;
+        w[c] = ww;
     }
 }
 
@@ -110,23 +112,29 @@ static int grid_for(long long n, int block) {
 template <typename S>
 static cudaError_t macro_go(bool thermal, const Geom& g, const void* f, const void* gt,
                             const void* F, double rho0, double inv, double* rho, double* u,
-                            double* v, double* w, double* T, cudaStream_t s) {
+                            double* v, double* w, double* T, bool ordered, cudaStream_t s) {
     int gr = grid_for(g.plane, 256);
-    if (thermal)
-        k_macro<S, true><<<gr, 256, 0, s>>>((const S*)f, (const typename GType<S>::T*)gt, F, g, rho0, inv, rho, u, v, w, T);
+    using G = typename GType<S>::T;
+    constexpr bool kRed = !std::is_same<S, double>::value;
+    if (thermal && ordered && kRed)
+        k_macro<S, true, kRed><<<gr, 256, 0, s>>>((const S*)f, (const G*)gt, F, g, rho0, inv, rho, u, v, w, T);
+    else if (thermal)
+        k_macro<S, true, false><<<gr, 256, 0, s>>>((const S*)f, (const G*)gt, F, g, rho0, inv, rho, u, v, w, T);
+    else if (ordered && kRed)
+        k_macro<S, false, kRed><<<gr, 256, 0, s>>>((const S*)f, nullptr, nullptr, g, rho0, inv, rho, u, v, w, T);
     else
-        k_macro<S, false><<<gr, 256, 0, s>>>((const S*)f, nullptr, nullptr, g, rho0, inv, rho, u, v, w, T);
+        k_macro<S, false, false><<<gr, 256, 0, s>>>((const S*)f, nullptr, nullptr, g, rho0, inv, rho, u, v, w, T);
     return cudaGetLastError();
 }
 
 cudaError_t launch_macro(int form, bool thermal, const Geom& g, const void* f, const void* gt,
                          const void* F, double rho0, float inv_scale, double* rho, double* u,
-                         double* v, double* w, double* T, cudaStream_t s) {
+                         double* v, double* w, double* T, bool ordered, cudaStream_t s) {
     switch (form) {
-        case FORM_FP64: return macro_go<double>(thermal, g, f, gt, F, rho0, 1.0, rho, u, v, w, T, s);
-        case FORM_FP32: return macro_go<float>(thermal, g, f, gt, F, rho0, 1.0, rho, u, v, w, T, s);
-        case FORM_FP16: return macro_go<__half>(thermal, g, f, gt, F, rho0, inv_scale, rho, u, v, w, T, s);
-        case FORM_BF16: return macro_go<__nv_bfloat16>(thermal, g, f, gt, F, rho0, 1.0, rho, u, v, w, T, s);
+        case FORM_FP64: return macro_go<double>(thermal, g, f, gt, F, rho0, 1.0, rho, u, v, w, T, ordered, s);
+        case FORM_FP32: return macro_go<float>(thermal, g, f, gt, F, rho0, 1.0, rho, u, v, w, T, ordered, s);
+        case FORM_FP16: return macro_go<__half>(thermal, g, f, gt, F, rho0, inv_scale, rho, u, v, w, T, ordered, s);
+        case FORM_BF16: return macro_go<__nv_bfloat16>(thermal, g, f, gt, F, rho0, 1.0, rho, u, v, w, T, ordered, s);
     }
     return cudaErrorInvalidValue;
 }

@@ -32,6 +32,7 @@
 
 #include <atomic>
 
+#include "macro64.cuh"
 #include "particles.cuh"
 
 namespace mglc {
@@ -1032,20 +1033,18 @@ __global__ void k_pmacro(const S* f, const int* owner, PartParams p, bool first,
             u[c] = v[c] = w[c] = 0.0;
             continue;
         }
-        double fq[Q19];
-        for (int q = 0; q < Q19; q++) fq[q] = pabs<S>(f, q * P + c, q, p.rho0);
-        double r = fq[0];
-        for (int q = 1; q < Q19; q++) r += fq[q];
-        double jx = 0.0, jy = 0.0, jz = 0.0;
-        for (int q = 1; q < Q19; q++) {
-            jx += ex19(q) * fq[q];
-            jy += ey19(q) * fq[q];
-            jz += ez19(q) * fq[q];
-        }
+        double r, jx, jy, jz, uu, vv, ww;
+        typename PC<S>::C fq[Q19];
+#pragma unroll
+        for (int q = 0; q < Q19; q++) fq[q] = f[q * P + c];
+        if constexpr (PSt<S>::SHIFT) macro_sums(fq, 1.0f, p.rho0, r, jx, jy, jz);
+        else macro_sums(fq, r, jx, jy, jz);
+        div_by(jx + 0.5 * (r * p.body_force[0]), jy + 0.5 * (r * p.body_force[1]),
+               jz + 0.5 * (r * p.body_force[2]), r, uu, vv, ww);
         rho[c] = r;
-        u[c] = (jx + 0.5 * (r * p.body_force[0])) / r;
-        v[c] = (jy + 0.5 * (r * p.body_force[1])) / r;
-        w[c] = (jz + 0.5 * (r * p.body_force[2])) / r;
+        u[c] = uu;
+        v[c] = vv;
+        w[c] = ww;
     }
 }
 

@@ -58,10 +58,12 @@ cudaError_t launch_thermal_step(int form, bool first, const void* fin, void* fou
                                 const void* gin, void* gout, void* F, const ThermalStepArgs& a,
                                 cudaStream_t s);
 
-// macroscopic fields from the current state (reference macro()/macroT() order)
+// macroscopic fields from the current state (reference macro()/macroT() order);
+// ordered: reduced forms sum in the reference's order too (the first step after
+// a load starts from these fields)
 cudaError_t launch_macro(int form, bool thermal, const Geom& g, const void* f, const void* gt,
                          const void* F, double rho0, float inv_scale, double* rho, double* u,
-                         double* v, double* w, double* T, cudaStream_t s);
+                         double* v, double* w, double* T, bool ordered, cudaStream_t s);
 
 // equilibrium initialisation from rho,u,v,w (and T): reference initial()
 cudaError_t launch_equilibrium(int form, bool thermal, const Geom& g, const double* rho,

@@ -198,3 +198,22 @@ def test_collision_is_closer_to_exact_than_fp64():
             sums[0] += float(err) ** 2
             sums[1] += float(abs(Fr(float(ref[q])) - want[q])) ** 2
     assert sums[0] < sums[1], (math.sqrt(sums[0]), math.sqrt(sums[1]))
+
+
+def test_sums_round_like_fp64():
+    """rn53 (macro64.cuh) after an exact integer sum is FP64's rounding of that sum."""
+    def rn53(v):
+        hi = v >> 32
+        r = max(11 - (32 - (hi ^ (hi >> 63)).bit_length()), 0)
+        m = (1 << r) - 1
+        return (v + (m >> 1) + ((v >> r) & m & 1)) & ~m
+
+    rng = random.Random(6)
+    for k in range(20000):
+        v = rng.choice([1, -1]) * rng.getrandbits(rng.randint(1, 62))
+        if k % 3 == 0 and abs(v) > 1 << 55:  # ties
+            r = abs(v).bit_length() - 53
+            v = (v >> r << r) + (1 << (r - 1))
+        elif k % 5 == 0:
+            v = rng.choice([1, -1]) << rng.randint(50, 62)
+        assert Fr(rn53(v), ONE) == Fr(float(Fr(v, ONE))), v
