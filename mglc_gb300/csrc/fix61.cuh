@@ -13,7 +13,9 @@
 // the exact collision than the FP64 evaluation's, whose sums and products round
 // on the way (tests/test_fix61_host.py; velocity error after six steps of 384^3
 // 2.1e-13 against 3.3e-13).  About a thousand integer instructions a lid cell:
-// 384^3 in 3.31 ms a step (17.1 GLUPS, 77% of HBM) against 15.7 ms in FP64.
+// 384^3 in 3.31 ms a step (17.1 GLUPS, 77% of HBM) against 15.7 ms in FP64;
+// the heated cavity at 128^3, whose temperature populations stay in FP64, in 234 us
+// (9.0 GLUPS) against 813.
 // Cells outside its range (a population outside [2^-8, 1/8), the rest
 // population outside [1/8, 1/2), negative and non-finite ones among them, rho
 // below 1/4 or a velocity component of 1/2 or more) take the FP64 form; inside,
@@ -55,10 +57,11 @@ __device__ __forceinline__ double fix61_store(long long v) {
     const unsigned long long m = w >> r;
     return __longlong_as_double((long long)(m + ((unsigned long long)(unsigned)(1024 - lz) << 52)));
 }
-// the same for any v, on the FP64 unit
+// v * 2^-Q for any v, on the FP64 unit
+template <int Q = 61>
 __device__ __forceinline__ double fix61_store_any(long long v) {
     const long long b = __double_as_longlong((double)v);
-    return __longlong_as_double(v ? b - (61LL << 52) : 0LL);
+    return __longlong_as_double(v ? b - ((long long)Q << 52) : 0LL);
 }
 
 // v = h * 2^32 + l in balanced digits
@@ -71,6 +74,7 @@ __device__ __forceinline__ FixD fix_dig(long long v) {
     d.h = (int)(v >> 32) + (int)((unsigned)d.l >> 31);
     return d;
 }
+__device__ __forceinline__ long long join(FixD d) { return ((long long)d.h << 32) + d.l; }
 // a + (v * c) / 2^64, the product rounded to nearest
 __device__ __forceinline__ long long fix_mad(FixD v, FixC c, long long a) {
     long long x = (long long)v.h * c.l + (0x80000000LL + __mulhi(v.l, c.l));
@@ -102,12 +106,6 @@ __device__ __forceinline__ long long fix_recip(long long rho, FixD rd) {
     return x1 + (((long long)(int)(x1 >> 32) * e1 + (1LL << 28)) >> 29);
 }
 
-// populations converted back on the FP64 unit (the others with integer
-// operations), balancing the two
-#ifndef FIX_CVT_OUT
-#define FIX_CVT_OUT 10
-#endif
-
 __device__ __forceinline__ void fix_pair(long long* F, int a, int b, const FixK& k, long long E,
                                          long long O) {
     const long long p = fix_mad(F[a] + F[b], k.c1, E), m = fix_mad(F[a] - F[b], k.c2, O);
@@ -115,7 +113,13 @@ __device__ __forceinline__ void fix_pair(long long* F, int a, int b, const FixK&
     F[b] = p - m;
 }
 
-// integer populations to doubles; v below 2^-8 or negative (rare): the FP64 unit
+// integer populations to doubles, the first NFP of them on the FP64 unit, the
+// others with integer operations (all on the FP64 unit when one is below 2^-8 or
+// negative, which is rare): the lid kernels, which need that unit for nothing
+// else, run best with 10 (3309 us a step at 384^3; 3456 with none, 3326 with all),
+// the heated ones, whose temperature part runs on it, with none (234 us at 128^3;
+// 238 with 6)
+template <int NFP>
 __device__ __forceinline__ void fix61_store_all(const long long (&F)[Q19], double (&f)[Q19]) {
     int least = 0x7fffffff;
 #pragma unroll
@@ -123,81 +127,123 @@ __device__ __forceinline__ void fix61_store_all(const long long (&F)[Q19], doubl
     if (least >= 0x200000) {
 #pragma unroll
         for (int q = 0; q < Q19; q++)
-            f[q] = q < FIX_CVT_OUT ? fix61_store_any(F[q]) : fix61_store(F[q]);
+            f[q] = q < NFP ? fix61_store_any(F[q]) : fix61_store(F[q]);
     } else {
 #pragma unroll
         for (int q = 0; q < Q19; q++) f[q] = fix61_store_any(F[q]);
     }
 }
 
-// The lid collision (pair_collide_lid) in place of a cell's populations as
-// integers; false, with nothing changed, when the density or the velocity is
-// out of range.  rho: the density of the equilibrium.  FIRST (the step after
-// initial or load): rho and u come from the macro arrays (rho0, u0, v0, w0),
-// and the projections of the populations on the conserved density and momentum
-// are taken back out (trt_collide_lid, CONS).
+// Density, momentum and velocity of a cell, as the collision takes them.
+struct FixFlow {
+    long long r;                // density
+    FixD rd, Jx, Jy, Jz;        // and rho u
+    FixD ux, uy, uz;            // velocity, units of 2^-63
+    long long ex, ey, ez, d19;  // 2 (j - rho u); FIRST: Snu/19 (sum f - rho)
+};
+// From the populations and half the force carried from the previous step
+// (hx, hy, hz; rho u = j + Fp/2), or, FIRST (the step after initial or load),
+// from the macro arrays; false when the density or the velocity is out of range.
 template <bool FIRST>
-__device__ __forceinline__ bool fix61_collide_lid(long long (&F)[Q19], const FixK& k,
-                                                  long long& rho, double rho0 = 0.0,
-                                                  double u0 = 0.0, double v0 = 0.0,
-                                                  double w0 = 0.0) {
+__device__ __forceinline__ bool fix61_flow(const long long (&F)[Q19], const FixK& k, long long hx,
+                                           long long hy, long long hz, double rho0, double u0,
+                                           double v0, double w0, FixFlow& o) {
     long long r, jx, jy, jz;
     moments0(F, r, jx, jy, jz);
-    FixD rd, dx, dy, dz, di, ux, uy, uz;
-    long long inv, hx = 0, hy = 0, hz = 0, d19 = 0;
     if (FIRST) {
         if (!(rho0 >= 0.25 && rho0 < 2.75 && fabs(u0) < 0.5 && fabs(v0) < 0.5 && fabs(w0) < 0.5))
             return false;
-        const long long rf = r, ax = jx, ay = jy, az = jz;
-        r = __double2ll_rn(rho0 * FIX_ONE);
-        ux = fix_dig(__double2ll_rn(u0 * (4.0 * FIX_ONE)));
-        uy = fix_dig(__double2ll_rn(v0 * (4.0 * FIX_ONE)));
-        uz = fix_dig(__double2ll_rn(w0 * (4.0 * FIX_ONE)));
-        rd = fix_dig(r);
-        inv = fix_recip(r, rd);
-        di = fix_dig(inv);
-        jx = fix_mul<63>(rd, ux);
-        jy = fix_mul<63>(rd, uy);
-        jz = fix_mul<63>(rd, uz);
-        dx = fix_dig(jx);
-        dy = fix_dig(jy);
-        dz = fix_dig(jz);
-        d19 = fix_mad(rf - r, k.l19, 0);
-        hx = fix_mad(ax - jx, k.l10, 0);
-        hy = fix_mad(ay - jy, k.l10, 0);
-        hz = fix_mad(az - jz, k.l10, 0);
-    } else {
-        const long long half = r >> 1;
-        if (!(r >= (1LL << 59) && jx < half && -jx < half && jy < half && -jy < half &&
-              jz < half && -jz < half))
-            return false;
-        rd = fix_dig(r);
-        dx = fix_dig(jx);
-        dy = fix_dig(jy);
-        dz = fix_dig(jz);
-        inv = fix_recip(r, rd);
-        di = fix_dig(inv);
-        // u in units of 2^-63
-        ux = fix_dig(fix_mul<58>(dx, di));
-        uy = fix_dig(fix_mul<58>(dy, di));
-        uz = fix_dig(fix_mul<58>(dz, di));
+        o.r = __double2ll_rn(rho0 * FIX_ONE);
+        o.rd = fix_dig(o.r);
+        o.ux = fix_dig(__double2ll_rn(u0 * (4.0 * FIX_ONE)));
+        o.uy = fix_dig(__double2ll_rn(v0 * (4.0 * FIX_ONE)));
+        o.uz = fix_dig(__double2ll_rn(w0 * (4.0 * FIX_ONE)));
+        const long long Jx = fix_mul<63>(o.rd, o.ux), Jy = fix_mul<63>(o.rd, o.uy),
+                        Jz = fix_mul<63>(o.rd, o.uz);
+        o.Jx = fix_dig(Jx);
+        o.Jy = fix_dig(Jy);
+        o.Jz = fix_dig(Jz);
+        o.ex = 2 * (jx - Jx);
+        o.ey = 2 * (jy - Jy);
+        o.ez = 2 * (jz - Jz);
+        o.d19 = fix_mad(r - o.r, k.l19, 0);
+        return true;
     }
-    rho = r;
-    // Snu/8 rho u in units of 2^-62
-    const FixD kx = fix_dig(fix_mad(dx, k.l8, 0)), ky = fix_dig(fix_mad(dy, k.l8, 0)),
-               kz = fix_dig(fix_mad(dz, k.l8, 0));
-    const long long X = fix_mul<64>(kx, ux), Y = fix_mul<64>(ky, uy), Z = fix_mul<64>(kz, uz);
-    const long long cxy = 2 * fix_mul<64>(kx, uy), cxz = 2 * fix_mul<64>(kx, uz),
-                    cyz = 2 * fix_mul<64>(ky, uz);
-    // half the lid quirk's term, (Y - Z)(1 - 1/rho)/6
-    const long long qh = fix_mul<60>(fix_dig(fix_mad(Y - Z, k.sixth, 0)), fix_dig((1LL << 60) - inv));
+    jx += hx;
+    jy += hy;
+    jz += hz;
+    const long long half = r >> 1;
+    if (!(r >= (1LL << 59) && jx < half && -jx < half && jy < half && -jy < half && jz < half &&
+          -jz < half))
+        return false;
+    o.r = r;
+    o.rd = fix_dig(r);
+    o.Jx = fix_dig(jx);
+    o.Jy = fix_dig(jy);
+    o.Jz = fix_dig(jz);
+    const FixD di = fix_dig(fix_recip(r, o.rd));
+    o.ux = fix_dig(fix_mul<58>(o.Jx, di));
+    o.uy = fix_dig(fix_mul<58>(o.Jy, di));
+    o.uz = fix_dig(fix_mul<58>(o.Jz, di));
+    o.ex = -2 * hx;
+    o.ey = -2 * hy;
+    o.ez = -2 * hz;
+    o.d19 = 0;
+    return true;
+}
+
+// The collision in place of a cell's populations as integers.
+// LID: the lid operator's quirk (pair_collide_lid).  FORCE: 0 none, 1 F_z only,
+// 2 all components (pair_collide_forced; fx, fy, fz this step's force); DF: the
+// force changes from step to step.
+template <bool LID, int FORCE, bool FIRST, bool DF>
+__device__ __forceinline__ void fix61_collide(long long (&F)[Q19], const FixK& k, const FixFlow& o,
+                                              long long fx, long long fy, long long fz) {
+    // Snu/8 V in units of 2^-62, V = rho u + (1 - Snu/2)/(Snu/2) F
+    long long vx = fix_mad(o.Jx, k.l8, 0), vy = fix_mad(o.Jy, k.l8, 0), vz = fix_mad(o.Jz, k.l8, 0);
+    // Sq/12 W, W = rho u + (1 - Sq/2)/Sq F
+    long long gx = fix_mad(o.Jx, k.l6, 0), gy = fix_mad(o.Jy, k.l6, 0), gz = fix_mad(o.Jz, k.l6, 0);
+    if (FORCE == 2) {
+        const FixD dx = fix_dig(fx), dy = fix_dig(fy);
+        vx = fix_mad(dx, k.kv, vx);
+        vy = fix_mad(dy, k.kv, vy);
+        gx = fix_mad(dx, k.kw, gx);
+        gy = fix_mad(dy, k.kw, gy);
+    }
+    if (FORCE) {
+        const FixD dz = fix_dig(fz);
+        vz = fix_mad(dz, k.kv, vz);
+        gz = fix_mad(dz, k.kw, gz);
+    }
+    const FixD kx = fix_dig(vx), ky = fix_dig(vy), kz = fix_dig(vz);
+    const long long X = fix_mul<64>(kx, o.ux), Y = fix_mul<64>(ky, o.uy), Z = fix_mul<64>(kz, o.uz);
+    // u_a V_b + u_b V_a: equal products where neither component has a force
+    const long long cxy = FORCE == 2 ? fix_mul<64>(kx, o.uy) + fix_mul<64>(ky, o.ux)
+                                     : 2 * fix_mul<64>(kx, o.uy);
+    const long long cxz = FORCE ? fix_mul<64>(kx, o.uz) + fix_mul<64>(kz, o.ux)
+                                : 2 * fix_mul<64>(kx, o.uz);
+    const long long cyz = FORCE ? fix_mul<64>(ky, o.uz) + fix_mul<64>(kz, o.uy)
+                                : 2 * fix_mul<64>(ky, o.uz);
     const long long S = X + Y + Z;
-    const long long b = fix_mad(rd, k.l18, fix_mad(S, k.third, 0)), b2 = 2 * b + d19, be = b + d19;
-    const long long gx = fix_mad(dx, k.l6, 0), gy = fix_mad(dy, k.l6, 0), gz = fix_mad(dz, k.l6, 0);
-    const long long ox = gx + hx, oy = gy + hy, oz = gz + hz;
-    const long long q = 2 * qh;
-    const long long bxy = be + qh + X + Y, bxz = be - qh + X + Z, byz = be + Y + Z;
-    F[0] = 2 * fix_mad(F[0], k.c1, fix_mad(rd, k.l0, -2 * S)) + d19;
+    const long long b = fix_mad(o.rd, k.l18, fix_mad(S, k.third, 0));
+    const long long b2 = 2 * b + o.d19, be = b + o.d19;
+    // what the conserved momentum leaves in the odd part: Sq/20 (2 (j - rho u) + F)
+    long long ox = gx, oy = gy, oz = gz;
+    if (FIRST || (DF && FORCE == 2)) {
+        ox = fix_mad(o.ex + (FORCE == 2 ? fx : 0), k.l20, gx);
+        oy = fix_mad(o.ey + (FORCE == 2 ? fy : 0), k.l20, gy);
+    }
+    if (FIRST || (DF && FORCE)) oz = fix_mad(o.ez + (FORCE ? fz : 0), k.l20, gz);
+    long long bxy = be + X + Y, bxz = be + X + Z, q = 0;
+    const long long byz = be + Y + Z;
+    if (LID) {  // (Y - Z)(1 - 1/rho)/3, half of it on the edges
+        const long long w = (1LL << 60) - fix_recip(o.r, o.rd);
+        const long long qh = fix_mul<60>(fix_dig(fix_mad(Y - Z, k.sixth, 0)), fix_dig(w));
+        q = 2 * qh;
+        bxy += qh;
+        bxz -= qh;
+    }
+    F[0] = 2 * fix_mad(F[0], k.c1, fix_mad(o.rd, k.l0, -2 * S)) + o.d19;
     fix_pair(F, 1, 2, k, b2 + 2 * X, gx + ox);
     fix_pair(F, 3, 4, k, b2 - q + 2 * Y, gy + oy);
     fix_pair(F, 5, 6, k, b2 + q + 2 * Z, gz + oz);
@@ -207,7 +253,6 @@ __device__ __forceinline__ bool fix61_collide_lid(long long (&F)[Q19], const Fix
     fix_pair(F, 13, 12, k, bxz - cxz, ox - oz);
     fix_pair(F, 15, 18, k, byz + cyz, oy + oz);
     fix_pair(F, 17, 16, k, byz - cyz, oy - oz);
-    return true;
 }
 
 }  // namespace mglc

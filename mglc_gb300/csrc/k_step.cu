@@ -29,23 +29,8 @@ __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
                                 K.seed);
 }
 
-// 4 blocks of 128 per SM (128 registers): measured faster than the 168-register
-// allocation at 3 blocks and than 5 blocks with spills
-template <bool FIRST, bool ROT, typename IDX>
-__global__ void __launch_bounds__(128, 4)
-    k_thermal_step_fx(const double* __restrict__ fin, double* __restrict__ fout,
-                      const double* __restrict__ gin, double* __restrict__ gout,
-                      double* __restrict__ F, FxTK K, IDX P, const double* __restrict__ mrho,
-                      const double* __restrict__ mu, const double* __restrict__ mv,
-                      const double* __restrict__ mw, const double* __restrict__ mT) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K.nx) return;
-    thermal_cell_fx<FIRST, ROT, IDX>(i, blockIdx.y, blockIdx.z, fin, fout, gin, gout, F, K, P,
-                                     mrho, mu, mv, mw, mT);
-}
-
 template <typename S, bool FIRST, bool ROT, typename IDX, bool SR>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, ThermalMinBlocks<S>::value)
     k_thermal_step(const S* __restrict__ fin, S* __restrict__ fout,
                    const typename St<S>::C* __restrict__ gin, typename St<S>::C* __restrict__ gout,
                    typename St<S>::C* __restrict__ F, StepK<typename St<S>::C> K, IDX P,
@@ -110,7 +95,7 @@ cudaError_t launch_lid_step(int form, bool first, const void* fin, void* fout,
 
 template <typename S>
 static cudaError_t th_go(bool first, const void* fin, void* fout, const void* gin, void* gout,
-                         void* F, const ThermalStepArgs& a, cudaStream_t s) {
+                         void* F, const ThermalStepArgs& a, cudaStream_t s, bool box = false) {
     using C = typename St<S>::C;
     StepK<C> K = make_k<C>(a.g, a.cd, 0.0, a.rho0, a.scale, a.inv_scale);
     K.seed = a.seed;
@@ -121,6 +106,7 @@ static cudaError_t th_go(bool first, const void* fin, void* fout, const void* gi
     K.ccold = (C)((6.0 + a.para_a) / 21.0 * a.t_cold);
     K.bc_y = a.bc_y; K.bc_z = a.bc_z;
     pair_k_heat(K.pk, a.para_a, a.qd, a.qnu);
+    set_box(K.pk, box);
     dim3 b = step_block(a.g.nx), gr = step_grid(a.g, b);
     const bool rot = a.omega_rot != 0.0;
     const bool small = (long long)Q19 * a.g.plane < (1ll << 31);
@@ -150,42 +136,11 @@ static cudaError_t th_go(bool first, const void* fin, void* fout, const void* gi
     return cudaGetLastError();
 }
 
-static cudaError_t th_go_fx(bool first, const void* fin, void* fout, const void* gin, void* gout,
-                            void* F, const ThermalStepArgs& a, cudaStream_t s) {
-    FxTK K;
-    K.nx = a.g.nx; K.ny = a.g.ny; K.nz = a.g.nz; K.bc_y = a.bc_y; K.bc_z = a.bc_z;
-    K.t = make_fx_thermal(a.cd, a.gbeta, a.omega_rot, a.t_ref, a.para_a, a.qd, a.qnu, a.t_hot,
-                          a.t_cold);
-    dim3 b = step_block(a.g.nx), gr = step_grid(a.g, b);
-    const bool rot = a.omega_rot != 0.0;
-    const bool small = (long long)Q19 * a.g.plane < (1ll << 31);
-    const double* fi = (const double*)fin;
-    const double* gi = (const double*)gin;
-    double* fo = (double*)fout;
-    double* go = (double*)gout;
-    double* Fp = (double*)F;
-#define THX_LAUNCH(FI, RO, IT) \
-    k_thermal_step_fx<FI, RO, IT><<<gr, b, 0, s>>>(fi, fo, gi, go, Fp, K, (IT)a.g.plane, a.rho, a.u, a.v, a.w, a.T)
-#define THX_ROT(IT)                                 \
-    if (first && rot) THX_LAUNCH(true, true, IT);    \
-    else if (first) THX_LAUNCH(true, false, IT);     \
-    else if (rot) THX_LAUNCH(false, true, IT);       \
-    else THX_LAUNCH(false, false, IT);
-    if (small) {
-        THX_ROT(unsigned)
-    } else {
-        THX_ROT(long long)
-    }
-#undef THX_ROT
-#undef THX_LAUNCH
-    return cudaGetLastError();
-}
-
 cudaError_t launch_thermal_step(int form, bool first, const void* fin, void* fout,
                                 const void* gin, void* gout, void* F, const ThermalStepArgs& a,
                                 cudaStream_t s) {
     switch (form) {
-        case FORM_FX64: return th_go_fx(first, fin, fout, gin, gout, F, a, s);
+        case FORM_FX64: return th_go<double>(first, fin, fout, gin, gout, F, a, s, true);
         case FORM_FP64: return th_go<double>(first, fin, fout, gin, gout, F, a, s);
         case FORM_FP32: return th_go<float>(first, fin, fout, gin, gout, F, a, s);
         case FORM_FP16: return th_go<__half>(first, fin, fout, gin, gout, F, a, s);

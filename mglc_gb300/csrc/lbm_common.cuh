@@ -496,7 +496,8 @@ inline long long fix_ratio(double x, int d) {
 // coefficients of the collision on the integer pipe (fix61.cuh)
 struct FixK {
     FixC c1, c2, l18, l0, l8, l6;  // (1-Snu)/2, (1-Sq)/2, Snu/36, Snu/6, Snu/4, Sq/12
-    FixC l19, l10, third, sixth;   // Snu/19, Sq/10, -1/3, 1/6
+    FixC l19, l20, third, sixth;   // Snu/19, Sq/20, -1/3, 1/6
+    FixC kv, kw;                   // forced: (1 - Snu/2)/2, (1 - Sq/2)/12
     int on;                        // the rates are in range
 };
 inline FixK make_fix_k(double snu, double sq) {
@@ -514,7 +515,9 @@ inline FixK make_fix_k(double snu, double sq) {
     k.l8 = fix_coef(fix_ratio(snu, 4));
     k.l6 = fix_coef(fix_ratio(sq, 12));
     k.l19 = fix_coef(fix_ratio(snu, 19));
-    k.l10 = fix_coef(fix_ratio(sq, 10));
+    k.l20 = fix_coef(fix_ratio(sq, 20));
+    k.kv = fix_coef(2 * (half - fix_ratio(snu, 8)));
+    k.kw = fix_coef(1537228672809129301LL - fix_ratio(sq, 24));  // 2^64/12 - ...
     k.third = fix_coef(-6148914691236517205LL);
     k.sixth = fix_coef(3074457345618258603LL);
     return k;

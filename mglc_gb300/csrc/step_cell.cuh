@@ -8,7 +8,6 @@
 #include <type_traits>
 
 #include "fix61.cuh"
-#include "fixed64.cuh"
 #include "kernels.cuh"
 
 namespace mglc {
@@ -168,6 +167,13 @@ struct LidMinBlocks {
     static constexpr int value = std::is_same<S, double>::value ? 5 : 0;
 };
 
+// and for the heated cavity's (128^3 FP64: 234 us a step at 5, 251 at 4, 246 at 3,
+// 253 at 6)
+template <typename S>
+struct ThermalMinBlocks {
+    static constexpr int value = std::is_same<S, double>::value ? 5 : 0;
+};
+
 // Scalar constants converted once on the host to the arithmetic type.
 template <typename C>
 struct StepK {
@@ -299,15 +305,18 @@ __device__ __forceinline__ void lid_cell_from(int i, int j, int k, const S (&raw
         // in range: on the integer pipe (fix61.cuh); else the FP64 pair form
         bool ok = K.pk.fix.on && fix61_ok(f);
         if (ok) {
-            long long F[Q19], r = 0;
+            long long F[Q19];
 #pragma unroll
             for (int q = 0; q < Q19; q++) F[q] = fix61_load(f[q]);
+            FixFlow fl;
             if (FIRST)
-                ok = fix61_collide_lid<true>(F, K.pk.fix, r, mrho[cell], mu[cell], mv[cell], mw[cell]);
+                ok = fix61_flow<true>(F, K.pk.fix, 0, 0, 0, mrho[cell], mu[cell], mv[cell],
+                                      mw[cell], fl);
             else
-                ok = fix61_collide_lid<false>(F, K.pk.fix, r);
-            rho = (double)r * (1.0 / FIX_ONE);
-            fix61_store_all(F, f);  // (out of range after all: the same values back)
+                ok = fix61_flow<false>(F, K.pk.fix, 0, 0, 0, 0.0, 0.0, 0.0, 0.0, fl);
+            if (ok) fix61_collide<true, 0, FIRST, false>(F, K.pk.fix, fl, 0, 0, 0);
+            rho = fix61_store_any(fl.r);
+            fix61_store_all<10>(F, f);  // (out of range after all: the same values back)
             if (K.pk.box && rho >= 2.0) set_nan(f);
         }
         if (!ok) {
@@ -470,15 +479,6 @@ __device__ __forceinline__ void lid_cell(int i, int j, int k, const S* __restric
     lid_cell_from<S, FIRST, IDX, SR>(i, j, k, raw, fout, K, P, mrho, mu, mv, mw, seed);
 }
 
-// populations converted on the FP64 unit (the rest with integer bit
-// operations), balancing that unit against the integer pipe
-#ifndef FX_CVT_IN
-#define FX_CVT_IN 17
-#endif
-#ifndef FX_CVT_OUT
-#define FX_CVT_OUT 17
-#endif
-
 // -------------------------------------------------------- thermal kernel --
 // Temperature populations are kept in the arithmetic type (FP64, or FP32 for
 // the reduced forms): g_0 ~ 0.7 T has a 16-bit ulp (~2e-4) far above the
@@ -518,76 +518,150 @@ __device__ __forceinline__ void thermal_cell_from(
     // storage scale sc (1 unless SCALED); rho, u, T and the carried force are
     // unscaled
     const C sc = St<S>::SCALED ? (C)K.scale : C(1);
-    C rho_m, rho, ux, uy, uz, temp, jx, jy, jz;  // j: rho u
     const C fxp = fp[0], fyp = fp[1], fzp = fp[2];  // carried from the previous step
-    if (FIRST) {
-        rho = (C)mrho[cell];
-        ux = (C)mu[cell];
-        uy = (C)mv[cell];
-        uz = (C)mw[cell];
-        temp = (C)mT[cell];
-        rho_m = St<S>::SHIFT ? (rho - K.rho0) * sc : rho;
-    } else {
-        moments0(f, rho_m, jx, jy, jz);
-        if (St<S>::SCALED) {
-            jx = jx * (C)K.inv_scale;
-            jy = jy * (C)K.inv_scale;
-            jz = jz * (C)K.inv_scale;
+    auto force = [&](C rho, C ux, C uy, C temp, C& fx, C& fy, C& fz) {
+        // body force from (rho,u,T) of the previous macro (bouyancy3d_mpi.F90:743-745)
+        fx = fy = C(0);
+        if (ROT) {
+            fx = C(-2) * rho * uy * K.omega_rot;
+            fy = C(2) * rho * ux * K.omega_rot;
+            if (!oob(P + cell, (IDX)3 * P)) {
+                F[cell] = fx;
+                F[P + cell] = fy;
+            }
         }
-        rho = St<S>::SHIFT ? K.rho0 + (St<S>::SCALED ? rho_m * (C)K.inv_scale : rho_m) : rho_m;
-        const C inv = recip(rho);
-        // u^n = (sum f e + F^n/2)/rho^n with the force carried from the previous step
-        jx = jx + C(0.5) * fxp;
-        jy = jy + C(0.5) * fyp;
-        jz = jz + C(0.5) * fzp;
-        ux = jx * inv;
-        uy = jy * inv;
-        uz = jz * inv;
-        temp = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
-    }
-    // body force from (rho,u,T) of the previous macro (bouyancy3d_mpi.F90:743-745)
-    C fx = C(0), fy = C(0);
-    if (ROT) {
-        fx = C(-2) * rho * uy * K.omega_rot;
-        fy = C(2) * rho * ux * K.omega_rot;
-        if (!oob(P + cell, (IDX)3 * P)) {
-            F[cell] = fx;
-            F[P + cell] = fy;
+        fz = rho * K.gbeta * (temp - K.t_ref);
+        if (!oob(fz_off + cell, fz_off + P)) F[fz_off + cell] = fz;
+    };
+    if constexpr (std::is_same<S, double>::value) {
+        // flow: in range on the integer pipe (fix61.cuh), else the FP64 pair form;
+        // the temperature populations, of either sign and down to zero, in FP64
+        constexpr int FO = ROT ? 2 : 1;
+        const double small = 0.125;
+        double temp = FIRST ? mT[cell]
+                            : ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
+        double rho, ux, uy, uz, fx, fy, fz;
+        bool ok = K.pk.fix.on && fix61_ok(f) && fabs(fxp) < small && fabs(fyp) < small &&
+                  fabs(fzp) < small, bad = false;
+        long long L[Q19];
+        FixFlow fl;
+        if (ok) {
+#pragma unroll
+            for (int q = 0; q < Q19; q++) L[q] = fix61_load(f[q]);
+            if (FIRST) {
+                ok = fix61_flow<true>(L, K.pk.fix, 0, 0, 0, mrho[cell], mu[cell], mv[cell],
+                                      mw[cell], fl);
+            } else {
+                const double h = 0.5 * FIX_ONE;
+                ok = fix61_flow<false>(L, K.pk.fix, ROT ? __double2ll_rn(fxp * h) : 0,
+                                       ROT ? __double2ll_rn(fyp * h) : 0, __double2ll_rn(fzp * h),
+                                       0.0, 0.0, 0.0, 0.0, fl);
+            }
         }
-    }
-    const C fz = rho * K.gbeta * (temp - K.t_ref);
-    if (!oob(fz_off + cell, fz_off + P)) F[fz_off + cell] = fz;
-    // the pair form where its equilibrium rounding stays below the storage
-    // error (FP64 and the 16-bit forms; see lid_cell_from)
-    if constexpr (std::is_same<S, float>::value) {
-        mrt_collide<C, true, false>(f, rho_m, rho, ux, uy, uz, fx, fy, fz, K.c);
-    } else if constexpr (std::is_same<S, double>::value && !FIRST) {
-        pair_collide_forced<ROT, true>(f, rho, jx, jy, jz, ux, uy, uz, fx, fy, fz, fx - fxp,
-                                       fy - fyp, fz - fzp, K.pk);
-    } else if constexpr (FIRST) {
-        // rho, u from the macro arrays: the odd term is e.(2 (j - rho u) + F)/10
-        // and the density projection goes back in (trt_collide_forced)
-        C rf;
-        moments0(f, rf, jx, jy, jz);
-        const C rhos = rho * sc;
-        trt_collide_forced<C, ROT, true>(
-            f, rho_m, rhos, ux, uy, uz, fx * sc, fy * sc, fz * sc,
-            fx * sc + C(2) * (jx - rhos * ux), fy * sc + C(2) * (jy - rhos * uy),
-            fz * sc + C(2) * (jz - rhos * uz), K.c, rf - rho_m);
+        if (ok) {
+            rho = fix61_store_any(fl.r);
+            ux = FIRST ? mu[cell] : fix61_store_any<63>(join(fl.ux));
+            uy = FIRST ? mv[cell] : fix61_store_any<63>(join(fl.uy));
+            uz = FIRST ? mw[cell] : fix61_store_any<63>(join(fl.uz));
+        } else if (FIRST) {
+            rho = mrho[cell];
+            ux = mu[cell];
+            uy = mv[cell];
+            uz = mw[cell];
+        } else {
+            moments0(f, rho, ux, uy, uz);
+            const double inv = recip(rho);
+            // u^n = (sum f e + F^n/2)/rho^n with the force carried from the previous step
+            ux = (ux + 0.5 * fxp) * inv;
+            uy = (uy + 0.5 * fyp) * inv;
+            uz = (uz + 0.5 * fzp) * inv;
+        }
+        force(rho, ux, uy, temp, fx, fy, fz);
+        if (ok && fabs(fx) < small && fabs(fy) < small && fabs(fz) < small) {
+            fix61_collide<false, FO, FIRST, true>(
+                L, K.pk.fix, fl, ROT ? __double2ll_rn(fx * FIX_ONE) : 0,
+                ROT ? __double2ll_rn(fy * FIX_ONE) : 0, __double2ll_rn(fz * FIX_ONE));
+            fix61_store_all<0>(L, f);
+        } else {
+#pragma unroll
+            for (int q = 0; q < Q19; q++) bad |= !(fabs(f[q]) < 1.0);
+            double rf, jx, jy, jz;
+            moments0(f, rf, jx, jy, jz);
+            if (FIRST) {
+                // rho, u from the macro arrays: the odd term is e.(2 (j - rho u) + F)/10
+                // and the density projection goes back in (trt_collide_forced)
+                trt_collide_forced<C, ROT, true>(f, rho, rho, ux, uy, uz, fx, fy, fz,
+                                                 fx + 2.0 * (jx - rho * ux),
+                                                 fy + 2.0 * (jy - rho * uy),
+                                                 fz + 2.0 * (jz - rho * uz), K.c, rf - rho);
+            } else {
+                pair_collide_forced<ROT, true>(f, rho, jx + 0.5 * fxp, jy + 0.5 * fyp,
+                                               jz + 0.5 * fzp, ux, uy, uz, fx, fy, fz, fx - fxp,
+                                               fy - fyp, fz - fzp, K.pk);
+            }
+        }
+        if (K.pk.box) {  // FX64's range box, with |g| and |T| below 2
+#pragma unroll
+            for (int q = 0; q < Q7; q++) bad |= !(fabs(g[q]) < 2.0);
+            bad = bad || !(fabs(temp) < 2.0) || out_of_box(rho, ux, uy, uz);
+        }
+        if (FIRST) {
+            const double sg = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
+            trt_collide_t<C, true>(g, temp, ux, uy, uz, K.para_a, K.qd, K.qnu, sg - temp);
+        } else {
+            pair_collide_t(g, temp, ux, uy, uz, K.pk);
+        }
+        if (K.pk.box && bad) {
+            set_nan(f);
+            set_nan(g);
+        }
     } else {
-        trt_collide_forced<C, ROT>(f, rho_m, rho * sc, ux, uy, uz, fx * sc, fy * sc, fz * sc,
-                                   (fx - fxp) * sc, (fy - fyp) * sc, (fz - fzp) * sc, K.c);
-    }
-    // D3Q7: the pair form in FP64; the FP32 temperature populations of the
-    // reduced forms keep the moment form (its rounding does not leak into
-    // the conserved sum of g; see lid_cell_from for the FP32 measurement)
-    if constexpr (!std::is_same<C, double>::value) {
+        C rho_m, rho, ux, uy, uz, temp, jx, jy, jz;
+        if (FIRST) {
+            rho = (C)mrho[cell];
+            ux = (C)mu[cell];
+            uy = (C)mv[cell];
+            uz = (C)mw[cell];
+            temp = (C)mT[cell];
+            rho_m = St<S>::SHIFT ? (rho - K.rho0) * sc : rho;
+        } else {
+            moments0(f, rho_m, jx, jy, jz);
+            if (St<S>::SCALED) {
+                jx = jx * (C)K.inv_scale;
+                jy = jy * (C)K.inv_scale;
+                jz = jz * (C)K.inv_scale;
+            }
+            rho = St<S>::SHIFT ? K.rho0 + (St<S>::SCALED ? rho_m * (C)K.inv_scale : rho_m) : rho_m;
+            const C inv = recip(rho);
+            // u^n = (sum f e + F^n/2)/rho^n with the force carried from the previous step
+            ux = (jx + C(0.5) * fxp) * inv;
+            uy = (jy + C(0.5) * fyp) * inv;
+            uz = (jz + C(0.5) * fzp) * inv;
+            temp = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
+        }
+        C fx, fy, fz;
+        force(rho, ux, uy, temp, fx, fy, fz);
+        // the pair form where its equilibrium rounding stays below the storage
+        // error (the 16-bit forms; see lid_cell_from)
+        if constexpr (std::is_same<S, float>::value) {
+            mrt_collide<C, true, false>(f, rho_m, rho, ux, uy, uz, fx, fy, fz, K.c);
+        } else if constexpr (FIRST) {
+            // rho, u from the macro arrays, as above
+            C rf;
+            moments0(f, rf, jx, jy, jz);
+            const C rhos = rho * sc;
+            trt_collide_forced<C, ROT, true>(
+                f, rho_m, rhos, ux, uy, uz, fx * sc, fy * sc, fz * sc,
+                fx * sc + C(2) * (jx - rhos * ux), fy * sc + C(2) * (jy - rhos * uy),
+                fz * sc + C(2) * (jz - rhos * uz), K.c, rf - rho_m);
+        } else {
+            trt_collide_forced<C, ROT>(f, rho_m, rho * sc, ux, uy, uz, fx * sc, fy * sc, fz * sc,
+                                       (fx - fxp) * sc, (fy - fyp) * sc, (fz - fzp) * sc, K.c);
+        }
+        // D3Q7: the FP32 temperature populations of the reduced forms keep the
+        // moment form (its rounding does not leak into the conserved sum of g; see
+        // lid_cell_from for the FP32 measurement)
         mrt_collide_t<C>(g, temp, ux, uy, uz, K.para_a, K.qd, K.qnu);
-    } else if constexpr (FIRST) {
-        const C sg = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
-        trt_collide_t<C, true>(g, temp, ux, uy, uz, K.para_a, K.qd, K.qnu, sg - temp);
-    } else {
-        pair_collide_t(g, temp, ux, uy, uz, K.pk);
     }
 
     const IDX sy = (IDX)nx, sz = (IDX)nx * (IDX)ny;
@@ -710,141 +784,6 @@ __device__ __forceinline__ void thermal_load_aa(int i, int j, int k, const S* f,
     load_carried<typename St<S>::C, ROT, IDX>(F, P, cell, fz_off, fp);
 #pragma unroll
     for (int q = 0; q < Q19; q++) fv[q] = St<S>::cvt_s(raw[q]);  // in units of the storage scale
-}
-
-// -------------------------------------------------- heated cavity, FX64 --
-// FP64 storage (f, g and the carried force as in the FP64 form); forced
-// D3Q19 and D3Q7 collisions in Q55 (fixed64.cuh); the streaming, bounce-back
-// and anti-bounce-back of thermal_cell.
-// temperature populations converted on the FP64 unit (the rest with integer
-// bit operations)
-#ifndef FXT_CVT_G
-#define FXT_CVT_G 4
-#endif
-struct FxTK {
-    int nx, ny, nz, bc_y, bc_z;
-    FxThermalCoef t;
-};
-
-// AAM: 0 push, 1 in-place even step, 2 in-place odd step (as lid_cell_fx)
-template <bool FIRST, bool ROT, typename IDX, int AAM = 0>
-__device__ __forceinline__ void thermal_cell_fx(
-    int i, int j, int k, const double* fin, double* fout, const double* gin, double* gout,
-    double* __restrict__ F,
-    const FxTK& K, IDX P, const double* __restrict__ mrho, const double* __restrict__ mu,
-    const double* __restrict__ mv, const double* __restrict__ mw, const double* __restrict__ mT) {
-    using ll = long long;
-    const int nx = K.nx, ny = K.ny, nz = K.nz;
-    const IDX cell = (IDX)i + (IDX)nx * ((IDX)j + (IDX)ny * (IDX)k);
-    ll f[Q19], g[Q7];
-    bool bad = false;
-    {
-        double rf[Q19], rg[Q7];
-        if (AAM == 0) {
-#pragma unroll
-            for (int q = 0; q < Q19; q++) rf[q] = oob((IDX)q * P + cell, (IDX)Q19 * P) ? 0.0 : __ldg(fin + ((IDX)q * P + cell));
-#pragma unroll
-            for (int q = 0; q < Q7; q++) rg[q] = oob((IDX)q * P + cell, (IDX)Q7 * P) ? 0.0 : __ldg(gin + ((IDX)q * P + cell));
-        } else {
-            const IDX sy = (IDX)nx, sz = (IDX)nx * (IDX)ny;
-            const unsigned bm = face_mask(i, j, k, nx, ny, nz);
-            auto src = [&](int q) -> IDX {
-                const int dx = ex19(q), dy = ey19(q), dz = ez19(q);
-                if (AAM != 2 || (bm & leave_bits(-dx, -dy, -dz)) != 0) return (IDX)q * P + cell;
-                return (IDX)opp19(q) * P + cell - (IDX)(dx + dy * (int)sy) - (IDX)dz * sz;
-            };
-#pragma unroll
-            for (int q = 0; q < Q19; q++) rf[q] = fin[src(q)];
-#pragma unroll
-            for (int q = 0; q < Q7; q++) rg[q] = oob(src(q), (IDX)Q7 * P) ? 0.0 : __ldcg(gin + src(q));
-        }
-#pragma unroll
-        for (int q = 0; q < Q19; q++) {
-            bad |= fx_bad(rf[q]);
-            f[q] = q < FX_CVT_IN ? d2q_cvt(rf[q]) : d2q(rf[q]);
-        }
-#pragma unroll
-        for (int q = 0; q < Q7; q++) {
-            bad |= fx_bad2(rg[q]);
-            g[q] = q < FXT_CVT_G ? d2q_cvt(rg[q]) : d2q(rg[q]);
-        }
-    }
-    ll rho, ux, uy, uz, temp, rux, ruy, ruz;
-    if (FIRST) {
-        const double r = mrho[cell], a = mu[cell], b = mv[cell], c = mw[cell], t = mT[cell];
-        bad |= ((unsigned)(__double_as_longlong(r) >> 52) & 0x7FFu) >= 1024u;
-        bad |= fx_bad(a) || fx_bad(b) || fx_bad(c) || fx_bad2(t);
-        rho = d2q(r); ux = d2q(a); uy = d2q(b); uz = d2q(c); temp = d2q(t);
-        rux = qmul(rho, ux); ruy = qmul(rho, uy); ruz = qmul(rho, uz);
-    } else {
-        // u = (sum f e + F/2) / rho with the force carried from the previous step
-        ll fxp = 0, fyp = 0;
-        if (ROT) {
-            fxp = d2q(oob(P + cell, (IDX)3 * P) ? 0.0 : F[cell]);
-            fyp = d2q(oob(P + cell, (IDX)3 * P) ? 0.0 : F[P + cell]);
-        }
-        const ll fzp = d2q(oob((IDX)2 * P + cell, (IDX)3 * P) ? 0.0 : F[2 * P + cell]);
-        const ll s1 = f[1] + f[2], s2 = f[3] + f[4], s3 = f[5] + f[6];
-        const ll s4 = f[7] + f[10], s5 = f[9] + f[8], s6 = f[11] + f[14], s7 = f[13] + f[12];
-        const ll s8 = f[15] + f[18], s9 = f[17] + f[16];
-        rho = f[0] + (s1 + s2 + s3) + ((s4 + s5) + (s6 + s7) + (s8 + s9));
-        const ll d4 = f[7] - f[10], d5 = f[9] - f[8], d6 = f[11] - f[14], d7 = f[13] - f[12];
-        const ll d8 = f[15] - f[18], d9 = f[17] - f[16];
-        rux = (f[1] - f[2]) + (d4 + d5) + (d6 + d7) + (fxp >> 1);
-        ruy = (f[3] - f[4]) + (d4 - d5) + (d8 + d9) + (fyp >> 1);
-        ruz = (f[5] - f[6]) + (d6 - d7) + (d8 - d9) + (fzp >> 1);
-        const ll inv = fx_recip(rho);
-        ux = qmul(rux, inv);
-        uy = qmul(ruy, inv);
-        uz = qmul(ruz, inv);
-        temp = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
-    }
-    // body force from (rho, u, T) of the previous macro (bouyancy3d_mpi.F90:743-745)
-    ll fx = 0, fy = 0;
-    if (ROT) {
-        fx = -qmul(qmul(rho, uy), K.t.omega2);
-        fy = qmul(qmul(rho, ux), K.t.omega2);
-        if (!oob(P + cell, (IDX)3 * P)) {
-            F[cell] = q2d(fx);
-            F[P + cell] = q2d(fy);
-        }
-    }
-    const ll fz = qmul(rho, qmulc(temp - K.t.t_ref, K.t.gbeta));
-    if (!oob((IDX)2 * P + cell, (IDX)3 * P)) F[2 * P + cell] = q2d(fz);
-    bad |= !mrt_collide_fx_forced(f, rho, ux, uy, uz, rux, ruy, ruz, fx, fy, fz, K.t);
-    mrt_collide_t_fx(g, temp, ux, uy, uz, K.t);
-
-    const double nan = __longlong_as_double(0x7ff8000000000000LL);
-    const IDX sy = (IDX)nx, sz = (IDX)nx * (IDX)ny;
-    const unsigned bm = face_mask(i, j, k, nx, ny, nz);
-#pragma unroll
-    for (int q = 0; q < Q19; q++) {
-        const int dx = ex19(q), dy = ey19(q), dz = ez19(q);
-        const double o = bad ? nan : (q < FX_CVT_OUT ? q2d_cvt(f[q]) : q2d(f[q]));
-        if (AAM == 1)  // in-place even step: own cell, slot opp(q)
-            st_chk(fout, (IDX)((IDX)opp19(q) * P + cell), (IDX)Q19 * P, o);
-        else if ((bm & leave_bits(dx, dy, dz)) == 0)
-            st_chk(fout, (IDX)((IDX)q * P + cell + (IDX)(dx + dy * (int)sy) + (IDX)dz * sz), (IDX)Q19 * P, o);
-        else
-            st_chk(fout, (IDX)((IDX)opp19(q) * P + cell), (IDX)Q19 * P, o);
-    }
-    // D3Q7: adiabatic walls reflect, constant-T walls anti-bounce-back
-#pragma unroll
-    for (int q = 0; q < Q7; q++) {
-        const int dx = ex19(q), dy = ey19(q), dz = ez19(q);
-        if ((bm & leave_bits(dx, dy, dz)) == 0) {
-            const double o = bad ? nan : (q < FXT_CVT_G ? q2d_cvt(g[q]) : q2d(g[q]));
-            if (AAM == 1)
-                st_chk(gout, (IDX)((IDX)opp19(q) * P + cell), (IDX)Q7 * P, o);
-            else
-                st_chk(gout, (IDX)((IDX)q * P + cell + (IDX)(dx + dy * (int)sy) + (IDX)dz * sz), (IDX)Q7 * P, o);
-        } else {
-            ll val = g[q];
-            if (dy != 0 && K.bc_y) val = -val + (dy < 0 ? K.t.chot : K.t.ccold);
-            if (dz != 0 && K.bc_z) val = -val + (dz < 0 ? K.t.chot : K.t.ccold);
-            st_chk(gout, (IDX)((IDX)opp19(q) * P + cell), (IDX)Q7 * P, bad ? nan : (q < FXT_CVT_G ? q2d_cvt(val) : q2d(val)));
-        }
-    }
 }
 
 }  // namespace mglc

@@ -82,6 +82,34 @@ def test_lid_matches_oracle_over_relaxation_times(mg, reynolds):
         _close(c.get_f(), o.s.f, 2)
 
 
+@pytest.mark.parametrize("ekman", [0.0, 1e-3])
+@pytest.mark.parametrize("macros", [False, True])
+@pytest.mark.parametrize("kind", ["flow", "dense", "fast", "edge", "mixed"])
+def test_heated_matches_oracle_in_and_out_of_range(mg, kind, macros, ekman):
+    nx, ny, nz = 33, 6, 5
+    ra = 1e5
+    f = _state(kind, (nz, ny, nx), 9)
+    rng = np.random.default_rng(10)
+    m = _macros(f)
+    o = O.ThermalOracle(nx, ny, nz, ra, 0.71, 0.1, ekman, 0.5, -0.5, 0.0)
+    T = rng.random((nz, ny, nx)) - 0.5
+    g = T[..., None] * (np.array([0.4] + [0.1] * 6) * (1 + 0.02 * (rng.random((nz, ny, nx, 7)) - 0.5)))
+    T = g.sum(-1)
+    if macros:
+        m, T = (np.full_like(m[0], 1.0), 0.5 * m[1], 0.5 * m[2], 0.5 * m[3]), 0.9 * T
+    o.f[:], o.g[:], o.T[:] = f, g, T
+    o.rho[:], o.u[:], o.v[:], o.w[:] = m
+    with mg.BuoyancyCavity(nx, ny, nz, rayleigh=ra, prandtl=0.71, mach=0.1, t_hot=0.5, t_cold=-0.5,
+                           ekman=ekman) as c:
+        c.load_state(f, g, *m, T) if macros else c.load_state(f, g)
+        for n in (1, 2):
+            c.step(1)
+            o.run(1)
+            gf, gg = c.get_f()
+            _close(gf, o.f, n)
+            _close(gg, o.g, n)
+
+
 def test_non_finite_cells_stay_non_finite(mg):
     """A NaN and an infinity take the FP64 form and spread with the stream, as in FP64."""
     f = _state("flow", (6, 6, 34), 7)
