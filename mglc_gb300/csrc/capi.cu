@@ -122,9 +122,9 @@ void release(mglc_ctx* c) {
     for (void* p : ptrs)
         if (p) cudaFree(p);
     PartDev& d = c->pd;
-    void* pptrs[] = {d.owner_cur, d.owner_new, d.xc, d.uc, d.om, d.xc_old, d.uc_old, d.om_old,
+    void* pptrs[] = {d.owner_cur, d.owner_new, d.xc, d.uc, d.om, d.xc_new, d.uc_new, d.om_new,
                      d.flink, d.tlink, d.corr, d.ftot, d.ttot, d.prep_sum, d.prep_cnt,
-                     d.partials, d.n_fluid, d.rho_avg, d.status};
+                     d.partials, d.n_fluid, d.rho_avg, d.status, d.done, d.rf_count, d.rf_list};
     for (void* p : pptrs)
         if (p) cudaFree(p);
     for (int h = 0; h < 2; h++) {
@@ -633,17 +633,22 @@ int mglc_step(mglc_ctx* c, int nsteps) {
                                                  c->f[nxt], c->pp, c->pd, c->stream);
             if (e != cudaSuccess) return cuda_fail(c, e, "particle step launch");
             std::swap(c->pd.owner_cur, c->pd.owner_new);
+            c->pd.par ^= 1;
             c->cur = nxt;
             c->first_pending = false;
             c->macros_valid = false;
             c->itc++;
         }
         // particle failures (overlap, wall penetration, ...) are reported here
-        int st[3] = {0, 0, 0};
+        int st[4] = {0, 0, 0, 0};
         CK(cudaMemcpyAsync(st, c->pd.status, sizeof st, cudaMemcpyDeviceToHost, c->stream),
            "read particle status");
         CK(cudaStreamSynchronize(c->stream), "synchronize");
         if (st[0]) {
+            if (st[3] != c->pd.par) {  // the mask the state is frozen with
+                std::swap(c->pd.owner_cur, c->pd.owner_new);
+                c->pd.par ^= 1;
+            }
             static const char* what[] = {"", "no particle owns a solid boundary node",
                                          "interpolation fraction q outside [0,1]",
                                          "particle-particle interpenetration",
@@ -917,21 +922,25 @@ int mglc_particle_create(const mglc_particle_params* p, const double* centers, i
     if ((rc = dalloc(c, (void**)&d.owner_cur, n * sizeof(int), "owner mask"))) return rc;
     if ((rc = dalloc(c, (void**)&d.owner_new, n * sizeof(int), "owner mask"))) return rc;
     const size_t v3 = sizeof(double) * 3 * (size_t)(np > 0 ? np : 1);
-    double** p3[] = {&d.xc, &d.uc, &d.om, &d.xc_old, &d.uc_old, &d.om_old, &d.ftot, &d.ttot};
+    double** p3[] = {&d.xc, &d.uc, &d.om, &d.xc_new, &d.uc_new, &d.om_new, &d.ftot, &d.ttot};
     for (double** a : p3)
         if ((rc = dalloc(c, (void**)a, v3, "particle state"))) return rc;
     // per-particle, per-slab partial sums of the boundary-link kernel
     if ((rc = dalloc(c, (void**)&d.flink, PART_NSLAB * v3, "link sums"))) return rc;
     if ((rc = dalloc(c, (void**)&d.tlink, PART_NSLAB * v3, "link sums"))) return rc;
     if ((rc = dalloc(c, (void**)&d.corr, PART_NSLAB * v3 / 3, "link sums"))) return rc;
-    if ((rc = dalloc(c, (void**)&d.prep_sum, v3 / 3, "particle sums"))) return rc;
-    if ((rc = dalloc(c, (void**)&d.prep_cnt, sizeof(int) * (size_t)(np > 0 ? np : 1), "particle sums"))) return rc;
+    const size_t n1 = (size_t)(np > 0 ? np : 1);
+    if ((rc = dalloc(c, (void**)&d.prep_sum, PART_NSLAB * v3 / 3, "particle sums"))) return rc;
+    if ((rc = dalloc(c, (void**)&d.prep_cnt, PART_NSLAB * sizeof(int) * n1, "particle sums"))) return rc;
+    if ((rc = dalloc(c, (void**)&d.rf_count, sizeof(int) * n1, "refill list"))) return rc;
+    if ((rc = dalloc(c, (void**)&d.rf_list, sizeof(long long) * PART_REFILL * n1, "refill list"))) return rc;
     d.nblocks = particle_bulk_blocks(pp);
-    // bulk partials (2 per warp) and the 2 x 32 stage-two sums of the finish kernel
-    if ((rc = dalloc(c, (void**)&d.partials, sizeof(double) * (2 * (size_t)d.nblocks + 64), "bulk partials"))) return rc;
+    // bulk partials (2 per warp) and the finish kernel's sums
+    if ((rc = dalloc(c, (void**)&d.partials, sizeof(double) * (2 * (size_t)d.nblocks + PART_FINISH), "bulk partials"))) return rc;
+    if ((rc = dalloc(c, (void**)&d.done, 4 * sizeof(unsigned), "block counters"))) return rc;
     if ((rc = dalloc(c, (void**)&d.n_fluid, 2 * sizeof(long long), "fluid count"))) return rc;
     if ((rc = dalloc(c, (void**)&d.rho_avg, 4 * sizeof(double), "average density"))) return rc;
-    if ((rc = dalloc(c, (void**)&d.status, 3 * sizeof(int), "particle status"))) return rc;
+    if ((rc = dalloc(c, (void**)&d.status, 4 * sizeof(int), "particle status"))) return rc;
     return MGLC_OK;
 }
 
@@ -946,7 +955,9 @@ int particle_initial(mglc_ctx* c) {
     CK(cudaMemsetAsync(d.om, 0, v3, c->stream), "zero rotation");
     CK(cudaMemsetAsync(d.ftot, 0, v3, c->stream), "zero forces");
     CK(cudaMemsetAsync(d.ttot, 0, v3, c->stream), "zero torques");
-    CK(cudaMemsetAsync(d.status, 0, 3 * sizeof(int), c->stream), "zero status");
+    CK(cudaMemsetAsync(d.status, 0, 4 * sizeof(int), c->stream), "zero status");
+    CK(cudaMemsetAsync(d.rf_count, 0, sizeof(int) * (size_t)(np > 0 ? np : 1), c->stream), "zero counters");
+    CK(cudaMemsetAsync(d.done, 0, 4 * sizeof(unsigned), c->stream), "zero counters");
     CK(cudaMemsetAsync(d.rho_avg, 0, 4 * sizeof(double), c->stream), "zero average");
     const size_t b = c->n * sizeof(double);
     CK(cudaMemsetAsync(c->up, 0, b, c->stream), "zero up");

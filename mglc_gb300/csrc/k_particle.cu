@@ -15,14 +15,15 @@
 //               streamed array: fp(a,y) sits in f(a, y+e_a) after the push
 //               (including solid destination cells, which only fluid pushes
 //               write).  Writes f(abar,x) and accumulates the Wen 2014
-//               momentum exchange (particle_force.F90:59-66) in FP64.
-//   k_pforce    one warp per particle: springs, gravity, body force
-//               (particle_force.F90:96-190)
-//   k_pmove     explicit update (particle_update.F90:26-50)
-//   k_pmark     new owner mask from the new centres (particle_update.F90:80-93)
-//   k_pprep     density bookkeeping of nodes that change phase
-//   k_prefill   refill of nodes that left a particle (:134-193), two phases
-//               per particle (all reads, then all writes).
+//               momentum exchange (particle_force.F90:59-66)
+//   k_pmark     springs, gravity and body force (:96-190), the particle's motion
+//               (particle_update.F90:26-50) and the owner mask of its new
+//               centre (:80-93), cleared by k_pbulk
+//   k_pphase    density bookkeeping of nodes that change phase and the list of
+//               nodes that left a particle
+//   k_prefill   refill of those nodes (:134-193), two phases per particle (all
+//               reads, then all writes), and the particle's new state.
+// Six launches a step instead of twelve.
 // Any kernel that detects a failure (no owner, q out of range, overlap, wall
 // penetration) writes a status code; every kernel returns at once while the
 // status is set, so the state freezes at the failing step and the host
@@ -31,7 +32,9 @@
 #include <cuda_fp16.h>
 
 #include <atomic>
+#include <cmath>
 
+#include "fix61.cuh"
 #include "macro64.cuh"
 #include "particles.cuh"
 
@@ -39,7 +42,6 @@ namespace mglc {
 
 constexpr int PB = 256;             // threads of the per-particle kernels
 constexpr int NSLAB = PART_NSLAB;   // CTAs per particle in k_plinks
-constexpr int REFILL_MAX = 256;     // refilled nodes one particle may produce per step
 
 template <typename S>
 struct PSt;
@@ -69,7 +71,7 @@ __device__ __forceinline__ void pset(S* f, long long idx, int q, double v, doubl
 
 // Signed x separation with the nearest periodic image.  Centres stay in
 // [0.5, nx + 0.5) and nodes in [1, nx], so one shift by L brings d into
-// [-L/2, L/2]; a larger |d| (a centre that jumped, which k_pmove reports)
+// [-L/2, L/2]; a larger |d| (a centre that jumped, which k_pmark reports)
 // takes the closed form d - L rint(d/L).  A non-finite d is returned as is:
 // no loop depends on it.
 __device__ __forceinline__ double dxp(double a, double b, const PartParams& p) {
@@ -90,6 +92,16 @@ __device__ __forceinline__ bool inside(double x, double y, double z, const doubl
     return d <= __dmul_rn(R, R);
 }
 __device__ __forceinline__ int wrapx(int i, int nx) { return i < 0 ? i + nx : (i >= nx ? i - nx : i); }
+
+// par: which owner buffer holds the mask that the state is frozen with (before
+// the particles move this step's, in the refill the new one)
+__device__ __forceinline__ void pfail(const PartDev& d, int code, int c, int other, int par) {
+    if (atomicCAS(d.status, 0, code) == 0) {
+        d.status[1] = c;
+        d.status[2] = other;
+        d.status[3] = par;
+    }
+}
 
 template <int NV>
 __device__ __forceinline__ void block_sum_to(double (&v)[NV], double* out, int stride) {
@@ -122,25 +134,153 @@ template <> struct PC<float> { using C = float; };
 // once on the host: double -> float conversions are slow on the device)
 template <typename C> struct PBulkK {
     C rho0, ax, ay, az;
+    MrtCoef<C> cd;
 };
+static PBulkK<float> bulk_k(const PartParams& p, float) {
+    return {(float)p.rho0, (float)p.body_force[0], (float)p.body_force[1], (float)p.body_force[2],
+            cast_coef<float>(make_mrt_coef(p.snu, p.sq))};
+}
+static PBulkK<double> bulk_k(const PartParams& p, double) {
+    return {p.rho0, p.body_force[0], p.body_force[1], p.body_force[2], make_mrt_coef(p.snu, p.sq)};
+}
+
+// The fluid collision of one cell: f in place; rho_m the density as stored
+// (less rho0 for deviations).
+template <bool FIRST>
+__device__ __forceinline__ void pcollide(float (&f)[Q19], const PBulkK<float>& k, float& rho_m) {
+    float rho, ux, uy, uz;
+    if (FIRST) {  // the reference's initial fields: rho0, u = 0
+        rho = k.rho0;
+        rho_m = 0.0f;
+        ux = uy = uz = 0.0f;
+    } else {
+        float jx, jy, jz;
+        moments0(f, rho_m, jx, jy, jz);
+        rho = k.rho0 + rho_m;
+        // u = (sum f e + F/2)/rho with F = rho*a (thermal macro form)
+        const float inv = __frcp_rn(rho);
+        ux = (jx + 0.5f * (rho * k.ax)) * inv;
+        uy = (jy + 0.5f * (rho * k.ay)) * inv;
+        uz = (jz + 0.5f * (rho * k.az)) * inv;
+    }
+    mrt_collide<float, true, false>(f, rho_m, rho, ux, uy, uz, rho * k.ax, rho * k.ay, rho * k.az,
+                                    k.cd);
+}
+// The FP64 form's torques nearly cancel, so the rounding of every population
+// shows in them and the collision keeps the operations of the moment form.  It
+// is bound by the FP64 pipe (a warp's instruction holds the unit for 16 clocks),
+// while nine tenths of the issue slots are empty; so the additions of the
+// forward transform, a third of its operations, run on integers: populations in
+// [2^-6, 1/2) are exact in units of 2^-58, and an integer addition followed by
+// rounding to 53 significant bits (rn53) is the FP64 addition bit for bit.
+struct Fix58 {
+    long long v;
+};
+__device__ __forceinline__ Fix58 operator+(Fix58 a, Fix58 b) { return {rn53(a.v + b.v)}; }
+__device__ __forceinline__ Fix58 operator-(Fix58 a, Fix58 b) { return {rn53(a.v - b.v)}; }
+__device__ __forceinline__ bool fix58_ok(const double (&f)[Q19]) {
+    unsigned worst = 0;
+#pragma unroll
+    for (int q = 1; q < Q19; q++)
+        worst = max(worst, (unsigned)__double2hiint(f[q]) - 0x3F900000u);  // 2^-6
+    return worst < 0x00300000u &&                                          // below 2^-3
+           (unsigned)__double2hiint(f[0]) - 0x3F900000u < 0x00500000u;     // below 1/2
+}
+// a value of at most 53 significant bits as the double it is
+__device__ __forceinline__ double fix58_out(long long v) {
+    const long long sg = v >> 63;
+    const unsigned long long a = (unsigned long long)((v ^ sg) - sg);
+    const int lz = __clzll((long long)a);
+    const unsigned long long m = a << (lz & 63) >> 11;  // the leading bit at bit 52
+    const unsigned long long b = m + ((unsigned long long)(unsigned)(1022 + 63 - 58 - lz) << 52);
+    return __longlong_as_double((long long)(a ? b | ((unsigned long long)sg << 63) : 0ull));
+}
+__device__ __forceinline__ void fix58_moments(const double (&f)[Q19], MrtMom<double>& o,
+                                              double& rho, double& jx, double& jy, double& jz) {
+    Fix58 F[Q19];
+#pragma unroll
+    for (int q = 0; q < Q19; q++) F[q].v = fix61_load(f[q]) >> 3;  // exact
+    Fix58 r, x, y, z;
+    moments0(F, r, x, y, z);
+    const Fix58 s1 = F[1] + F[2], d1 = F[1] - F[2], s2 = F[3] + F[4], d2 = F[3] - F[4];
+    const Fix58 s3 = F[5] + F[6], d3 = F[5] - F[6], s4 = F[7] + F[10], d4 = F[7] - F[10];
+    const Fix58 s5 = F[9] + F[8], d5 = F[9] - F[8], s6 = F[11] + F[14], d6 = F[11] - F[14];
+    const Fix58 s7 = F[13] + F[12], d7 = F[13] - F[12], s8 = F[15] + F[18], d8 = F[15] - F[18];
+    const Fix58 s9 = F[17] + F[16], d9 = F[17] - F[16];
+    const Fix58 sa = s1 + s2 + s3, se = (s4 + s5) + (s6 + s7) + (s8 + s9);
+    // the fused multiply-adds of mrt_moments as nvcc contracts them: one rounding
+    // of the exact value (8 se + RN(-11 sa) in m1)
+    o.m1 = fix58_out(rn53(-30 * F[0].v + rn53(8 * se.v + rn53(-11 * sa.v))));
+    o.m2 = fix58_out(rn53(12 * F[0].v + rn53(-4 * sa.v + se.v)));
+    const Fix58 a45 = d4 + d5, b45 = d4 - d5, a67 = d6 + d7, b67 = d6 - d7, a89 = d8 + d9,
+                b89 = d8 - d9;
+    o.m4 = fix58_out(rn53(-4 * d1.v + (a45 + a67).v));
+    o.m6 = fix58_out(rn53(-4 * d2.v + (b45 + a89).v));
+    o.m8 = fix58_out(rn53(-4 * d3.v + (b67 + b89).v));
+    const Fix58 sxy = s4 + s5, sxz = s6 + s7, syz = s8 + s9, s23 = s2 + s3, t23 = s2 - s3;
+    const Fix58 sp = sxy + sxz, sm = sxy - sxz;
+    o.m9 = fix58_out(rn53((Fix58{rn53(2 * s1.v - s23.v)} + sp).v - 2 * syz.v));
+    o.m10 = fix58_out(rn53((Fix58{rn53(-4 * s1.v + 2 * s23.v)} + sp).v - 2 * syz.v));
+    o.m11 = fix58_out((t23 + sm).v);
+    o.m12 = fix58_out(rn53(-2 * t23.v + sm.v));
+    o.m13 = fix58_out((s4 - s5).v);
+    o.m14 = fix58_out((s8 - s9).v);
+    o.m15 = fix58_out((s6 - s7).v);
+    o.m16 = fix58_out((a45 - a67).v);
+    o.m17 = fix58_out(rn53(-b45.v + a89.v));
+    o.m18 = fix58_out((b67 - b89).v);
+    rho = fix58_out(r.v);
+    jx = fix58_out(x.v);
+    jy = fix58_out(y.v);
+    jz = fix58_out(z.v);
+}
+template <bool FIRST>
+__device__ __forceinline__ void pcollide(double (&f)[Q19], const PBulkK<double>& k, double& rho) {
+    double ux = 0.0, uy = 0.0, uz = 0.0;
+    MrtMom<double> m;
+    if (FIRST) {
+        rho = k.rho0;
+        m = mrt_moments(f);
+    } else {
+        double jx, jy, jz;
+        if (fix58_ok(f)) {
+            fix58_moments(f, m, rho, jx, jy, jz);
+        } else {
+            moments0(f, rho, jx, jy, jz);
+            m = mrt_moments(f);
+        }
+        // u = (sum f e + F/2)/rho with F = rho*a (thermal macro form)
+        div_by(jx + 0.5 * (rho * k.ax), jy + 0.5 * (rho * k.ay), jz + 0.5 * (rho * k.az), rho, ux,
+               uy, uz);
+    }
+    mrt_relax<double, true, false>(f, m, rho, rho, ux, uy, uz, rho * k.ax, rho * k.ay, rho * k.az,
+                                   k.cd);
+}
 
 // One thread per node of an x-row segment.  Fluid nodes collide and push
 // their populations (walls at y, z and, unless periodic, x bounce them back in
 // place); solid nodes do nothing.  Each warp writes its partial sums of the
 // fluid density before collision and of the post-collision mass to its own
 // slot, so no block barrier is needed and the totals are added in a fixed
-// order by k_pfinish.
-// resident 128-thread blocks per SM the FP32 bulk kernel holds its registers to
+// order by k_pfinish.  The FP32 form writes its two FP32 sums and its count of
+// fluid nodes and leaves FP64 to k_pfinish (a warp's FP64 instruction holds the
+// unit for 16 clocks, and there were seven for every 32 cells); the FP64 form's
+// collision conserves mass to its rounding, so the density serves as both sums.
+// The owner mask that the next positions will be marked in is cleared on the
+// way.
+// resident 128-thread blocks per SM the bulk kernel holds its registers to
 #ifndef MGLC_PBULK_MINB
 #define MGLC_PBULK_MINB 8
 #endif
+#ifndef MGLC_PBULK_MINB64
+#define MGLC_PBULK_MINB64 5
+#endif
 template <typename S, bool FIRST, typename IDX>
-__global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : 4))
+__global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : MGLC_PBULK_MINB64))
     k_pbulk(const S* __restrict__ fin, S* __restrict__ fout, const int* __restrict__ owner,
-            PartParams p, MrtCoef<typename PC<S>::C> cd, PBulkK<typename PC<S>::C> bk,
+            int* __restrict__ owner_new, PartParams p, PBulkK<typename PC<S>::C> bk,
             double* partials, const int* status) {
     using C = typename PC<S>::C;
-    constexpr bool DEV = PSt<S>::SHIFT;
     if (status[0]) return;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -157,37 +297,15 @@ __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : 4))
         for (int q = 0; q < Q19; q++) f[q] = (C)__ldg(fin + (q * P + cell));
     }
     const bool fluid = active && __ldg(owner + cell) < 0;
+    if (active) owner_new[cell] = -1;
     if (fluid) {
-        const C rho0 = bk.rho0, ax = bk.ax, ay = bk.ay, az = bk.az;
-        C rho_m, rho, ux, uy, uz;
-        if (FIRST) {  // the reference's initial fields: rho0, u = 0
-            rho = rho0;
-            rho_m = DEV ? C(0) : rho0;
-            ux = uy = uz = C(0);
-        } else {
-            C jx, jy, jz;
-            moments0(f, rho_m, jx, jy, jz);
-            rho = DEV ? rho0 + rho_m : rho_m;
-            // u = (sum f e + F/2)/rho with F = rho*a (thermal macro form); FP32
-            // multiplies by the correctly rounded reciprocal, FP64 divides
-            if constexpr (sizeof(C) == 4) {
-                const C inv = __frcp_rn(rho);
-                ux = (jx + C(0.5) * (rho * ax)) * inv;
-                uy = (jy + C(0.5) * (rho * ay)) * inv;
-                uz = (jz + C(0.5) * (rho * az)) * inv;
-            } else {
-                ux = (jx + C(0.5) * (rho * ax)) / rho;
-                uy = (jy + C(0.5) * (rho * ay)) / rho;
-                uz = (jz + C(0.5) * (rho * az)) / rho;
-            }
-        }
-        // deviation storage sums deviations (rho0 added back per warp)
-        cacc[0] = DEV ? rho_m : rho;
-        mrt_collide<C, true, false>(f, rho_m, rho, ux, uy, uz, rho * ax, rho * ay, rho * az, cd);
-        C m = C(0);
+        pcollide<FIRST>(f, bk, cacc[0]);
+        if (sizeof(C) == 4) {
+            C m = C(0);
 #pragma unroll
-        for (int q = 0; q < Q19; q++) m += f[q];
-        cacc[1] = m;
+            for (int q = 0; q < Q19; q++) m += f[q];
+            cacc[1] = m;
+        }
         const IDX sy = nx, sz = (IDX)nx * ny;
         if (i > 0 && i < nx - 1 && j > 0 && j < ny - 1 && k > 0 && k < nz - 1) {
             // interior node: every population streams, no wrap
@@ -209,82 +327,84 @@ __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : 4))
             }
         }
     }
+    constexpr int NS = sizeof(C) == 4 ? 2 : 1;
 #pragma unroll
-    for (int q = 0; q < 2; q++)
+    for (int q = 0; q < NS; q++)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) cacc[q] += __shfl_down_sync(0xffffffffu, cacc[q], o);
     // fluid cells of this warp (deviation storage adds rho0 for each of them)
     const unsigned fl = __ballot_sync(0xffffffffu, fluid);
-    if ((threadIdx.x & 31) == 0) {  // FP64 only for the warp leaders
+    if ((threadIdx.x & 31) == 0) {
         const int nw = blockDim.x >> 5;
         const int b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
         const int slot = b * nw + (threadIdx.x >> 5);
         const int nslot = gridDim.x * gridDim.y * gridDim.z * nw;
-        const double nf = DEV ? (double)__popc(fl) * p.rho0 : 0.0;
-        partials[slot] = (double)cacc[0] + nf;
-        partials[nslot + slot] = (double)cacc[1] + nf;
+        if constexpr (sizeof(C) == 4) {
+            ((float2*)partials)[slot] = make_float2(cacc[0], cacc[1]);
+            ((int*)(partials + nslot))[slot] = __popc(fl);
+        } else {
+            partials[slot] = cacc[0];
+        }
     }
 }
 
-constexpr int FINISH_BLOCKS = 32;
+// blocks: the FP64 form's torques nearly cancel and show the rounding of the
+// average, so its ranges stay 32 (7 us for 16384 partials); the FP32 form, whose
+// partials are eight times as many in the channel, spreads over the SMs
+template <typename S>
+constexpr int FINISH_BLOCKS = PSt<S>::SHIFT ? 128 : 32;
 
-// stage 1: FINISH_BLOCKS contiguous ranges of the bulk partials
-__global__ void k_pfinish(PartDev d, int nblocks) {
+// rho_avg at bounce-back and the post-collision mass from the bulk partials:
+// FINISH_BLOCKS contiguous ranges; the last block to finish adds their sums by
+// a fixed shuffle tree (as two launches: 14 + 4 us)
+template <typename S>
+__global__ void __launch_bounds__(256) k_pfinish(PartDev d, int nblocks, double rho0) {
     if (d.status[0]) return;
-    const int per = (nblocks + FINISH_BLOCKS - 1) / FINISH_BLOCKS;
+    __shared__ int last;
+    constexpr int NB = FINISH_BLOCKS<S>;
+    const int per = (nblocks + NB - 1) / NB;
     const int b0 = blockIdx.x * per, b1 = min(nblocks, b0 + per);
+    double* part = d.partials + 2 * (size_t)nblocks;
     double acc[2] = {0.0, 0.0};
+#pragma unroll 4
     for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) {
-        acc[0] += d.partials[b];
-        acc[1] += d.partials[nblocks + b];
+        if constexpr (PSt<S>::SHIFT) {
+            const float2 v = ((const float2*)d.partials)[b];
+            const double nf = (double)((const int*)(d.partials + nblocks))[b] * rho0;
+            acc[0] += (double)v.x + nf;
+            acc[1] += (double)v.y + nf;
+        } else {
+            acc[0] += d.partials[b];
+        }
     }
     __shared__ double out[2];
     block_sum_to<2>(acc, out, 1);
     if (threadIdx.x == 0) {
-        d.partials[2 * nblocks + blockIdx.x] = out[0];
-        d.partials[2 * nblocks + FINISH_BLOCKS + blockIdx.x] = out[1];
+        part[blockIdx.x] = out[0];
+        part[NB + blockIdx.x] = PSt<S>::SHIFT ? out[1] : out[0];
+        __threadfence();
+        last = atomicAdd(d.done, 1u) == gridDim.x - 1;
     }
-}
-// stage 2 (one warp): rho_avg at bounce-back and the post-collision mass
-__global__ void k_pfinish2(PartDev d, int nblocks) {
-    if (d.status[0]) return;
-    const int lane = threadIdx.x;
-    double a0 = d.partials[2 * nblocks + lane], a1 = d.partials[2 * nblocks + FINISH_BLOCKS + lane];
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return;
+    __threadfence();
+    double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+    for (int q = 0; q < NB; q += 32) {
+        a0 += __ldcg(part + q + threadIdx.x);
+        a1 += __ldcg(part + NB + q + threadIdx.x);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         a0 += __shfl_down_sync(0xffffffffu, a0, o);
         a1 += __shfl_down_sync(0xffffffffu, a1, o);
     }
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
         d.rho_avg[0] = a0 / (double)d.n_fluid[0];
         d.rho_avg[2] = a1;
+        *d.done = 0;
     }
 }
-// average density over the new fluid set, used by the refill (one warp,
-// fixed order): (mass after bounce-back + link corrections + phase changes)
-// / (fluid count + its change)
-__global__ void k_prefill_avg(PartParams p, PartDev d) {
-    if (d.status[0]) return;
-    const int lane = threadIdx.x;
-    double sum = 0.0;
-    long long cnt = 0;
-    for (int q = lane; q < p.np; q += 32) {
-        for (int sl = 0; sl < NSLAB; sl++) sum += d.corr[q * NSLAB + sl];
-        sum += d.prep_sum[q];
-        cnt += d.prep_cnt[q];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sum += __shfl_down_sync(0xffffffffu, sum, o);
-        cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-    }
-    if (lane == 0) {
-        const long long n1 = d.n_fluid[0] + cnt;
-        d.rho_avg[1] = (d.rho_avg[2] + sum) / (double)n1;
-        d.n_fluid[1] = n1;  // moved into slot 0 by k_pcommit
-    }
-}
-
 // --------------------------------------------------- boundary links (IBB) --
 // Deviation f - w rho0 of the post-collision value fp(q, c) of node c
 // (coordinates as 0-based indices), read from the streamed array; nodes
@@ -373,58 +493,197 @@ __device__ __forceinline__ bool node_avail(int i, int j, int k, const PartParams
 // TILE: the owner ids of the slab's box plus a one-node halo are staged in
 // dynamic shared memory (walls and, without periodicity, the x faces as -2),
 // so the scan's 19 lookups per node stay on chip.
+// FP64 instructions are what the FP32 form spends its time on if they are left
+// in (each holds the SM's unit for 16 clocks or more, whatever lanes are
+// active), so: the centre's conversions are one warp's; the node's distance to
+// the surface is an exact fixed-point one; the few links that need an FP64 root
+// are collected and take it together; the slab's sums are integers and pairs of
+// FP32 values (TwoSum).  A link's values and masks are loaded before any is used
+// (one latency a link instead of three), after the roots, so that the warps need
+// no barrier between their links.  200 spheres of radius 5, FP32: 95 -> 48 us
+// (1.3 waves of blocks, a quarter of the issue slots waiting at barriers);
+// blocks of 128 threads, one wave: 69 us.  24 spheres, FP64: 59 -> 46 us, the
+// FP64 unit of the 96 SMs that have a block.
+// What a block of k_plinks needs of its particle's centre, converted once.
+template <typename L>
+struct LinkCentre {
+    double X0, X1, X2;
+    L ox, oy, oz;           // spin
+    L ux, uy, uz, ravg;     // velocity, average density
+    float xf0, xf1, xf2, reach2;
+    // FP32 form: floor of the centre, its fraction in units of 2^-52, R^2 in
+    // units of 2^-(2 sh - 64); sh: shift that takes distances below R + 2 to 62
+    // bits (0: the centre is not a multiple of 2^-52, or R is too large)
+    int fi, fj, fk, sh;
+    long long qi, qj, qk, r2;
+};
+
+// |v| * |v| / 2^64
+__device__ __forceinline__ long long sq_hi(long long v) {
+    const unsigned long long a = (unsigned long long)(v < 0 ? -v : v);
+    return (long long)__umul64hi(a, a);
+}
+
+// resident blocks per SM the FP32 link kernel holds its registers to
+#ifndef MGLC_PLINKS_MINB
+#define MGLC_PLINKS_MINB 4
+#endif
 template <typename S, bool TILE>
-__global__ void __launch_bounds__(PB) k_plinks(S* __restrict__ f, PartParams p, PartDev d) {
+__global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
+    k_plinks(S* __restrict__ f, PartParams p, PartDev d) {
     using L = typename PC<S>::C;
     if (d.status[0]) return;
+    __shared__ LinkCentre<L> s_c;
+    __shared__ int s_box[3];
+    __shared__ int s_list[LINK_CAP];  // box index * 32 + direction
+    __shared__ int s_wsum[2][PB / 32];
+    __shared__ float s_hi[PB / 32][7], s_lo[PB / 32][7];
+    __shared__ double s_av[PB / 32][7], s_out[13];
+    __shared__ int s_int[PB / 32][6];
+    __shared__ int s_def[PB], s_nd;  // listed links that take the FP64 root,
+    __shared__ float s_q[PB];        // and the roots
+    extern __shared__ int s_own[];
     const int c = blockIdx.x, slab = blockIdx.y;
-    const double X0 = d.xc[3 * c], X1 = d.xc[3 * c + 1], X2 = d.xc[3 * c + 2];
-    const L Ux = (L)d.uc[3 * c], Uy = (L)d.uc[3 * c + 1], Uz = (L)d.uc[3 * c + 2];
-    const L Ox = (L)d.om[3 * c], Oy = (L)d.om[3 * c + 1], Oz = (L)d.om[3 * c + 2];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const double R = p.radius;
-    const L ravg = (L)d.rho_avg[0];
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const long long P = (long long)nx * ny * nz;
     // box of nodes within R+2 of the centre (1-based coordinate = index + 1)
+    if (threadIdx.x < 3) s_box[threadIdx.x] = (int)floor(d.xc[3 * c + threadIdx.x]);
+    if (threadIdx.x == 0) s_nd = 0;
     const int h = (int)ceil(R) + 2;
-    const int ci = (int)floor(X0) - 1, cj = (int)floor(X1) - 1, ck = (int)floor(X2) - 1;
+    __syncthreads();
+    const int ci = s_box[0] - 1, cj = s_box[1] - 1, ck = s_box[2] - 1;
     const int bw = 2 * h + 2;
     const int kz0 = slab * bw / NSLAB, kz1 = (slab + 1) * bw / NSLAB;
     const int nbox = bw * bw * (kz1 - kz0);
-    const float reach2f = (float)((R + 1.8) * (R + 1.8));  // |x - X| <= R + sqrt(2) for a link
-    const float Xf0 = (float)X0, Xf1 = (float)X1, Xf2 = (float)X2, Lf = (float)p.nx;
+    const int TX = bw + 2, TY = bw + 2, TZ = kz1 - kz0 + 2;
+    if (TILE) {
+        // a thread walks the tile in strides of PB without divisions, TU loads in flight
+        int ti = (int)threadIdx.x % TX, tj = (int)threadIdx.x / TX % TY, tk = (int)threadIdx.x / (TX * TY);
+        const int ai = PB % TX, aj = PB / TX % TY, ak = PB / (TX * TY), nt_ = TX * TY * TZ;
+        constexpr int TU = 6;
+        for (int e = threadIdx.x; e < nt_; e += TU * PB) {
+            int o[TU];
+#pragma unroll
+            for (int u = 0; u < TU; u++) {
+                int i = ci - h + ti - 1;
+                const int j = cj - h + tj - 1, k = ck - h + kz0 + tk - 1;
+                if (p.periodic_x) i = i < 0 ? i + nx : (i >= nx ? i - nx : i);
+                const bool in = e + u * PB < nt_ && j >= 0 && j < ny && k >= 0 && k < nz && i >= 0 && i < nx;
+                o[u] = in ? d.owner_cur[i + (long long)nx * (j + (long long)ny * k)] : -2;
+                ti += ai;
+                int carry = ti >= TX;
+                if (carry) ti -= TX;
+                tj += aj + carry;
+                carry = tj >= TY;
+                if (carry) tj -= TY;
+                tk += ak + carry;
+            }
+#pragma unroll
+            for (int u = 0; u < TU; u++)
+                if (e + u * PB < nt_) s_own[e + u * PB] = o[u];
+        }
+    }
+    if (wid == PB / 32 - 1) {
+        const double X0 = d.xc[3 * c], X1 = d.xc[3 * c + 1], X2 = d.xc[3 * c + 2];
+        LinkCentre<L> v;
+        v.X0 = X0; v.X1 = X1; v.X2 = X2;
+        v.ux = (L)d.uc[3 * c]; v.uy = (L)d.uc[3 * c + 1]; v.uz = (L)d.uc[3 * c + 2];
+        v.ox = (L)d.om[3 * c]; v.oy = (L)d.om[3 * c + 1]; v.oz = (L)d.om[3 * c + 2];
+        v.ravg = (L)d.rho_avg[0];
+        v.reach2 = (float)((R + 1.8) * (R + 1.8));  // |x - X| <= R + sqrt(2) for a link
+        v.xf0 = (float)X0; v.xf1 = (float)X1; v.xf2 = (float)X2;
+        v.sh = 0;
+        if (sizeof(L) == 4) {
+            const double one = 4503599627370496.0;  // 2^52
+            const double f0 = floor(X0), f1 = floor(X1), f2 = floor(X2);
+            const double q0 = (X0 - f0) * one, q1 = (X1 - f1) * one, q2 = (X2 - f2) * one;
+            const int bits = 32 - __clz(h);  // distances below 2^bits
+            if (q0 == floor(q0) && q1 == floor(q1) && q2 == floor(q2) && bits <= 9) {
+                v.fi = s_box[0]; v.fj = s_box[1]; v.fk = s_box[2];
+                v.qi = (long long)q0; v.qj = (long long)q1; v.qk = (long long)q2;
+                v.sh = 62 - bits;
+                v.r2 = __double2ll_rn(ldexp(R * R, 2 * v.sh - 64));
+            }
+        }
+        if (lane == 0) s_c = v;
+    }
+    __syncthreads();
+    const double X0 = s_c.X0, X1 = s_c.X1, X2 = s_c.X2;
+    const L Ux = s_c.ux, Uy = s_c.uy, Uz = s_c.uz, Ox = s_c.ox, Oy = s_c.oy, Oz = s_c.oz;
+    const L ravg = s_c.ravg;
+    const float reach2f = s_c.reach2, Xf0 = s_c.xf0, Xf1 = s_c.xf1, Xf2 = s_c.xf2, Lf = (float)p.nx;
+    const int sh = s_c.sh;
     int nf[3] = {0, 0, 0};  // sum m e
     int nt[3] = {0, 0, 0};  // sum m (n x e)
     L av[7] = {L(0), L(0), L(0), L(0), L(0), L(0), L(0)};  // variable force, torque, mass change
-    // Links are listed (box index, direction) over the scan rounds of PB box
-    // nodes, in a deterministic order, and processed one per thread once the
-    // list is nearly full or the box is done.
-    __shared__ int s_t[LINK_CAP];
-    __shared__ unsigned char s_dir[LINK_CAP];
-    __shared__ int s_n;
-    __shared__ int s_wsum[PB / 32];
-    extern __shared__ int s_own[];
-    const int TX = bw + 2, TY = bw + 2, TZ = kz1 - kz0 + 2;
-    if (TILE) {
-        for (int e = threadIdx.x; e < TX * TY * TZ; e += PB) {
-            const int ti = e % TX, tj = (e / TX) % TY, tk = e / (TX * TY);
-            int i = ci - h + ti - 1;
-            const int j = cj - h + tj - 1, k = ck - h + kz0 + tk - 1;
-            int o = -2;
-            if (j >= 0 && j < ny && k >= 0 && k < nz) {
-                if (p.periodic_x) i = i < 0 ? i + nx : (i >= nx ? i - nx : i);
-                if (i >= 0 && i < nx) o = d.owner_cur[i + (long long)nx * (j + (long long)ny * k)];
-            }
-            s_own[e] = o;
-        }
-    }
     auto own_at = [&](int bi, int bj, int bk) {  // box coordinates, bk absolute in the box
         return s_own[(bi + 1) + TX * ((bj + 1) + TY * (bk - kz0 + 1))];
     };
-    if (threadIdx.x == 0) s_n = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int t0 = 0; t0 < nbox; t0 += PB) {
+    // The fraction q of listed link le: ray-sphere root from the node (calQ2,
+    // particle_bounceback.F90:144-185), FP64 (false: out of range, status set).
+    // The node lies within R + 1.8 < nx / 2 of the centre: the unwrapped difference
+    // is the periodic minimum image.
+    auto root64 = [&](int le, double& qd) {
+        const int tt = le >> 5, a = le & 31;
+        const int ea = e_rt(EX_PACK, a), eb = e_rt(EY_PACK, a), ec = e_rt(EZ_PACK, a);
+        const double ox = (double)(ci - h + tt % bw + 1) - X0, oy = (double)(cj - h + tt / bw % bw + 1) - X1,
+                     oz = (double)(ck - h + kz0 + tt / (bw * bw) + 1) - X2;
+        const double sx = ea > 0 ? ox : (ea < 0 ? -ox : 0.0);
+        const double sy = eb > 0 ? oy : (eb < 0 ? -oy : 0.0);
+        const double sz = ec > 0 ? oz : (ec < 0 ? -oz : 0.0);
+        const double cc = ox * ox + oy * oy + oz * oz - R * R;
+        const double cb = 2.0 * (sx + sy + sz);
+        const double delta = cb * cb - (a <= 6 ? 4.0 : 8.0) * cc;
+        if (delta < 0) { pfail(d, PS_Q_RANGE, c, 0, d.par); return false; }
+        qd = (-cb - sqrt(delta)) * (a <= 6 ? 0.5 : 0.25);  // /(2 |e|^2), exact
+        if (qd > 1.0 || qd < 0.0) { pfail(d, PS_Q_RANGE, c, 0, d.par); return false; }
+        return true;
+    };
+    // FP32 form: |x - X|^2 - R^2 (the cancelling part) beyond FP32, the root in FP32.
+    // Its error grows where the ray is nearly tangent (small delta) and matters
+    // where q is near 0 or 1, the ends the range check tests: those links (false)
+    // take the FP64 root, so the FP32 and FP64 forms accept and reject the same links.
+    auto root32 = [&](int le, float& ox, float& oy, float& oz, float& q) {
+        const int tt = le >> 5, a = le & 31;
+        const int iu = ci - h + tt % bw, j = cj - h + tt / bw % bw, k = ck - h + kz0 + tt / (bw * bw);
+        const int ea = e_rt(EX_PACK, a), eb = e_rt(EY_PACK, a), ec = e_rt(EZ_PACK, a);
+        float cbf, ccf;
+        if (sh) {
+            // x - X exactly, in units of 2^-52, and its square to 2^-52 or so
+            const long long wx = ((long long)(iu + 1 - s_c.fi) << 52) - s_c.qi;
+            const long long wy = ((long long)(j + 1 - s_c.fj) << 52) - s_c.qj;
+            const long long wz = ((long long)(k + 1 - s_c.fk) << 52) - s_c.qk;
+            const long long w = wx * ea + wy * eb + wz * ec;
+            const int up = sh - 52;
+            const long long cc = sq_hi(wx << up) + sq_hi(wy << up) + sq_hi(wz << up) - s_c.r2;
+            ox = (float)wx * 0x1p-52f;
+            oy = (float)wy * 0x1p-52f;
+            oz = (float)wz * 0x1p-52f;
+            cbf = 2.0f * ((float)w * 0x1p-52f);
+            ccf = (float)cc * __int_as_float((127 - (2 * sh - 64)) << 23);
+        } else {
+            const double x = (double)(iu + 1) - X0, y = (double)(j + 1) - X1, z = (double)(k + 1) - X2;
+            const double sx = ea > 0 ? x : (ea < 0 ? -x : 0.0);
+            const double sy = eb > 0 ? y : (eb < 0 ? -y : 0.0);
+            const double sz = ec > 0 ? z : (ec < 0 ? -z : 0.0);
+            ox = (float)x;
+            oy = (float)y;
+            oz = (float)z;
+            cbf = 2.0f * (float)(sx + sy + sz);
+            ccf = (float)(x * x + y * y + z * z - R * R);
+        }
+        const float delta = cbf * cbf - (a <= 6 ? 4.0f : 8.0f) * ccf;
+        q = (-cbf - sqrtf(fmaxf(delta, 0.0f))) * (a <= 6 ? 0.5f : 0.25f);
+        return delta > 1e-2f * cbf * cbf + 1e-3f && q > 1e-3f && q < 1.0f - 1e-3f;
+    };
+    // Links are listed (box index, direction) over the scan rounds of PB box
+    // nodes, in a deterministic order, and processed one per thread once the
+    // list is nearly full or the box is done.
+    int nl = 0;  // listed so far, the same in every thread
+    int par = 0;
+    for (int t0 = 0; t0 < nbox; t0 += PB, par ^= 1) {
         unsigned my_dirs = 0;  // bit a: direction a is a boundary link of my node
         const int t = t0 + threadIdx.x;
         if (t < nbox) {
@@ -473,63 +732,90 @@ __global__ void __launch_bounds__(PB) k_plinks(S* __restrict__ f, PartParams p, 
             const int v = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += v;
         }
-        if (lane == 31) s_wsum[wid] = incl;
+        if (lane == 31) s_wsum[par][wid] = incl;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            int run = s_n;
-            for (int q = 0; q < PB / 32; q++) {
-                const int v = s_wsum[q];
-                s_wsum[q] = run;
-                run += v;
-            }
-            s_n = run;
+        int slot = nl + incl - cnt;
+#pragma unroll
+        for (int q = 0; q < PB / 32; q++) {
+            const int v = s_wsum[par][q];
+            if (q < wid) slot += v;
+            nl += v;
         }
-        __syncthreads();
-        int slot = s_wsum[wid] + incl - cnt;
-        for (unsigned m = my_dirs; m; m &= m - 1) {
-            s_t[slot] = t;
-            s_dir[slot] = (unsigned char)(__ffs(m) - 1);
-            slot++;
-        }
-        const int nl = s_n;
+        for (unsigned m = my_dirs; m; m &= m - 1) s_list[slot++] = t * 32 + __ffs(m) - 1;
         if (nl <= LINK_CAP - PB * 18 && t0 + PB < nbox) continue;  // uniform over the block
         __syncthreads();
+        if constexpr (sizeof(L) == 4) {
+            // the links that need it take their FP64 root together, over the
+            // whole list, before any is processed (s_def full: where they are)
+            for (int e = threadIdx.x; e < nl; e += PB) {
+                const int le = s_list[e];
+                float ox, oy, oz, q;
+                if (root32(le, ox, oy, oz, q)) continue;
+                const int slot = atomicAdd(&s_nd, 1);
+                if (slot < PB) {
+                    s_def[slot] = le;
+                    s_list[e] = -1 - slot;
+                }
+            }
+            __syncthreads();
+            if (threadIdx.x < s_nd) {
+                const int le = s_def[threadIdx.x];
+                double qd;
+                s_q[threadIdx.x] = root64(le, qd) ? (float)qd : -1.0f;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) s_nd = 0;
+        }
         for (int e = threadIdx.x; e < nl; e += PB) {
-            const int tt = s_t[e], a = s_dir[e];
+            int le = s_list[e];
+            L ox, oy, oz, q;
+            if constexpr (sizeof(L) == 4) {
+                bool have = false;
+                if (le < 0) {
+                    q = s_q[-1 - le];
+                    le = s_def[-1 - le];
+                    have = true;
+                    if (q < 0.0f) continue;
+                }
+                float qf;
+                const bool near = root32(le, ox, oy, oz, qf);
+                if (!have) q = qf;
+                if (!have && !near) {
+                    double qd;
+                    if (!root64(le, qd)) continue;
+                    q = (float)qd;
+                }
+            } else {
+                if (!root64(le, q)) continue;
+            }
+            const int tt = le >> 5, a = le & 31;
             const int bi = tt % bw, bj = (tt / bw) % bw, bk = kz0 + tt / (bw * bw);
             const int iu = ci - h + bi, j = cj - h + bj, k = ck - h + bk;  // iu: unwrapped
             const int i = p.periodic_x ? wrapx(iu, nx) : iu;
             const int ea = e_rt(EX_PACK, a), eb = e_rt(EY_PACK, a), ec = e_rt(EZ_PACK, a);
             const int m = a <= 6 ? 2 : 1;
-            // the node lies within R + 1.8 < nx / 2 of the centre: the unwrapped
-            // difference is the periodic minimum image
-            const double ox = (double)(iu + 1) - X0, oy = (double)(j + 1) - X1,
-                         oz = (double)(k + 1) - X2;
-            // q: ray-sphere root from the node (calQ2, particle_bounceback.F90:144-185)
-            const double sx = ea > 0 ? ox : (ea < 0 ? -ox : 0.0);
-            const double sy = eb > 0 ? oy : (eb < 0 ? -oy : 0.0);
-            const double sz = ec > 0 ? oz : (ec < 0 ? -oz : 0.0);
-            const double cc = ox * ox + oy * oy + oz * oz - R * R;
-            double qd = -1.0;
-            bool exact = true;
-            if constexpr (sizeof(L) == 4) {
-                // FP32 form: |x - X|^2 - R^2 (the cancelling part) in FP64, the
-                // root in FP32.  Its error grows where the ray is nearly tangent
-                // (small delta) and matters where q is near 0 or 1, the ends
-                // the range check tests: those links take the FP64 root, so the
-                // FP32 and FP64 forms accept and reject the same links.
-                const float cbf = 2.0f * (float)(sx + sy + sz);
-                const float delta = cbf * cbf - (a <= 6 ? 4.0f : 8.0f) * (float)cc;
-                const float qf = (-cbf - sqrtf(fmaxf(delta, 0.0f))) * (a <= 6 ? 0.5f : 0.25f);
-                exact = !(delta > 1e-2f * cbf * cbf + 1e-3f && qf > 1e-3f && qf < 1.0f - 1e-3f);
-                if (!exact) qd = (double)qf;
+            if constexpr (sizeof(L) == 8) {
+                ox = (double)(iu + 1) - X0;
+                oy = (double)(j + 1) - X1;
+                oz = (double)(k + 1) - X2;
             }
-            if (exact) {
-                const double cb = 2.0 * (sx + sy + sz);
-                const double delta = cb * cb - (a <= 6 ? 4.0 : 8.0) * cc;
-                if (delta < 0) { atomicCAS(d.status, 0, PS_Q_RANGE); d.status[1] = c; continue; }
-                qd = (-cb - sqrt(delta)) * (a <= 6 ? 0.5 : 0.25);  // /(2 |e|^2), exact
-                if (qd > 1.0 || qd < 0.0) { atomicCAS(d.status, 0, PS_Q_RANGE); d.status[1] = c; continue; }
+            // interpolation nodes inside a solid have no post-collision value
+            // of this step: fall back to the linear IBB, then to simple
+            // bounce-back (nodes beyond the walls are ghosts and available).
+            // All values are loaded before any is used.
+            const int ra = opp_rt(a);
+            const bool lo = q < L(0.5);
+            const bool av1 = TILE ? own_at(bi - ea, bj - eb, bk - ec) < 0
+                                  : node_avail(i - ea, j - eb, k - ec, p, d.owner_cur);
+            const L dpa = fp_dev<S, L>(f, a, i, j, k, p);
+            const int s1 = lo ? 1 : 0, qs = lo ? a : ra;
+            L v1 = L(0), v2 = L(0);
+            bool av2 = false;
+            if (lo ? av1 : true) v1 = fp_dev<S, L>(f, qs, i - s1 * ea, j - s1 * eb, k - s1 * ec, p);
+            if (av1) {
+                const int s2 = s1 + 1;
+                v2 = fp_dev<S, L>(f, qs, i - s2 * ea, j - s2 * eb, k - s2 * ec, p);
+                av2 = !lo || node_avail(i - 2 * ea, j - 2 * eb, k - 2 * ec, p, d.owner_cur);
             }
             // constant parts (integers)
             const int n0 = iu + 1, n1 = j + 1, n2 = k + 1;
@@ -540,43 +826,29 @@ __global__ void __launch_bounds__(PB) k_plinks(S* __restrict__ f, PartParams p, 
             nt[1] += m * (n2 * ea - n0 * ec);
             nt[2] += m * (n0 * eb - n1 * ea);
             // wall point relative to the centre and its velocity U + Omega x r
-            const L q = (L)qd;
             const L rx = (L)ox + q * (L)ea, ry = (L)oy + q * (L)eb, rz = (L)oz + q * (L)ec;
             const L uw0 = Ux + (Oy * rz - Oz * ry);
             const L uw1 = Uy + (Oz * rx - Ox * rz);
             const L uw2 = Uz + (Ox * ry - Oy * rx);
-            const int ra = opp_rt(a);
             const L w = a <= 6 ? L(1.0 / 18.0) : L(1.0 / 36.0);
             const L mv = L(6) * w * ravg * (-(L)ea * uw0 - (L)eb * uw1 - (L)ec * uw2);  // moving wall
-            const L dpa = fp_dev<S, L>(f, a, i, j, k, p);
-            // interpolation nodes inside a solid have no post-collision value
-            // of this step: fall back to the linear IBB, then to simple
-            // bounce-back (nodes beyond the walls are ghosts and available)
-            const bool av1 = node_avail(i - ea, j - eb, k - ec, p, d.owner_cur);
             L dn;
-            if (q < L(0.5)) {
-                const bool av2 = node_avail(i - 2 * ea, j - 2 * eb, k - 2 * ec, p, d.owner_cur);
+            if (lo) {
                 if (av1 && av2) {
                     const L c0 = q * (L(1) + L(2) * q), c1 = L(1) - L(4) * q * q,
                             c2 = q * (L(1) - L(2) * q);
-                    const L d1 = fp_dev<S, L>(f, a, i - ea, j - eb, k - ec, p);
-                    const L d2 = fp_dev<S, L>(f, a, i - 2 * ea, j - 2 * eb, k - 2 * ec, p);
-                    dn = c0 * dpa + c1 * d1 - c2 * d2 + mv;
+                    dn = c0 * dpa + c1 * v1 - c2 * v2 + mv;
                 } else if (av1) {  // case1/mpi_complete/particle_bounceback.F90:66-69
-                    const L d1 = fp_dev<S, L>(f, a, i - ea, j - eb, k - ec, p);
-                    dn = L(2) * q * dpa + (L(1) - L(2) * q) * d1 + mv;
+                    dn = L(2) * q * dpa + (L(1) - L(2) * q) * v1 + mv;
                 } else {
                     dn = dpa + mv;
                 }
             } else if (av1) {
                 const L iq = L(1) / q, i2 = L(1) / (L(1) + L(2) * q), a2 = L(2) * q - L(1);
-                const L g0 = fp_dev<S, L>(f, ra, i, j, k, p);
-                const L g1 = fp_dev<S, L>(f, ra, i - ea, j - eb, k - ec, p);
-                dn = (iq * i2) * dpa + (a2 * iq) * g0 - (a2 * i2) * g1 + (iq * i2) * mv;
+                dn = (iq * i2) * dpa + (a2 * iq) * v1 - (a2 * i2) * v2 + (iq * i2) * mv;
             } else {  // case1/mpi_complete/particle_bounceback.F90:70-73
                 const L h = L(0.5) / q;
-                const L g0 = fp_dev<S, L>(f, ra, i, j, k, p);
-                dn = h * dpa + (L(1) - h) * g0 + h * mv;
+                dn = h * dpa + (L(1) - h) * v1 + h * mv;
             }
             const long long fslot = ra * P + (i + (long long)nx * (j + (long long)ny * k));
             if (PSt<S>::SHIFT) {
@@ -600,31 +872,82 @@ __global__ void __launch_bounds__(PB) k_plinks(S* __restrict__ f, PartParams p, 
             av[6] += dn - dpa;
         }
         __syncthreads();
-        if (threadIdx.x == 0) s_n = 0;
+        nl = 0;
     }
-    double acc[13];
-#pragma unroll
-    for (int q = 0; q < 7; q++) acc[q] = (double)av[q];
+    // the warp's sums: exact integers, and the variable parts
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-        acc[7 + q] = (double)nf[q];  // integers: the block sums are exact
-        acc[10 + q] = (double)nt[q];
-    }
-    __shared__ double out[13];
-    block_sum_to<13>(acc, out, 1);
-    if (threadIdx.x == 0) {
-        const double k0 = p.rho0 / 18.0;
-        const double NF0 = out[7], NF1 = out[8], NF2 = out[9];
-        const double fc[3] = {k0 * NF0, k0 * NF1, k0 * NF2};
-        const double tc[3] = {k0 * (out[10] - (X1 * NF2 - X2 * NF1)),
-                              k0 * (out[11] - (X2 * NF0 - X0 * NF2)),
-                              k0 * (out[12] - (X0 * NF1 - X1 * NF0))};
-        const int sl = c * NSLAB + slab;  // per-slab partials, summed in slab order by readers
-        for (int q = 0; q < 3; q++) {
-            d.flink[3 * sl + q] = fc[q] + out[q];
-            d.tlink[3 * sl + q] = tc[q] + out[3 + q];
+        const int a = __reduce_add_sync(0xffffffffu, nf[q]), b = __reduce_add_sync(0xffffffffu, nt[q]);
+        if (lane == 0) {
+            s_int[wid][q] = a;
+            s_int[wid][3 + q] = b;
         }
-        d.corr[sl] = out[6];
+    }
+#pragma unroll
+    for (int q = 0; q < 7; q++) {
+        if constexpr (sizeof(L) == 4) {
+            float hi = av[q], lo = 0.0f;  // TwoSum over the lanes
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
+                lo += __shfl_xor_sync(0xffffffffu, lo, o);
+                two_sum(hi, lo, oh);
+            }
+            if (lane == 0) {
+                s_hi[wid][q] = hi;
+                s_lo[wid][q] = lo;
+            }
+        } else {
+            double v = av[q];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) s_av[wid][q] = v;
+        }
+    }
+    __syncthreads();
+    if (wid == 0) {
+        if constexpr (sizeof(L) == 4) {
+            // 8 lanes per sum add the warps' pairs
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const int q = min(4 * r + (lane >> 3), 6), w = lane & 7;
+                float hi = s_hi[w][q], lo = s_lo[w][q];
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) {
+                    const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
+                    lo += __shfl_xor_sync(0xffffffffu, lo, o);
+                    two_sum(hi, lo, oh);
+                }
+                if (w == 0) s_out[q] = (double)hi + (double)lo;
+            }
+        } else if (lane < 7) {  // the warps' parts in order
+            double v = 0.0;
+#pragma unroll
+            for (int w = 0; w < PB / 32; w++) v += s_av[w][lane];
+            s_out[lane] = v;
+        }
+        if (lane < 6) {
+            int v = 0;
+#pragma unroll
+            for (int w = 0; w < PB / 32; w++) v += s_int[w][lane];
+            s_out[7 + lane] = (double)v;
+        }
+        __syncwarp();
+        const double* out = s_out;
+        if (lane == 0) {
+            const double k0 = p.rho0 / 18.0;
+            const double NF0 = out[7], NF1 = out[8], NF2 = out[9];
+            const double fc[3] = {k0 * NF0, k0 * NF1, k0 * NF2};
+            const double tc[3] = {k0 * (out[10] - (X1 * NF2 - X2 * NF1)),
+                                  k0 * (out[11] - (X2 * NF0 - X0 * NF2)),
+                                  k0 * (out[12] - (X0 * NF1 - X1 * NF0))};
+            const int sl = c * NSLAB + slab;  // per-slab partials, summed in slab order
+            for (int q = 0; q < 3; q++) {
+                d.flink[3 * sl + q] = fc[q] + out[q];
+                d.tlink[3 * sl + q] = tc[q] + out[3 + q];
+            }
+            d.corr[sl] = out[6];
+        }
     }
 }
 
@@ -634,6 +957,16 @@ __global__ void __launch_bounds__(PB) k_plinks(S* __restrict__ f, PartParams p, 
 struct BoxWalk {
     int bi, bj, bk, ai, aj, ak, bw;
     __device__ BoxWalk(long long t0, int bw_) : bw(bw_) {
+        if (bw_ < 1024) {  // 32-bit divisions
+            const int t = (int)t0, b2 = bw_ * bw_;
+            bi = t % bw_;
+            bj = t / bw_ % bw_;
+            bk = t / b2;
+            ai = PB % bw_;
+            aj = PB / bw_ % bw_;
+            ak = PB / b2;
+            return;
+        }
         const long long b2 = (long long)bw_ * bw_;
         bi = (int)(t0 % bw_);
         bj = (int)((t0 / bw_) % bw_);
@@ -653,23 +986,56 @@ struct BoxWalk {
     }
 };
 
-// ----------------------------------------------------------- update --------
-// particle_force.F90:96-190 in 3-D: one warp per particle; the lanes split the
-// pair loop and a fixed shuffle tree adds their spring forces.
-__global__ void k_pforce(PartParams p, PartDev d) {
-    if (d.status[0]) return;
+// ------------------------------------------- force, motion, new mask --------
+// mass, volume and moment of inertia of a sphere
+struct SphereK {
+    double vol, M, I;
+};
+inline SphereK sphere_k(const PartParams& p) {
+    const double R0 = p.radius;
+    SphereK k;
+    k.vol = 4.0 / 3.0 * p.pi * R0 * R0 * R0;
+    k.M = p.rho_solid * 4.0 / 3.0 * p.pi * R0 * R0 * R0;
+    k.I = 0.4 * k.M * R0 * R0;
+    return k;
+}
+
+// The FP64 value *x cut to FP32, on integers (2^-20 relative; tiny values 0,
+// huge ones, infinities and NaN: NaN)
+__device__ __forceinline__ float top32(const double* x) {
+    const int2 w = *reinterpret_cast<const int2*>(x);
+    const int e = (w.y >> 20) & 0x7ff;
+    const unsigned m = ((unsigned)(e - 896) << 23) | ((unsigned)(w.y & 0xfffff) << 3);
+    if (e >= 896 + 255) return __int_as_float(0x7fc00000);
+    return e <= 896 ? 0.0f : __int_as_float((int)(m | ((unsigned)w.y & 0x80000000u)));
+}
+
+// Force, torque (particle_force.F90:96-190 in 3-D) and motion
+// (particle_update.F90:26-50) of particle c by one block; the new centre is left
+// in Xn and d.*_new, the state moves on once every particle has done so.  false:
+// the particle has left the range a step may take.
+__device__ bool pmotion(const PartParams& p, const SphereK& sk, const PartDev& d, int c, double* Xn) {
+    __shared__ double fij[3];
+    __shared__ int s_ok;
     const int np = p.np;
-    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (c >= np) return;
-    const double R0 = p.radius, ravg = d.rho_avg[0];
-    const double vol = 4.0 / 3.0 * p.pi * R0 * R0 * R0;
+    const double R0 = p.radius, Rc = p.radius;
     const double* X = d.xc + 3 * c;
-    double fij[3] = {0.0, 0.0, 0.0};
-    const double Rc = R0;
-    for (int c2 = lane; c2 < np; c2 += 32) {
+    double fp[3] = {0.0, 0.0, 0.0};
+    bool hit = false;
+    // FP64 only for the pairs whose top 20 bits do not rule them out: y and z are
+    // below 2^16 (a difference off by 2^-3), x below 2 nx
+    const float xt[3] = {top32(X), top32(X + 1), top32(X + 2)}, Lf = (float)p.nx;
+    const float far = (float)(Rc + R0 + p.thr_part) * 1.001f + 0.3f + 4e-6f * Lf;
+    for (int c2 = threadIdx.x; c2 < np; c2 += PB) {
         if (c2 == c) continue;
         const double* X2 = d.xc + 3 * c2;
+        float g0 = top32(X2) - xt[0];
+        if (p.periodic_x) {
+            if (g0 > 0.5f * Lf) g0 -= Lf;
+            else if (g0 < -0.5f * Lf) g0 += Lf;
+        }
+        if (fabsf(g0) > far || fabsf(top32(X2 + 1) - xt[1]) > far || fabsf(top32(X2 + 2) - xt[2]) > far)
+            continue;  // certainly out of range (not taken for a NaN)
         const double d0 = dxp(X[0], X2[0], p), d1 = X[1] - X2[1], d2 = X[2] - X2[2];
         const double thr = p.thr_part;
         const double reach = Rc + R0 + thr;
@@ -678,96 +1044,98 @@ __global__ void k_pforce(PartParams p, PartDev d) {
         if (dij >= Rc + R0 + thr) {
         } else if (dij >= Rc + R0) {
             const double t = (dij - Rc - R0 - thr) / thr;
-            fij[0] = fij[0] + p.scale_part * (t * t) * d0 / dij;
-            fij[1] = fij[1] + p.scale_part * (t * t) * d1 / dij;
-            fij[2] = fij[2] + p.scale_part * (t * t) * d2 / dij;
+            fp[0] = fp[0] + p.scale_part * (t * t) * d0 / dij;
+            fp[1] = fp[1] + p.scale_part * (t * t) * d1 / dij;
+            fp[2] = fp[2] + p.scale_part * (t * t) * d2 / dij;
+            hit = true;
         } else {
-            if (atomicCAS(d.status, 0, PS_OVERLAP) == 0) {
-                d.status[1] = c;
-                d.status[2] = c2;
-            }
+            pfail(d, PS_OVERLAP, c, c2, d.par);
         }
     }
-#pragma unroll
-    for (int q = 0; q < 3; q++)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) fij[q] += __shfl_down_sync(0xffffffffu, fij[q], o);
-    if (lane != 0) return;
-    double fw[3] = {0.0, 0.0, 0.0};
-    const double thw = p.thr_wall;
-    for (int ax = 0; ax < 3; ax++) {
-        if (ax == 0 && p.periodic_x) continue;
-        const int nax = ax == 0 ? p.nx : (ax == 1 ? p.ny : p.nz);
-        double dw = X[ax] - Rc - 1.0;
-        if (dw < 0) {
-            if (atomicCAS(d.status, 0, PS_WALL) == 0) d.status[1] = c;
-        } else if (dw < thw) {
-            fw[ax] = fw[ax] + p.scale_wall * ((dw - thw) / thw) * ((dw - thw) / thw);
+    if (__syncthreads_or(hit)) block_sum_to<3>(fp, fij, 1);
+    else if (threadIdx.x == 0) fij[0] = fij[1] = fij[2] = 0.0;
+    __syncthreads();
+    if (threadIdx.x < 32) {  // lane q: component q
+        const int q = min((int)threadIdx.x, 2);
+        const double ravg = d.rho_avg[0], thw = p.thr_wall;
+        double fw = 0.0;
+        if (q > 0 || !p.periodic_x) {
+            const int nax = q == 0 ? p.nx : (q == 1 ? p.ny : p.nz);
+            double dw = X[q] - Rc - 1.0;
+            if (dw < 0) pfail(d, PS_WALL, c, 0, d.par);
+            else if (dw < thw) fw = fw + p.scale_wall * ((dw - thw) / thw) * ((dw - thw) / thw);
+            dw = (double)nax - X[q] - Rc;
+            if (dw < 0) pfail(d, PS_WALL, c, 0, d.par);
+            else if (dw < thw) fw = fw - p.scale_wall * ((dw - thw) / thw) * ((dw - thw) / thw);
         }
-        dw = (double)nax - X[ax] - Rc;
-        if (dw < 0) {
-            if (atomicCAS(d.status, 0, PS_WALL) == 0) d.status[1] = c;
-        } else if (dw < thw) {
-            fw[ax] = fw[ax] - p.scale_wall * ((dw - thw) / thw) * ((dw - thw) / thw);
-        }
-    }
-    for (int q = 0; q < 3; q++) {
         double fl = 0.0, tl = 0.0;
+#pragma unroll
         for (int sl = 0; sl < NSLAB; sl++) {
             fl += d.flink[3 * (c * NSLAB + sl) + q];
             tl += d.tlink[3 * (c * NSLAB + sl) + q];
         }
-        double tot = fl + (p.rho_solid - ravg) * vol * p.gravity[q] + fij[q] + fw[q];
-        tot = tot + ravg * vol * p.body_force[q];
-        d.ftot[3 * c + q] = tot;
-        d.ttot[3 * c + q] = tl;
+        double tot = fl + (p.rho_solid - ravg) * sk.vol * (q == 0 ? p.gravity[0] : q == 1 ? p.gravity[1] : p.gravity[2]) + fij[q] + fw;
+        tot = tot + ravg * sk.vol * (q == 0 ? p.body_force[0] : q == 1 ? p.body_force[1] : p.body_force[2]);
+        const double a = tot / sk.M;
+        const double u = d.uc[3 * c + q] + a, om = d.om[3 * c + q] + tl / sk.I;
+        double x = X[q] + d.uc[3 * c + q] + 0.5 * a;
+        bool ok = isfinite(x) && isfinite(u) && isfinite(om);
+        if (q == 0 && p.periodic_x) {
+            // one wrap per step is enough only while the step moves the centre by
+            // less than half the periodic length
+            const double L = (double)p.nx;
+            ok = ok && fabs(x - X[0]) < 0.5 * L;
+            if (x >= L + 0.5) x -= L;
+            if (x < 0.5) x += L;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (threadIdx.x < 3) {
+            d.ftot[3 * c + q] = tot;
+            d.ttot[3 * c + q] = tl;
+            d.xc_new[3 * c + q] = x;
+            d.uc_new[3 * c + q] = u;
+            d.om_new[3 * c + q] = om;
+            Xn[q] = x;
+        }
+        if (threadIdx.x == 0) s_ok = ok;
     }
+    __syncthreads();
+    return s_ok;
 }
 
-// particle_update.F90:26-50 in 3-D, one thread per particle
-__global__ void k_pmove(PartParams p, PartDev d) {
-    if (d.status[0]) return;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= p.np) return;
-    const double R0 = p.radius;
-    const double M = p.rho_solid * 4.0 / 3.0 * p.pi * R0 * R0 * R0;
-    const double I = 0.4 * M * R0 * R0;
-    bool ok = true;
-    for (int q = 0; q < 3; q++) {
-        d.xc_old[3 * c + q] = d.xc[3 * c + q];
-        d.uc_old[3 * c + q] = d.uc[3 * c + q];
-        d.om_old[3 * c + q] = d.om[3 * c + q];
-        const double a = d.ftot[3 * c + q] / M;
-        d.uc[3 * c + q] = d.uc_old[3 * c + q] + a;
-        d.om[3 * c + q] = d.om_old[3 * c + q] + d.ttot[3 * c + q] / I;
-        d.xc[3 * c + q] = d.xc_old[3 * c + q] + d.uc_old[3 * c + q] + 0.5 * a;
-        ok = ok && isfinite(d.xc[3 * c + q]) && isfinite(d.uc[3 * c + q]) &&
-             isfinite(d.om[3 * c + q]);
-    }
-    if (p.periodic_x) {
-        // one wrap per step is enough only while the step moves the centre by
-        // less than half the periodic length
-        const double L = (double)p.nx;
-        ok = ok && fabs(d.xc[3 * c] - d.xc_old[3 * c]) < 0.5 * L;
-        if (d.xc[3 * c] >= L + 0.5) d.xc[3 * c] -= L;
-        if (d.xc[3 * c] < 0.5) d.xc[3 * c] += L;
-    }
-    if (!ok && atomicCAS(d.status, 0, PS_DIVERGED) == 0) d.status[1] = c;
-}
-
-// -------------------------------------------------------------- new mask --
-__global__ void __launch_bounds__(PB) k_pmark(int* owner, const double* xc, PartParams p,
-                                                const int* status, bool check_status) {
-    if (check_status && status[0]) return;
+// MOVE: the particle's force and motion first (as a launch of its own, a warp per
+// particle and one block that moved them all, 46 us for 200 spheres; in
+// k_plinks's last block, longer still, waiting in the fence for that SM's
+// scattered stores).
+template <bool MOVE>
+__global__ void __launch_bounds__(PB) k_pmark(int* owner, PartParams p, SphereK sk, PartDev d) {
+    if (MOVE && d.status[0]) return;
     const int c = blockIdx.x;
-    const double* X = xc + 3 * c;
+    __shared__ double X[3];
+    if constexpr (MOVE) {
+        if (!pmotion(p, sk, d, c, X)) {
+            if (threadIdx.x == 0) atomicCAS(d.done + 1, 0u, (unsigned)c + 1u);
+            return;
+        }
+    } else {
+        if (threadIdx.x < 3) X[threadIdx.x] = d.xc[3 * c + threadIdx.x];
+        __syncthreads();
+    }
+    __shared__ int s_c[3];
+    __shared__ float s_f[3];
+    if (threadIdx.x < 3) {
+        s_c[threadIdx.x] = (int)floor(X[threadIdx.x]) - 1;
+        s_f[threadIdx.x] = (float)X[threadIdx.x];
+    }
+    __syncthreads();
     const double R = p.radius;
     const int h = (int)ceil(R) + 1;
-    const int ci = (int)floor(X[0]) - 1, cj = (int)floor(X[1]) - 1, ck = (int)floor(X[2]) - 1;
+    const int ci = s_c[0], cj = s_c[1], ck = s_c[2];
     const int bw = 2 * h + 2;
     const long long nbox = (long long)bw * bw * bw;
-    const float Xf0 = (float)X[0], Xf1 = (float)X[1], Xf2 = (float)X[2], Lf = (float)p.nx;
+    const float Xf0 = s_f[0], Xf1 = s_f[1], Xf2 = s_f[2], Lf = (float)p.nx;
     const float Xmax = fmaxf(fabsf(Xf0), fmaxf(fabsf(Xf1), fabsf(Xf2))) + Lf;  // wrapped nodes too
+    const float r2 = (float)(R * R);
     BoxWalk bw_it(threadIdx.x, bw);
     for (long long t = threadIdx.x; t < nbox; t += PB, bw_it.next()) {
         const int bi = bw_it.bi, bj = bw_it.bj, bk = bw_it.bk;
@@ -786,7 +1154,7 @@ __global__ void __launch_bounds__(PB) k_pmark(int* owner, const double* xc, Part
             else if (fx < -0.5f * Lf) fx += Lf;
         }
         const float fy = (float)(j + 1) - Xf1, fz = (float)(k + 1) - Xf2;
-        const float d2 = fx * fx + fy * fy + fz * fz, r2 = (float)(R * R);
+        const float d2 = fx * fx + fy * fy + fz * fz;
         const float tol = 1e-3f * r2 + 4e-6f * (float)(h + 1) * (Xmax + (float)(h + 1)) + 1e-6f * d2;
         bool in;
         if (fabsf(d2 - r2) > tol) in = d2 < r2;
@@ -795,48 +1163,105 @@ __global__ void __launch_bounds__(PB) k_pmark(int* owner, const double* xc, Part
     }
 }
 
-// nodes that change phase: density bookkeeping of the average used by the refill
+// Nodes that change phase: the density bookkeeping of the average used by the
+// refill, and each particle's list of nodes to refill.  PREP_SLAB blocks per
+// particle walk a z slab of its old box and, where that differs, of its new one;
+// the last block to finish forms the average: (mass after bounce-back + link
+// corrections + phase changes) / (fluid count + its change).  (As three
+// launches, the boxes walked three times by one block each: 17 + 8 + 15 us.)
+constexpr int PREP_SLAB = PART_NSLAB;
+#ifndef MGLC_PU
+#define MGLC_PU 2
+#endif
+constexpr int PU = MGLC_PU;
 template <typename S>
-__global__ void __launch_bounds__(PB) k_pprep(const S* __restrict__ f, PartParams p, PartDev d) {
+__global__ void __launch_bounds__(PB) k_pphase(const S* __restrict__ f, PartParams p, PartDev d) {
     if (d.status[0]) return;
-    const int c = blockIdx.x;
+    const int c = blockIdx.x, slab = blockIdx.y;
+    if (d.done[1]) {  // a particle went out of range: the state moves and freezes
+        if (c == 0 && slab == 0 && threadIdx.x == 0) pfail(d, PS_DIVERGED, (int)d.done[1] - 1, 0, d.par);
+        return;
+    }
     const long long P = (long long)p.nx * p.ny * p.nz;
     double sum = 0.0;
     int cnt = 0;
-    for (int pass = 0; pass < 2; pass++) {
-        const double* X = (pass == 0 ? d.xc_old : d.xc) + 3 * c;
-        const int h = (int)ceil(p.radius) + 1;
-        const int ci = (int)floor(X[0]) - 1, cj = (int)floor(X[1]) - 1, ck = (int)floor(X[2]) - 1;
+    __shared__ int s_c[6];  // corner node of the old and the new box, less h
+    if (threadIdx.x < 6)
+        s_c[threadIdx.x] = (int)floor(threadIdx.x < 3 ? d.xc[3 * c + threadIdx.x] : d.xc_new[3 * c + threadIdx.x - 3]) - 1;
+    __syncthreads();
+    // the second box only where it is another one; the first pass then looks for
+    // entering nodes too
+    const bool same = s_c[0] == s_c[3] && s_c[1] == s_c[4] && s_c[2] == s_c[5];
+    const int h = (int)ceil(p.radius) + 1;
+    for (int pass = 0; pass < (same ? 1 : 2); pass++) {
+        const int ci = s_c[3 * pass], cj = s_c[3 * pass + 1], ck = s_c[3 * pass + 2];
         const int bw = 2 * h + 2;
-        const long long nbox = (long long)bw * bw * bw;
-        BoxWalk bw_it(threadIdx.x, bw);
-        for (long long t = threadIdx.x; t < nbox; t += PB, bw_it.next()) {
-            const int bi = bw_it.bi, bj = bw_it.bj, bk = bw_it.bk;
-            int i = ci - h + bi;
-            const int j = cj - h + bj, k = ck - h + bk;
-            if (j < 0 || j >= p.ny || k < 0 || k >= p.nz) continue;
-            if (p.periodic_x) i = wrapx(i, p.nx);
-            else if (i < 0 || i >= p.nx) continue;
-            const long long cell = i + (long long)p.nx * (j + (long long)p.ny * k);
-            const int oc = d.owner_cur[cell], on = d.owner_new[cell];
-            if (pass == 0 && oc == c && on < 0) {  // leaves particle c: counted with rho_solid
-                sum += p.rho_solid;
-                cnt += 1;
+        const int k0 = slab * bw / PREP_SLAB, k1 = (slab + 1) * bw / PREP_SLAB;
+        const long long t1 = (long long)bw * bw * k1;
+        BoxWalk bw_it((long long)bw * bw * k0 + threadIdx.x, bw);
+        for (long long t = (long long)bw * bw * k0 + threadIdx.x; t < t1; t += PU * PB) {
+            // PU nodes' masks in flight
+            long long cell[PU];
+            int oc[PU], on[PU];
+#pragma unroll
+            for (int u = 0; u < PU; u++, bw_it.next()) {
+                int i = ci - h + bw_it.bi;
+                const int j = cj - h + bw_it.bj, k = ck - h + bw_it.bk;
+                bool in = t + u * PB < t1 && j >= 0 && j < p.ny && k >= 0 && k < p.nz;
+                if (p.periodic_x) i = wrapx(i, p.nx);
+                else in = in && i >= 0 && i < p.nx;
+                cell[u] = i + (long long)p.nx * (j + (long long)p.ny * k);
+                oc[u] = in ? d.owner_cur[cell[u]] : c;  // outside: no change of phase
+                on[u] = in ? d.owner_new[cell[u]] : c;
             }
-            if (pass == 1 && oc < 0 && on == c) {  // enters particle c: drop its density
-                double r = 0.0;
-                for (int q = 0; q < Q19; q++) r += pabs<S>(f, q * P + cell, q, p.rho0);
-                sum -= r;
-                cnt -= 1;
+#pragma unroll
+            for (int u = 0; u < PU; u++) {
+                if (pass == 0 && oc[u] == c && on[u] < 0) {  // leaves particle c: counted with rho_solid
+                    sum += p.rho_solid;
+                    cnt += 1;
+                    const int slot = atomicAdd(d.rf_count + c, 1);
+                    if (slot < PART_REFILL) d.rf_list[(size_t)c * PART_REFILL + slot] = cell[u];
+                }
+                if ((pass == 1 || same) && oc[u] < 0 && on[u] == c) {  // enters particle c: drop its density
+                    double r = 0.0;
+                    for (int q = 0; q < Q19; q++) r += pabs<S>(f, q * P + cell[u], q, p.rho0);
+                    sum -= r;
+                    cnt -= 1;
+                }
             }
         }
     }
-    double acc[2] = {sum, (double)cnt};
+    // most blocks have nothing to add
     __shared__ double out[2];
-    block_sum_to<2>(acc, out, 1);
+    __shared__ int last;
+    if (__syncthreads_or(cnt != 0 || sum != 0.0)) {
+        double acc[2] = {sum, (double)cnt};
+        block_sum_to<2>(acc, out, 1);
+    } else if (threadIdx.x == 0) {
+        out[0] = out[1] = 0.0;
+    }
     if (threadIdx.x == 0) {
-        d.prep_sum[c] = out[0];
-        d.prep_cnt[c] = (int)llround(out[1]);
+        d.prep_sum[c * PREP_SLAB + slab] = out[0];
+        d.prep_cnt[c * PREP_SLAB + slab] = (int)llround(out[1]);
+        __threadfence();
+        last = atomicAdd(d.done + 2, 1u) == gridDim.x * gridDim.y - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double acc[2] = {0.0, 0.0};
+    for (int q = threadIdx.x; q < p.np * PREP_SLAB; q += PB) {
+        acc[0] += __ldcg(d.corr + q) + __ldcg(d.prep_sum + q);
+        acc[1] += (double)__ldcg(d.prep_cnt + q);
+    }
+    block_sum_to<2>(acc, out, 1);
+    for (int q = threadIdx.x; q < p.np; q += PB)
+        if (__ldcg(d.rf_count + q) > PART_REFILL) pfail(d, PS_REFILL_FULL, q, 0, d.par ^ 1);
+    if (threadIdx.x == 0) {
+        const long long n1 = d.n_fluid[0] + llround(out[1]);
+        d.rho_avg[1] = (d.rho_avg[2] + out[0]) / (double)n1;
+        d.n_fluid[0] = n1;
+        d.done[2] = 0;
     }
 }
 
@@ -904,38 +1329,30 @@ __device__ void inverse19d(const double* m, double* f) {
 // rho_avg times the wall velocity.  All of a particle's refills read before
 // any of them is written.
 template <typename S>
-__global__ void __launch_bounds__(PB) k_prefill(S* __restrict__ f, PartParams p, PartDev d,
-                                                int nblocks_bulk) {
-    if (d.status[0]) return;
+__global__ void __launch_bounds__(PB) k_prefill(S* __restrict__ f, PartParams p, PartDev d) {
     const int c = blockIdx.x;
-    const long long P = (long long)p.nx * p.ny * p.nz;
-    __shared__ double s_val[REFILL_MAX][Q19];
-    __shared__ long long s_cell[REFILL_MAX];
-    __shared__ int s_n;
-    __shared__ double s_ravg;
-    if (threadIdx.x == 0) {
-        s_n = 0;
-        s_ravg = d.rho_avg[1];
+    // the particle moves on, with an error too if that came after the motion
+    // (status from an earlier step: the values are those of now)
+    const int code = d.status[0];
+    if (threadIdx.x < 3 && (!code || code == PS_REFILL_FULL || code == PS_NO_REFILL_DIR || code == PS_DIVERGED)) {
+        const int q = 3 * c + threadIdx.x;
+        d.xc[q] = d.xc_new[q];
+        d.uc[q] = d.uc_new[q];
+        d.om[q] = d.om_new[q];
     }
-    __syncthreads();
-    const double* X = d.xc + 3 * c;       // new centre
-    const double* Xo = d.xc_old + 3 * c;  // old centre: the nodes it covered
-    const double* U = d.uc + 3 * c;
-    const double* O = d.om + 3 * c;
-    const int h = (int)ceil(p.radius) + 1;
-    const int ci = (int)floor(Xo[0]) - 1, cj = (int)floor(Xo[1]) - 1, ck = (int)floor(Xo[2]) - 1;
-    const int bw = 2 * h + 2;
-    const long long nbox = (long long)bw * bw * bw;
-    BoxWalk bw_it(threadIdx.x, bw);
-    for (long long t = threadIdx.x; t < nbox; t += PB, bw_it.next()) {
-        const int bi = bw_it.bi, bj = bw_it.bj, bk = bw_it.bk;
-        int i = ci - h + bi;
-        const int j = cj - h + bj, k = ck - h + bk;
-        if (j < 0 || j >= p.ny || k < 0 || k >= p.nz) continue;
-        if (p.periodic_x) i = wrapx(i, p.nx);
-        else if (i < 0 || i >= p.nx) continue;
-        const long long cell = i + (long long)p.nx * (j + (long long)p.ny * k);
-        if (!(d.owner_cur[cell] == c && d.owner_new[cell] < 0)) continue;
+    if (__syncthreads_or(code)) return;
+    const int n = d.rf_count[c];  // at most PART_REFILL: k_pphase has failed where more
+    if (n == 0) return;
+    const long long P = (long long)p.nx * p.ny * p.nz;
+    __shared__ double s_val[PART_REFILL][Q19];
+    const double s_ravg = d.rho_avg[1];
+    const double* X = d.xc_new + 3 * c;
+    const double* U = d.uc_new + 3 * c;
+    const double* O = d.om_new + 3 * c;
+    for (int slot = threadIdx.x; slot < n; slot += PB) {
+        const long long cell = d.rf_list[(size_t)c * PART_REFILL + slot];
+        const int i = (int)(cell % p.nx), j = (int)(cell / p.nx % p.ny),
+                  k = (int)(cell / ((long long)p.nx * p.ny));
         const double rx = dxp((double)(i + 1), X[0], p), ry = (double)(j + 1) - X[1],
                      rz = (double)(k + 1) - X[2];
         double out = 0.0;
@@ -950,7 +1367,7 @@ __global__ void __launch_bounds__(PB) k_prefill(S* __restrict__ f, PartParams p,
             }
         }
         if (ec == 0) {
-            atomicCAS(d.status, 0, PS_NO_REFILL_DIR);
+            pfail(d, PS_NO_REFILL_DIR, c, 0, d.par ^ 1);
             continue;
         }
         const int e0 = ex19(ec), e1 = ey19(ec), e2 = ez19(ec);
@@ -975,25 +1392,16 @@ __global__ void __launch_bounds__(PB) k_prefill(S* __restrict__ f, PartParams p,
         m[5] = s_ravg * (U[1] + (O[2] * qx - O[0] * qz));
         m[7] = s_ravg * (U[2] + (O[0] * qy - O[1] * qx));
         inverse19d(m, fl);
-        const int slot = atomicAdd(&s_n, 1);
-        if (slot >= REFILL_MAX) {
-            atomicCAS(d.status, 0, PS_REFILL_FULL);
-            continue;
-        }
-        s_cell[slot] = cell;
         for (int a = 0; a < Q19; a++) s_val[slot][a] = fl[a];
     }
+    // a node without a direction has set the status: nothing is written
     __syncthreads();
-    const int n = min(s_n, REFILL_MAX);
+    if (threadIdx.x == 0) d.rf_count[c] = 0;
+    if (__ldcg(d.status)) return;
     for (int t = threadIdx.x; t < n * Q19; t += PB) {
         const int slot = t / Q19, a = t % Q19;
-        pset<S>(f, a * P + s_cell[slot], a, s_val[slot][a], p.rho0);
+        pset<S>(f, a * P + d.rf_list[(size_t)c * PART_REFILL + slot], a, s_val[slot][a], p.rho0);
     }
-}
-
-__global__ void k_pcommit(PartDev d) {
-    if (d.status[0]) return;
-    d.n_fluid[0] = d.n_fluid[1];
 }
 
 // ------------------------------------------------------------ initialise --
@@ -1064,19 +1472,17 @@ static cudaError_t pstep_go(bool first, const void* fin, void* fout, const PartP
                             const PartDev& d, cudaStream_t s) {
     using C = typename PC<S>::C;
     dim3 b = pblock(p.nx), g((p.nx + b.x - 1) / b.x, p.ny, p.nz);
-    MrtCoef<C> cd = cast_coef<C>(make_mrt_coef(p.snu, p.sq));
-    const PBulkK<C> bk = {(C)p.rho0, (C)p.body_force[0], (C)p.body_force[1], (C)p.body_force[2]};
+    const PBulkK<C> bk = bulk_k(p, C());
     // 32-bit indices while every population index (and the +-1 neighbour
     // offsets) fits in int
     const bool i32 = (long long)p.nx * p.ny * p.nz * (Q19 + 1) < (1LL << 31);
     const S* fi = (const S*)fin;
     S* fo = (S*)fout;
-    if (first && i32) k_pbulk<S, true, int><<<g, b, 0, s>>>(fi, fo, d.owner_cur, p, cd, bk, d.partials, d.status);
-    else if (first) k_pbulk<S, true, long long><<<g, b, 0, s>>>(fi, fo, d.owner_cur, p, cd, bk, d.partials, d.status);
-    else if (i32) k_pbulk<S, false, int><<<g, b, 0, s>>>(fi, fo, d.owner_cur, p, cd, bk, d.partials, d.status);
-    else k_pbulk<S, false, long long><<<g, b, 0, s>>>(fi, fo, d.owner_cur, p, cd, bk, d.partials, d.status);
-    k_pfinish<<<FINISH_BLOCKS, 256, 0, s>>>(d, d.nblocks);
-    k_pfinish2<<<1, 32, 0, s>>>(d, d.nblocks);
+    if (first && i32) k_pbulk<S, true, int><<<g, b, 0, s>>>(fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
+    else if (first) k_pbulk<S, true, long long><<<g, b, 0, s>>>(fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
+    else if (i32) k_pbulk<S, false, int><<<g, b, 0, s>>>(fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
+    else k_pbulk<S, false, long long><<<g, b, 0, s>>>(fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
+    k_pfinish<S><<<FINISH_BLOCKS<S>, 256, 0, s>>>(d, d.nblocks, p.rho0);
     if (p.np > 0) {
         const int bw = 2 * ((int)ceil(p.radius) + 2) + 2;
         const size_t tile = sizeof(int) * (size_t)(bw + 2) * (bw + 2) * ((bw + NSLAB - 1) / NSLAB + 2);
@@ -1097,18 +1503,9 @@ static cudaError_t pstep_go(bool first, const void* fin, void* fout, const PartP
         } else {
             k_plinks<S, false><<<dim3(p.np, NSLAB), PB, 0, s>>>((S*)fout, p, d);
         }
-        // one warp per particle, one warp per block: the particles spread over the SMs
-        k_pforce<<<p.np, 32, 0, s>>>(p, d);
-        k_pmove<<<(p.np + 31) / 32, 32, 0, s>>>(p, d);
-    }
-    cudaError_t e = cudaMemsetAsync(d.owner_new, 0xFF, sizeof(int) * (size_t)p.nx * p.ny * p.nz, s);
-    if (e != cudaSuccess) return e;
-    if (p.np > 0) {
-        k_pmark<<<p.np, PB, 0, s>>>(d.owner_new, d.xc, p, d.status, true);
-        k_pprep<S><<<p.np, PB, 0, s>>>((const S*)fout, p, d);
-        k_prefill_avg<<<1, 32, 0, s>>>(p, d);
-        k_prefill<S><<<p.np, PB, 0, s>>>((S*)fout, p, d, d.nblocks);
-        k_pcommit<<<1, 1, 0, s>>>(d);
+        k_pmark<true><<<p.np, PB, 0, s>>>(d.owner_new, p, sphere_k(p), d);
+        k_pphase<S><<<dim3(p.np, PREP_SLAB), PB, 0, s>>>((const S*)fout, p, d);
+        k_prefill<S><<<p.np, PB, 0, s>>>((S*)fout, p, d);
     }
     return cudaGetLastError();
 }
@@ -1125,7 +1522,7 @@ cudaError_t launch_particle_init(int form, void* f, const PartParams& p, const P
     const long long n = (long long)p.nx * p.ny * p.nz;
     cudaError_t e = cudaMemsetAsync(d.owner_cur, 0xFF, sizeof(int) * (size_t)n, s);
     if (e != cudaSuccess) return e;
-    if (p.np > 0) k_pmark<<<p.np, PB, 0, s>>>(d.owner_cur, d.xc, p, d.status, false);
+    if (p.np > 0) k_pmark<false><<<p.np, PB, 0, s>>>(d.owner_cur, p, sphere_k(p), d);
     int gb = (int)std::min<long long>((n + 255) / 256, 152 * 16);
     if (form == FORM_FP64) k_pinit_f<double><<<gb, 256, 0, s>>>((double*)f, d.owner_cur, p);
     else k_pinit_f<float><<<gb, 256, 0, s>>>((float*)f, d.owner_cur, p);

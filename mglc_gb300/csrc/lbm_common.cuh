@@ -110,10 +110,14 @@ __device__ __forceinline__ void moments0(const T* f, T& rho_m, T& jx, T& jy, T& 
 //  LID_MEQ12: lid operator quirk, meq(12) without the factor rho (collision.f90:85)
 //  msc  : scale of f, rho_m, rho and the forces (the lid quirk's meq(12), which
 //         carries no rho, is multiplied by it); 1 for unscaled arithmetic
-template <typename T, bool FORCED, bool LID_MEQ12>
-__device__ __forceinline__ void mrt_collide(T* f, T rho_m, T rho, T ux, T uy, T uz, T fx, T fy,
-                                            T fz, const MrtCoef<T>& c, T msc = T(1)) {
-    const T two = T(2), four = T(4), half = T(0.5);
+// The moments m = M f that the collision relaxes (mrt_relax).
+template <typename T>
+struct MrtMom {
+    T m1, m2, m4, m6, m8, m9, m10, m11, m12, m13, m14, m15, m16, m17, m18;
+};
+template <typename T>
+__device__ __forceinline__ MrtMom<T> mrt_moments(const T* f) {
+    const T two = T(2), four = T(4);
     // opposite pairs: (a,b) = (1,2) (3,4) (5,6) (7,10) (9,8) (11,14) (13,12) (15,18) (17,16)
     T s1 = f[1] + f[2], d1 = f[1] - f[2];
     T s2 = f[3] + f[4], d2 = f[3] - f[4];
@@ -126,25 +130,36 @@ __device__ __forceinline__ void mrt_collide(T* f, T rho_m, T rho, T ux, T uy, T 
     T s9 = f[17] + f[16], d9 = f[17] - f[16];
     T sa = s1 + s2 + s3;                    // axis sum
     T se = (s4 + s5) + (s6 + s7) + (s8 + s9); // edge sum
-    T m1 = T(-30) * f[0] + (T(-11) * sa + T(8) * se);
-    T m2 = T(12) * f[0] + (T(-4) * sa + se);
+    MrtMom<T> o;
+    o.m1 = T(-30) * f[0] + (T(-11) * sa + T(8) * se);
+    o.m2 = T(12) * f[0] + (T(-4) * sa + se);
     T ex_ = (d4 + d5) + (d6 + d7);
     T ey_ = (d4 - d5) + (d8 + d9);
     T ez_ = (d6 - d7) + (d8 - d9);
-    T m4 = T(-4) * d1 + ex_;
-    T m6 = T(-4) * d2 + ey_;
-    T m8 = T(-4) * d3 + ez_;
+    o.m4 = T(-4) * d1 + ex_;
+    o.m6 = T(-4) * d2 + ey_;
+    o.m8 = T(-4) * d3 + ez_;
     T sxy = s4 + s5, sxz = s6 + s7, syz = s8 + s9;
-    T m9 = two * s1 - (s2 + s3) + (sxy + sxz) - two * syz;
-    T m10 = -four * s1 + two * (s2 + s3) + (sxy + sxz) - two * syz;
-    T m11 = (s2 - s3) + (sxy - sxz);
-    T m12 = -two * (s2 - s3) + (sxy - sxz);
-    T m13 = s4 - s5;
-    T m14 = s8 - s9;
-    T m15 = s6 - s7;
-    T m16 = (d4 + d5) - (d6 + d7);
-    T m17 = (d5 - d4) + (d8 + d9);
-    T m18 = (d6 - d7) - (d8 - d9);
+    o.m9 = two * s1 - (s2 + s3) + (sxy + sxz) - two * syz;
+    o.m10 = -four * s1 + two * (s2 + s3) + (sxy + sxz) - two * syz;
+    o.m11 = (s2 - s3) + (sxy - sxz);
+    o.m12 = -two * (s2 - s3) + (sxy - sxz);
+    o.m13 = s4 - s5;
+    o.m14 = s8 - s9;
+    o.m15 = s6 - s7;
+    o.m16 = (d4 + d5) - (d6 + d7);
+    o.m17 = (d5 - d4) + (d8 + d9);
+    o.m18 = (d6 - d7) - (d8 - d9);
+    return o;
+}
+template <typename T, bool FORCED, bool LID_MEQ12>
+__device__ __forceinline__ void mrt_relax(T* f, const MrtMom<T>& o, T rho_m, T rho, T ux, T uy,
+                                          T uz, T fx, T fy, T fz, const MrtCoef<T>& c,
+                                          T msc = T(1)) {
+    const T two = T(2), four = T(4), half = T(0.5);
+    const T m1 = o.m1, m2 = o.m2, m4 = o.m4, m6 = o.m6, m8 = o.m8, m9 = o.m9, m10 = o.m10,
+            m11 = o.m11, m12 = o.m12, m13 = o.m13, m14 = o.m14, m15 = o.m15, m16 = o.m16,
+            m17 = o.m17, m18 = o.m18;
 
     // equilibrium parts
     T ux2 = ux * ux, uy2 = uy * uy, uz2 = uz * uz;
@@ -227,6 +242,12 @@ __device__ __forceinline__ void mrt_collide(T* f, T rho_m, T rho, T ux, T uy, T 
     // P9 (17,16)
     E = bz - r14; O = Y - Z + (r17 + r18);
     f[17] -= E + O; f[16] -= E - O;
+}
+
+template <typename T, bool FORCED, bool LID_MEQ12>
+__device__ __forceinline__ void mrt_collide(T* f, T rho_m, T rho, T ux, T uy, T uz, T fx, T fy,
+                                            T fz, const MrtCoef<T>& c, T msc = T(1)) {
+    mrt_relax<T, FORCED, LID_MEQ12>(f, mrt_moments(f), rho_m, rho, ux, uy, uz, fx, fy, fz, c, msc);
 }
 
 // The lid-driven cavity's MRT collision (collision.f90:15-202) in its pair

@@ -10,6 +10,10 @@ namespace mglc {
 // CTAs per particle in the boundary-link kernel (z slabs of the node box);
 // the link sums are kept per (particle, slab) and added in slab order
 constexpr int PART_NSLAB = 4;
+// sums that the finish kernel keeps behind the bulk partials
+constexpr int PART_FINISH = 2 * 128;
+// nodes that may leave one particle in one step
+constexpr int PART_REFILL = 256;
 
 // Status codes written by the particle kernels (mirrors orc_pt_step's codes).
 enum PartStatus {
@@ -36,16 +40,21 @@ struct PartDev {
     int* owner_cur;   // -1 fluid, p >= 0 solid node of particle p (interior cells)
     int* owner_new;
     double *xc, *uc, *om;              // np*3, current
-    double *xc_old, *uc_old, *om_old;  // np*3
+    double *xc_new, *uc_new, *om_new;  // np*3, after this step's motion
     double *flink, *tlink, *corr;      // np*PART_NSLAB*3 (x2), np*PART_NSLAB: link sums per slab
     double *ftot, *ttot;               // np*3: total force and torque of the last step
-    double* prep_sum;                  // np: refill bookkeeping (density)
-    int* prep_cnt;                     // np: refill bookkeeping (fluid count change)
-    double* partials;                  // bulk-kernel block partials, 2 per block
+    double* prep_sum;                  // refill bookkeeping per slab: density
+    int* prep_cnt;                     // and fluid count change, np*PART_NSLAB each
+    int* rf_count;                     // np: nodes that left the particle this step,
+    long long* rf_list;                // np*PART_REFILL: and their cells
+    int par;                           // which of the two mask buffers owner_cur is
+    double* partials;                  // bulk-kernel partials, 2 per warp, and the finish sums
     int nblocks;                       // number of bulk-kernel partial slots (one per warp)
     long long* n_fluid;                // device scalar
     double* rho_avg;                   // device scalars: [0] at bounce-back, [1] after update
-    int* status;                       // device: [0] code, [1] particle, [2] other particle
+    unsigned* done;                    // blocks that have finished (last-block sums)
+    int* status;                       // device: [0] code, [1] particle, [2] other particle,
+                                       // [3] mask buffer of the frozen state
 };
 
 // one fused step of the particle flow (collide + stream + bounce-back on

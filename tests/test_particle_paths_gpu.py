@@ -1,0 +1,71 @@
+"""Branches of the sphere step against the general path.
+
+FP64 cells take the integer form of the forward transform while f_1..18 lie in
+[2^-6, 2^-3) and f_0 in [2^-6, 1/2), the FP64 form otherwise: rho0 = 0.5625 puts the
+diagonal weights on the lower limit, 1.5 the rest weight and 2.25 the axis weights
+on the upper ones (cells of both kinds side by side), 8 takes every cell to the FP64
+form.  The bounds are those of the unit-density flow: 1e-10 on the populations,
+1e-9 on the particle state."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tests.gpu_util import rel_l2
+from tests.test_particle_gpu import CASE, mg  # noqa: F401  (fixture)
+
+pytestmark = pytest.mark.gpu
+
+CENTERS = [[8.3, 11.7, 10.1], [21.6, 11.4, 10.2], [34.2, 10.8, 9.5]]
+
+
+def _flow(mg, precision, centers=CENTERS, **over):
+    kw = dict(CASE, nx=37, ny=23, nz=21)
+    kw.update(over)
+    nx, ny, nz, r = kw.pop("nx"), kw.pop("ny"), kw.pop("nz"), kw.pop("radius")
+    kw["periodic_x"] = bool(kw["periodic_x"])
+    return mg.ParticleFlow(nx, ny, nz, centers, r, precision=precision, **kw)
+
+
+@pytest.mark.parametrize("rho0", [0.5625, 1.5, 2.25, 8.0])
+def test_density_ranges_match_oracle(mg, rho0):  # noqa: F811
+    over = dict(nx=37, ny=23, nz=21, rho0=rho0, rho_solid=1.2 * rho0)
+    o = O.ParticleOracle(np.array(CENTERS), dim=3, qmode=1, **dict(CASE, **over))
+    assert o.step(30) == 0
+    ref = o.get()
+    with _flow(mg, "fp64", **over) as c:
+        c.initial()
+        c.step(30)
+        st, mask, f = c.state(), c.mask(), c.get_f()
+    fluid = ref["obst"] == 0
+    assert np.array_equal(mask < 0, fluid)
+    assert rel_l2(f[fluid], ref["f"][fluid]) <= 1e-10
+    for a, b in (("uc", "uc"), ("omega", "om"), ("force", "force"), ("torque", "torque")):
+        assert rel_l2(st[a], ref[b]) <= 1e-8, a
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("g", [-0.05, -0.06])
+def test_frozen_state_is_the_failing_steps(mg, precision, g):  # noqa: F811
+    """A sphere that falls into the wall freezes the same state whether the steps
+    come one by one or as many more in one call than were needed, an even or an
+    odd number (the mask buffers alternate)."""
+    over = dict(gravity=(0.0, 0.0, g), spring_scale_wall=0.0)
+    centers = [[8.3, 11.7, 5.3], [21.6, 11.4, 10.2]]
+
+    def run(chunks):
+        with _flow(mg, precision, centers, **over) as c:
+            c.initial()
+            n = 0
+            with pytest.raises(mg.MglcError):
+                for k in chunks:
+                    c.step(k)
+                    n += k
+            return n, c.mask(), c.state()
+
+    n, mask, st = run([1] * 200)
+    assert 0 < n < 199
+    for extra in (n + 6, n + 7):
+        _, m2, s2 = run([extra])
+        assert np.array_equal(mask, m2)
+        for k in ("xc", "uc", "omega"):
+            assert np.array_equal(st[k], s2[k]), k
