@@ -1,24 +1,30 @@
 // d2q9.cuh -- the D2Q9 MRT collision of the reference's 2-D codes, bit for bit
 // (Lid_driven_cavity/fortran/2d/2d_revised/mpi_blocked/evolution.f90:16-68 and
 // Micro_particles/fortran/case4/mpi_particle/fluid.F90:14-64), shared by the
-// 2-D cavity and the 2-D particle kernels.  Both are bound by the FP64 pipe,
-// so the fast path writes the statements with as few FP64 instructions as give
-// the same bits (about 132 a node and 12 for the two quotients of the macro,
-// where the statements as written took about 190 and 20):
+// 2-D cavity and the 2-D particle kernels.  Both are bound by the FP64 pipe (a
+// warp's instruction holds the SM's unit for 16 clocks or more), so the fast
+// path writes the statements with as few FP64 instructions as give the same bits:
+// 82 a node and 8 for the quotients of the macro, where the statements as written
+// took about 190 and 20 (2-D cavity, 1024^2: 404 us a step as written, 331 with
+// the first three of these, 221 with all; 22 are its bytes):
 //  * products by 2, 4, 1/2 and 1/4 are exact, so a sum with one is a single
 //    fused multiply-add with the same rounding, and a chain of sums of doubled
 //    terms is twice the chain of the terms;
 //  * the conserved moments relax at s = 0: m - 0 (m - meq) is m for finite
 //    values other than -0;
 //  * x/18 = 2 (x/36) and x/12 = (x/6)/2 exactly, so eight quotients serve all;
-//  * a quotient by 6, 9, 18 or 36 is one multiply and one fused multiply-add
-//    (div_const), and two quotients by rho share one reciprocal (div_pair).
+//    a quotient by 6, 9, 18 or 36 is one multiply and one fused multiply-add
+//    (div_const), and two quotients by rho share one reciprocal (div_pair);
+//  * the fifty additions of the moments, and most of that reciprocal, run on
+//    integers, each rounded as FP64 rounds (Fix9), in issue slots that are empty.
 // A node whose values are outside the ranges that these need (fast_ok) takes
 // the statements as the reference writes them.
 // Include only in files compiled with -fmad=false: the contractions are the
 // explicit __fma_rn.
 #pragma once
 #include <cuda_runtime.h>
+
+#include "fix61.cuh"
 
 namespace mglc {
 
@@ -79,16 +85,106 @@ __device__ __forceinline__ void div_pair(double a, double b, double r, double& q
     qb = __fma_rn(__fma_rn(-r, tb, b), y, tb);
 }
 
-// macro (evolution.f90:103-107, fluid.F90:164-184)
-__device__ __forceinline__ void d2q9_macro(const double (&f)[9], double& r, double& u, double& v) {
+// Sums of populations, each addition rounded as FP64's: populations in [2^-6, 1/2)
+// are exact in units of 2^-58, and there an addition is an integer one followed
+// by the rounding of the sum to 53 significant bits (rn53), bit for bit.
+__device__ __forceinline__ bool d2q9_fix_ok(const double (&f)[9]) {
+    unsigned worst = 0;
+#pragma unroll
+    for (int q = 1; q < 9; q++)
+        worst = max(worst, (unsigned)__double2hiint(f[q]) - 0x3F900000u);  // 2^-6
+    return worst < 0x00400000u &&                                          // below 1/4
+           (unsigned)__double2hiint(f[0]) - 0x3F900000u < 0x00500000u;     // below 1/2
+}
+struct Fix9 {
+    long long v;
+};
+__device__ __forceinline__ Fix9 operator+(Fix9 a, Fix9 b) { return {rn53(a.v + b.v)}; }
+__device__ __forceinline__ Fix9 operator-(Fix9 a, Fix9 b) { return {rn53(a.v - b.v)}; }
+// s a + b, one rounding
+__device__ __forceinline__ Fix9 fma9(int s, Fix9 a, Fix9 b) { return {rn53(s * a.v + b.v)}; }
+__device__ __forceinline__ double fma9(int s, double a, double b) { return __fma_rn((double)s, a, b); }
+__device__ __forceinline__ Fix9 neg9(Fix9 a) { return {-a.v}; }
+__device__ __forceinline__ double neg9(double a) { return -a; }
+__device__ __forceinline__ void d2q9_fix_load(const double (&f)[9], Fix9 (&F)[9]) {
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+        const unsigned hi = (unsigned)__double2hiint(f[q]), lo = (unsigned)__double2loint(f[q]);
+        const unsigned s = (hi >> 20) - 1017u;
+        const unsigned mh = (hi & 0xFFFFFu) | 0x100000u;
+        F[q].v = (long long)(((unsigned long long)__funnelshift_l(lo, mh, s) << 32) | (lo << s));
+    }
+}
+
+// moments of the macro (evolution.f90:103-107, fluid.F90:164-184)
+template <class T>
+__device__ __forceinline__ void d2q9_sums(const T (&f)[9], T& r, T& jx, T& jy) {
     r = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8];
-    const double jx = f[1] - f[3] + f[5] - f[6] - f[7] + f[8];
-    const double jy = f[2] - f[4] + f[5] + f[6] - f[7] - f[8];
+    jx = f[1] - f[3] + f[5] - f[6] - f[7] + f[8];
+    jy = f[2] - f[4] + f[5] + f[6] - f[7] - f[8];
+}
+// and of the collision.  GROUPED: m1 and m2 sum the equal terms first
+// (evolution.f90:17-18, case1 fluid.F90:15-16), else term by term (case4 fluid.F90)
+template <bool GROUPED, class T>
+__device__ __forceinline__ void d2q9_moments(const T (&f)[9], T (&m)[9]) {
+    d2q9_sums(f, m[0], m[3], m[5]);
+    T m1 = fma9(-4, f[0], neg9(f[1])) - f[2] - f[3] - f[4], m2;
+    if (GROUPED) {
+        m1 = fma9(2, f[5] + f[6] + f[7] + f[8], m1);
+        m2 = fma9(2, f[0], neg9(f[1] + f[2] + f[3] + f[4]));  // half of 4 f0 - 2 (...)
+    } else {
+        m1 = fma9(2, f[5], m1);
+        m1 = fma9(2, f[6], m1);
+        m1 = fma9(2, f[7], m1);
+        m1 = fma9(2, f[8], m1);
+        m2 = fma9(2, f[0], neg9(f[1])) - f[2] - f[3] - f[4];
+    }
+    m[1] = m1;
+    m[2] = fma9(2, m2, f[5]) + f[6] + f[7] + f[8];
+    m[4] = fma9(2, f[3] - f[1], f[5]) - f[6] - f[7] + f[8];
+    m[6] = fma9(2, f[4] - f[2], f[5]) + f[6] - f[7] - f[8];
+    m[7] = f[1] - f[2] + f[3] - f[4];
+    m[8] = f[5] - f[6] + f[7] - f[8];
+}
+
+// velocity from the sums as doubles
+__device__ __forceinline__ void d2q9_velocity(double r, double jx, double jy, double& u, double& v) {
     if (den_ok(r) && mid_or_pzero(jx) && mid_or_pzero(jy)) {
         div_pair(jx, jy, r, u, v);
     } else {
         u = jx / r;
         v = jy / r;
+    }
+}
+// and for a density of R >= 1/4 in units of 2^-58 (sums in range, so below 2.75): the
+// reciprocal to 2^-60 on integers, rounded, then div_pair's last step
+__device__ __forceinline__ void d2q9_velocity(long long R, double r, double jx, double jy,
+                                              double& u, double& v) {
+    if (R >= (1LL << 56) && den_ok(r)) {
+        double y = fix_out<60>(rn53(fix_recip(R << 3, fix_dig(R << 3))));
+        y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
+        const double ta = __dmul_rn(jx, y), tb = __dmul_rn(jy, y);
+        u = __fma_rn(__fma_rn(-r, ta, jx), y, ta);
+        v = __fma_rn(__fma_rn(-r, tb, jy), y, tb);
+    } else {
+        u = jx / r;
+        v = jy / r;
+    }
+}
+
+__device__ __forceinline__ void d2q9_macro(const double (&f)[9], double& r, double& u, double& v) {
+    double jx, jy;
+    if (d2q9_fix_ok(f)) {
+        Fix9 F[9], R, X, Y;
+        d2q9_fix_load(f, F);
+        d2q9_sums(F, R, X, Y);
+        r = fix_out<58>(R.v);
+        jx = fix_out<58>(X.v);
+        jy = fix_out<58>(Y.v);
+        d2q9_velocity(R.v, r, jx, jy, u, v);
+    } else {
+        d2q9_sums(f, r, jx, jy);
+        d2q9_velocity(r, jx, jy, u, v);
     }
 }
 
@@ -141,29 +237,25 @@ __device__ __noinline__ void d2q9_collide_plain(const double* f, double rho, dou
 }
 
 // post-collision populations fp of one node from its populations and rho, u, v
-template <bool GROUPED>
-__device__ __forceinline__ void d2q9_collide(const double (&f)[9], double rho, double u, double v,
+// (MACRO: which it forms first)
+template <bool GROUPED, bool MACRO>
+__device__ __forceinline__ void d2q9_collide(const double (&f)[9], double& rho, double& u, double& v,
                                              double snu, double sq, double (&fp)[9]) {
-    const double m0 = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8];
-    double m1 = __fma_rn(-4.0, f[0], -f[1]) - f[2] - f[3] - f[4];
-    double m2;
-    if (GROUPED) {
-        m1 = __fma_rn(2.0, f[5] + f[6] + f[7] + f[8], m1);
-        m2 = __fma_rn(2.0, f[0], -(f[1] + f[2] + f[3] + f[4]));  // half of 4 f0 - 2 (...)
+    double m[9];
+    if (d2q9_fix_ok(f)) {
+        Fix9 F[9], M[9];
+        d2q9_fix_load(f, F);
+        d2q9_moments<GROUPED>(F, M);
+#pragma unroll
+        for (int a = 0; a < 9; a++) m[a] = fix_out<58>(M[a].v);
+        if (MACRO) d2q9_velocity(M[0].v, m[0], m[3], m[5], u, v);
     } else {
-        m1 = __fma_rn(2.0, f[5], m1);
-        m1 = __fma_rn(2.0, f[6], m1);
-        m1 = __fma_rn(2.0, f[7], m1);
-        m1 = __fma_rn(2.0, f[8], m1);
-        m2 = __fma_rn(2.0, f[0], -f[1]) - f[2] - f[3] - f[4];
+        d2q9_moments<GROUPED>(f, m);
+        if (MACRO) d2q9_velocity(m[0], m[3], m[5], u, v);
     }
-    m2 = __fma_rn(2.0, m2, f[5]) + f[6] + f[7] + f[8];
-    const double m3 = f[1] - f[3] + f[5] - f[6] - f[7] + f[8];
-    const double m4 = __fma_rn(2.0, f[3] - f[1], f[5]) - f[6] - f[7] + f[8];
-    const double m5 = f[2] - f[4] + f[5] + f[6] - f[7] - f[8];
-    const double m6 = __fma_rn(2.0, f[4] - f[2], f[5]) + f[6] - f[7] - f[8];
-    const double m7 = f[1] - f[2] + f[3] - f[4];
-    const double m8 = f[5] - f[6] + f[7] - f[8];
+    if (MACRO) rho = m[0];
+    const double m0 = m[0], m1 = m[1], m2 = m[2], m3 = m[3], m4 = m[4], m5 = m[5], m6 = m[6],
+                 m7 = m[7], m8 = m[8];
     const double u2 = u * u, v2 = v * v, t3 = 3.0 * (u2 + v2);
     const double ru = rho * u, rv = rho * v;
     const double p1 = m1 - snu * (m1 - rho * (-2.0 + t3));

@@ -64,6 +64,26 @@ __device__ __forceinline__ double fix61_store_any(long long v) {
     return __longlong_as_double(v ? b - ((long long)Q << 52) : 0LL);
 }
 
+// v rounded to 53 significant bits, to nearest even; |v| < 2^63
+__device__ __forceinline__ long long rn53(long long v) {
+    const int hi = (int)(v >> 32);
+    const int r = max(11 - __clz(hi ^ (hi >> 31)), 0);
+    const unsigned m = (1u << r) - 1u;  // the bits to drop
+    const unsigned odd = (unsigned)(v >> r) & m & 1u;
+    return (v + (long long)(m >> 1) + (long long)odd) & ~(long long)m;
+}
+
+// v * 2^-Q for a v of at most 53 significant bits, with integer operations
+template <int Q>
+__device__ __forceinline__ double fix_out(long long v) {
+    const long long sg = v >> 63;
+    const unsigned long long a = (unsigned long long)((v ^ sg) - sg);
+    const int lz = __clzll((long long)a);
+    const unsigned long long m = a << (lz & 63) >> 11;  // the leading bit at bit 52
+    const unsigned long long b = m + ((unsigned long long)(unsigned)(1022 + 63 - Q - lz) << 52);
+    return __longlong_as_double((long long)(a ? b | ((unsigned long long)sg << 63) : 0ull));
+}
+
 // v = h * 2^32 + l in balanced digits
 struct FixD {
     int h, l;

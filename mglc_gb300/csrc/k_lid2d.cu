@@ -18,9 +18,10 @@
 // arithmetic is FP64 in the reference's expression order and this file is
 // compiled without FMA contraction (device and host), so every value rounds
 // as the reference's statement does; the collision and the two quotients of
-// macro are d2q9.cuh's, which give those bits with about 150 FP64 instructions
-// a node.  The FP64 pipe bounds the step: 1024^2 takes 331 us (3.17 GLUPS)
-// against 404 us with the statements written out (about 190 instructions).
+// macro are d2q9.cuh's, which give those bits with about 90 FP64 instructions
+// a node and as many integer ones beside them as fit.  The FP64 pipe bounds the
+// step: 1024^2 takes 221 us (4.74 GLUPS) against 404 us with the statements
+// written out (about 190 FP64 instructions).
 // check() sums on the host in the reference's (j, i) loop order for the same
 // reason.
 #include <algorithm>
@@ -95,11 +96,9 @@ __global__ void __launch_bounds__(128) k_l2_step(L2K k) {
         r = k.rho[c];
         u = k.u[c];
         v = k.v[c];
-    } else {
-        d2q9_macro(f, r, u, v);
     }
     double fp[9];
-    d2q9_collide<true>(f, r, u, v, k.snu, k.sq, fp);
+    d2q9_collide<true, !FIRST>(f, r, u, v, k.snu, k.sq, fp);
     // streaming + bounceback, evolution.f90:81-90 and bounceback.f90:6-42
 #pragma unroll
     for (int a = 0; a < 9; a++) {

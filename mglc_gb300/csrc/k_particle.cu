@@ -186,15 +186,6 @@ __device__ __forceinline__ bool fix58_ok(const double (&f)[Q19]) {
     return worst < 0x00300000u &&                                          // below 2^-3
            (unsigned)__double2hiint(f[0]) - 0x3F900000u < 0x00500000u;     // below 1/2
 }
-// a value of at most 53 significant bits as the double it is
-__device__ __forceinline__ double fix58_out(long long v) {
-    const long long sg = v >> 63;
-    const unsigned long long a = (unsigned long long)((v ^ sg) - sg);
-    const int lz = __clzll((long long)a);
-    const unsigned long long m = a << (lz & 63) >> 11;  // the leading bit at bit 52
-    const unsigned long long b = m + ((unsigned long long)(unsigned)(1022 + 63 - 58 - lz) << 52);
-    return __longlong_as_double((long long)(a ? b | ((unsigned long long)sg << 63) : 0ull));
-}
 __device__ __forceinline__ void fix58_moments(const double (&f)[Q19], MrtMom<double>& o,
                                               double& rho, double& jx, double& jy, double& jz) {
     Fix58 F[Q19];
@@ -210,29 +201,29 @@ __device__ __forceinline__ void fix58_moments(const double (&f)[Q19], MrtMom<dou
     const Fix58 sa = s1 + s2 + s3, se = (s4 + s5) + (s6 + s7) + (s8 + s9);
     // the fused multiply-adds of mrt_moments as nvcc contracts them: one rounding
     // of the exact value (8 se + RN(-11 sa) in m1)
-    o.m1 = fix58_out(rn53(-30 * F[0].v + rn53(8 * se.v + rn53(-11 * sa.v))));
-    o.m2 = fix58_out(rn53(12 * F[0].v + rn53(-4 * sa.v + se.v)));
+    o.m1 = fix_out<58>(rn53(-30 * F[0].v + rn53(8 * se.v + rn53(-11 * sa.v))));
+    o.m2 = fix_out<58>(rn53(12 * F[0].v + rn53(-4 * sa.v + se.v)));
     const Fix58 a45 = d4 + d5, b45 = d4 - d5, a67 = d6 + d7, b67 = d6 - d7, a89 = d8 + d9,
                 b89 = d8 - d9;
-    o.m4 = fix58_out(rn53(-4 * d1.v + (a45 + a67).v));
-    o.m6 = fix58_out(rn53(-4 * d2.v + (b45 + a89).v));
-    o.m8 = fix58_out(rn53(-4 * d3.v + (b67 + b89).v));
+    o.m4 = fix_out<58>(rn53(-4 * d1.v + (a45 + a67).v));
+    o.m6 = fix_out<58>(rn53(-4 * d2.v + (b45 + a89).v));
+    o.m8 = fix_out<58>(rn53(-4 * d3.v + (b67 + b89).v));
     const Fix58 sxy = s4 + s5, sxz = s6 + s7, syz = s8 + s9, s23 = s2 + s3, t23 = s2 - s3;
     const Fix58 sp = sxy + sxz, sm = sxy - sxz;
-    o.m9 = fix58_out(rn53((Fix58{rn53(2 * s1.v - s23.v)} + sp).v - 2 * syz.v));
-    o.m10 = fix58_out(rn53((Fix58{rn53(-4 * s1.v + 2 * s23.v)} + sp).v - 2 * syz.v));
-    o.m11 = fix58_out((t23 + sm).v);
-    o.m12 = fix58_out(rn53(-2 * t23.v + sm.v));
-    o.m13 = fix58_out((s4 - s5).v);
-    o.m14 = fix58_out((s8 - s9).v);
-    o.m15 = fix58_out((s6 - s7).v);
-    o.m16 = fix58_out((a45 - a67).v);
-    o.m17 = fix58_out(rn53(-b45.v + a89.v));
-    o.m18 = fix58_out((b67 - b89).v);
-    rho = fix58_out(r.v);
-    jx = fix58_out(x.v);
-    jy = fix58_out(y.v);
-    jz = fix58_out(z.v);
+    o.m9 = fix_out<58>(rn53((Fix58{rn53(2 * s1.v - s23.v)} + sp).v - 2 * syz.v));
+    o.m10 = fix_out<58>(rn53((Fix58{rn53(-4 * s1.v + 2 * s23.v)} + sp).v - 2 * syz.v));
+    o.m11 = fix_out<58>((t23 + sm).v);
+    o.m12 = fix_out<58>(rn53(-2 * t23.v + sm.v));
+    o.m13 = fix_out<58>((s4 - s5).v);
+    o.m14 = fix_out<58>((s8 - s9).v);
+    o.m15 = fix_out<58>((s6 - s7).v);
+    o.m16 = fix_out<58>((a45 - a67).v);
+    o.m17 = fix_out<58>(rn53(-b45.v + a89.v));
+    o.m18 = fix_out<58>((b67 - b89).v);
+    rho = fix_out<58>(r.v);
+    jx = fix_out<58>(x.v);
+    jy = fix_out<58>(y.v);
+    jz = fix_out<58>(z.v);
 }
 template <bool FIRST>
 __device__ __forceinline__ void pcollide(double (&f)[Q19], const PBulkK<double>& k, double& rho) {

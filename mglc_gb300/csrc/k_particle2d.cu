@@ -135,7 +135,8 @@ __device__ __forceinline__ void collide_node(const D2& d, int c) {
     double f[9], fp[9];
 #pragma unroll
     for (int a = 0; a < 9; a++) f[a] = d.f[a * d.C + c];
-    d2q9_collide<GROUPED>(f, d.rho[c], d.u[c], d.v[c], d.p.snu, d.p.sq, fp);
+    double r = d.rho[c], u = d.u[c], v = d.v[c];
+    d2q9_collide<GROUPED, false>(f, r, u, v, d.p.snu, d.p.sq, fp);
 #pragma unroll
     for (int a = 0; a < 9; a++) d.fp[a * d.C + c] = fp[a];
 }

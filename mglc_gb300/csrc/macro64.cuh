@@ -18,15 +18,6 @@
 
 namespace mglc {
 
-// v rounded to 53 significant bits, to nearest even; |v| < 2^63
-__device__ __forceinline__ long long rn53(long long v) {
-    const int hi = (int)(v >> 32);
-    const int r = max(11 - __clz(hi ^ (hi >> 31)), 0);
-    const unsigned m = (1u << r) - 1u;  // the bits to drop
-    const unsigned odd = (unsigned)(v >> r) & m & 1u;
-    return (v + (long long)(m >> 1) + (long long)odd) & ~(long long)m;
-}
-
 // sum f and sum f e in the order of the populations, in FP64
 __device__ __forceinline__ void sums_fp64(const double (&f)[Q19], double& r, double& jx, double& jy,
                                           double& jz) {

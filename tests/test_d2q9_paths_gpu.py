@@ -73,3 +73,40 @@ def test_frozen_state_keeps_its_mask(mg):
         c.initial()
         c.step(1)
         assert (c.mask() >= 0).sum() > 0
+
+
+@pytest.mark.parametrize("kind", ["diagonal", "rest", "axis", "thin", "dense"])
+def test_lid2d_integer_sums_bitwise(mg, kind):
+    """Populations on either side of the range in which the sums run on integers
+    ([2^-6, 1/4), the rest population up to 1/2, density from 1/4): the limits
+    themselves, their neighbours and mixed cells."""
+    rng = np.random.default_rng(11)
+    nx, ny = 67, 5
+    w = np.array([4 / 9] + [1 / 9] * 4 + [1 / 36] * 4)
+    f = w * (1.0 + 0.2 * (rng.random((ny, nx, 9)) - 0.5))
+
+    def around(limit, n):  # the limit, its neighbours and values close by
+        near = np.array([limit, np.nextafter(limit, 0), np.nextafter(limit, 1)])
+        pick = rng.integers(0, 4, (ny, nx, n))
+        return np.where(pick < 3, near[np.minimum(pick, 2)], limit * (1 + 0.1 * (rng.random((ny, nx, n)) - 0.5)))
+
+    if kind == "diagonal":
+        f[..., 5:] = around(2.0 ** -6, 4)
+    elif kind == "rest":
+        f[..., :1] = around(0.5, 1)
+    elif kind == "axis":
+        f[..., 1:5] = around(0.25, 4)
+    elif kind == "thin":  # densities around 1/4 from populations in range
+        f = np.array([0.08] + [0.021] * 8) * (1.0 + 0.1 * (rng.random((ny, nx, 9)) - 0.5))
+    else:  # the largest density in range
+        f[..., 0] = np.nextafter(0.5, 0)
+        f[..., 1:] = np.where(rng.random((ny, nx, 8)) < 0.8, np.nextafter(0.25, 0), 0.2)
+    o = O.Lid2DOracle(nx, ny, 200.0, 0.1)
+    with mg.LidDrivenCavity2D(nx, ny, reynolds=200.0, u0=0.1) as c:
+        c.load_state(f)
+        rho, u, v = c.macro()
+        o.f[:], o.rho[:], o.u[:], o.v[:] = f, rho, u, v
+        for _ in range(3):
+            c.step(1)
+            o.run(1)
+            assert np.array_equal(c.get_f(), o.f)
