@@ -161,19 +161,13 @@ struct FixFlow {
     FixD ux, uy, uz;            // velocity, units of 2^-63
     long long ex, ey, ez, d19;  // 2 (j - rho u); FIRST: Snu/19 (sum f - rho)
 };
-// No force: half(rho, h) of fix61_flow.
-struct FixNoForce {
-    __device__ __forceinline__ void operator()(FixD, long long (&h)[3]) const {
-        h[0] = h[1] = h[2] = 0;
-    }
-};
-// From the populations and half the force that the velocity takes (half(rho, h);
-// rho u = j + h), or, FIRST (the step after initial or load), from the macro
-// arrays; false when the density or the velocity is out of range.
-template <bool FIRST, class Half>
-__device__ __forceinline__ bool fix61_flow(const long long (&F)[Q19], const FixK& k, Half half,
-                                           double rho0, double u0, double v0, double w0,
-                                           FixFlow& o) {
+// From the populations and half the force carried from the previous step
+// (hx, hy, hz; rho u = j + Fp/2), or, FIRST (the step after initial or load),
+// from the macro arrays; false when the density or the velocity is out of range.
+template <bool FIRST>
+__device__ __forceinline__ bool fix61_flow(const long long (&F)[Q19], const FixK& k, long long hx,
+                                           long long hy, long long hz, double rho0, double u0,
+                                           double v0, double w0, FixFlow& o) {
     long long r, jx, jy, jz;
     moments0(F, r, jx, jy, jz);
     if (FIRST) {
@@ -195,16 +189,15 @@ __device__ __forceinline__ bool fix61_flow(const long long (&F)[Q19], const FixK
         o.d19 = fix_mad(r - o.r, k.l19, 0);
         return true;
     }
+    jx += hx;
+    jy += hy;
+    jz += hz;
+    const long long half = r >> 1;
+    if (!(r >= (1LL << 59) && jx < half && -jx < half && jy < half && -jy < half && jz < half &&
+          -jz < half))
+        return false;
     o.r = r;
     o.rd = fix_dig(r);
-    long long h[3];
-    half(o.rd, h);
-    jx += h[0];
-    jy += h[1];
-    jz += h[2];
-    const long long r2 = r >> 1;
-    if (!(r >= (1LL << 59) && jx < r2 && -jx < r2 && jy < r2 && -jy < r2 && jz < r2 && -jz < r2))
-        return false;
     o.Jx = fix_dig(jx);
     o.Jy = fix_dig(jy);
     o.Jz = fix_dig(jz);
@@ -212,9 +205,9 @@ __device__ __forceinline__ bool fix61_flow(const long long (&F)[Q19], const FixK
     o.ux = fix_dig(fix_mul<58>(o.Jx, di));
     o.uy = fix_dig(fix_mul<58>(o.Jy, di));
     o.uz = fix_dig(fix_mul<58>(o.Jz, di));
-    o.ex = -2 * h[0];
-    o.ey = -2 * h[1];
-    o.ez = -2 * h[2];
+    o.ex = -2 * hx;
+    o.ey = -2 * hy;
+    o.ez = -2 * hz;
     o.d19 = 0;
     return true;
 }

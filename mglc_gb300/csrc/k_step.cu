@@ -14,45 +14,36 @@
 //   thermal: bouyancy3d_mpi.F90 collision :641-864, streaming :867-892,
 //            bounceback :895-983, collisionT :1014-1070, streamingT :1073-1098,
 //            bouncebackT :1101-1210, macro :986-1010, macroT :1215-1231
+#include "cell_map.cuh"
 #include "step_cell.cuh"
 
 namespace mglc {
 
-template <typename S, bool FIRST, typename IDX, bool SR>
+template <typename S, bool FIRST, typename IDX, bool SR, class MAP>
 __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
     k_lid_step(const S* __restrict__ fin, S* __restrict__ fout, StepK<typename St<S>::C> K,
-               IDX P, const double* __restrict__ mrho, const double* __restrict__ mu,
+               MAP map, IDX P, const double* __restrict__ mrho, const double* __restrict__ mu,
                const double* __restrict__ mv, const double* __restrict__ mw) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K.nx) return;
-    lid_cell<S, FIRST, IDX, SR>(i, blockIdx.y, blockIdx.z, fin, fout, K, P, mrho, mu, mv, mw,
-                                K.seed);
+    int i, j, k;
+    if (!map.at(K.nx, K.ny, P, i, j, k)) return;
+    lid_cell<S, FIRST, IDX, SR>(i, j, k, fin, fout, K, P, mrho, mu, mv, mw, K.seed);
 }
 
-template <typename S, bool FIRST, bool ROT, typename IDX, bool SR>
+template <typename S, bool FIRST, bool ROT, typename IDX, bool SR, class MAP>
 __global__ void __launch_bounds__(128, ThermalMinBlocks<S>::value)
     k_thermal_step(const S* __restrict__ fin, S* __restrict__ fout,
                    const typename St<S>::C* __restrict__ gin, typename St<S>::C* __restrict__ gout,
-                   typename St<S>::C* __restrict__ F, StepK<typename St<S>::C> K, IDX P,
+                   typename St<S>::C* __restrict__ F, StepK<typename St<S>::C> K, MAP map, IDX P,
                    const double* __restrict__ mrho, const double* __restrict__ mu,
                    const double* __restrict__ mv, const double* __restrict__ mw,
                    const double* __restrict__ mT) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K.nx) return;
-    thermal_cell<S, FIRST, ROT, IDX, SR>(i, blockIdx.y, blockIdx.z, fin, fout, gin, gout, F, K,
-                                         P, mrho, mu, mv, mw, mT, (IDX)2 * P, K.seed);
+    int i, j, k;
+    if (!map.at(K.nx, K.ny, P, i, j, k)) return;
+    thermal_cell<S, FIRST, ROT, IDX, SR>(i, j, k, fin, fout, gin, gout, F, K, P, mrho, mu, mv, mw,
+                                         mT, (IDX)2 * P, K.seed);
 }
 
 // --------------------------------------------------------------- launch --
-static dim3 step_block(int nx) {
-    int bx = ((nx + 31) / 32) * 32;
-    if (bx > 128) bx = 128;
-    return dim3(bx, 1, 1);
-}
-static dim3 step_grid(const Geom& g, dim3 b) {
-    return dim3((g.nx + b.x - 1) / b.x, g.ny, g.nz);
-}
-
 template <typename S>
 static cudaError_t lid_go(bool first, const void* fin, void* fout, const LidStepArgs& a,
                           cudaStream_t s, bool box = false) {
@@ -61,20 +52,22 @@ static cudaError_t lid_go(bool first, const void* fin, void* fout, const LidStep
     set_box(K.pk, box);
     K.seed = a.seed;
     K.sr = a.sr;
-    dim3 b = step_block(a.g.nx), gr = step_grid(a.g, b);
-    const bool small = (long long)Q19 * a.g.plane < (1ll << 31);
+    const CellLaunch l(a.g);
+    const bool small = index32(a.g);
     // stochastic rounding exists for the 16-bit storage types only
     constexpr bool kHalf = sizeof(S) == 2;
-#define LID_LAUNCH(FI, IT, SRV)                                                          \
-    k_lid_step<S, FI, IT, SRV><<<gr, b, 0, s>>>((const S*)fin, (S*)fout, K, (IT)a.g.plane, \
-                                                a.rho, a.u, a.v, a.w)
-#define LID_SR(FI, IT)                                  \
-    if (kHalf && a.sr) LID_LAUNCH(FI, IT, kHalf);        \
-    else LID_LAUNCH(FI, IT, false);
-    if (small) {
-        if (first) { LID_SR(true, unsigned) } else { LID_SR(false, unsigned) }
+#define LID_LAUNCH(FI, IT, SRV, MAP)                                                              \
+    k_lid_step<S, FI, IT, SRV, MAP><<<l.grid, l.block, 0, s>>>((const S*)fin, (S*)fout, K, MAP(a.g), \
+                                                               (IT)a.g.plane, a.rho, a.u, a.v, a.w)
+#define LID_SR(FI, IT, MAP)                              \
+    if (kHalf && a.sr) LID_LAUNCH(FI, IT, kHalf, MAP);   \
+    else LID_LAUNCH(FI, IT, false, MAP);
+    if (linear_cells(a.g)) {
+        if (first) { LID_SR(true, unsigned, CellMap) } else { LID_SR(false, unsigned, CellMap) }
+    } else if (small) {
+        if (first) { LID_SR(true, unsigned, RowMap) } else { LID_SR(false, unsigned, RowMap) }
     } else {
-        if (first) { LID_SR(true, long long) } else { LID_SR(false, long long) }
+        if (first) { LID_SR(true, long long, RowMap) } else { LID_SR(false, long long, RowMap) }
     }
 #undef LID_SR
 #undef LID_LAUNCH
@@ -107,28 +100,30 @@ static cudaError_t th_go(bool first, const void* fin, void* fout, const void* gi
     K.bc_y = a.bc_y; K.bc_z = a.bc_z;
     pair_k_heat(K.pk, a.para_a, a.qd, a.qnu);
     set_box(K.pk, box);
-    dim3 b = step_block(a.g.nx), gr = step_grid(a.g, b);
+    const CellLaunch l(a.g);
     const bool rot = a.omega_rot != 0.0;
-    const bool small = (long long)Q19 * a.g.plane < (1ll << 31);
+    const bool small = index32(a.g);
     constexpr bool kHalf = sizeof(S) == 2;
-#define TH_LAUNCH2(FI, RO, IT, SRV)                                                            \
-    k_thermal_step<S, FI, RO, IT, SRV><<<gr, b, 0, s>>>((const S*)fin, (S*)fout, (const C*)gin, \
-                                                        (C*)gout, (C*)F, K, (IT)a.g.plane,     \
-                                                        a.rho, a.u, a.v, a.w, a.T)
-#define TH_LAUNCH(FI, RO, IT)                                   \
+#define TH_LAUNCH2(FI, RO, IT, SRV, MAP)                                                     \
+    k_thermal_step<S, FI, RO, IT, SRV, MAP><<<l.grid, l.block, 0, s>>>(                      \
+        (const S*)fin, (S*)fout, (const C*)gin, (C*)gout, (C*)F, K, MAP(a.g), (IT)a.g.plane, \
+        a.rho, a.u, a.v, a.w, a.T)
+#define TH_LAUNCH(FI, RO, IT, MAP)                              \
     do {                                                        \
-        if (kHalf && a.sr) TH_LAUNCH2(FI, RO, IT, kHalf);       \
-        else TH_LAUNCH2(FI, RO, IT, false);                     \
+        if (kHalf && a.sr) TH_LAUNCH2(FI, RO, IT, kHalf, MAP);  \
+        else TH_LAUNCH2(FI, RO, IT, false, MAP);                \
     } while (0)
-#define TH_ROT(IT)                                       \
-    if (first && rot) TH_LAUNCH(true, true, IT);          \
-    else if (first) TH_LAUNCH(true, false, IT);           \
-    else if (rot) TH_LAUNCH(false, true, IT);             \
-    else TH_LAUNCH(false, false, IT);
-    if (small) {
-        TH_ROT(unsigned)
+#define TH_ROT(IT, MAP)                                  \
+    if (first && rot) TH_LAUNCH(true, true, IT, MAP);     \
+    else if (first) TH_LAUNCH(true, false, IT, MAP);      \
+    else if (rot) TH_LAUNCH(false, true, IT, MAP);        \
+    else TH_LAUNCH(false, false, IT, MAP);
+    if (linear_cells(a.g)) {
+        TH_ROT(unsigned, CellMap)
+    } else if (small) {
+        TH_ROT(unsigned, RowMap)
     } else {
-        TH_ROT(long long)
+        TH_ROT(long long, RowMap)
     }
 #undef TH_ROT
 #undef TH_LAUNCH

@@ -8,18 +8,18 @@
 // post-stream layout (the reference's f), which getters and checkpoints read.
 // Same reference routines as k_step.cu (mpi_3d_blocked/{collision.f90:15-202,
 // streaming.f90:8-20, bounce_back.f90:6-83, macro.f90:6-25}).
+#include "cell_map.cuh"
 #include "step_cell.cuh"
 
 namespace mglc {
 
-template <typename S, bool FIRST, typename IDX, bool SR, bool ODD>
+template <typename S, bool FIRST, typename IDX, bool SR, bool ODD, class MAP>
 __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
-    k_lid_step_aa(S* f, StepK<typename St<S>::C> K, IDX P, const double* __restrict__ mrho,
+    k_lid_step_aa(S* f, StepK<typename St<S>::C> K, MAP map, IDX P, const double* __restrict__ mrho,
                   const double* __restrict__ mu, const double* __restrict__ mv,
                   const double* __restrict__ mw) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K.nx) return;
-    const int j = blockIdx.y, k = blockIdx.z;
+    int i, j, k;
+    if (!map.at(K.nx, K.ny, P, i, j, k)) return;
     S raw[Q19];  // every load is issued before the first store
     lid_load_aa<S, IDX, ODD>(i, j, k, f, K.nx, K.ny, K.nz, P, raw);
     lid_cell_from<S, FIRST, IDX, SR, !ODD>(i, j, k, raw, f, K, P, mrho, mu, mv, mw, K.seed);
@@ -27,16 +27,15 @@ __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
 
 // Heated cavity in place: flow and temperature populations each on one
 // buffer; the carried force is the cell's own (read, then written).
-template <typename S, bool FIRST, bool ROT, typename IDX, bool SR, bool ODD>
+template <typename S, bool FIRST, bool ROT, typename IDX, bool SR, bool ODD, class MAP>
 __global__ void __launch_bounds__(128, ThermalMinBlocks<S>::value)
     k_thermal_step_aa(S* f, typename St<S>::C* g, typename St<S>::C* __restrict__ F,
-                      StepK<typename St<S>::C> K, IDX P, const double* __restrict__ mrho,
+                      StepK<typename St<S>::C> K, MAP map, IDX P, const double* __restrict__ mrho,
                       const double* __restrict__ mu, const double* __restrict__ mv,
                       const double* __restrict__ mw, const double* __restrict__ mT) {
     using C = typename St<S>::C;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K.nx) return;
-    const int j = blockIdx.y, k = blockIdx.z;
+    int i, j, k;
+    if (!map.at(K.nx, K.ny, P, i, j, k)) return;
     C fv[Q19], gv[Q7], fp[3];  // every load is issued before the first store
     thermal_load_aa<S, IDX, ODD, ROT>(i, j, k, f, g, F, (IDX)2 * P, K, P, fv, gv, fp);
     thermal_cell_from<S, FIRST, ROT, IDX, SR, !ODD>(i, j, k, fv, gv, fp, f, g, F, K, P, mrho, mu,
@@ -48,11 +47,10 @@ __global__ void __launch_bounds__(128, ThermalMinBlocks<S>::value)
 // without collision.  The pair is owned by the thread of x, so the exchange
 // is race-free; where x - e_q is outside, slot q of x already holds the
 // reflected population.
-template <typename S, int Q, typename IDX>
-__global__ void __launch_bounds__(128) k_aa_swap(S* f, int nx, int ny, int nz, IDX P) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nx) return;
-    const int j = blockIdx.y, k = blockIdx.z;
+template <typename S, int Q, typename IDX, class MAP>
+__global__ void __launch_bounds__(128) k_aa_swap(S* f, int nx, int ny, int nz, MAP map, IDX P) {
+    int i, j, k;
+    if (!map.at(nx, ny, P, i, j, k)) return;
     const IDX cell = (IDX)i + (IDX)nx * ((IDX)j + (IDX)ny * (IDX)k);
     const IDX sy = (IDX)nx, sz = (IDX)nx * (IDX)ny;
     const unsigned bm = face_mask(i, j, k, nx, ny, nz);
@@ -74,12 +72,6 @@ __global__ void __launch_bounds__(128) k_aa_swap(S* f, int nx, int ny, int nz, I
 
 namespace {
 
-dim3 aa_block(int nx) {
-    int bx = ((nx + 31) / 32) * 32;
-    if (bx > 128) bx = 128;
-    return dim3(bx, 1, 1);
-}
-
 template <typename S>
 cudaError_t lid_go_aa(bool first, bool odd, void* f, const LidStepArgs& a, cudaStream_t s,
                       bool box = false) {
@@ -88,28 +80,31 @@ cudaError_t lid_go_aa(bool first, bool odd, void* f, const LidStepArgs& a, cudaS
     set_box(K.pk, box);
     K.seed = a.seed;
     K.sr = a.sr;
-    const dim3 b = aa_block(a.g.nx), gr((a.g.nx + b.x - 1) / b.x, a.g.ny, a.g.nz);
-    const bool small = (long long)Q19 * a.g.plane < (1ll << 31);
+    const CellLaunch l(a.g);
+    const bool small = index32(a.g);
     constexpr bool kHalf = sizeof(S) == 2;  // stochastic rounding: 16-bit storage only
     const bool sr = kHalf && a.sr;
     S* fp = (S*)f;
-#define AA_LAUNCH(FI, IT, SRV, OD) \
-    k_lid_step_aa<S, FI, IT, SRV, OD><<<gr, b, 0, s>>>(fp, K, (IT)a.g.plane, a.rho, a.u, a.v, a.w)
-#define AA_PICK(IT)                                                        \
+#define AA_LAUNCH(FI, IT, SRV, OD, MAP)                                       \
+    k_lid_step_aa<S, FI, IT, SRV, OD, MAP><<<l.grid, l.block, 0, s>>>(        \
+        fp, K, MAP(a.g), (IT)a.g.plane, a.rho, a.u, a.v, a.w)
+#define AA_PICK(IT, MAP)                                                   \
     if (odd) {                                                             \
-        if (sr) AA_LAUNCH(false, IT, kHalf, true);                         \
-        else AA_LAUNCH(false, IT, false, true);                            \
+        if (sr) AA_LAUNCH(false, IT, kHalf, true, MAP);                    \
+        else AA_LAUNCH(false, IT, false, true, MAP);                       \
     } else if (first) {                                                    \
-        if (sr) AA_LAUNCH(true, IT, kHalf, false);                         \
-        else AA_LAUNCH(true, IT, false, false);                            \
+        if (sr) AA_LAUNCH(true, IT, kHalf, false, MAP);                    \
+        else AA_LAUNCH(true, IT, false, false, MAP);                       \
     } else {                                                               \
-        if (sr) AA_LAUNCH(false, IT, kHalf, false);                        \
-        else AA_LAUNCH(false, IT, false, false);                           \
+        if (sr) AA_LAUNCH(false, IT, kHalf, false, MAP);                   \
+        else AA_LAUNCH(false, IT, false, false, MAP);                      \
     }
-    if (small) {
-        AA_PICK(unsigned)
+    if (linear_cells(a.g)) {
+        AA_PICK(unsigned, CellMap)
+    } else if (small) {
+        AA_PICK(unsigned, RowMap)
     } else {
-        AA_PICK(long long)
+        AA_PICK(long long, RowMap)
     }
 #undef AA_PICK
 #undef AA_LAUNCH
@@ -118,11 +113,13 @@ cudaError_t lid_go_aa(bool first, bool odd, void* f, const LidStepArgs& a, cudaS
 
 template <typename S, int Q>
 cudaError_t swap_go(const Geom& g, void* f, cudaStream_t s) {
-    const dim3 b = aa_block(g.nx), gr((g.nx + b.x - 1) / b.x, g.ny, g.nz);
-    if ((long long)Q19 * g.plane < (1ll << 31))
-        k_aa_swap<S, Q, unsigned><<<gr, b, 0, s>>>((S*)f, g.nx, g.ny, g.nz, (unsigned)g.plane);
+    const CellLaunch l(g);
+    if (linear_cells(g))
+        k_aa_swap<S, Q, unsigned><<<l.grid, l.block, 0, s>>>((S*)f, g.nx, g.ny, g.nz, CellMap(g), (unsigned)g.plane);
+    else if (index32(g))
+        k_aa_swap<S, Q, unsigned><<<l.grid, l.block, 0, s>>>((S*)f, g.nx, g.ny, g.nz, RowMap(g), (unsigned)g.plane);
     else
-        k_aa_swap<S, Q, long long><<<gr, b, 0, s>>>((S*)f, g.nx, g.ny, g.nz, (long long)g.plane);
+        k_aa_swap<S, Q, long long><<<l.grid, l.block, 0, s>>>((S*)f, g.nx, g.ny, g.nz, RowMap(g), (long long)g.plane);
     return cudaGetLastError();
 }
 
@@ -140,30 +137,32 @@ cudaError_t th_go_aa(bool first, bool odd, void* f, void* g, void* F, const Ther
     K.bc_y = a.bc_y; K.bc_z = a.bc_z;
     pair_k_heat(K.pk, a.para_a, a.qd, a.qnu);
     set_box(K.pk, box);
-    const dim3 b = aa_block(a.g.nx), gr((a.g.nx + b.x - 1) / b.x, a.g.ny, a.g.nz);
+    const CellLaunch l(a.g);
     const bool rot = a.omega_rot != 0.0;
-    const bool small = (long long)Q19 * a.g.plane < (1ll << 31);
+    const bool small = index32(a.g);
     constexpr bool kHalf = sizeof(S) == 2;
     const bool sr = kHalf && a.sr;
     S* fp = (S*)f;
     C* gp = (C*)g;
     C* Fp = (C*)F;
-#define TA_LAUNCH(FI, RO, IT, SRV, OD)                                                       \
-    k_thermal_step_aa<S, FI, RO, IT, SRV, OD><<<gr, b, 0, s>>>(fp, gp, Fp, K, (IT)a.g.plane, \
-                                                               a.rho, a.u, a.v, a.w, a.T)
-#define TA_SR(FI, RO, IT, OD)                        \
-    do {                                             \
-        if (sr) TA_LAUNCH(FI, RO, IT, kHalf, OD);    \
-        else TA_LAUNCH(FI, RO, IT, false, OD);       \
+#define TA_LAUNCH(FI, RO, IT, SRV, OD, MAP)                                      \
+    k_thermal_step_aa<S, FI, RO, IT, SRV, OD, MAP><<<l.grid, l.block, 0, s>>>(   \
+        fp, gp, Fp, K, MAP(a.g), (IT)a.g.plane, a.rho, a.u, a.v, a.w, a.T)
+#define TA_SR(FI, RO, IT, OD, MAP)                        \
+    do {                                                  \
+        if (sr) TA_LAUNCH(FI, RO, IT, kHalf, OD, MAP);    \
+        else TA_LAUNCH(FI, RO, IT, false, OD, MAP);       \
     } while (0)
-#define TA_PICK(RO, IT)                              \
-    if (odd) TA_SR(false, RO, IT, true);             \
-    else if (first) TA_SR(true, RO, IT, false);      \
-    else TA_SR(false, RO, IT, false);
-    if (small) {
-        if (rot) { TA_PICK(true, unsigned) } else { TA_PICK(false, unsigned) }
+#define TA_PICK(RO, IT, MAP)                              \
+    if (odd) TA_SR(false, RO, IT, true, MAP);             \
+    else if (first) TA_SR(true, RO, IT, false, MAP);      \
+    else TA_SR(false, RO, IT, false, MAP);
+    if (linear_cells(a.g)) {
+        if (rot) { TA_PICK(true, unsigned, CellMap) } else { TA_PICK(false, unsigned, CellMap) }
+    } else if (small) {
+        if (rot) { TA_PICK(true, unsigned, RowMap) } else { TA_PICK(false, unsigned, RowMap) }
     } else {
-        if (rot) { TA_PICK(true, long long) } else { TA_PICK(false, long long) }
+        if (rot) { TA_PICK(true, long long, RowMap) } else { TA_PICK(false, long long, RowMap) }
     }
 #undef TA_PICK
 #undef TA_SR

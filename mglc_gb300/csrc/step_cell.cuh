@@ -310,10 +310,10 @@ __device__ __forceinline__ void lid_cell_from(int i, int j, int k, const S (&raw
             for (int q = 0; q < Q19; q++) F[q] = fix61_load(f[q]);
             FixFlow fl;
             if (FIRST)
-                ok = fix61_flow<true>(F, K.pk.fix, FixNoForce(), mrho[cell], mu[cell], mv[cell],
+                ok = fix61_flow<true>(F, K.pk.fix, 0, 0, 0, mrho[cell], mu[cell], mv[cell],
                                       mw[cell], fl);
             else
-                ok = fix61_flow<false>(F, K.pk.fix, FixNoForce(), 0.0, 0.0, 0.0, 0.0, fl);
+                ok = fix61_flow<false>(F, K.pk.fix, 0, 0, 0, 0.0, 0.0, 0.0, 0.0, fl);
             if (ok) fix61_collide<true, 0, FIRST, false>(F, K.pk.fix, fl, 0, 0, 0);
             rho = fix61_store_any(fl.r);
             fix61_store_all<10>(F, f);  // (out of range after all: the same values back)
@@ -549,16 +549,13 @@ __device__ __forceinline__ void thermal_cell_from(
 #pragma unroll
             for (int q = 0; q < Q19; q++) L[q] = fix61_load(f[q]);
             if (FIRST) {
-                ok = fix61_flow<true>(L, K.pk.fix, FixNoForce(), mrho[cell], mu[cell], mv[cell],
+                ok = fix61_flow<true>(L, K.pk.fix, 0, 0, 0, mrho[cell], mu[cell], mv[cell],
                                       mw[cell], fl);
             } else {
-                auto carried = [&](FixD, long long (&h)[3]) {
-                    const double s = 0.5 * FIX_ONE;
-                    h[0] = ROT ? __double2ll_rn(fxp * s) : 0;
-                    h[1] = ROT ? __double2ll_rn(fyp * s) : 0;
-                    h[2] = __double2ll_rn(fzp * s);
-                };
-                ok = fix61_flow<false>(L, K.pk.fix, carried, 0.0, 0.0, 0.0, 0.0, fl);
+                const double h = 0.5 * FIX_ONE;
+                ok = fix61_flow<false>(L, K.pk.fix, ROT ? __double2ll_rn(fxp * h) : 0,
+                                       ROT ? __double2ll_rn(fyp * h) : 0, __double2ll_rn(fzp * h),
+                                       0.0, 0.0, 0.0, 0.0, fl);
             }
         }
         if (ok) {
