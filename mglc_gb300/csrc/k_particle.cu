@@ -298,8 +298,11 @@ __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : MGLC_
             cacc[1] = m;
         }
         const IDX sy = nx, sz = (IDX)nx * ny;
-        if (i > 0 && i < nx - 1 && j > 0 && j < ny - 1 && k > 0 && k < nz - 1) {
-            // interior node: every population streams, no wrap
+        // asked of the warp's fluid nodes together: apart, a row's two end warps
+        // would store twice
+        const bool edge = i == 0 || i == nx - 1 || j == 0 || j == ny - 1 || k == 0 || k == nz - 1;
+        if (!__any_sync(__activemask(), edge)) {
+            // every population streams, no wrap
 #pragma unroll
             for (int q = 0; q < Q19; q++)
                 fout[q * P + cell + (IDX)ex19(q) + (IDX)ey19(q) * sy + (IDX)ez19(q) * sz] = (S)f[q];
@@ -309,12 +312,11 @@ __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : MGLC_
                 const int dx = ex19(q), dy = ey19(q), dz = ez19(q);
                 const int jj = j + dy, kk = k + dz, ir = i + dx;
                 const bool xwall = !p.periodic_x && (ir < 0 || ir >= nx);
-                if (xwall || jj < 0 || jj >= ny || kk < 0 || kk >= nz) {
-                    fout[opp19(q) * P + cell] = (S)f[q];  // no-slip wall
-                } else {
-                    const int ii = wrapx(ir, nx);
-                    fout[q * P + ((IDX)ii + sy * jj + sz * kk)] = (S)f[q];
-                }
+                const bool wall = xwall || jj < 0 || jj >= ny || kk < 0 || kk >= nz;
+                // no-slip wall: back into the node's opposite slot
+                const IDX to = wall ? opp19(q) * P + cell
+                                    : q * P + ((IDX)wrapx(ir, nx) + sy * jj + sz * kk);
+                fout[to] = (S)f[q];
             }
         }
     }
