@@ -73,6 +73,14 @@ __device__ __forceinline__ long long rn53(long long v) {
     return (v + (long long)(m >> 1) + (long long)odd) & ~(long long)m;
 }
 
+// the same for v >= 0
+__device__ __forceinline__ long long rn53_pos(long long v) {
+    const int r = max(11 - __clz((int)(v >> 32)), 0);
+    const unsigned m = (1u << r) - 1u;
+    const unsigned odd = (unsigned)(v >> r) & m & 1u;
+    return (v + (long long)(m >> 1) + (long long)odd) & ~(long long)m;
+}
+
 // v * 2^-Q for a v of at most 53 significant bits, with integer operations
 template <int Q>
 __device__ __forceinline__ double fix_out(long long v) {

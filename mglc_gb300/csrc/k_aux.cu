@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "kernels.cuh"
+#include "cell_map.cuh"
 #include "macro64.cuh"
 
 namespace mglc {
@@ -58,23 +59,51 @@ __device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float
 template <typename S, bool THERMAL, bool ORDERED>
 __global__ void __launch_bounds__(256) k_macro(const S* __restrict__ f,
                         const typename GType<S>::T* __restrict__ gt, const void* Fv,
-                        Geom g, double rho0, double inv_scale, double* rho, double* u, double* v,
-                        double* w, double* T) {
+                        Geom g, double rho0, double inv_scale, Fix60K fk, double* rho, double* u,
+                        double* v, double* w, double* T) {
     const long long n = g.plane;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
          c += (long long)gridDim.x * blockDim.x) {
         double r, jx, jy, jz;
+        long long R = 0;
         if constexpr (std::is_same<S, double>::value) {
             double fq[Q19];
 #pragma unroll
             for (int q = 0; q < Q19; q++) fq[q] = f[q * n + c];
-            macro_sums(fq, r, jx, jy, jz);
+            macro_sums<!THERMAL>(fq, r, jx, jy, jz, R);
         } else {
             float fq[Q19];
 #pragma unroll
             for (int q = 0; q < Q19; q++) fq[q] = to_f(f[q * n + c]);
-            if (ORDERED) macro_sums_ordered(fq, inv_scale, rho0, r, jx, jy, jz);
-            else macro_sums(fq, (float)inv_scale, rho0, r, jx, jy, jz);
+            if constexpr (!ORDERED) {
+                float F[3] = {0.0f, 0.0f, 0.0f}, gq[Q7];
+                if (THERMAL) {
+#pragma unroll
+                    for (int a = 0; a < 3; a++) F[a] = ((const float*)Fv)[a * n + c];
+#pragma unroll
+                    for (int q = 0; q < Q7; q++) gq[q] = gt[q * n + c];
+                }
+                long long r60, j[3], t60 = 0;
+                bool ok = fix60_sums(fq, fk, r60, j);
+                if (THERMAL) {
+                    int worst = 0, hot = 0;
+#pragma unroll
+                    for (int a = 0; a < 3; a++) j[a] += fix60_load<124>(F[a], -1, worst);
+#pragma unroll
+                    for (int q = 0; q < Q7; q++) t60 += fix60_load<127>(gq[q], 0, hot);
+                    ok = ok && worst < 124 && hot < 127;  // forces below 1/4, g below 1
+                }
+                if (ok && fix60_flow(r60, j)) {
+                    const FixD y = fix_dig(fix_recip(2 * r60, fix_dig(2 * r60)));
+                    rho[c] = fix61_store_any<60>(r60);
+                    u[c] = fix61_store_any<60>(fix_mul<60>(fix_dig(j[0]), y));
+                    v[c] = fix61_store_any<60>(fix_mul<60>(fix_dig(j[1]), y));
+                    w[c] = fix61_store_any<60>(fix_mul<60>(fix_dig(j[2]), y));
+                    if (THERMAL) T[c] = fix61_store_any<60>(t60);
+                    continue;
+                }
+            }
+            macro_sums_ordered(fq, inv_scale, rho0, r, jx, jy, jz);
         }
         if (THERMAL) {
             double Fx, Fy, Fz;
@@ -95,7 +124,7 @@ __global__ void __launch_bounds__(256) k_macro(const S* __restrict__ f,
         }
         rho[c] = r;
         double uu, vv, ww;
-        div_by(jx, jy, jz, r, uu, vv, ww);
+        div_by(jx, jy, jz, r, uu, vv, ww, R);
         u[c] = uu;
         v[c] = vv;
         w[c] = ww;
@@ -116,14 +145,15 @@ static cudaError_t macro_go(bool thermal, const Geom& g, const void* f, const vo
     int gr = grid_for(g.plane, 256);
     using G = typename GType<S>::T;
     constexpr bool kRed = !std::is_same<S, double>::value;
+    const Fix60K fk = make_fix60(rho0, inv);
     if (thermal && ordered && kRed)
-        k_macro<S, true, kRed><<<gr, 256, 0, s>>>((const S*)f, (const G*)gt, F, g, rho0, inv, rho, u, v, w, T);
+        k_macro<S, true, kRed><<<gr, 256, 0, s>>>((const S*)f, (const G*)gt, F, g, rho0, inv, fk, rho, u, v, w, T);
     else if (thermal)
-        k_macro<S, true, false><<<gr, 256, 0, s>>>((const S*)f, (const G*)gt, F, g, rho0, inv, rho, u, v, w, T);
+        k_macro<S, true, false><<<gr, 256, 0, s>>>((const S*)f, (const G*)gt, F, g, rho0, inv, fk, rho, u, v, w, T);
     else if (ordered && kRed)
-        k_macro<S, false, kRed><<<gr, 256, 0, s>>>((const S*)f, nullptr, nullptr, g, rho0, inv, rho, u, v, w, T);
+        k_macro<S, false, kRed><<<gr, 256, 0, s>>>((const S*)f, nullptr, nullptr, g, rho0, inv, fk, rho, u, v, w, T);
     else
-        k_macro<S, false, false><<<gr, 256, 0, s>>>((const S*)f, nullptr, nullptr, g, rho0, inv, rho, u, v, w, T);
+        k_macro<S, false, false><<<gr, 256, 0, s>>>((const S*)f, nullptr, nullptr, g, rho0, inv, fk, rho, u, v, w, T);
     return cudaGetLastError();
 }
 
@@ -317,22 +347,24 @@ __global__ void __launch_bounds__(RED_BLOCK)
     block_sum<4>(acc, partials + 4 * blockIdx.x);
 }
 
+// one warp per value: each lane sums a strided subset in order, eight loads in
+// flight, then a fixed tree (one warp for all, a load at a time: 16 us for 1216
+// blocks)
 template <int NV>
 __global__ void k_finish(int nblocks, const double* partials, double* out) {
-    // one warp: each lane sums a strided subset in order, then a fixed tree
-    double acc[NV];
+    const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    double acc = 0.0;
+    for (int b0 = lane; b0 < nblocks; b0 += 8 * 32) {
+        double x[8];
 #pragma unroll
-    for (int k = 0; k < NV; k++) acc[k] = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += 32)
+        for (int q = 0; q < 8; q++) x[q] = b0 + 32 * q < nblocks ? partials[NV * (b0 + 32 * q) + k] : 0.0;
 #pragma unroll
-        for (int k = 0; k < NV; k++) acc[k] += partials[NV * b + k];
+        for (int q = 0; q < 8; q++)
+            if (b0 + 32 * q < nblocks) acc += x[q];
+    }
 #pragma unroll
-    for (int k = 0; k < NV; k++)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], o);
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < NV; k++) out[k] = acc[k];
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) out[k] = acc;
 }
 
 cudaError_t launch_residual(long long n, const double* u, const double* v, const double* w,
@@ -340,7 +372,7 @@ cudaError_t launch_residual(long long n, const double* u, const double* v, const
                             bool with_w, double* partials, double* out4, cudaStream_t s) {
     int nb = reduce_blocks(n);
     k_residual<<<nb, RED_BLOCK, 0, s>>>(n, u, v, w, T, up, vp, wp, Tp, with_w, partials);
-    k_finish<4><<<1, 32, 0, s>>>(nb, partials, out4);
+    k_finish<4><<<1, 4 * 32, 0, s>>>(nb, partials, out4);
     return cudaGetLastError();
 }
 
@@ -363,7 +395,7 @@ cudaError_t launch_totals(long long n, const double* rho, const double* u, const
                           cudaStream_t s) {
     int nb = reduce_blocks(n);
     k_totals<<<nb, RED_BLOCK, 0, s>>>(n, rho, u, v, w, T, partials);
-    k_finish<3><<<1, 32, 0, s>>>(nb, partials, out3);
+    k_finish<3><<<1, 3 * 32, 0, s>>>(nb, partials, out3);
     return cudaGetLastError();
 }
 
@@ -371,8 +403,8 @@ cudaError_t launch_totals(long long n, const double* rho, const double* u, const
 // hot/cold wall Nusselt numbers.  The wall sits half a cell outside the first
 // node, so dT/dn|wall = (9 T_1 - T_2 - 8 T_wall)/3 (second order).
 __global__ void __launch_bounds__(RED_BLOCK)
-    k_thermal_stats(Geom g, const double* u, const double* v, const double* w, const double* T,
-                    int wall_axis, double* partials) {
+    k_thermal_stats(Geom g, DivBy byx, DivBy byy, const double* u, const double* v, const double* w,
+                    const double* T, int wall_axis, double* partials) {
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     const long long n = g.plane;
     const long long sxy = (long long)g.nx * g.ny;
@@ -382,13 +414,18 @@ __global__ void __launch_bounds__(RED_BLOCK)
         acc[0] += ww * t;
         acc[1] += uu * uu + vv * vv + ww * ww;
         if (wall_axis == 1) {
-            const int j = (int)((c / g.nx) % g.ny);
+            int j;  // by multiplication below 2^31 cells (64-bit divisions: 54 us for 128^3)
+            if (n < (1LL << 31)) {
+                const unsigned row = byx((unsigned)c);
+                j = (int)(row - byy(row) * (unsigned)g.ny);
+            } else {
+                j = (int)((c / g.nx) % g.ny);
+            }
             if (j == 0) acc[2] += 9.0 * t - T[c + g.nx];
             if (j == g.ny - 1) acc[3] += 9.0 * t - T[c - g.nx];
         } else if (wall_axis == 2) {
-            const long long k = c / sxy;
-            if (k == 0) acc[2] += 9.0 * t - T[c + sxy];
-            if (k == g.nz - 1) acc[3] += 9.0 * t - T[c - sxy];
+            if (c < sxy) acc[2] += 9.0 * t - T[c + sxy];
+            if (c >= n - sxy) acc[3] += 9.0 * t - T[c - sxy];
         }
     }
     block_sum<4>(acc, partials + 4 * blockIdx.x);
@@ -398,8 +435,8 @@ cudaError_t launch_thermal_stats(const Geom& g, const double* u, const double* v
                                  const double* T, int wall_axis, double* partials, double* out4,
                                  cudaStream_t s) {
     int nb = reduce_blocks(g.plane);
-    k_thermal_stats<<<nb, RED_BLOCK, 0, s>>>(g, u, v, w, T, wall_axis, partials);
-    k_finish<4><<<1, 32, 0, s>>>(nb, partials, out4);
+    k_thermal_stats<<<nb, RED_BLOCK, 0, s>>>(g, make_div(g.nx), make_div(g.ny), u, v, w, T, wall_axis, partials);
+    k_finish<4><<<1, 4 * 32, 0, s>>>(nb, partials, out4);
     return cudaGetLastError();
 }
 

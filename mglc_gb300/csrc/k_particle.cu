@@ -187,7 +187,8 @@ __device__ __forceinline__ bool fix58_ok(const double (&f)[Q19]) {
            (unsigned)__double2hiint(f[0]) - 0x3F900000u < 0x00500000u;     // below 1/2
 }
 __device__ __forceinline__ void fix58_moments(const double (&f)[Q19], MrtMom<double>& o,
-                                              double& rho, double& jx, double& jy, double& jz) {
+                                              double& rho, double& jx, double& jy, double& jz,
+                                              long long& R) {
     Fix58 F[Q19];
 #pragma unroll
     for (int q = 0; q < Q19; q++) F[q].v = fix61_load(f[q]) >> 3;  // exact
@@ -221,6 +222,7 @@ __device__ __forceinline__ void fix58_moments(const double (&f)[Q19], MrtMom<dou
     o.m17 = fix_out<58>(rn53(-b45.v + a89.v));
     o.m18 = fix_out<58>((b67 - b89).v);
     rho = fix_out<58>(r.v);
+    R = r.v < (11LL << 56) ? r.v << 3 : 0;  // in units of 2^-61
     jx = fix_out<58>(x.v);
     jy = fix_out<58>(y.v);
     jz = fix_out<58>(z.v);
@@ -234,15 +236,16 @@ __device__ __forceinline__ void pcollide(double (&f)[Q19], const PBulkK<double>&
         m = mrt_moments(f);
     } else {
         double jx, jy, jz;
+        long long R = 0;
         if (fix58_ok(f)) {
-            fix58_moments(f, m, rho, jx, jy, jz);
+            fix58_moments(f, m, rho, jx, jy, jz, R);
         } else {
             moments0(f, rho, jx, jy, jz);
             m = mrt_moments(f);
         }
         // u = (sum f e + F/2)/rho with F = rho*a (thermal macro form)
         div_by(jx + 0.5 * (rho * k.ax), jy + 0.5 * (rho * k.ay), jz + 0.5 * (rho * k.az), rho, ux,
-               uy, uz);
+               uy, uz, R);
     }
     mrt_relax<double, true, false>(f, m, rho, rho, ux, uy, uz, rho * k.ax, rho * k.ay, rho * k.az,
                                    k.cd);
@@ -1419,7 +1422,7 @@ __global__ void k_pcount(const int* owner, long long n, long long* out) {
 }
 
 template <typename S>
-__global__ void k_pmacro(const S* f, const int* owner, PartParams p, bool first, double* rho,
+__global__ void k_pmacro(const S* f, const int* owner, PartParams p, Fix60K fk, bool first, double* rho,
                          double* u, double* v, double* w) {
     const long long P = (long long)p.nx * p.ny * p.nz;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < P;
@@ -1438,10 +1441,24 @@ __global__ void k_pmacro(const S* f, const int* owner, PartParams p, bool first,
         typename PC<S>::C fq[Q19];
 #pragma unroll
         for (int q = 0; q < Q19; q++) fq[q] = f[q * P + c];
-        if constexpr (PSt<S>::SHIFT) macro_sums(fq, 1.0f, p.rho0, r, jx, jy, jz);
-        else macro_sums(fq, r, jx, jy, jz);
+        long long R = 0;
+        if constexpr (PSt<S>::SHIFT) {
+            long long j[3];
+            if (fix60_sums(fq, fk, R, j)) {
+                r = fix61_store_any<60>(R);
+                jx = fix61_store_any<60>(j[0]);
+                jy = fix61_store_any<60>(j[1]);
+                jz = fix61_store_any<60>(j[2]);
+                R *= 2;
+            } else {
+                macro_sums_ordered(fq, 1.0, p.rho0, r, jx, jy, jz);
+                R = 0;
+            }
+        } else {
+            macro_sums<false>(fq, r, jx, jy, jz, R);
+        }
         div_by(jx + 0.5 * (r * p.body_force[0]), jy + 0.5 * (r * p.body_force[1]),
-               jz + 0.5 * (r * p.body_force[2]), r, uu, vv, ww);
+               jz + 0.5 * (r * p.body_force[2]), r, uu, vv, ww, R);
         rho[c] = r;
         u[c] = uu;
         v[c] = vv;
@@ -1529,9 +1546,9 @@ cudaError_t launch_particle_macro(int form, bool first, const void* f, const Par
     const long long n = (long long)p.nx * p.ny * p.nz;
     int gb = (int)std::min<long long>((n + 255) / 256, 152 * 16);
     if (form == FORM_FP64)
-        k_pmacro<double><<<gb, 256, 0, s>>>((const double*)f, d.owner_cur, p, first, rho, u, v, w);
+        k_pmacro<double><<<gb, 256, 0, s>>>((const double*)f, d.owner_cur, p, make_fix60(p.rho0, 1.0), first, rho, u, v, w);
     else
-        k_pmacro<float><<<gb, 256, 0, s>>>((const float*)f, d.owner_cur, p, first, rho, u, v, w);
+        k_pmacro<float><<<gb, 256, 0, s>>>((const float*)f, d.owner_cur, p, make_fix60(p.rho0, 1.0), first, rho, u, v, w);
     return cudaGetLastError();
 }
 

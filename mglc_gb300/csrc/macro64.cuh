@@ -8,11 +8,19 @@
 //    addition has to round as FP64's; with the populations exact in units of
 //    2^-61 (fix61.cuh) an addition is an integer one followed by the rounding
 //    of the sum to 53 significant bits, to nearest even.
-//  * reduced forms: the stored deviations are summed in pairs of FP32 values
-//    (Knuth's TwoSum), good to 2^-45 of the largest, below the rounding of the
-//    FP64 sum with w rho0; scale and rho0 come in at the end.
-//  * the three quotients by rho share one reciprocal (div_by).
+//  * reduced forms: the stored deviations, rho0, half the force and the
+//    temperature populations are summed in units of 2^-60, exactly but for what
+//    lies below 2^-60, and the velocity is a product with the integer reciprocal,
+//    to 2^-61: closer to the exact quotient of the stored values than the FP64
+//    sums with w rho0, which round at 2^-54.  Four conversions a cell remain of
+//    33 FP64 instructions.
+//  * FP64 storage: the three quotients by rho share one reciprocal, taken from
+//    integers where the density is one (div_by).
+// FP16 256^3 1028 -> 479 us (174 are its bytes), FP32 97x63x129 60 -> 29, heated and
+// rotating 81x97x72 67 -> 29.
 #pragma once
+#include <cmath>
+
 #include "d2q9.cuh"
 #include "fix61.cuh"
 
@@ -37,22 +45,35 @@ __device__ __forceinline__ void sums_fp64(const double (&f)[Q19], double& r, dou
 
 // sum f and sum f e in the order of the populations, each addition rounded as
 // FP64 rounds it
+// (R: the density times 2^61, 0 where the sums ran in FP64).  Z64: the z momentum on
+// the FP64 unit, which the lid's kernel leaves idle otherwise (256^3 with a 134 MB
+// copy: 800 us so, 918 all on integers, 850 with the quotients there instead; heated
+// 128^3, with sums of its own: 145 without).
+template <bool Z64>
 __device__ __forceinline__ void macro_sums(const double (&f)[Q19], double& r, double& jx,
-                                           double& jy, double& jz) {
+                                           double& jy, double& jz, long long& R) {
+    R = 0;
     if (fix61_ok(f)) {
-        long long R = 0, J[3] = {0, 0, 0};
+        long long J[3] = {0, 0, 0};
 #pragma unroll
         for (int q = 0; q < Q19; q++) {
             const long long F = fix61_load(f[q]);
-            R = q ? rn53(R + F) : F;
+            R = q ? rn53_pos(R + F) : F;
             if (ex19(q)) J[0] = rn53(ex19(q) > 0 ? J[0] + F : J[0] - F);
             if (ey19(q)) J[1] = rn53(ey19(q) > 0 ? J[1] + F : J[1] - F);
-            if (ez19(q)) J[2] = rn53(ez19(q) > 0 ? J[2] + F : J[2] - F);
+            if (!Z64 && ez19(q)) J[2] = rn53(ez19(q) > 0 ? J[2] + F : J[2] - F);
         }
-        r = fix61_store_any(R);
-        jx = fix61_store_any(J[0]);
-        jy = fix61_store_any(J[1]);
-        jz = fix61_store_any(J[2]);
+        r = fix_out<61>(R);
+        jx = fix_out<61>(J[0]);
+        jy = fix_out<61>(J[1]);
+        if (Z64) {
+            jz = f[5];
+#pragma unroll
+            for (int q = 6; q < Q19; q++)
+                if (ez19(q)) jz = __dadd_rn(jz, ez19(q) * f[q]);
+        } else {
+            jz = fix_out<61>(J[2]);
+        }
         return;
     }
     sums_fp64(f, r, jx, jy, jz);
@@ -73,38 +94,82 @@ __device__ __forceinline__ void two_sum(float& h, float& l, float x) {
     l += (h - (s - b)) + (x - b);
     h = s;
 }
-// the same sums of stored deviations f = (f_abs - w rho0) / inv (inv a power of
-// two); not finite or huge: in FP64 as the populations would be
-__device__ __forceinline__ void macro_sums(const float (&f)[Q19], float inv, double rho0,
-                                           double& r, double& jx, double& jy, double& jz) {
-    float h = f[0], l = 0.0f, H[3] = {f[1], f[3], f[5]}, L[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int q = 1; q < Q19; q++) {
-        two_sum(h, l, f[q]);
-        if (ex19(q) && q != 1) two_sum(H[0], L[0], ex19(q) > 0 ? f[q] : -f[q]);
-        if (ey19(q) && q != 3) two_sum(H[1], L[1], ey19(q) > 0 ? f[q] : -f[q]);
-        if (ez19(q) && q != 5) two_sum(H[2], L[2], ez19(q) > 0 ? f[q] : -f[q]);
-    }
-    const float big = fabsf(h) + fabsf(H[0]) + fabsf(H[1]) + fabsf(H[2]);
-    if (big < 1e30f) {
-        const double s = (double)inv;
-        r = fma((double)h + (double)l, s, rho0);
-        jx = ((double)H[0] + (double)L[0]) * s;
-        jy = ((double)H[1] + (double)L[1]) * s;
-        jz = ((double)H[2] + (double)L[2]) * s;
-        return;
-    }
-    macro_sums_ordered(f, (double)inv, rho0, r, jx, jy, jz);
+// x 2^e2 in units of 2^-60, cut towards zero, for |x| 2^e2 < 2^(L - 127); `worst` takes
+// the exponent field, above L - 1 where x is out of range (infinities and NaN too)
+template <int L>
+__device__ __forceinline__ long long fix60_load(float x, int e2, int& worst) {
+    const int b = __float_as_int(x);
+    const int e = ((b >> 23) & 0xff) + e2;
+    // (a subnormal, taken for a normal of the least exponent, is below 2^-60 too)
+    worst = max(worst, ((b >> 23) & 0xff) == 0xff ? 0x7fff : e);
+    const unsigned m = ((unsigned)b & 0x7fffffu) | 0x800000u;
+    // the significand at the place of exponent L - 1, then down
+    constexpr int TOP = L - 1 - 150 + 60;
+    const long long v = (long long)(((unsigned long long)m << TOP) >> min(max(L - 1 - e, 0), 63));
+    const long long sg = b >> 31;
+    return (v ^ sg) - sg;
 }
 
-// a/r, b/r and c/r, correctly rounded (div_pair, d2q9.cuh)
+// Scale, rho0 and range of the reduced forms' sums; on: rho0 in [0, 4) and a
+// power-of-two scale.
+struct Fix60K {
+    int on, e2;
+    long long rho0;
+};
+inline Fix60K make_fix60(double rho0, double inv) {
+    Fix60K k{};
+    int e = 0;
+    const bool pow2 = inv > 0.0 && std::frexp(inv, &e) == 0.5;
+    k.on = pow2 && e > -60 && e < 60 && rho0 >= 0.0 && rho0 < 4.0;
+    k.e2 = e - 1;
+    if (k.on) k.rho0 = std::llrint(std::ldexp(rho0, 60));
+    return k;
+}
+
+// rho and the momenta of stored deviations (units of 2^-60); false: a population of
+// 1/8 or more (19 of them and rho0 stay below 8), or not finite
+__device__ __forceinline__ bool fix60_sums(const float (&f)[Q19], const Fix60K& k, long long& r,
+                                           long long (&j)[3]) {
+    int worst = 0;
+    r = k.rho0;
+    j[0] = j[1] = j[2] = 0;
+#pragma unroll
+    for (int q = 0; q < Q19; q++) {
+        const long long v = fix60_load<124>(f[q], k.e2, worst);
+        r += v;
+        if (ex19(q)) j[0] = ex19(q) > 0 ? j[0] + v : j[0] - v;
+        if (ey19(q)) j[1] = ey19(q) > 0 ? j[1] + v : j[1] - v;
+        if (ez19(q)) j[2] = ez19(q) > 0 ? j[2] + v : j[2] - v;
+    }
+    return k.on && worst < 124;
+}
+// rho (units of 2^-60) has an integer reciprocal and the momenta are below it
+__device__ __forceinline__ bool fix60_flow(long long r, const long long (&j)[3]) {
+    return r >= (1LL << 58) && r < (11LL << 58) && j[0] < r && -j[0] < r && j[1] < r && -j[1] < r &&
+           j[2] < r && -j[2] < r;
+}
+
+// 1/r, correctly rounded, for r of significand not all ones (den_ok) and R = r 2^61 in
+// [2^59, 11 2^59): the integer reciprocal, rounded, and one Newton step
+__device__ __forceinline__ double recip_of(long long R, double r) {
+    const double y = fix_out<60>(rn53(fix_recip(R, fix_dig(R))));
+    return __fma_rn(__fma_rn(-r, y, 1.0), y, y);
+}
+
+// a/r, b/r and c/r, correctly rounded (div_pair, d2q9.cuh); R: r 2^61 where it is known
+// as an integer, else 0
 __device__ __forceinline__ void div_by(double a, double b, double c, double r, double& qa,
-                                       double& qb, double& qc) {
+                                       double& qb, double& qc, long long R = 0) {
     if (den_ok(r) && mid_or_pzero(a) && mid_or_pzero(b) && mid_or_pzero(c)) {
-        double y = (double)__frcp_rn((float)r);
-        y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
-        y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
-        y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
+        double y;
+        if (R >= (1LL << 59) && R < (11LL << 59)) {
+            y = recip_of(R, r);
+        } else {
+            y = (double)__frcp_rn((float)r);
+            y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
+            y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
+            y = __fma_rn(__fma_rn(-r, y, 1.0), y, y);
+        }
         const double ta = __dmul_rn(a, y), tb = __dmul_rn(b, y), tc = __dmul_rn(c, y);
         qa = __fma_rn(__fma_rn(-r, ta, a), y, ta);
         qb = __fma_rn(__fma_rn(-r, tb, b), y, tb);
