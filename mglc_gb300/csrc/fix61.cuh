@@ -14,8 +14,8 @@
 // on the way (tests/test_fix61_host.py; velocity error after six steps of 384^3
 // 2.1e-13 against 3.3e-13).  About a thousand integer instructions a lid cell:
 // 384^3 in 3.31 ms a step (17.1 GLUPS, 77% of HBM) against 15.7 ms in FP64;
-// the heated cavity at 128^3, whose temperature populations stay in FP64, in 234 us
-// (9.0 GLUPS) against 813.
+// the heated cavity at 128^3, temperature populations alike (fix_heat; 235 with those
+// in FP64), in 205 us (10.2 GLUPS) against 813.
 // Cells outside its range (a population outside [2^-8, 1/8), the rest
 // population outside [1/8, 1/2), negative and non-finite ones among them, rho
 // below 1/4 or a velocity component of 1/2 or more) take the FP64 form; inside,
@@ -145,8 +145,8 @@ __device__ __forceinline__ void fix_pair(long long* F, int a, int b, const FixK&
 // others with integer operations (all on the FP64 unit when one is below 2^-8 or
 // negative, which is rare): the lid kernels, which need that unit for nothing
 // else, run best with 10 (3309 us a step at 384^3; 3456 with none, 3326 with all),
-// the heated ones, whose temperature part runs on it, with none (234 us at 128^3;
-// 238 with 6)
+// the heated ones, which store their temperature populations through it too, with 5
+// (205 us at 128^3; 208 with none, 209 with 10)
 template <int NFP>
 __device__ __forceinline__ void fix61_store_all(const long long (&F)[Q19], double (&f)[Q19]) {
     int least = 0x7fffffff;
@@ -281,6 +281,43 @@ __device__ __forceinline__ void fix61_collide(long long (&F)[Q19], const FixK& k
     fix_pair(F, 13, 12, k, bxz - cxz, ox - oz);
     fix_pair(F, 15, 18, k, byz + cyz, oy + oz);
     fix_pair(F, 17, 16, k, byz - cyz, oy - oz);
+}
+
+// The temperature part.  Its populations are of either sign and down to zero: below
+// 2^-9 loading rounds them to 2^-61, which is less than the rounding that an FP64
+// step leaves in their neighbours (2^-56 for populations of 1/10).
+// Every |g| below 1/2?
+__device__ __forceinline__ bool fix_heat_ok(const double (&g)[Q7]) {
+    unsigned worst = 0;
+#pragma unroll
+    for (int q = 0; q < Q7; q++) worst = max(worst, (unsigned)__double2hiint(g[q]) & 0x7fffffffu);
+    return worst < 0x3FE00000u;
+}
+// x * 2^61 rounded to nearest, |x| < 1/2
+__device__ __forceinline__ long long fix61_load_any(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int s = min(1023 - (int)((hi >> 20) & 0x7ffu), 63);
+    const unsigned long long m =
+        ((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32 | lo) << 10;
+    const long long v = (long long)(((m >> s) + 1) >> 1), sg = (int)hi >> 31;
+    return (v ^ sg) - sg;
+}
+// D3Q7 collision (pair_collide_t) in place, |T| < 1
+__device__ __forceinline__ void fix_heat(long long (&G)[Q7], long long T, const FixHeatK& k,
+                                         const FixFlow& o) {
+    const FixD t = fix_dig(T);
+    const long long E = fix_mad(t, k.gE, 0);
+    const FixD h = fix_dig(2 * fix_mad(t, k.hd, 0));
+    G[0] = 2 * fix_mad(G[0], k.g1, 2 * fix_mad(t, k.c0, 0));
+    const FixD u[3] = {o.ux, o.uy, o.uz};
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const int q = 2 * a + 1;
+        const long long p = fix_mad(G[q] + G[q + 1], k.g1, E);
+        const long long m = fix_mad(G[q] - G[q + 1], k.g2, fix_mul<63>(h, u[a]));
+        G[q] = p + m;
+        G[q + 1] = p - m;
+    }
 }
 
 }  // namespace mglc

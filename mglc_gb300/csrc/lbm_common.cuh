@@ -543,6 +543,24 @@ inline FixK make_fix_k(double snu, double sq) {
     k.sixth = fix_coef(3074457345618258603LL);
     return k;
 }
+// and of the D3Q7 part: (1-qnu)/2, (1-qd)/2, ge0/4, gE, qd/4 (pair_k_heat)
+struct FixHeatK {
+    FixC g1, g2, c0, gE, hd;
+    int on;
+};
+inline FixHeatK make_fix_heat_k(double qd, double qnu, double ge0, double gE) {
+    FixHeatK k;
+    auto in = [](double s) { return s >= 0x1p-20 && s <= 2.0 - 0x1p-20; };
+    k.on = in(qd) && in(qnu) && ge0 >= 0.0 && ge0 < 2.0 && gE >= 0.0 && gE < 0.5;
+    if (!k.on) return FixHeatK{};
+    const long long half = 1LL << 62;  // 1/4
+    k.g1 = fix_coef(2 * (half - fix_ratio(qnu, 4)));
+    k.g2 = fix_coef(2 * (half - fix_ratio(qd, 4)));
+    k.c0 = fix_coef(fix_ratio(ge0, 4));
+    k.gE = fix_coef(fix_ratio(4.0 * gE, 4));
+    k.hd = fix_coef(fix_ratio(qd, 4));
+    return k;
+}
 // Coefficients, converted once on the host; empty for the other types.
 template <typename T>
 struct PairK {};
@@ -555,6 +573,7 @@ struct PairK<double> {
     FixK fix;                         // the collision on integers (fix61.cuh)
     int box;                          // FX64: a cell outside its range box writes NaN
     double g1, g2, gom, ge0, gE, gd;  // D3Q7: (1-qnu)/2, (1-qd)/2, 1-qnu, its equilibria, qd/2
+    FixHeatK heat;                    // the same on integers
 };
 template <typename T>
 inline PairK<T> make_pair_k(double, double) { return PairK<T>{}; }
@@ -578,6 +597,7 @@ inline void pair_k_heat(PairK<double>& k, double para_a, double qd, double qnu) 
     k.ge0 = qnu * (1.0 - para_a) / 7.0;
     k.gE = 0.5 * qnu * (6.0 + para_a) / 21.0;
     k.gd = 0.5 * qd;
+    k.heat = make_fix_heat_k(qd, qnu, k.ge0, k.gE);
 }
 template <typename T>
 inline void pair_k_heat(PairK<T>&, double, double, double) {}

@@ -177,11 +177,10 @@ struct LidMinBlocks {
     static constexpr int value = std::is_same<S, double>::value ? 5 : 0;
 };
 
-// and for the heated cavity's (128^3 FP64: 234 us a step at 5, 251 at 4, 246 at 3,
-// 253 at 6)
+// and for the heated cavity's (128^3 FP64: 205 us a step at 4, 211 at 3, 234 at 5)
 template <typename S>
 struct ThermalMinBlocks {
-    static constexpr int value = std::is_same<S, double>::value ? 5 : 0;
+    static constexpr int value = std::is_same<S, double>::value ? 4 : 0;
 };
 
 // Scalar constants converted once on the host to the arithmetic type.
@@ -544,12 +543,23 @@ __device__ __forceinline__ void thermal_cell_from(
         if (!oob(fz_off + cell, fz_off + P)) F[fz_off + cell] = fz;
     };
     if constexpr (std::is_same<S, double>::value) {
-        // flow: in range on the integer pipe (fix61.cuh), else the FP64 pair form;
-        // the temperature populations, of either sign and down to zero, in FP64
+        // in range on the integer pipe (fix61.cuh), else the FP64 pair forms
         constexpr int FO = ROT ? 2 : 1;
         const double small = 0.125;
-        double temp = FIRST ? mT[cell]
-                            : ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
+        double temp;
+        long long G[Q7], T = 0;
+        bool hot = !FIRST && K.pk.heat.on && fix_heat_ok(g);
+        if (hot) {
+#pragma unroll
+            for (int q = 0; q < Q7; q++) {
+                G[q] = fix61_load_any(g[q]);
+                T += G[q];
+            }
+            hot = T < (1LL << 61) && -T < (1LL << 61);
+            temp = fix61_store_any(T);
+        } else {
+            temp = FIRST ? mT[cell] : ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
+        }
         double rho, ux, uy, uz, fx, fy, fz;
         bool ok = K.pk.fix.on && fix61_ok(f) && fabs(fxp) < small && fabs(fyp) < small &&
                   fabs(fzp) < small, bad = false;
@@ -570,9 +580,13 @@ __device__ __forceinline__ void thermal_cell_from(
         }
         if (ok) {
             rho = fix61_store_any(fl.r);
-            ux = FIRST ? mu[cell] : fix61_store_any<63>(join(fl.ux));
-            uy = FIRST ? mv[cell] : fix61_store_any<63>(join(fl.uy));
-            uz = FIRST ? mw[cell] : fix61_store_any<63>(join(fl.uz));
+            if (FIRST || ROT || K.pk.box || !hot) {
+                ux = FIRST ? mu[cell] : fix61_store_any<63>(join(fl.ux));
+                uy = FIRST ? mv[cell] : fix61_store_any<63>(join(fl.uy));
+                uz = FIRST ? mw[cell] : fix61_store_any<63>(join(fl.uz));
+            } else {
+                ux = uy = uz = 0.0;  // used as integers only
+            }
         } else if (FIRST) {
             rho = mrho[cell];
             ux = mu[cell];
@@ -591,12 +605,17 @@ __device__ __forceinline__ void thermal_cell_from(
             fix61_collide<false, FO, FIRST, true>(
                 L, K.pk.fix, fl, ROT ? __double2ll_rn(fx * FIX_ONE) : 0,
                 ROT ? __double2ll_rn(fy * FIX_ONE) : 0, __double2ll_rn(fz * FIX_ONE));
-            fix61_store_all<0>(L, f);
+            fix61_store_all<5>(L, f);
         } else {
 #pragma unroll
             for (int q = 0; q < Q19; q++) bad |= !(fabs(f[q]) < 1.0);
             double rf, jx, jy, jz;
             moments0(f, rf, jx, jy, jz);
+            if (!FIRST && ok) {  // (a force of 1/8 or more)
+                ux = fix61_store_any<63>(join(fl.ux));
+                uy = fix61_store_any<63>(join(fl.uy));
+                uz = fix61_store_any<63>(join(fl.uz));
+            }
             if (FIRST) {
                 // rho, u from the macro arrays: the odd term is e.(2 (j - rho u) + F)/10
                 // and the density projection goes back in (trt_collide_forced)
@@ -615,7 +634,11 @@ __device__ __forceinline__ void thermal_cell_from(
             for (int q = 0; q < Q7; q++) bad |= !(fabs(g[q]) < 2.0);
             bad = bad || !(fabs(temp) < 2.0) || out_of_box(rho, ux, uy, uz);
         }
-        if (FIRST) {
+        if (ok && hot) {
+            fix_heat(G, T, K.pk.heat, fl);
+#pragma unroll
+            for (int q = 0; q < Q7; q++) g[q] = fix61_store_any(G[q]);
+        } else if (FIRST) {
             const double sg = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
             trt_collide_t<C, true>(g, temp, ux, uy, uz, K.para_a, K.qd, K.qnu, sg - temp);
         } else {
