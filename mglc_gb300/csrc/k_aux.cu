@@ -8,6 +8,7 @@
 
 #include "kernels.cuh"
 #include "cell_map.cuh"
+#include "launch.cuh"
 #include "macro64.cuh"
 
 namespace mglc {
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(256) k_macro(const S* __restrict__ f,
                         const typename GType<S>::T* __restrict__ gt, const void* Fv,
                         Geom g, double rho0, double inv_scale, Fix60K fk, double* rho, double* u,
                         double* v, double* w, double* T) {
+    after_previous();
     const long long n = g.plane;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n;
          c += (long long)gridDim.x * blockDim.x) {
@@ -147,13 +149,13 @@ static cudaError_t macro_go(bool thermal, const Geom& g, const void* f, const vo
     constexpr bool kRed = !std::is_same<S, double>::value;
     const Fix60K fk = make_fix60(rho0, inv);
     if (thermal && ordered && kRed)
-        k_macro<S, true, kRed><<<gr, 256, 0, s>>>((const S*)f, (const G*)gt, F, g, rho0, inv, fk, rho, u, v, w, T);
+        launch_next(k_macro<S, true, kRed>, gr, 256, 0, s, (const S*)f, (const G*)gt, F, g, rho0, inv, fk, rho, u, v, w, T);
     else if (thermal)
-        k_macro<S, true, false><<<gr, 256, 0, s>>>((const S*)f, (const G*)gt, F, g, rho0, inv, fk, rho, u, v, w, T);
+        launch_next(k_macro<S, true, false>, gr, 256, 0, s, (const S*)f, (const G*)gt, F, g, rho0, inv, fk, rho, u, v, w, T);
     else if (ordered && kRed)
-        k_macro<S, false, kRed><<<gr, 256, 0, s>>>((const S*)f, nullptr, nullptr, g, rho0, inv, fk, rho, u, v, w, T);
+        launch_next(k_macro<S, false, kRed>, gr, 256, 0, s, (const S*)f, nullptr, nullptr, g, rho0, inv, fk, rho, u, v, w, T);
     else
-        k_macro<S, false, false><<<gr, 256, 0, s>>>((const S*)f, nullptr, nullptr, g, rho0, inv, fk, rho, u, v, w, T);
+        launch_next(k_macro<S, false, false>, gr, 256, 0, s, (const S*)f, nullptr, nullptr, g, rho0, inv, fk, rho, u, v, w, T);
     return cudaGetLastError();
 }
 
@@ -327,6 +329,7 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* out) {
 __global__ void __launch_bounds__(RED_BLOCK)
     k_residual(long long n, const double* u, const double* v, const double* w, const double* T,
                double* up, double* vp, double* wp, double* Tp, bool with_w, double* partials) {
+    after_previous();
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (long long c = blockIdx.x * (long long)RED_BLOCK + threadIdx.x; c < n;
          c += (long long)gridDim.x * RED_BLOCK) {
@@ -352,6 +355,7 @@ __global__ void __launch_bounds__(RED_BLOCK)
 // blocks)
 template <int NV>
 __global__ void k_finish(int nblocks, const double* partials, double* out) {
+    after_previous();
     const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
     double acc = 0.0;
     for (int b0 = lane; b0 < nblocks; b0 += 8 * 32) {
@@ -371,14 +375,15 @@ cudaError_t launch_residual(long long n, const double* u, const double* v, const
                             const double* T, double* up, double* vp, double* wp, double* Tp,
                             bool with_w, double* partials, double* out4, cudaStream_t s) {
     int nb = reduce_blocks(n);
-    k_residual<<<nb, RED_BLOCK, 0, s>>>(n, u, v, w, T, up, vp, wp, Tp, with_w, partials);
-    k_finish<4><<<1, 4 * 32, 0, s>>>(nb, partials, out4);
+    launch_next(k_residual, nb, RED_BLOCK, 0, s, n, u, v, w, T, up, vp, wp, Tp, with_w, partials);
+    launch_next(k_finish<4>, 1, 4 * 32, 0, s, nb, partials, out4);
     return cudaGetLastError();
 }
 
 __global__ void __launch_bounds__(RED_BLOCK)
     k_totals(long long n, const double* rho, const double* u, const double* v, const double* w,
              const double* T, double* partials) {
+    after_previous();
     double acc[3] = {0.0, 0.0, 0.0};
     for (long long c = blockIdx.x * (long long)RED_BLOCK + threadIdx.x; c < n;
          c += (long long)gridDim.x * RED_BLOCK) {
@@ -394,8 +399,8 @@ cudaError_t launch_totals(long long n, const double* rho, const double* u, const
                           const double* w, const double* T, double* partials, double* out3,
                           cudaStream_t s) {
     int nb = reduce_blocks(n);
-    k_totals<<<nb, RED_BLOCK, 0, s>>>(n, rho, u, v, w, T, partials);
-    k_finish<3><<<1, 3 * 32, 0, s>>>(nb, partials, out3);
+    launch_next(k_totals, nb, RED_BLOCK, 0, s, n, rho, u, v, w, T, partials);
+    launch_next(k_finish<3>, 1, 3 * 32, 0, s, nb, partials, out3);
     return cudaGetLastError();
 }
 
@@ -405,6 +410,7 @@ cudaError_t launch_totals(long long n, const double* rho, const double* u, const
 __global__ void __launch_bounds__(RED_BLOCK)
     k_thermal_stats(Geom g, DivBy byx, DivBy byy, const double* u, const double* v, const double* w,
                     const double* T, int wall_axis, double* partials) {
+    after_previous();
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     const long long n = g.plane;
     const long long sxy = (long long)g.nx * g.ny;
@@ -435,8 +441,8 @@ cudaError_t launch_thermal_stats(const Geom& g, const double* u, const double* v
                                  const double* T, int wall_axis, double* partials, double* out4,
                                  cudaStream_t s) {
     int nb = reduce_blocks(g.plane);
-    k_thermal_stats<<<nb, RED_BLOCK, 0, s>>>(g, make_div(g.nx), make_div(g.ny), u, v, w, T, wall_axis, partials);
-    k_finish<4><<<1, 4 * 32, 0, s>>>(nb, partials, out4);
+    launch_next(k_thermal_stats, nb, RED_BLOCK, 0, s, g, make_div(g.nx), make_div(g.ny), u, v, w, T, wall_axis, partials);
+    launch_next(k_finish<4>, 1, 4 * 32, 0, s, nb, partials, out4);
     return cudaGetLastError();
 }
 

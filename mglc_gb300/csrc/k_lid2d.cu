@@ -31,6 +31,7 @@
 
 #include "mglc.h"
 #include "d2q9.cuh"
+#include "launch.cuh"
 #include "lid2d.cuh"
 
 namespace mglc {
@@ -84,6 +85,7 @@ __global__ void k_l2_initial(double* __restrict__ f, double* __restrict__ rho,
 
 template <bool FIRST>
 __global__ void __launch_bounds__(128) k_l2_step(L2K k) {
+    after_previous();
     const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (c >= k.n) return;
     const int j = (int)(c / k.nx), i = (int)(c - (long long)j * k.nx);
@@ -121,6 +123,7 @@ __global__ void k_l2_macro(const double* __restrict__ f, const double* __restric
                            const double* __restrict__ su, const double* __restrict__ sv,
                            int stored, long long n, double* __restrict__ rho,
                            double* __restrict__ u, double* __restrict__ v) {
+    after_previous();
     const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (c >= n) return;
     double r, uu, vv;
@@ -283,9 +286,9 @@ int l2d_step(L2Ctx* c, int nsteps, std::string& err) {
         k.fin = c->f[c->cur];
         k.fout = c->f[c->cur ^ 1];
         if (c->first_pending)
-            k_l2_step<true><<<blocks_of(c->n), 128, 0, c->s>>>(k);
+            launch_next(k_l2_step<true>, blocks_of(c->n), 128, 0, c->s, k);
         else
-            k_l2_step<false><<<blocks_of(c->n), 128, 0, c->s>>>(k);
+            launch_next(k_l2_step<false>, blocks_of(c->n), 128, 0, c->s, k);
         c->first_pending = false;
         c->cur ^= 1;
         c->itc++;
@@ -307,7 +310,7 @@ int l2d_get_f(L2Ctx* c, double* f, std::string& err) {
 
 namespace {
 int l2_macro_launch(L2Ctx* c, double* rho, double* u, double* v, std::string& err) {
-    k_l2_macro<<<blocks_of(c->n), 128, 0, c->s>>>(c->f[c->cur], c->rho, c->u, c->v,
+    launch_next(k_l2_macro, blocks_of(c->n), 128, 0, c->s, c->f[c->cur], c->rho, c->u, c->v,
                                                    c->first_pending ? 1 : 0, c->n, rho, u, v);
     return ck(cudaGetLastError(), "macro launch", err);
 }

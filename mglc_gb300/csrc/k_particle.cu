@@ -35,6 +35,7 @@
 #include <cmath>
 
 #include "fix61.cuh"
+#include "launch.cuh"
 #include "macro64.cuh"
 #include "particles.cuh"
 
@@ -274,6 +275,7 @@ __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : MGLC_
     k_pbulk(const S* __restrict__ fin, S* __restrict__ fout, const int* __restrict__ owner,
             int* __restrict__ owner_new, PartParams p, PBulkK<typename PC<S>::C> bk,
             double* partials, const int* status) {
+    after_previous();
     using C = typename PC<S>::C;
     if (status[0]) return;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
@@ -355,6 +357,7 @@ constexpr int FINISH_BLOCKS = PSt<S>::SHIFT ? 128 : 32;
 // a fixed shuffle tree (as two launches: 14 + 4 us)
 template <typename S>
 __global__ void __launch_bounds__(256) k_pfinish(PartDev d, int nblocks, double rho0) {
+    after_previous();
     if (d.status[0]) return;
     __shared__ int last;
     constexpr int NB = FINISH_BLOCKS<S>;
@@ -527,6 +530,7 @@ __device__ __forceinline__ long long sq_hi(long long v) {
 template <typename S, bool TILE>
 __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
     k_plinks(S* __restrict__ f, PartParams p, PartDev d) {
+    after_previous();
     using L = typename PC<S>::C;
     if (d.status[0]) return;
     __shared__ LinkCentre<L> s_c;
@@ -1105,6 +1109,7 @@ __device__ bool pmotion(const PartParams& p, const SphereK& sk, const PartDev& d
 // scattered stores).
 template <bool MOVE>
 __global__ void __launch_bounds__(PB) k_pmark(int* owner, PartParams p, SphereK sk, PartDev d) {
+    after_previous();
     if (MOVE && d.status[0]) return;
     const int c = blockIdx.x;
     __shared__ double X[3];
@@ -1172,6 +1177,7 @@ constexpr int PREP_SLAB = PART_NSLAB;
 constexpr int PU = MGLC_PU;
 template <typename S>
 __global__ void __launch_bounds__(PB) k_pphase(const S* __restrict__ f, PartParams p, PartDev d) {
+    after_previous();
     if (d.status[0]) return;
     const int c = blockIdx.x, slab = blockIdx.y;
     if (d.done[1]) {  // a particle went out of range: the state moves and freezes
@@ -1326,6 +1332,7 @@ __device__ void inverse19d(const double* m, double* f) {
 // any of them is written.
 template <typename S>
 __global__ void __launch_bounds__(PB) k_prefill(S* __restrict__ f, PartParams p, PartDev d) {
+    after_previous();
     const int c = blockIdx.x;
     // the particle moves on, with an error too if that came after the motion
     // (status from an earlier step: the values are those of now)
@@ -1424,6 +1431,7 @@ __global__ void k_pcount(const int* owner, long long n, long long* out) {
 template <typename S>
 __global__ void k_pmacro(const S* f, const int* owner, PartParams p, Fix60K fk, bool first, double* rho,
                          double* u, double* v, double* w) {
+    after_previous();
     const long long P = (long long)p.nx * p.ny * p.nz;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < P;
          c += (long long)gridDim.x * blockDim.x) {
@@ -1488,11 +1496,11 @@ static cudaError_t pstep_go(bool first, const void* fin, void* fout, const PartP
     const bool i32 = (long long)p.nx * p.ny * p.nz * (Q19 + 1) < (1LL << 31);
     const S* fi = (const S*)fin;
     S* fo = (S*)fout;
-    if (first && i32) k_pbulk<S, true, int><<<g, b, 0, s>>>(fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
-    else if (first) k_pbulk<S, true, long long><<<g, b, 0, s>>>(fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
-    else if (i32) k_pbulk<S, false, int><<<g, b, 0, s>>>(fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
-    else k_pbulk<S, false, long long><<<g, b, 0, s>>>(fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
-    k_pfinish<S><<<FINISH_BLOCKS<S>, 256, 0, s>>>(d, d.nblocks, p.rho0);
+    if (first && i32) launch_next(k_pbulk<S, true, int>, g, b, 0, s, fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
+    else if (first) launch_next(k_pbulk<S, true, long long>, g, b, 0, s, fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
+    else if (i32) launch_next(k_pbulk<S, false, int>, g, b, 0, s, fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
+    else launch_next(k_pbulk<S, false, long long>, g, b, 0, s, fi, fo, d.owner_cur, d.owner_new, p, bk, d.partials, d.status);
+    launch_next(k_pfinish<S>, FINISH_BLOCKS<S>, 256, 0, s, d, d.nblocks, p.rho0);
     if (p.np > 0) {
         const int bw = 2 * ((int)ceil(p.radius) + 2) + 2;
         const size_t tile = sizeof(int) * (size_t)(bw + 2) * (bw + 2) * ((bw + NSLAB - 1) / NSLAB + 2);
@@ -1509,13 +1517,13 @@ static cudaError_t pstep_go(bool first, const void* fin, void* fout, const PartP
                 if (e != cudaSuccess) return e;
                 opted.fetch_or(bit);
             }
-            k_plinks<S, true><<<dim3(p.np, NSLAB), PB, tile, s>>>((S*)fout, p, d);
+            launch_next(k_plinks<S, true>, dim3(p.np, NSLAB), PB, tile, s, (S*)fout, p, d);
         } else {
-            k_plinks<S, false><<<dim3(p.np, NSLAB), PB, 0, s>>>((S*)fout, p, d);
+            launch_next(k_plinks<S, false>, dim3(p.np, NSLAB), PB, 0, s, (S*)fout, p, d);
         }
-        k_pmark<true><<<p.np, PB, 0, s>>>(d.owner_new, p, sphere_k(p), d);
-        k_pphase<S><<<dim3(p.np, PREP_SLAB), PB, 0, s>>>((const S*)fout, p, d);
-        k_prefill<S><<<p.np, PB, 0, s>>>((S*)fout, p, d);
+        launch_next(k_pmark<true>, p.np, PB, 0, s, d.owner_new, p, sphere_k(p), d);
+        launch_next(k_pphase<S>, dim3(p.np, PREP_SLAB), PB, 0, s, (const S*)fout, p, d);
+        launch_next(k_prefill<S>, p.np, PB, 0, s, (S*)fout, p, d);
     }
     return cudaGetLastError();
 }
@@ -1532,7 +1540,7 @@ cudaError_t launch_particle_init(int form, void* f, const PartParams& p, const P
     const long long n = (long long)p.nx * p.ny * p.nz;
     cudaError_t e = cudaMemsetAsync(d.owner_cur, 0xFF, sizeof(int) * (size_t)n, s);
     if (e != cudaSuccess) return e;
-    if (p.np > 0) k_pmark<false><<<p.np, PB, 0, s>>>(d.owner_cur, p, sphere_k(p), d);
+    if (p.np > 0) launch_next(k_pmark<false>, p.np, PB, 0, s, d.owner_cur, p, sphere_k(p), d);
     int gb = (int)std::min<long long>((n + 255) / 256, 152 * 16);
     if (form == FORM_FP64) k_pinit_f<double><<<gb, 256, 0, s>>>((double*)f, d.owner_cur, p);
     else k_pinit_f<float><<<gb, 256, 0, s>>>((float*)f, d.owner_cur, p);
@@ -1546,9 +1554,9 @@ cudaError_t launch_particle_macro(int form, bool first, const void* f, const Par
     const long long n = (long long)p.nx * p.ny * p.nz;
     int gb = (int)std::min<long long>((n + 255) / 256, 152 * 16);
     if (form == FORM_FP64)
-        k_pmacro<double><<<gb, 256, 0, s>>>((const double*)f, d.owner_cur, p, make_fix60(p.rho0, 1.0), first, rho, u, v, w);
+        launch_next(k_pmacro<double>, gb, 256, 0, s, (const double*)f, d.owner_cur, p, make_fix60(p.rho0, 1.0), first, rho, u, v, w);
     else
-        k_pmacro<float><<<gb, 256, 0, s>>>((const float*)f, d.owner_cur, p, make_fix60(p.rho0, 1.0), first, rho, u, v, w);
+        launch_next(k_pmacro<float>, gb, 256, 0, s, (const float*)f, d.owner_cur, p, make_fix60(p.rho0, 1.0), first, rho, u, v, w);
     return cudaGetLastError();
 }
 

@@ -54,6 +54,7 @@
 
 #include "mglc.h"
 #include "d2q9.cuh"
+#include "launch.cuh"
 #include "particles2d.cuh"
 
 namespace mglc {
@@ -144,6 +145,7 @@ __device__ __forceinline__ void collide_node(const D2& d, int c) {
 // on still holds) are being refilled beside this kernel, and collided there
 template <bool GROUPED>
 __global__ void __launch_bounds__(128) k2_collide(D2 d, bool refilling) {
+    after_previous();
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y;
     if (i > d.p.nx || d.status[0]) return;
     const int c = IX(d, i, j);
@@ -166,6 +168,7 @@ constexpr int r2(int a) { return a == 0 ? 0 : (a <= 4 ? (a + 1) % 4 + 1 : (a - 3
 // reading the populations again (400x800: 26 + 8 + 40 us as three kernels).
 template <bool SHEAR>
 __global__ void __launch_bounds__(128) k2_stream(D2 d) {
+    after_previous();
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y;
     if (i > d.p.nx || d.status[0]) return;
     const int nx = d.p.nx, ny = d.p.ny, c = IX(d, i, j);
@@ -513,6 +516,7 @@ __device__ void chunk_split(int base, int total, const bool (&fc)[EPT], const do
 
 template <class Fetch>
 __global__ void __launch_bounds__(SB) k_gs_part(Fetch fetch, int total, GsBuf b) {
+    after_previous();
     __shared__ double ws[SB / 32];
     __shared__ int wc[SB / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x;
@@ -704,6 +708,7 @@ __device__ __forceinline__ int gs_binade(long long v, int E) {
 // sum to fetch.finish (with every thread of the block)
 template <class Fetch>
 __global__ void __launch_bounds__(SB) k_gs_map(Fetch fetch, int total, int nch, GsBuf b) {
+    after_previous();
     if (fetch.stop()) return;
     __shared__ GsShared sh;
     __shared__ double ws[SB / 32], wall[SB / 32], s_x[GS_PIECES];
@@ -956,8 +961,8 @@ int gs_chunks(long long total) { return (int)((total + CH - 1) / CH) > 0 ? (int)
 template <class Fetch>
 void gs_launch(const Fetch& f, int total, const GsBuf& b, cudaStream_t s) {
     const int nch = gs_chunks(total);
-    k_gs_part<<<nch, SB, 0, s>>>(f, total, b);
-    k_gs_map<<<nch, SB, 0, s>>>(f, total, nch, b);
+    launch_next(k_gs_part<Fetch>, nch, SB, 0, s, f, total, b);
+    launch_next(k_gs_map<Fetch>, nch, SB, 0, s, f, total, nch, b);
 }
 
 // calQ / calQ2 from node (x, y) along direction a towards circle c
@@ -1097,6 +1102,7 @@ __device__ __forceinline__ void link_force(const D2& d, int i, int j, int a, int
 // with bisections one after another the bounce-back took 187 us and a second
 // evaluation for the forces 169 (400x800, three circles of radius 10).
 __global__ void __launch_bounds__(256) k2_boundary(D2 d) {
+    after_previous();
     if (d.status[0]) return;
     // per direction: the first circle that owns the solid end, for the forces,
     // and the last one, whose bounce-back stands (they differ only where
@@ -1290,6 +1296,7 @@ __device__ __forceinline__ int box_hi(double x, double r, int margin, int lo, in
 // The last block to finish moves every circle.
 constexpr int FB = 1024, FT = 512;
 __global__ void __launch_bounds__(FB) k2_force(D2 d) {
+    after_previous();
     if (d.status[0]) return;
     __shared__ int list[8 * FB];  // place * 8 + direction - 1; negative (~): evaluate
     __shared__ double term[3][FT];
@@ -1413,6 +1420,7 @@ __global__ void __launch_bounds__(FB) k2_force(D2 d) {
 // a cleared mask, a block per circle and its box; interior solid nodes get
 // rho_s and u = 0 (:94-102)
 __global__ void __launch_bounds__(256) k2_mark(D2 d, int* mask, bool set_macro) {
+    after_previous();
     if (d.status[0]) return;
     const int c = blockIdx.x;
     const double R0 = d.p.radius, xcc = d.xc[3 * c], ycc = d.xc[3 * c + 1];
@@ -1823,7 +1831,7 @@ int p2d_initial(P2Ctx* c, std::string& err) {
             return rc;
         if ((rc = ck(cudaStreamSynchronize(c->s), "velocities", err))) return rc;
     }
-    if (d.p.np > 0) k2_mark<<<d.p.np, 256, 0, c->s>>>(d, d.ob, false);
+    if (d.p.np > 0) launch_next(k2_mark, d.p.np, 256, 0, c->s, d, d.ob, false);
     k2_init_fields<<<dim3((d.p.nx + 6 + 127) / 128, d.p.ny + 6), 128, 0, c->s>>>(d);
     c->itc = 0;
     return ck(cudaStreamSynchronize(c->s), "initial", err);
@@ -1846,15 +1854,15 @@ int p2d_step(P2Ctx* c, int nsteps, std::string& err) {
         if (n > 0) gs_launch(RhoFetch<true>{prev, true}, total, d.gb, c->side);
         gs_launch(RhoFetch<false>{d, false}, total, d.ga, c->side);
         if ((rc = ck(cudaEventRecord(c->join, c->side), "join", err))) return rc;
-        if (shear) k2_collide<true><<<g, 128, 0, c->s>>>(d, n > 0);
-        else k2_collide<false><<<g, 128, 0, c->s>>>(d, n > 0);
+        if (shear) launch_next(k2_collide<true>, g, 128, 0, c->s, d, n > 0);
+        else launch_next(k2_collide<false>, g, 128, 0, c->s, d, n > 0);
         if ((rc = ck(cudaStreamWaitEvent(c->s, c->join, 0), "join", err))) return rc;
-        if (shear) k2_stream<true><<<g, 128, 0, c->s>>>(d);
-        else k2_stream<false><<<g, 128, 0, c->s>>>(d);
+        if (shear) launch_next(k2_stream<true>, g, 128, 0, c->s, d);
+        else launch_next(k2_stream<false>, g, 128, 0, c->s, d);
         if (d.p.np > 0) {
-            k2_boundary<<<bg, 256, 0, c->s>>>(d);
-            k2_force<<<d.p.np, FB, 0, c->s>>>(d);
-            k2_mark<<<d.p.np, 256, 0, c->s>>>(d, d.on, true);
+            launch_next(k2_boundary, bg, 256, 0, c->s, d);
+            launch_next(k2_force, d.p.np, FB, 0, c->s, d);
+            launch_next(k2_mark, d.p.np, 256, 0, c->s, d, d.on, true);
         }
         prev = d;
         std::swap(d.ob, d.on);

@@ -15,6 +15,7 @@
 //            bounceback :895-983, collisionT :1014-1070, streamingT :1073-1098,
 //            bouncebackT :1101-1210, macro :986-1010, macroT :1215-1231
 #include "cell_map.cuh"
+#include "launch.cuh"
 #include "step_cell.cuh"
 
 namespace mglc {
@@ -24,6 +25,7 @@ __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
     k_lid_step(const S* __restrict__ fin, S* __restrict__ fout, StepK<typename St<S>::C> K,
                MAP map, IDX P, const double* __restrict__ mrho, const double* __restrict__ mu,
                const double* __restrict__ mv, const double* __restrict__ mw) {
+    after_previous();
     int i, j, k;
     if (!map.at(K.nx, K.ny, P, i, j, k)) return;
     lid_cell<S, FIRST, IDX, SR>(i, j, k, fin, fout, K, P, mrho, mu, mv, mw, K.seed);
@@ -37,6 +39,7 @@ __global__ void __launch_bounds__(128, ThermalMinBlocks<S>::value)
                    const double* __restrict__ mrho, const double* __restrict__ mu,
                    const double* __restrict__ mv, const double* __restrict__ mw,
                    const double* __restrict__ mT) {
+    after_previous();
     int i, j, k;
     if (!map.at(K.nx, K.ny, P, i, j, k)) return;
     thermal_cell<S, FIRST, ROT, IDX, SR>(i, j, k, fin, fout, gin, gout, F, K, P, mrho, mu, mv, mw,
@@ -57,7 +60,7 @@ static cudaError_t lid_go(bool first, const void* fin, void* fout, const LidStep
     // stochastic rounding exists for the 16-bit storage types only
     constexpr bool kHalf = sizeof(S) == 2;
 #define LID_LAUNCH(FI, IT, SRV, MAP)                                                              \
-    k_lid_step<S, FI, IT, SRV, MAP><<<l.grid, l.block, 0, s>>>((const S*)fin, (S*)fout, K, MAP(a.g), \
+    launch_next(k_lid_step<S, FI, IT, SRV, MAP>, l.grid, l.block, 0, s, (const S*)fin, (S*)fout, K, MAP(a.g), \
                                                                (IT)a.g.plane, a.rho, a.u, a.v, a.w)
 #define LID_SR(FI, IT, MAP)                              \
     if (kHalf && a.sr) LID_LAUNCH(FI, IT, kHalf, MAP);   \
@@ -105,7 +108,7 @@ static cudaError_t th_go(bool first, const void* fin, void* fout, const void* gi
     const bool small = index32(a.g);
     constexpr bool kHalf = sizeof(S) == 2;
 #define TH_LAUNCH2(FI, RO, IT, SRV, MAP)                                                     \
-    k_thermal_step<S, FI, RO, IT, SRV, MAP><<<l.grid, l.block, 0, s>>>(                      \
+    launch_next(k_thermal_step<S, FI, RO, IT, SRV, MAP>, l.grid, l.block, 0, s,                \
         (const S*)fin, (S*)fout, (const C*)gin, (C*)gout, (C*)F, K, MAP(a.g), (IT)a.g.plane, \
         a.rho, a.u, a.v, a.w, a.T)
 #define TH_LAUNCH(FI, RO, IT, MAP)                              \

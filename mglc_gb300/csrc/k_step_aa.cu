@@ -9,6 +9,7 @@
 // Same reference routines as k_step.cu (mpi_3d_blocked/{collision.f90:15-202,
 // streaming.f90:8-20, bounce_back.f90:6-83, macro.f90:6-25}).
 #include "cell_map.cuh"
+#include "launch.cuh"
 #include "step_cell.cuh"
 
 namespace mglc {
@@ -18,6 +19,7 @@ __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
     k_lid_step_aa(S* f, StepK<typename St<S>::C> K, MAP map, IDX P, const double* __restrict__ mrho,
                   const double* __restrict__ mu, const double* __restrict__ mv,
                   const double* __restrict__ mw) {
+    after_previous();
     int i, j, k;
     if (!map.at(K.nx, K.ny, P, i, j, k)) return;
     S raw[Q19];  // every load is issued before the first store
@@ -33,6 +35,7 @@ __global__ void __launch_bounds__(128, ThermalMinBlocks<S>::value)
                       StepK<typename St<S>::C> K, MAP map, IDX P, const double* __restrict__ mrho,
                       const double* __restrict__ mu, const double* __restrict__ mv,
                       const double* __restrict__ mw, const double* __restrict__ mT) {
+    after_previous();
     using C = typename St<S>::C;
     int i, j, k;
     if (!map.at(K.nx, K.ny, P, i, j, k)) return;
@@ -49,6 +52,7 @@ __global__ void __launch_bounds__(128, ThermalMinBlocks<S>::value)
 // reflected population.
 template <typename S, int Q, typename IDX, class MAP>
 __global__ void __launch_bounds__(128) k_aa_swap(S* f, int nx, int ny, int nz, MAP map, IDX P) {
+    after_previous();
     int i, j, k;
     if (!map.at(nx, ny, P, i, j, k)) return;
     const IDX cell = (IDX)i + (IDX)nx * ((IDX)j + (IDX)ny * (IDX)k);
@@ -86,7 +90,7 @@ cudaError_t lid_go_aa(bool first, bool odd, void* f, const LidStepArgs& a, cudaS
     const bool sr = kHalf && a.sr;
     S* fp = (S*)f;
 #define AA_LAUNCH(FI, IT, SRV, OD, MAP)                                       \
-    k_lid_step_aa<S, FI, IT, SRV, OD, MAP><<<l.grid, l.block, 0, s>>>(        \
+    launch_next(k_lid_step_aa<S, FI, IT, SRV, OD, MAP>, l.grid, l.block, 0, s,   \
         fp, K, MAP(a.g), (IT)a.g.plane, a.rho, a.u, a.v, a.w)
 #define AA_PICK(IT, MAP)                                                   \
     if (odd) {                                                             \
@@ -115,11 +119,11 @@ template <typename S, int Q>
 cudaError_t swap_go(const Geom& g, void* f, cudaStream_t s) {
     const CellLaunch l(g);
     if (linear_cells(g))
-        k_aa_swap<S, Q, unsigned><<<l.grid, l.block, 0, s>>>((S*)f, g.nx, g.ny, g.nz, CellMap(g), (unsigned)g.plane);
+        launch_next(k_aa_swap<S, Q, unsigned, CellMap>, l.grid, l.block, 0, s, (S*)f, g.nx, g.ny, g.nz, CellMap(g), (unsigned)g.plane);
     else if (index32(g))
-        k_aa_swap<S, Q, unsigned><<<l.grid, l.block, 0, s>>>((S*)f, g.nx, g.ny, g.nz, RowMap(g), (unsigned)g.plane);
+        launch_next(k_aa_swap<S, Q, unsigned, RowMap>, l.grid, l.block, 0, s, (S*)f, g.nx, g.ny, g.nz, RowMap(g), (unsigned)g.plane);
     else
-        k_aa_swap<S, Q, long long><<<l.grid, l.block, 0, s>>>((S*)f, g.nx, g.ny, g.nz, RowMap(g), (long long)g.plane);
+        launch_next(k_aa_swap<S, Q, long long, RowMap>, l.grid, l.block, 0, s, (S*)f, g.nx, g.ny, g.nz, RowMap(g), (long long)g.plane);
     return cudaGetLastError();
 }
 
@@ -146,7 +150,7 @@ cudaError_t th_go_aa(bool first, bool odd, void* f, void* g, void* F, const Ther
     C* gp = (C*)g;
     C* Fp = (C*)F;
 #define TA_LAUNCH(FI, RO, IT, SRV, OD, MAP)                                      \
-    k_thermal_step_aa<S, FI, RO, IT, SRV, OD, MAP><<<l.grid, l.block, 0, s>>>(   \
+    launch_next(k_thermal_step_aa<S, FI, RO, IT, SRV, OD, MAP>, l.grid, l.block, 0, s,    \
         fp, gp, Fp, K, MAP(a.g), (IT)a.g.plane, a.rho, a.u, a.v, a.w, a.T)
 #define TA_SR(FI, RO, IT, OD, MAP)                        \
     do {                                                  \
