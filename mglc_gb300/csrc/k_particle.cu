@@ -496,13 +496,55 @@ __device__ __forceinline__ bool node_avail(int i, int j, int k, const PartParams
 // in (each holds the SM's unit for 16 clocks or more, whatever lanes are
 // active), so: the centre's conversions are one warp's; the node's distance to
 // the surface is an exact fixed-point one; the few links that need an FP64 root
-// are collected and take it together; the slab's sums are integers and pairs of
-// FP32 values (TwoSum).  A link's values and masks are loaded before any is used
+// are collected and take it together; the slab's sums are integers and triples
+// of FP32 values (Sum3).  A link's values and masks are loaded before any is used
 // (one latency a link instead of three), after the roots, so that the warps need
 // no barrier between their links.  200 spheres of radius 5, FP32: 95 -> 48 us
 // (1.3 waves of blocks, a quarter of the issue slots waiting at barriers);
 // blocks of 128 threads, one wave: 69 us.  24 spheres, FP64: 59 -> 46 us, the
 // FP64 unit of the 96 SMs that have a block.
+// A sum of FP32 values as three of them, errors kept by TwoSum: good to about 2^-70 of
+// the largest partial sum (FP64: 2^-53).
+struct Sum3 {
+    float h, m, l;
+    __device__ __forceinline__ Sum3 from_lane(int o) const {  // the one of lane ^ o
+        return {__shfl_xor_sync(0xffffffffu, h, o), __shfl_xor_sync(0xffffffffu, m, o),
+                __shfl_xor_sync(0xffffffffu, l, o)};
+    }
+    __device__ __forceinline__ void operator+=(Sum3 x) {
+        float e1 = 0.0f, e2 = 0.0f;
+        two_sum(h, e1, x.h);
+        two_sum(m, e2, x.m);
+        two_sum(m, e2, e1);
+        l += x.l + e2;
+    }
+};
+struct Sum64 {
+    double h;
+    __device__ __forceinline__ Sum64 from_lane(int o) const { return {__shfl_xor_sync(0xffffffffu, h, o)}; }
+    __device__ __forceinline__ void operator+=(Sum64 x) { h += x.h; }
+};
+// Eight sums over the warp, each by the pairwise tree over the lanes' bits 4 to 0: at the
+// first three levels a lane gives half of its values away and keeps the other half,
+// nine additions instead of forty.  Lane l ends with sum 4 b4 + 2 b3 + b2 of its bits.
+template <class T>
+__device__ __forceinline__ T warp_sum8(T (&v)[8], int lane) {
+#pragma unroll
+    for (int n = 4, o = 16; n > 0; n >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const T give = up ? v[i] : v[i + n];
+            T keep = up ? v[i + n] : v[i];
+            keep += give.from_lane(o);
+            v[i] = keep;
+        }
+    }
+    v[0] += v[0].from_lane(2);
+    v[0] += v[0].from_lane(1);
+    return v[0];
+}
+
 // What a block of k_plinks needs of its particle's centre, converted once.
 template <typename L>
 struct LinkCentre {
@@ -537,7 +579,7 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
     __shared__ int s_box[3];
     __shared__ int s_list[LINK_CAP];  // box index * 32 + direction
     __shared__ int s_wsum[2][PB / 32];
-    __shared__ float s_hi[PB / 32][7], s_lo[PB / 32][7];
+    __shared__ Sum3 s_sum[PB / 32][7];
     __shared__ double s_av[PB / 32][7], s_out[13];
     __shared__ int s_int[PB / 32][6];
     __shared__ int s_def[PB], s_nd;  // listed links that take the FP64 root,
@@ -883,42 +925,33 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
             s_int[wid][3 + q] = b;
         }
     }
-#pragma unroll
-    for (int q = 0; q < 7; q++) {
+    {
+        const int sum = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
         if constexpr (sizeof(L) == 4) {
-            float hi = av[q], lo = 0.0f;  // TwoSum over the lanes
+            Sum3 v[8];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
-                lo += __shfl_xor_sync(0xffffffffu, lo, o);
-                two_sum(hi, lo, oh);
-            }
-            if (lane == 0) {
-                s_hi[wid][q] = hi;
-                s_lo[wid][q] = lo;
-            }
+            for (int q = 0; q < 8; q++) v[q] = {q < 7 ? av[q] : 0.0f, 0.0f, 0.0f};
+            const Sum3 t = warp_sum8(v, lane);
+            if ((lane & 3) == 0 && sum < 7) s_sum[wid][sum] = t;
         } else {
-            double v = av[q];
+            Sum64 v[8];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) s_av[wid][q] = v;
+            for (int q = 0; q < 8; q++) v[q].h = q < 7 ? av[q] : 0.0;
+            const Sum64 t = warp_sum8(v, lane);
+            if ((lane & 3) == 0 && sum < 7) s_av[wid][sum] = t.h;
         }
     }
     __syncthreads();
     if (wid == 0) {
         if constexpr (sizeof(L) == 4) {
-            // 8 lanes per sum add the warps' pairs
+            // 8 lanes per sum add the warps' parts
 #pragma unroll
             for (int r = 0; r < 2; r++) {
                 const int q = min(4 * r + (lane >> 3), 6), w = lane & 7;
-                float hi = s_hi[w][q], lo = s_lo[w][q];
+                Sum3 v = s_sum[w][q];
 #pragma unroll
-                for (int o = 4; o > 0; o >>= 1) {
-                    const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
-                    lo += __shfl_xor_sync(0xffffffffu, lo, o);
-                    two_sum(hi, lo, oh);
-                }
-                if (w == 0) s_out[q] = (double)hi + (double)lo;
+                for (int o = 4; o > 0; o >>= 1) v += v.from_lane(o);
+                if (w == 0) s_out[q] = (double)v.h + ((double)v.m + (double)v.l);
             }
         } else if (lane < 7) {  // the warps' parts in order
             double v = 0.0;
