@@ -305,24 +305,35 @@ int reduce_blocks(long long n) {
 }
 
 // block-wide sum of NV values, warp shuffles then shared memory; fixed order
+// Each of the NV (3 or 4) sums by the pairwise tree over the lanes, then over the warps in
+// order.  Over the first two levels a lane gives half of its values away and keeps the
+// other half: six additions a warp instead of twenty, each of which holds the SM's
+// FP64 unit for 16 clocks.
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double* out) {
     __shared__ double sh[RED_BLOCK / 32][NV];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double x[4];
 #pragma unroll
-    for (int k = 0; k < NV; k++)
+    for (int k = 0; k < 4; k++) x[k] = k < NV ? v[k] : 0.0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-    if (lane == 0)
+    for (int n = 2, o = 16; n > 0; n >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
 #pragma unroll
-        for (int k = 0; k < NV; k++) sh[wid][k] = v[k];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < NV; k++) {
-            double t = 0.0;
-            for (int wv = 0; wv < RED_BLOCK / 32; wv++) t += sh[wv][k];
-            out[k] = t;
+        for (int i = 0; i < n; i++) {
+            const double give = up ? x[i] : x[i + n];
+            x[i] = (up ? x[i + n] : x[i]) + __shfl_xor_sync(0xffffffffu, give, o);
         }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+    const int mine = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
+    if ((lane & 7) == 0 && mine < NV) sh[wid][mine] = x[0];
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        double t = 0.0;
+        for (int wv = 0; wv < RED_BLOCK / 32; wv++) t += sh[wv][threadIdx.x];
+        out[threadIdx.x] = t;
     }
 }
 
@@ -414,13 +425,17 @@ __global__ void __launch_bounds__(RED_BLOCK)
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     const long long n = g.plane;
     const long long sxy = (long long)g.nx * g.ny;
-    for (long long c = blockIdx.x * (long long)RED_BLOCK + threadIdx.x; c < n;
-         c += (long long)gridDim.x * RED_BLOCK) {
-        const double uu = u[c], vv = v[c], ww = w[c], t = T[c];
+    const long long step = (long long)gridDim.x * RED_BLOCK;
+    long long c = blockIdx.x * (long long)RED_BLOCK + threadIdx.x;
+    double nu = 0.0, nv = 0.0, nw = 0.0, nt = 0.0;  // the next cell's, loaded ahead
+    if (c < n) nu = u[c], nv = v[c], nw = w[c], nt = T[c];
+    for (; c < n; c += step) {
+        const double uu = nu, vv = nv, ww = nw, t = nt;
+        if (c + step < n) nu = u[c + step], nv = v[c + step], nw = w[c + step], nt = T[c + step];
         acc[0] += ww * t;
         acc[1] += uu * uu + vv * vv + ww * ww;
         if (wall_axis == 1) {
-            int j;  // by multiplication below 2^31 cells (64-bit divisions: 54 us for 128^3)
+            int j;  // by multiplication below 2^31 cells
             if (n < (1LL << 31)) {
                 const unsigned row = byx((unsigned)c);
                 j = (int)(row - byy(row) * (unsigned)g.ny);
