@@ -250,6 +250,16 @@ __device__ __forceinline__ void d2q9_collide(const double (&f)[9], double& rho, 
         for (int a = 0; a < 9; a++) m[a] = fix_out<58>(M[a].v);
         if (MACRO) d2q9_velocity(M[0].v, m[0], m[3], m[5], u, v);
     } else {
+        // A density that is not finite: the conserved moment relaxes to m0 - 0 (m0 - rho),
+        // a NaN, and every population takes it (a cavity of NaN ran at 0.57 of the speed that
+        // the statements as written had, without this).
+        const double m0 = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8];
+        if (!isfinite(m0)) {
+            if (MACRO) rho = m0;
+#pragma unroll
+            for (int a = 0; a < 9; a++) fp[a] = __longlong_as_double(0x7ff8000000000000LL);
+            return;
+        }
         d2q9_moments<GROUPED>(f, m);
         if (MACRO) d2q9_velocity(m[0], m[3], m[5], u, v);
     }

@@ -216,6 +216,18 @@ __device__ __forceinline__ bool out_of_box(double rho, double ux, double uy, dou
     return !(rho >= 0.25 && rho < 2.0 && fabs(ux) < 0.5 && fabs(uy) < 0.5 && fabs(uz) < 0.5);
 }
 template <int N>
+__device__ __forceinline__ bool beyond_one(const double (&f)[N]) {  // |f| >= 1, or not finite
+    unsigned worst = 0;
+#pragma unroll
+    for (int q = 0; q < N; q++) worst = max(worst, (unsigned)__double2hiint(f[q]) & 0x7fffffffu);
+    return worst >= 0x3FF00000u;
+}
+// A density that is not finite makes every population NaN (each takes a term with
+// rho, and u is NaN); said here, not computed, as a diverged solve is all such cells.
+__device__ __forceinline__ bool not_finite(double r) {
+    return ((unsigned)__double2hiint(r) & 0x7ff00000u) == 0x7ff00000u;
+}
+template <int N>
 __device__ __forceinline__ void set_nan(double (&f)[N]) {
 #pragma unroll
     for (int q = 0; q < N; q++) f[q] = __longlong_as_double(0x7ff8000000000000LL);
@@ -330,11 +342,11 @@ __device__ __forceinline__ void lid_cell_from(int i, int j, int k, const S (&raw
         }
         if (!ok) {
             C jx, jy, jz, ux, uy, uz;
-            bool bad = false;
-#pragma unroll
-            for (int q = 0; q < Q19; q++) bad |= !(fabs(f[q]) < 1.0);
+            const bool bad = K.pk.box && beyond_one(f);
             moments0(f, rho, jx, jy, jz);
-            if (FIRST) {
+            if (!FIRST && (bad || not_finite(rho))) {
+                set_nan(f);
+            } else if (FIRST) {
                 const double rf = rho;
                 rho = mrho[cell];
                 ux = mu[cell];
@@ -562,7 +574,7 @@ __device__ __forceinline__ void thermal_cell_from(
         }
         double rho, ux, uy, uz, fx, fy, fz;
         bool ok = K.pk.fix.on && fix61_ok(f) && fabs(fxp) < small && fabs(fyp) < small &&
-                  fabs(fzp) < small, bad = false;
+                  fabs(fzp) < small, bad = false, none = false;
         long long L[Q19];
         FixFlow fl;
         if (ok) {
@@ -594,7 +606,8 @@ __device__ __forceinline__ void thermal_cell_from(
             uz = mw[cell];
         } else {
             moments0(f, rho, ux, uy, uz);
-            const double inv = recip(rho);
+            none = not_finite(rho);
+            const double inv = none ? rho - rho : recip(rho);  // (NaN)
             // u^n = (sum f e + F^n/2)/rho^n with the force carried from the previous step
             ux = (ux + 0.5 * fxp) * inv;
             uy = (uy + 0.5 * fyp) * inv;
@@ -606,9 +619,11 @@ __device__ __forceinline__ void thermal_cell_from(
                 L, K.pk.fix, fl, ROT ? __double2ll_rn(fx * FIX_ONE) : 0,
                 ROT ? __double2ll_rn(fy * FIX_ONE) : 0, __double2ll_rn(fz * FIX_ONE));
             fix61_store_all<5>(L, f);
+        } else if (none) {
+            bad = true;
+            set_nan(f);
         } else {
-#pragma unroll
-            for (int q = 0; q < Q19; q++) bad |= !(fabs(f[q]) < 1.0);
+            bad = beyond_one(f);
             double rf, jx, jy, jz;
             moments0(f, rf, jx, jy, jz);
             if (!FIRST && ok) {  // (a force of 1/8 or more)
@@ -634,7 +649,10 @@ __device__ __forceinline__ void thermal_cell_from(
             for (int q = 0; q < Q7; q++) bad |= !(fabs(g[q]) < 2.0);
             bad = bad || !(fabs(temp) < 2.0) || out_of_box(rho, ux, uy, uz);
         }
-        if (ok && hot) {
+        if (K.pk.box && bad) {
+            set_nan(f);
+            set_nan(g);
+        } else if (ok && hot) {
             fix_heat(G, T, K.pk.heat, fl);
 #pragma unroll
             for (int q = 0; q < Q7; q++) g[q] = fix61_store_any(G[q]);
@@ -643,10 +661,6 @@ __device__ __forceinline__ void thermal_cell_from(
             trt_collide_t<C, true>(g, temp, ux, uy, uz, K.para_a, K.qd, K.qnu, sg - temp);
         } else {
             pair_collide_t(g, temp, ux, uy, uz, K.pk);
-        }
-        if (K.pk.box && bad) {
-            set_nan(f);
-            set_nan(g);
         }
     } else {
         C rho_m, rho, ux, uy, uz, temp, jx, jy, jz;

@@ -49,3 +49,31 @@ def test_temperature_matches_oracle(mg, kind, ekman, in_place):  # noqa: F811
             for got, want in ((gf, o.f), (gg, o.g)):
                 bound = n * (900 * 2.0 ** -53 * np.abs(want).max() + 8 * 2.0 ** -61)
                 assert np.abs(got - want).max() <= bound
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_non_finite_cells_spread_as_in_the_oracle(mg, bad):  # noqa: F811
+    """Cells whose density is not finite: not finite where the oracle is not (which of
+    infinity and NaN a population becomes depends on the form of the sums), its
+    values elsewhere."""
+    nx, ny, nz = 34, 6, 7
+    f = _state("flow", (nz, ny, nx), 8)
+    T = 0.3 * np.sin(np.arange(nz * ny * nx)).reshape(nz, ny, nx)
+    g = T[..., None] * (np.array([0.4] + [0.1] * 6))
+    from tests.test_fix61_gpu import _macros
+    m = _macros(f)
+    f[3, 2, 16, 5] = bad
+    o = O.ThermalOracle(nx, ny, nz, 1e5, 0.71, 0.1, 0.0, 0.5, -0.5, 0.0)
+    o.f[:], o.g[:], o.T[:] = f, g, g.sum(-1)
+    o.rho[:], o.u[:], o.v[:], o.w[:] = m
+    with mg.BuoyancyCavity(nx, ny, nz, rayleigh=1e5, prandtl=0.71, mach=0.1, t_hot=0.5, t_cold=-0.5) as c, \
+            np.errstate(all="ignore"):
+        c.load_state(f, g, *m, g.sum(-1))
+        for n in (1, 2, 3):
+            c.step(1)
+            o.run(1)
+            for got, want in zip(c.get_f(), (o.f, o.g)):
+                assert np.array_equal(np.isfinite(got), np.isfinite(want))
+                ok = np.isfinite(want)
+                bound = n * (900 * 2.0 ** -53 * np.abs(want[ok]).max() + 8 * 2.0 ** -61)
+                assert np.abs(got[ok] - want[ok]).max() <= bound
