@@ -5,8 +5,8 @@ Re=1000, U=0.1, FP64 plain method (the drop-in).  A "step" is one fused time
 step over the whole lattice.  ``value`` is MLUPS with the state resident in
 HBM; ``e2e`` is the same metric through the C-ABI with host buffers (initial
 state uploaded from pinned host memory, K steps, macroscopic fields read back)
-inside the timed region.  The other forms (FX64: FP64 storage with the
-fixed-point collision; FP32 / FP16 / BF16 deviations with FP32 arithmetic) are
+inside the timed region.  The other forms (FX64: as FP64, with a
+range box; FP32 / FP16 / BF16 deviations with FP32 arithmetic) are
 timed on the same workload and reported under ``forms``.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl mglc|reference]
@@ -42,7 +42,7 @@ WORKLOADS = {
     "thermal128": dict(kind="thermal", n=128, rayleigh=1e5, prandtl=0.71, mach=0.1, error_steps=20000,
                        desc="differentially heated cavity D3Q19+D3Q7 128^3 Ra=1e5 Pr=0.71"),
     "particles": dict(kind="particle", n=(256, 128, 128), np=200, radius=5.0, ratio=1.2,
-                      body_force=1e-6, tauf=0.65, seed=2026, launches_per_step=11,
+                      body_force=1e-6, tauf=0.65, seed=2026, launches_per_step=6,
                       error_steps=10000,
                       data="synthetic (seeded sphere placement, fluid at rest, no dataset)",
                       desc="particle-laden channel D3Q19 256x128x128, 200 spheres R=5, "
@@ -555,7 +555,7 @@ def side_workload(torch, mg, key, steps, warmup, peak, probe, cpu=True, errors=T
         rf = {"bound": "fp64" if "fp64_frac" in head else "hbm", "achieved": head["achieved_gbs"],
               "peak": peak, "unit": "GB/s", "frac": head["frac"],
               "bytes_per_cell": head["bytes_per_cell"],
-              "kernel": "particle step (k_pbulk + 10 small kernels)" if kind == "particle"
+              "kernel": "particle step (k_pbulk + 5 small kernels)" if kind == "particle"
               else f"k_thermal_step<{forms[0]}>"}
         for k in ("fp64_achieved", "fp64_peak", "fp64_unit", "fp64_frac", "fp64_mix_roof_mlups",
                   "fp64_mix_frac", "fp64_instr_per_cell", "alt_layout_bytes_per_cell"):
@@ -1026,7 +1026,7 @@ def main():
         "metric": METRIC, "value": round(value, 3), "unit": "MLUPS", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(ms_step, 4),
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": {"fp64": "f64", "fx64": "i64 Q55 fixed point (f64 storage)"}.get(args.form, "f32"),
+        "dtype": {"fp64": "f64", "fx64": "i64 Q61 fixed point (f64 storage)"}.get(args.form, "f32"),
         "data": wl.get("data", "synthetic (analytic cavity initial state, no dataset)"),
         "config": mglc_config(wl, args.form, world, args.in_place),
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
