@@ -12,8 +12,8 @@
 // 2^-61 is finer than an FP64 ulp from 2^-8 up, so every result lies closer to
 // the exact collision than the FP64 evaluation's, whose sums and products round
 // on the way (tests/test_fix61_host.py; velocity error after six steps of 384^3
-// 2.1e-13 against 3.3e-13).  About a thousand integer instructions a lid cell:
-// 384^3 in 3.31 ms a step (17.1 GLUPS, 77% of HBM) against 15.7 ms in FP64;
+// 2.1e-13 against 3.3e-13).  1554 instructions a lid cell, twelve of them FP64 (ncu):
+// 384^3 in 3.26 ms a step (17.4 GLUPS, 78% of HBM) against 15.7 ms in FP64;
 // the heated cavity at 128^3, temperature populations alike (fix_heat; 235 with those
 // in FP64), in 205 us (10.2 GLUPS) against 813.
 // Cells outside its range (a population outside [2^-8, 1/8), the rest

@@ -18,7 +18,7 @@
 // arithmetic is FP64 in the reference's expression order and this file is
 // compiled without FMA contraction (device and host), so every value rounds
 // as the reference's statement does; the collision and the two quotients of
-// macro are d2q9.cuh's, which give those bits with about 90 FP64 instructions
+// macro are d2q9.cuh's, which give those bits with 108 FP64 instructions
 // a node and as many integer ones beside them as fit.  The FP64 pipe bounds the
 // step: 1024^2 takes 221 us (4.74 GLUPS) against 404 us with the statements
 // written out (about 190 FP64 instructions).

@@ -44,9 +44,9 @@
 // Case4 at 400x800 with three circles: 1118 us a step before (19 launches:
 // the node-wise collision 210, the averages 2 x 140, bounce-back 187 and links
 // 169 with calQ's bisections one after another in a thread, the forces 203 on
-// one warp a circle), 200 us now: k2_collide 97 (FP64 pipe), k2_stream 31,
-// k2_boundary 18, k2_force 29 (190 dependent adds at ~90 clocks), k2_mark 6; the
-// two averages, 7 + 32 each, run beside k2_collide.
+// one warp a circle), 198 us now: k2_collide 64 (FP64 pipe), k2_stream 24,
+// k2_boundary 17, k2_force 29 (190 dependent adds at ~90 clocks), k2_mark 7; the
+// two averages, 7 + 32 each, run beside k2_collide and k2_stream.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
