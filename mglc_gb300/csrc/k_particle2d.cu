@@ -67,6 +67,11 @@ __device__ __constant__ int c_r[9] = {0, 3, 4, 1, 2, 7, 8, 5, 6};
 __device__ __constant__ double c_w[9] = {4.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0,
                                          1.0 / 36.0, 1.0 / 36.0, 1.0 / 36.0, 1.0 / 36.0};
 
+// what a listed boundary node keeps: the owner of each of its eight links, and
+// each link's F_x, F_y and torque.  Any fluid node may be listed (circles of one
+// node three apart list eight of nine), so the arrays hold every node.
+constexpr int NODE_LINKS = 8, LINK_TERMS = 3, NODE_TERMS = NODE_LINKS * LINK_TERMS;
+
 enum { S_NO_OWNER = 1, S_Q = 2, S_OVERLAP = 3, S_WALL = 4, S_NO_DIR = 5 };
 
 // Records of one ordered density sum (GsPiece below): per chunk of addends its
@@ -1160,7 +1165,7 @@ __global__ void __launch_bounds__(256) k2_boundary(D2 d) {
                     fra = F(d, ra, i, j);
                     double Fx, Fy, T;
                     link_force(d, i, j, a, c0, s_x0[0][b], s_y0[0][b], Fx, Fy, T);
-                    double* o = d.lt + 3 * (8 * (size_t)pos + b);
+                    double* o = d.lt + LINK_TERMS * (NODE_LINKS * (size_t)pos + b);
                     o[0] = Fx;
                     o[1] = Fy;
                     o[2] = T;
@@ -1360,7 +1365,7 @@ __global__ void __launch_bounds__(FB) k2_force(D2 d) {
                 const int e = list[k0 + threadIdx.x];
                 double Fx = 0.0, Fy = 0.0, T = 0.0;
                 if (e >= 0) {
-                    const double* o = d.lt + 3 * (size_t)e;
+                    const double* o = d.lt + LINK_TERMS * (size_t)e;
                     Fx = o[0];
                     Fy = o[1];
                     T = o[2];
@@ -1753,7 +1758,8 @@ int p2d_create(const P2Params& p, const double* centers_xy, P2Ctx** out, std::st
         if ((rc = dal(c, a, np3, err))) return rc;
     const size_t nodes = (size_t)p.nx * p.ny;
     if ((rc = dal(c, &d.bl_list, nodes, err)) || (rc = dal(c, &d.bl_pos, cells, err)) ||
-        (rc = dal(c, &d.lc, 8 * nodes, err)) || (rc = dal(c, &d.lt, 16 * nodes, err)) ||
+        (rc = dal(c, &d.lc, NODE_LINKS * nodes, err)) ||
+        (rc = dal(c, &d.lt, NODE_TERMS * nodes, err)) ||
         (rc = dal(c, &d.done, 2, err)))
         return rc;
     const size_t nch = (size_t)gs_chunks((long long)p.nx * p.ny);
@@ -1920,7 +1926,7 @@ __global__ void __launch_bounds__(128) k2_pack_f(D2 d, double* out) {
 
 int p2d_get_f(P2Ctx* c, double* f, std::string& err) {
     const D2& d = c->d;
-    // lt (24 doubles per node) holds nothing between steps
+    static_assert(NODE_TERMS >= 9, "lt takes the populations");  // it holds nothing between steps
     k2_pack_f<<<rows_grid(d), 128, 0, c->s>>>(d, d.lt);
     int rc = ck(cudaGetLastError(), "copy to host", err);
     if (rc) return rc;
