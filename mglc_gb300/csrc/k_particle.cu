@@ -104,6 +104,11 @@ __device__ __forceinline__ void pfail(const PartDev& d, int code, int c, int oth
     }
 }
 
+// Has a step failed?  One answer for the whole block, so that it leaves together:
+// other blocks of the same launch may be setting the status, and warps that read it
+// late would leave the others to barriers and shared values that they never wrote.
+__device__ __forceinline__ bool stopped(const PartDev& d) { return __syncthreads_or(d.status[0]); }
+
 template <int NV>
 __device__ __forceinline__ void block_sum_to(double (&v)[NV], double* out, int stride) {
     __shared__ double sh[32][NV];
@@ -358,7 +363,7 @@ constexpr int FINISH_BLOCKS = PSt<S>::SHIFT ? 128 : 32;
 template <typename S>
 __global__ void __launch_bounds__(256) k_pfinish(PartDev d, int nblocks, double rho0) {
     after_previous();
-    if (d.status[0]) return;
+    if (stopped(d)) return;
     __shared__ int last;
     constexpr int NB = FINISH_BLOCKS<S>;
     const int per = (nblocks + NB - 1) / NB;
@@ -574,7 +579,7 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
     k_plinks(S* __restrict__ f, PartParams p, PartDev d) {
     after_previous();
     using L = typename PC<S>::C;
-    if (d.status[0]) return;
+    if (stopped(d)) return;
     __shared__ LinkCentre<L> s_c;
     __shared__ int s_box[3];
     __shared__ int s_list[LINK_CAP];  // box index * 32 + direction
@@ -1143,7 +1148,7 @@ __device__ bool pmotion(const PartParams& p, const SphereK& sk, const PartDev& d
 template <bool MOVE>
 __global__ void __launch_bounds__(PB) k_pmark(int* owner, PartParams p, SphereK sk, PartDev d) {
     after_previous();
-    if (MOVE && d.status[0]) return;
+    if (MOVE && stopped(d)) return;
     const int c = blockIdx.x;
     __shared__ double X[3];
     if constexpr (MOVE) {
@@ -1211,7 +1216,7 @@ constexpr int PU = MGLC_PU;
 template <typename S>
 __global__ void __launch_bounds__(PB) k_pphase(const S* __restrict__ f, PartParams p, PartDev d) {
     after_previous();
-    if (d.status[0]) return;
+    if (stopped(d)) return;
     const int c = blockIdx.x, slab = blockIdx.y;
     if (d.done[1]) {  // a particle went out of range: the state moves and freezes
         if (c == 0 && slab == 0 && threadIdx.x == 0) pfail(d, PS_DIVERGED, (int)d.done[1] - 1, 0, d.par);

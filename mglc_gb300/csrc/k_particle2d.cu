@@ -126,6 +126,13 @@ __device__ void fail(const D2& d, int code, int c, int par) {
     }
 }
 
+// Has a step failed?  One answer for the whole block, so that it leaves together:
+// other blocks of the same launch may be setting the status, and warps that read it
+// late would leave the others to barriers and shared values that they never wrote.
+// (Counters that such a block does not advance are reset by p2d_initial; until then
+// the state is frozen.)
+__device__ __forceinline__ bool stopped(const D2& d) { return __syncthreads_or(d.status[0]); }
+
 // x index of a population read: case1 is periodic in x (its MPI exchange
 // fills the ghost columns with the periodic partner's values); case4 reads
 // its own ghost columns
@@ -714,7 +721,7 @@ __device__ __forceinline__ int gs_binade(long long v, int E) {
 template <class Fetch>
 __global__ void __launch_bounds__(SB) k_gs_map(Fetch fetch, int total, int nch, GsBuf b) {
     after_previous();
-    if (fetch.stop()) return;
+    if (__syncthreads_or(fetch.stop())) return;
     __shared__ GsShared sh;
     __shared__ double ws[SB / 32], wall[SB / 32], s_x[GS_PIECES];
     __shared__ long long wt[SB / 32];
@@ -1108,7 +1115,7 @@ __device__ __forceinline__ void link_force(const D2& d, int i, int j, int a, int
 // evaluation for the forces 169 (400x800, three circles of radius 10).
 __global__ void __launch_bounds__(256) k2_boundary(D2 d) {
     after_previous();
-    if (d.status[0]) return;
+    if (stopped(d)) return;
     // per direction: the first circle that owns the solid end, for the forces,
     // and the last one, whose bounce-back stands (they differ only where
     // circles overlap)
@@ -1302,7 +1309,7 @@ __device__ __forceinline__ int box_hi(double x, double r, int margin, int lo, in
 constexpr int FB = 1024, FT = 512;
 __global__ void __launch_bounds__(FB) k2_force(D2 d) {
     after_previous();
-    if (d.status[0]) return;
+    if (stopped(d)) return;
     __shared__ int list[8 * FB];  // place * 8 + direction - 1; negative (~): evaluate
     __shared__ double term[3][FT];
     __shared__ int wcount[FB / 32];
