@@ -257,6 +257,30 @@ __device__ __forceinline__ void pcollide(double (&f)[Q19], const PBulkK<double>&
                                    k.cd);
 }
 
+// The mass of the collided populations, added in their order.  FP64: where they are
+// exact in units of 2^-61, integer additions rounded as FP64 rounds, bit for bit (the
+// unit that the collision waits for stays free: 18 additions a cell on it against
+// none).  The density before the collision is not that mass: the first step's
+// density is rho0, whatever the populations are.
+__device__ __forceinline__ float pmass(const float (&f)[Q19]) {
+    float m = 0.0f;
+#pragma unroll
+    for (int q = 0; q < Q19; q++) m += f[q];
+    return m;
+}
+__device__ __forceinline__ double pmass(const double (&f)[Q19]) {
+    if (fix61_ok(f)) {
+        long long R = fix61_load(f[0]);
+#pragma unroll
+        for (int q = 1; q < Q19; q++) R = rn53_pos(R + fix61_load(f[q]));
+        return fix_out<61>(R);
+    }
+    double m = f[0];
+#pragma unroll
+    for (int q = 1; q < Q19; q++) m = __dadd_rn(m, f[q]);
+    return m;
+}
+
 // One thread per node of an x-row segment.  Fluid nodes collide and push
 // their populations (walls at y, z and, unless periodic, x bounce them back in
 // place); solid nodes do nothing.  Each warp writes its partial sums of the
@@ -264,8 +288,7 @@ __device__ __forceinline__ void pcollide(double (&f)[Q19], const PBulkK<double>&
 // slot, so no block barrier is needed and the totals are added in a fixed
 // order by k_pfinish.  The FP32 form writes its two FP32 sums and its count of
 // fluid nodes and leaves FP64 to k_pfinish (a warp's FP64 instruction holds the
-// unit for 16 clocks, and there were seven for every 32 cells); the FP64 form's
-// collision conserves mass to its rounding, so the density serves as both sums.
+// unit for 16 clocks, and there were seven for every 32 cells).
 // The owner mask that the next positions will be marked in is cleared on the
 // way.
 // resident 128-thread blocks per SM the bulk kernel holds its registers to
@@ -287,7 +310,7 @@ __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : MGLC_
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, k = blockIdx.z;
     const IDX P = (IDX)nx * ny * nz;
-    C cacc[2] = {C(0), C(0)};  // per-cell sums in the arithmetic type, widened per warp
+    C cacc[2] = {C(0), C(0)};  // per-cell sums, added over the warp in the arithmetic type
     const bool active = i < nx;
     const IDX cell = (IDX)i + (IDX)nx * ((IDX)j + (IDX)ny * k);
     // the populations are loaded before the mask answers (solid cells read
@@ -301,12 +324,7 @@ __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : MGLC_
     if (active) owner_new[cell] = -1;
     if (fluid) {
         pcollide<FIRST>(f, bk, cacc[0]);
-        if (sizeof(C) == 4) {
-            C m = C(0);
-#pragma unroll
-            for (int q = 0; q < Q19; q++) m += f[q];
-            cacc[1] = m;
-        }
+        cacc[1] = pmass(f);
         const IDX sy = nx, sz = (IDX)nx * ny;
         // asked of the warp's fluid nodes together: apart, a row's two end warps
         // would store twice
@@ -330,9 +348,8 @@ __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : MGLC_
             }
         }
     }
-    constexpr int NS = sizeof(C) == 4 ? 2 : 1;
 #pragma unroll
-    for (int q = 0; q < NS; q++)
+    for (int q = 0; q < 2; q++)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) cacc[q] += __shfl_down_sync(0xffffffffu, cacc[q], o);
     // fluid cells of this warp (deviation storage adds rho0 for each of them)
@@ -347,6 +364,7 @@ __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : MGLC_
             ((int*)(partials + nslot))[slot] = __popc(fl);
         } else {
             partials[slot] = cacc[0];
+            partials[nslot + slot] = cacc[1];
         }
     }
 }
@@ -379,13 +397,14 @@ __global__ void __launch_bounds__(256) k_pfinish(PartDev d, int nblocks, double 
             acc[1] += (double)v.y + nf;
         } else {
             acc[0] += d.partials[b];
+            acc[1] += d.partials[nblocks + b];
         }
     }
     __shared__ double out[2];
     block_sum_to<2>(acc, out, 1);
     if (threadIdx.x == 0) {
         part[blockIdx.x] = out[0];
-        part[NB + blockIdx.x] = PSt<S>::SHIFT ? out[1] : out[0];
+        part[NB + blockIdx.x] = out[1];
         __threadfence();
         last = atomicAdd(d.done, 1u) == gridDim.x - 1;
     }

@@ -69,3 +69,22 @@ def test_frozen_state_is_the_failing_steps(mg, precision, g):  # noqa: F811
         assert np.array_equal(mask, m2)
         for k in ("xc", "uc", "omega"):
             assert np.array_equal(st[k], s2[k]), k
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("fp32", 1e-4)])
+@pytest.mark.parametrize("rho0", [1.0, 2.0])
+def test_node_refilled_in_the_first_step(mg, rho0, precision, tol):  # noqa: F811
+    """A node just inside the sphere leaves it in the first step; its refill takes the
+    average density of the collided populations, which start from w whatever rho0 is."""
+    over = dict(nx=37, ny=23, nz=21, rho0=rho0, rho_solid=1.2 * rho0, gravity=(0.0, 0.0, 0.05))
+    centers = [[18.0, 12.0, 10.499]]  # node (18, 12, 7) is 3.499 away
+    o = O.ParticleOracle(np.array(centers), dim=3, qmode=1, **dict(CASE, **over))
+    inside = o.get()["obst"][6, 11, 17]
+    assert o.step(1) == 0
+    ref = o.get()
+    assert inside != 0 and ref["obst"][6, 11, 17] == 0
+    with _flow(mg, precision, centers, **over) as c:
+        c.initial()
+        c.step(1)
+        f = c.get_f()[6, 11, 17]
+    assert np.abs(f - ref["f"][6, 11, 17]).max() <= tol * rho0
