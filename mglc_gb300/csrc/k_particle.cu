@@ -1077,14 +1077,13 @@ __device__ bool pmotion(const PartParams& p, const SphereK& sk, const PartDev& d
     const int np = p.np;
     const double R0 = p.radius, Rc = p.radius;
     const double* X = d.xc + 3 * c;
-    double fp[3] = {0.0, 0.0, 0.0};
-    bool hit = false;
     // FP64 only for the pairs whose top 20 bits do not rule them out: y and z are
     // below 2^16 (a difference off by 2^-3), x below 2 nx
     const float xt[3] = {top32(X), top32(X + 1), top32(X + 2)}, Lf = (float)p.nx;
     const float far = (float)(Rc + R0 + p.thr_part) * 1.001f + 0.3f + 4e-6f * Lf;
-    for (int c2 = threadIdx.x; c2 < np; c2 += PB) {
-        if (c2 == c) continue;
+    // the spring force of particle c2 added to fp; false: out of range
+    auto spring = [&](int c2, double (&fp)[3]) {
+        if (c2 == c) return false;
         const double* X2 = d.xc + 3 * c2;
         float g0 = top32(X2) - xt[0];
         if (p.periodic_x) {
@@ -1092,25 +1091,42 @@ __device__ bool pmotion(const PartParams& p, const SphereK& sk, const PartDev& d
             else if (g0 < -0.5f * Lf) g0 += Lf;
         }
         if (fabsf(g0) > far || fabsf(top32(X2 + 1) - xt[1]) > far || fabsf(top32(X2 + 2) - xt[2]) > far)
-            continue;  // certainly out of range (not taken for a NaN)
+            return false;  // certainly (not taken for a NaN)
         const double d0 = dxp(X[0], X2[0], p), d1 = X[1] - X2[1], d2 = X[2] - X2[2];
         const double thr = p.thr_part;
         const double reach = Rc + R0 + thr;
-        if (fabs(d0) >= reach || fabs(d1) >= reach || fabs(d2) >= reach) continue;  // out of range
+        if (fabs(d0) >= reach || fabs(d1) >= reach || fabs(d2) >= reach) return false;
         const double dij = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-        if (dij >= Rc + R0 + thr) {
-        } else if (dij >= Rc + R0) {
+        if (dij >= Rc + R0 + thr) return false;
+        if (dij >= Rc + R0) {
             const double t = (dij - Rc - R0 - thr) / thr;
             fp[0] = fp[0] + p.scale_part * (t * t) * d0 / dij;
             fp[1] = fp[1] + p.scale_part * (t * t) * d1 / dij;
             fp[2] = fp[2] + p.scale_part * (t * t) * d2 / dij;
-            hit = true;
-        } else {
-            pfail(d, PS_OVERLAP, c, c2, d.par);
+            return true;
         }
+        pfail(d, PS_OVERLAP, c, c2, d.par);
+        return false;
+    };
+    // The whole block looks for contacts; their forces, which are rare, are one
+    // warp's: a lane adds every 32nd particle's, then the tree over the lanes, so that
+    // the sums do not depend on how many threads look.
+    bool hit = false;
+    double none[3] = {0.0, 0.0, 0.0};
+    for (int c2 = threadIdx.x; c2 < np; c2 += PB) hit = spring(c2, none) || hit;
+    const bool any = __syncthreads_or(hit);
+    if (threadIdx.x < 32) {
+        double fp[3] = {0.0, 0.0, 0.0};
+        if (any) {
+            for (int c2 = threadIdx.x; c2 < np; c2 += 32) spring(c2, fp);
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) fp[q] += __shfl_down_sync(0xffffffffu, fp[q], o);
+        }
+        if (threadIdx.x == 0)
+            for (int q = 0; q < 3; q++) fij[q] = fp[q];
     }
-    if (__syncthreads_or(hit)) block_sum_to<3>(fp, fij, 1);
-    else if (threadIdx.x == 0) fij[0] = fij[1] = fij[2] = 0.0;
     __syncthreads();
     if (threadIdx.x < 32) {  // lane q: component q
         const int q = min((int)threadIdx.x, 2);

@@ -88,3 +88,46 @@ def test_node_refilled_in_the_first_step(mg, rho0, precision, tol):  # noqa: F81
         c.step(1)
         f = c.get_f()[6, 11, 17]
     assert np.abs(f - ref["f"][6, 11, 17]).max() <= tol * rho0
+
+
+def _contacts(case):
+    """80 spheres of radius 1.5 out of each other's reach but for four (with spaces of 33
+    and 72 between their numbers) around sphere 5.  Offsets are multiples of 1/16:
+    differences and squares are exact."""
+    offsets = {0: ([3.0, 1.0, 0.5], [-3.0, 1.25, 0.5], [0.5, -3.0, 1.0], [0.75, 1.0, 3.125]),
+               1: ([2.0, 2.0, 1.5], [-2.0, 2.0, -1.5], [1.5, -2.0, 2.0], [-1.75, -2.5, -0.75])}[case]
+    at = [[4.0 + 4.25 * i, 4.0 + 4.25 * j, 4.0 + 4.25 * k] for k in range(4) for j in range(4) for i in range(5)]
+    focus = np.array([36.0, 12.0, 12.0])
+    at[5] = list(focus)
+    for c2, o in zip((0, 33, 72, 41), offsets):
+        at[c2] = list(focus + o)
+    return np.array(at), focus
+
+
+@pytest.mark.parametrize("case", [0, 1])
+def test_contact_forces_are_added_in_a_stated_order(mg, case):  # noqa: F811
+    """Lane l of 32 adds the springs of particles l, l + 32, ..., then the lanes' sums by
+    halves: bit for bit, whatever number of threads looks for contacts."""
+    at, focus = _contacts(case)
+    r, thr = 1.5, 1.0
+    over = dict(nx=48, ny=24, nz=24, radius=r, threshold_particle=thr, threshold_wall=0.5,
+                gravity=(0.0, 0.0, 0.0), body_force=(0.0, 0.0, 0.0))
+    total = {}
+    for scale in (0.0, 0.7):
+        with _flow(mg, "fp64", at, spring_scale_particle=scale, **over) as c:
+            c.initial()
+            c.step(1)
+            total[scale] = c.state()["force"][5]
+    lanes = np.zeros((32, 3))
+    for c2 in range(len(at)):
+        d = focus - at[c2]
+        dij = np.sqrt((d * d).sum())
+        if c2 != 5 and dij < 2 * r + thr:
+            t = (dij - r - r - thr) / thr
+            lanes[c2 % 32] += 0.7 * (t * t) * d / dij
+    assert np.count_nonzero(lanes.any(1)) == 4
+    half = 16
+    while half:
+        lanes[:half] = lanes[:half] + lanes[half:2 * half]
+        half //= 2
+    assert np.array_equal(total[0.7], total[0.0] + lanes[0])
