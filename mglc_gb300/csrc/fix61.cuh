@@ -14,8 +14,8 @@
 // on the way (tests/test_fix61_host.py; velocity error after six steps of 384^3
 // 2.1e-13 against 3.3e-13).  1554 instructions a lid cell, twelve of them FP64 (ncu):
 // 384^3 in 3.26 ms a step (17.4 GLUPS, 78% of HBM) against 15.7 ms in FP64;
-// the heated cavity at 128^3, temperature populations alike (fix_heat; 235 with those
-// in FP64), in 205 us (10.2 GLUPS) against 813.
+// the heated cavity at 128^3, temperature populations on integers too, in units of
+// their own (fix_heat; 235 with those in FP64), in 205 us (10.2 GLUPS) against 813.
 // Cells outside its range (a population outside [2^-8, 1/8), the rest
 // population outside [1/8, 1/2), negative and non-finite ones among them, rho
 // below 1/4 or a velocity component of 1/2 or more) take the FP64 form; inside,
@@ -283,26 +283,48 @@ __device__ __forceinline__ void fix61_collide(long long (&F)[Q19], const FixK& k
     fix_pair(F, 17, 16, k, byz - cyz, oy - oz);
 }
 
-// The temperature part.  Its populations are of either sign and down to zero: below
-// 2^-9 loading rounds them to 2^-61, which is less than the rounding that an FP64
-// step leaves in their neighbours (2^-56 for populations of 1/10).
-// Every |g| below 1/2?
-__device__ __forceinline__ bool fix_heat_ok(const double (&g)[Q7]) {
+// The temperature part.  Its populations are of either sign, down to zero and of
+// whatever scale the walls set, so each cell has units of its own: the largest of its
+// seven populations lies in [2^(59 - head), 2^(60 - head)) units, smaller ones are
+// rounded to a unit, at most 2^-57 of the largest, where FP64's own half ulp of it is
+// 2^-54.  head leaves |T| below 2^61 (FixHeatK: from the equilibrium weights).  In fixed
+// units of 2^-61 a temperature of 1e-6 was 5e4 times less accurate than in FP64, and
+// walls of 1 and 0 put populations out of range.
+struct HeatUnit {
+    int top;  // exponent field of the largest population, plus head
+};
+// false: a population that is not finite, or all of them below 2^-959 but not zero
+__device__ __forceinline__ bool fix_heat_unit(const double (&g)[Q7], const FixHeatK& k,
+                                              HeatUnit& o) {
     unsigned worst = 0;
 #pragma unroll
     for (int q = 0; q < Q7; q++) worst = max(worst, (unsigned)__double2hiint(g[q]) & 0x7fffffffu);
-    return worst < 0x3FE00000u;
+    o.top = (int)(worst >> 20) + k.head;
+    if (worst < 64u << 20) {
+        unsigned any = 0;
+#pragma unroll
+        for (int q = 0; q < Q7; q++)
+            any |= (unsigned)__double2hiint(g[q]) << 1 | (unsigned)__double2loint(g[q]);
+        o.top = 1023;
+        return any == 0;
+    }
+    return worst < 2040u << 20;
 }
-// x * 2^61 rounded to nearest, |x| < 1/2
-__device__ __forceinline__ long long fix61_load_any(double x) {
+// x in the cell's units, rounded to nearest
+__device__ __forceinline__ long long fix_heat_load(double x, HeatUnit k) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const int s = min(1023 - (int)((hi >> 20) & 0x7ffu), 63);
+    const int s = min(k.top + 2 - (int)((hi >> 20) & 0x7ffu), 63);
     const unsigned long long m =
         ((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32 | lo) << 10;
     const long long v = (long long)(((m >> s) + 1) >> 1), sg = (int)hi >> 31;
     return (v ^ sg) - sg;
 }
-// D3Q7 collision (pair_collide_t) in place, |T| < 1
+__device__ __forceinline__ double fix_heat_store(long long v, HeatUnit k) {
+    const double b = (double)v;
+    // units of 2^(top - 1082)
+    return v ? __hiloint2double(__double2hiint(b) + (k.top - 1082) * (1 << 20), __double2loint(b)) : 0.0;
+}
+// D3Q7 collision (pair_collide_t) in place, |T| < 2^61 units
 __device__ __forceinline__ void fix_heat(long long (&G)[Q7], long long T, const FixHeatK& k,
                                          const FixFlow& o) {
     const FixD t = fix_dig(T);

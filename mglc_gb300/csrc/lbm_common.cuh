@@ -546,9 +546,10 @@ inline FixK make_fix_k(double snu, double sq) {
 // and of the D3Q7 part: (1-qnu)/2, (1-qd)/2, ge0/4, gE, qd/4 (pair_k_heat)
 struct FixHeatK {
     FixC g1, g2, c0, gE, hd;
+    int head;  // bits that the temperature may exceed the largest population by
     int on;
 };
-inline FixHeatK make_fix_heat_k(double qd, double qnu, double ge0, double gE) {
+inline FixHeatK make_fix_heat_k(double para_a, double qd, double qnu, double ge0, double gE) {
     FixHeatK k;
     auto in = [](double s) { return s >= 0x1p-20 && s <= 2.0 - 0x1p-20; };
     k.on = in(qd) && in(qnu) && ge0 >= 0.0 && ge0 < 2.0 && gE >= 0.0 && gE < 0.5;
@@ -559,6 +560,10 @@ inline FixHeatK make_fix_heat_k(double qd, double qnu, double ge0, double gE) {
     k.c0 = fix_coef(fix_ratio(ge0, 4));
     k.gE = fix_coef(fix_ratio(4.0 * gE, 4));
     k.hd = fix_coef(fix_ratio(qd, 4));
+    // at equilibrium T is the largest population over the largest weight; a fifth more
+    // stays below 2^(1 + head) of it, and seven populations always below 2^3
+    const double most = std::fmax(std::fabs(1.0 - para_a) / 7.0, std::fabs(6.0 + para_a) / 42.0);
+    k.head = most >= 0.6 ? 0 : most >= 0.3 ? 1 : 2;
     return k;
 }
 // Coefficients, converted once on the host; empty for the other types.
@@ -597,7 +602,7 @@ inline void pair_k_heat(PairK<double>& k, double para_a, double qd, double qnu) 
     k.ge0 = qnu * (1.0 - para_a) / 7.0;
     k.gE = 0.5 * qnu * (6.0 + para_a) / 21.0;
     k.gd = 0.5 * qd;
-    k.heat = make_fix_heat_k(qd, qnu, k.ge0, k.gE);
+    k.heat = make_fix_heat_k(para_a, qd, qnu, k.ge0, k.gE);
 }
 template <typename T>
 inline void pair_k_heat(PairK<T>&, double, double, double) {}

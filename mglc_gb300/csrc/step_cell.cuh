@@ -560,15 +560,16 @@ __device__ __forceinline__ void thermal_cell_from(
         const double small = 0.125;
         double temp;
         long long G[Q7], T = 0;
-        bool hot = !FIRST && K.pk.heat.on && fix_heat_ok(g);
+        HeatUnit hu;
+        bool hot = !FIRST && K.pk.heat.on && fix_heat_unit(g, K.pk.heat, hu);
         if (hot) {
 #pragma unroll
             for (int q = 0; q < Q7; q++) {
-                G[q] = fix61_load_any(g[q]);
+                G[q] = fix_heat_load(g[q], hu);
                 T += G[q];
             }
             hot = T < (1LL << 61) && -T < (1LL << 61);
-            temp = fix61_store_any(T);
+            temp = fix_heat_store(T, hu);
         } else {
             temp = FIRST ? mT[cell] : ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
         }
@@ -655,7 +656,7 @@ __device__ __forceinline__ void thermal_cell_from(
         } else if (ok && hot) {
             fix_heat(G, T, K.pk.heat, fl);
 #pragma unroll
-            for (int q = 0; q < Q7; q++) g[q] = fix61_store_any(G[q]);
+            for (int q = 0; q < Q7; q++) g[q] = fix_heat_store(G[q], hu);
         } else if (FIRST) {
             const double sg = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + g[6]);
             trt_collide_t<C, true>(g, temp, ux, uy, uz, K.para_a, K.qd, K.qnu, sg - temp);
