@@ -85,15 +85,14 @@ __global__ void __launch_bounds__(256) k_macro(const S* __restrict__ f,
 #pragma unroll
                     for (int q = 0; q < Q7; q++) gq[q] = gt[q * n + c];
                 }
-                long long r60, j[3], t60 = 0;
+                long long r60, j[3];
                 bool ok = fix60_sums(fq, fk, r60, j);
+                double t = 0.0;
                 if (THERMAL) {
-                    int worst = 0, hot = 0;
+                    int worst = 0;
 #pragma unroll
                     for (int a = 0; a < 3; a++) j[a] += fix60_load<124>(F[a], -1, worst);
-#pragma unroll
-                    for (int q = 0; q < Q7; q++) t60 += fix60_load<127>(gq[q], 0, hot);
-                    ok = ok && worst < 124 && hot < 127;  // forces below 1/4, g below 1
+                    ok = fix60_temperature(gq, t) && ok && worst < 124;  // forces below 1/4
                 }
                 if (ok && fix60_flow(r60, j)) {
                     const FixD y = fix_dig(fix_recip(2 * r60, fix_dig(2 * r60)));
@@ -101,7 +100,7 @@ __global__ void __launch_bounds__(256) k_macro(const S* __restrict__ f,
                     u[c] = fix61_store_any<60>(fix_mul<60>(fix_dig(j[0]), y));
                     v[c] = fix61_store_any<60>(fix_mul<60>(fix_dig(j[1]), y));
                     w[c] = fix61_store_any<60>(fix_mul<60>(fix_dig(j[2]), y));
-                    if (THERMAL) T[c] = fix61_store_any<60>(t60);
+                    if (THERMAL) T[c] = t;
                     continue;
                 }
             }

@@ -8,9 +8,9 @@
 //    addition has to round as FP64's; with the populations exact in units of
 //    2^-61 (fix61.cuh) an addition is an integer one followed by the rounding
 //    of the sum to 53 significant bits, to nearest even.
-//  * reduced forms: the stored deviations, rho0, half the force and the
-//    temperature populations are summed in units of 2^-60, exactly but for what
-//    lies below 2^-60, and the velocity is a product with the integer reciprocal,
+//  * reduced forms: the stored deviations, rho0 and half the force are summed in
+//    units of 2^-60, exactly but for what lies below 2^-60 (the temperature
+//    populations in units of their own scale), and the velocity is a product with the integer reciprocal,
 //    to 2^-61: closer to the exact quotient of the stored values than the FP64
 //    sums with w rho0, which round at 2^-54.  Four conversions a cell remain of
 //    33 FP64 instructions.
@@ -108,6 +108,24 @@ __device__ __forceinline__ long long fix60_load(float x, int e2, int& worst) {
     const long long v = (long long)(((unsigned long long)m << TOP) >> min(max(L - 1 - e, 0), 63));
     const long long sg = b >> 31;
     return (v ^ sg) - sg;
+}
+
+// The sum of temperature populations of any scale: in units of 2^-60 of the power of two
+// above the largest, so cut at 2^-59 of it or less (an FP64 sum rounds at 2^-53).  false:
+// one is not finite, or all are below 2^-65 but not zero
+__device__ __forceinline__ bool fix60_temperature(const float (&g)[Q7], double& t) {
+    unsigned big = 0;
+#pragma unroll
+    for (int q = 0; q < Q7; q++) big = max(big, (unsigned)__float_as_int(g[q]) & 0x7fffffffu);
+    const int e = (int)(big >> 23);
+    int worst = 0;
+    long long v = 0;
+#pragma unroll
+    for (int q = 0; q < Q7; q++) v += fix60_load<127>(g[q], 126 - e, worst);
+    const double b = (double)v;
+    t = v && big ? __hiloint2double(__double2hiint(b) + (e - 126 - 60) * (1 << 20), __double2loint(b))
+                 : 0.0;
+    return big == 0 || (e >= 62 && e < 255);
 }
 
 // Scale, rho0 and range of the reduced forms' sums; on: rho0 in [0, 4) and a

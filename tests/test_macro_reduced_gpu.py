@@ -67,3 +67,22 @@ def test_heated_fields(mg, precision):  # noqa: F811
     for got, e in ((fields[1], EX), (fields[2], EY)):  # no force in x and y
         assert (np.abs(got - (f2 * e).sum(-1) / r) * np.abs(r)).max() <= 2 * tol
     assert np.abs(fields[4] - g2.sum(-1)).max() <= 7 * 4 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp16s"])
+@pytest.mark.parametrize("scale", [0.0, 1e-16, 1e-11, 1e-6, 1.0, 300.0, 1e-30])
+def test_temperature_of_any_scale(mg, scale, precision):  # noqa: F811
+    """Bound: seven units of 2^-59 of the largest population, and the rounding of the sum."""
+    nx, ny, nz = 33, 5, 6
+    rng = np.random.default_rng(4)
+    f = _state("flow", (nz, ny, nx), 19, rng)
+    T = scale * (rng.random((nz, ny, nx)) - 0.5)
+    g = T[..., None] * (np.array([0.4] + [0.1] * 6)) * (1 + 0.1 * rng.random((nz, ny, nx, 7)))
+    with mg.BuoyancyCavity(nx, ny, nz, rayleigh=1e4, t_hot=0.5 * scale, t_cold=-0.5 * scale, precision=precision) as c:
+        c.load_state(f, g)
+        c.step(1)
+        got = c.macro()[4]
+        g2 = c.get_f()[1].astype(np.longdouble)
+    want = g2.sum(-1)
+    assert np.isfinite(got).all()
+    assert (np.abs(got - want) <= 7 * 2.0 ** -59 * np.abs(g2).max(-1) + 8 * 2.0 ** -53 * np.abs(g2).sum(-1)).all()
