@@ -488,6 +488,9 @@ constexpr size_t TILE_MAX_BYTES = 160 * 1024;
 // Link-list capacity of k_plinks: one scan round adds at most PB * 18 links,
 // so the list is processed as soon as fewer than that many slots are free.
 constexpr int LINK_CAP = PB * 27;
+// Nodes that a list spans at most: an entry is the node's distance from the list's first
+// scan round, and its direction, in 31 bits (a slab has 2^26 nodes from radius 320).
+constexpr int LINK_SPAN = 1 << 26;
 
 // Is node (i, j, k) (0-based, x unwrapped) a fluid node, or a ghost beyond a
 // wall?  Only those have a post-collision value of this step.
@@ -601,7 +604,7 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
     if (stopped(d)) return;
     __shared__ LinkCentre<L> s_c;
     __shared__ int s_box[3];
-    __shared__ int s_list[LINK_CAP];  // box index * 32 + direction
+    __shared__ int s_list[LINK_CAP];  // (box index - tb) * 32 + direction
     __shared__ int s_wsum[2][PB / 32];
     __shared__ Sum3 s_sum[PB / 32][7];
     __shared__ double s_av[PB / 32][7], s_out[13];
@@ -687,12 +690,13 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
     auto own_at = [&](int bi, int bj, int bk) {  // box coordinates, bk absolute in the box
         return s_own[(bi + 1) + TX * ((bj + 1) + TY * (bk - kz0 + 1))];
     };
+    int tb = 0;  // box index that the list counts from
     // The fraction q of listed link le: ray-sphere root from the node (calQ2,
     // particle_bounceback.F90:144-185), FP64 (false: out of range, status set).
     // The node lies within R + 1.8 < nx / 2 of the centre: the unwrapped difference
     // is the periodic minimum image.
     auto root64 = [&](int le, double& qd) {
-        const int tt = le >> 5, a = le & 31;
+        const int tt = tb + (le >> 5), a = le & 31;
         const int ea = e_rt(EX_PACK, a), eb = e_rt(EY_PACK, a), ec = e_rt(EZ_PACK, a);
         const double ox = (double)(ci - h + tt % bw + 1) - X0, oy = (double)(cj - h + tt / bw % bw + 1) - X1,
                      oz = (double)(ck - h + kz0 + tt / (bw * bw) + 1) - X2;
@@ -712,7 +716,7 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
     // where q is near 0 or 1, the ends the range check tests: those links (false)
     // take the FP64 root, so the FP32 and FP64 forms accept and reject the same links.
     auto root32 = [&](int le, float& ox, float& oy, float& oz, float& q) {
-        const int tt = le >> 5, a = le & 31;
+        const int tt = tb + (le >> 5), a = le & 31;
         const int iu = ci - h + tt % bw, j = cj - h + tt / bw % bw, k = ck - h + kz0 + tt / (bw * bw);
         const int ea = e_rt(EX_PACK, a), eb = e_rt(EY_PACK, a), ec = e_rt(EZ_PACK, a);
         float cbf, ccf;
@@ -807,8 +811,9 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
             if (q < wid) slot += v;
             nl += v;
         }
-        for (unsigned m = my_dirs; m; m &= m - 1) s_list[slot++] = t * 32 + __ffs(m) - 1;
-        if (nl <= LINK_CAP - PB * 18 && t0 + PB < nbox) continue;  // uniform over the block
+        for (unsigned m = my_dirs; m; m &= m - 1) s_list[slot++] = (t - tb) * 32 + __ffs(m) - 1;
+        // uniform over the block
+        if (nl <= LINK_CAP - PB * 18 && t0 + PB < nbox && t0 + 2 * PB - tb <= LINK_SPAN) continue;
         __syncthreads();
         if constexpr (sizeof(L) == 4) {
             // the links that need it take their FP64 root together, over the
@@ -854,7 +859,7 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
             } else {
                 if (!root64(le, q)) continue;
             }
-            const int tt = le >> 5, a = le & 31;
+            const int tt = tb + (le >> 5), a = le & 31;
             const int bi = tt % bw, bj = (tt / bw) % bw, bk = kz0 + tt / (bw * bw);
             const int iu = ci - h + bi, j = cj - h + bj, k = ck - h + bk;  // iu: unwrapped
             const int i = p.periodic_x ? wrapx(iu, nx) : iu;
@@ -939,6 +944,7 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
         }
         __syncthreads();
         nl = 0;
+        tb = t0 + PB;
     }
     // the warp's sums: exact integers, and the variable parts
 #pragma unroll
