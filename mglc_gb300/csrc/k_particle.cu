@@ -572,6 +572,15 @@ __device__ __forceinline__ T warp_sum8(T (&v)[8], int lane) {
     return v[0];
 }
 
+// The exact sum over the warp of integers of 32 bits, from their halves.  A slab's torque
+// sum is about 14 R^2 x, past 32 bits in lattices of some 6e8 nodes; a thread's share,
+// a few links in a thousand, stays below them in any lattice that fits the device.
+__device__ __forceinline__ long long warp_sum64(int v) {
+    const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)v & 0xffffu);
+    const int hi = __reduce_add_sync(0xffffffffu, v >> 16);
+    return (long long)hi * 65536 + (long long)lo;
+}
+
 // What a block of k_plinks needs of its particle's centre, converted once.
 template <typename L>
 struct LinkCentre {
@@ -608,7 +617,8 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
     __shared__ int s_wsum[2][PB / 32];
     __shared__ Sum3 s_sum[PB / 32][7];
     __shared__ double s_av[PB / 32][7], s_out[13];
-    __shared__ int s_int[PB / 32][6];
+    __shared__ int s_nf[PB / 32][3];
+    __shared__ long long s_nt[PB / 32][3];
     __shared__ int s_def[PB], s_nd;  // listed links that take the FP64 root,
     __shared__ float s_q[PB];        // and the roots
     extern __shared__ int s_own[];
@@ -949,10 +959,11 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
     // the warp's sums: exact integers, and the variable parts
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-        const int a = __reduce_add_sync(0xffffffffu, nf[q]), b = __reduce_add_sync(0xffffffffu, nt[q]);
+        const int a = __reduce_add_sync(0xffffffffu, nf[q]);
+        const long long b = warp_sum64(nt[q]);
         if (lane == 0) {
-            s_int[wid][q] = a;
-            s_int[wid][3 + q] = b;
+            s_nf[wid][q] = a;
+            s_nt[wid][q] = b;
         }
     }
     {
@@ -990,10 +1001,10 @@ __global__ void __launch_bounds__(PB, sizeof(S) == 4 ? MGLC_PLINKS_MINB : 2)
             s_out[lane] = v;
         }
         if (lane < 6) {
-            int v = 0;
+            long long v = 0;
 #pragma unroll
-            for (int w = 0; w < PB / 32; w++) v += s_int[w][lane];
-            s_out[7 + lane] = (double)v;
+            for (int w = 0; w < PB / 32; w++) v += lane < 3 ? (long long)s_nf[w][lane] : s_nt[w][lane - 3];
+            s_out[7 + lane] = (double)v;  // exact: far below 2^53
         }
         __syncwarp();
         const double* out = s_out;
