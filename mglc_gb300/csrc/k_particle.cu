@@ -206,8 +206,8 @@ __device__ __forceinline__ void fix58_moments(const double (&f)[Q19], MrtMom<dou
     const Fix58 s7 = F[13] + F[12], d7 = F[13] - F[12], s8 = F[15] + F[18], d8 = F[15] - F[18];
     const Fix58 s9 = F[17] + F[16], d9 = F[17] - F[16];
     const Fix58 sa = s1 + s2 + s3, se = (s4 + s5) + (s6 + s7) + (s8 + s9);
-    // the fused multiply-adds of mrt_moments as nvcc contracts them: one rounding
-    // of the exact value (8 se + RN(-11 sa) in m1)
+    // the roundings of mrt_energy; the other products of mrt_moments are by powers of
+    // two, exact, so that fused or not each sum rounds once
     o.m1 = fix_out<58>(rn53(-30 * F[0].v + rn53(8 * se.v + rn53(-11 * sa.v))));
     o.m2 = fix_out<58>(rn53(12 * F[0].v + rn53(-4 * sa.v + se.v)));
     const Fix58 a45 = d4 + d5, b45 = d4 - d5, a67 = d6 + d7, b67 = d6 - d7, a89 = d8 + d9,

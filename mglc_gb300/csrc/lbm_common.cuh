@@ -115,6 +115,17 @@ template <typename T>
 struct MrtMom {
     T m1, m2, m4, m6, m8, m9, m10, m11, m12, m13, m14, m15, m16, m17, m18;
 };
+// the two moments whose products are not exact; FP64 states its roundings, which the
+// spheres' integer form repeats (k_particle.cu: fix58_moments), FP32 leaves them to the
+// compiler
+__device__ __forceinline__ void mrt_energy(double f0, double sa, double se, double& m1, double& m2) {
+    m1 = __fma_rn(-30.0, f0, __fma_rn(8.0, se, __dmul_rn(-11.0, sa)));
+    m2 = __fma_rn(12.0, f0, __fma_rn(-4.0, sa, se));
+}
+__device__ __forceinline__ void mrt_energy(float f0, float sa, float se, float& m1, float& m2) {
+    m1 = -30.0f * f0 + (-11.0f * sa + 8.0f * se);
+    m2 = 12.0f * f0 + (-4.0f * sa + se);
+}
 template <typename T>
 __device__ __forceinline__ MrtMom<T> mrt_moments(const T* f) {
     const T two = T(2), four = T(4);
@@ -131,8 +142,7 @@ __device__ __forceinline__ MrtMom<T> mrt_moments(const T* f) {
     T sa = s1 + s2 + s3;                    // axis sum
     T se = (s4 + s5) + (s6 + s7) + (s8 + s9); // edge sum
     MrtMom<T> o;
-    o.m1 = T(-30) * f[0] + (T(-11) * sa + T(8) * se);
-    o.m2 = T(12) * f[0] + (T(-4) * sa + se);
+    mrt_energy(f[0], sa, se, o.m1, o.m2);
     T ex_ = (d4 + d5) + (d6 + d7);
     T ey_ = (d4 - d5) + (d8 + d9);
     T ez_ = (d6 - d7) + (d8 - d9);
