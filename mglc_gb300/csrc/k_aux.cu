@@ -58,8 +58,8 @@ __device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float
 // for the fields that the first step after a load starts from (another rounding
 // of them, however small, and the 16-bit stores round otherwise from there on)
 template <typename S, bool THERMAL, bool ORDERED>
-__global__ void __launch_bounds__(256) k_macro(const S* __restrict__ f,
-                        const typename GType<S>::T* __restrict__ gt, const void* Fv,
+__global__ void __launch_bounds__(256) k_macro(const S* f,
+                        const typename GType<S>::T* gt, const void* Fv,
                         Geom g, double rho0, double inv_scale, Fix60K fk, double* rho, double* u,
                         double* v, double* w, double* T) {
     after_previous();

@@ -56,7 +56,7 @@ static_assert(INV6_H == RH6 && INV6_L == RL6 && INV9_H == RH9 && INV9_L == RL9 &
               "the collision's reciprocal pairs");
 
 struct L2K {
-    const double* __restrict__ fin;
+    const double* fin;
     double* __restrict__ fout;
     const double *rho, *u, *v;  // stored fields, read by the first step only
     long long n;                // nx * ny
@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(128) k_l2_step(L2K k) {
 }
 
 // macro, evolution.f90:98-112 (or the stored fields before the first step)
-__global__ void k_l2_macro(const double* __restrict__ f, const double* __restrict__ srho,
-                           const double* __restrict__ su, const double* __restrict__ sv,
+__global__ void k_l2_macro(const double* f, const double* srho,
+                           const double* su, const double* sv,
                            int stored, long long n, double* __restrict__ rho,
                            double* __restrict__ u, double* __restrict__ v) {
     after_previous();

@@ -300,7 +300,7 @@ __device__ __forceinline__ double pmass(const double (&f)[Q19]) {
 #endif
 template <typename S, bool FIRST, typename IDX>
 __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : MGLC_PBULK_MINB64))
-    k_pbulk(const S* __restrict__ fin, S* __restrict__ fout, const int* __restrict__ owner,
+    k_pbulk(const S* fin, S* __restrict__ fout, const int* owner,
             int* __restrict__ owner_new, PartParams p, PBulkK<typename PC<S>::C> bk,
             double* partials, const int* status) {
     after_previous();
@@ -318,9 +318,9 @@ __global__ void __launch_bounds__(128, (sizeof(S) == 4 ? MGLC_PBULK_MINB : MGLC_
     C f[Q19];
     if (active) {
 #pragma unroll
-        for (int q = 0; q < Q19; q++) f[q] = (C)__ldg(fin + (q * P + cell));
+        for (int q = 0; q < Q19; q++) f[q] = (C)fin[q * P + cell];
     }
-    const bool fluid = active && __ldg(owner + cell) < 0;
+    const bool fluid = active && owner[cell] < 0;
     if (active) owner_new[cell] = -1;
     if (fluid) {
         pcollide<FIRST>(f, bk, cacc[0]);
@@ -495,7 +495,7 @@ constexpr int LINK_SPAN = 1 << 26;
 // Is node (i, j, k) (0-based, x unwrapped) a fluid node, or a ghost beyond a
 // wall?  Only those have a post-collision value of this step.
 __device__ __forceinline__ bool node_avail(int i, int j, int k, const PartParams& p,
-                                           const int* __restrict__ owner) {
+                                           const int* owner) {
     if (j < 0 || j >= p.ny || k < 0 || k >= p.nz) return true;
     if (i < 0 || i >= p.nx) {
         if (!p.periodic_x) return true;
@@ -1266,7 +1266,7 @@ constexpr int PREP_SLAB = PART_NSLAB;
 #endif
 constexpr int PU = MGLC_PU;
 template <typename S>
-__global__ void __launch_bounds__(PB) k_pphase(const S* __restrict__ f, PartParams p, PartDev d) {
+__global__ void __launch_bounds__(PB) k_pphase(const S* f, PartParams p, PartDev d) {
     after_previous();
     if (stopped(d)) return;
     const int c = blockIdx.x, slab = blockIdx.y;

@@ -22,9 +22,9 @@ namespace mglc {
 
 template <typename S, bool FIRST, typename IDX, bool SR, class MAP>
 __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
-    k_lid_step(const S* __restrict__ fin, S* __restrict__ fout, StepK<typename St<S>::C> K,
-               MAP map, IDX P, const double* __restrict__ mrho, const double* __restrict__ mu,
-               const double* __restrict__ mv, const double* __restrict__ mw) {
+    k_lid_step(const S* fin, S* __restrict__ fout, StepK<typename St<S>::C> K,
+               MAP map, IDX P, const double* mrho, const double* mu,
+               const double* mv, const double* mw) {
     after_previous();
     int i, j, k;
     if (!map.at(K.nx, K.ny, P, i, j, k)) return;
@@ -33,12 +33,12 @@ __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
 
 template <typename S, bool FIRST, bool ROT, typename IDX, bool SR, class MAP>
 __global__ void __launch_bounds__(128, ThermalMinBlocks<S>::value)
-    k_thermal_step(const S* __restrict__ fin, S* __restrict__ fout,
-                   const typename St<S>::C* __restrict__ gin, typename St<S>::C* __restrict__ gout,
+    k_thermal_step(const S* fin, S* __restrict__ fout,
+                   const typename St<S>::C* gin, typename St<S>::C* __restrict__ gout,
                    typename St<S>::C* __restrict__ F, StepK<typename St<S>::C> K, MAP map, IDX P,
-                   const double* __restrict__ mrho, const double* __restrict__ mu,
-                   const double* __restrict__ mv, const double* __restrict__ mw,
-                   const double* __restrict__ mT) {
+                   const double* mrho, const double* mu,
+                   const double* mv, const double* mw,
+                   const double* mT) {
     after_previous();
     int i, j, k;
     if (!map.at(K.nx, K.ny, P, i, j, k)) return;

@@ -16,9 +16,9 @@ namespace mglc {
 
 template <typename S, bool FIRST, typename IDX, bool SR, bool ODD, class MAP>
 __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
-    k_lid_step_aa(S* f, StepK<typename St<S>::C> K, MAP map, IDX P, const double* __restrict__ mrho,
-                  const double* __restrict__ mu, const double* __restrict__ mv,
-                  const double* __restrict__ mw) {
+    k_lid_step_aa(S* f, StepK<typename St<S>::C> K, MAP map, IDX P, const double* mrho,
+                  const double* mu, const double* mv,
+                  const double* mw) {
     after_previous();
     int i, j, k;
     if (!map.at(K.nx, K.ny, P, i, j, k)) return;
@@ -32,9 +32,9 @@ __global__ void __launch_bounds__(128, LidMinBlocks<S>::value)
 template <typename S, bool FIRST, bool ROT, typename IDX, bool SR, bool ODD, class MAP>
 __global__ void __launch_bounds__(128, ThermalMinBlocks<S>::value)
     k_thermal_step_aa(S* f, typename St<S>::C* g, typename St<S>::C* __restrict__ F,
-                      StepK<typename St<S>::C> K, MAP map, IDX P, const double* __restrict__ mrho,
-                      const double* __restrict__ mu, const double* __restrict__ mv,
-                      const double* __restrict__ mw, const double* __restrict__ mT) {
+                      StepK<typename St<S>::C> K, MAP map, IDX P, const double* mrho,
+                      const double* mu, const double* mv,
+                      const double* mw, const double* mT) {
     after_previous();
     using C = typename St<S>::C;
     int i, j, k;

@@ -5,8 +5,11 @@
 // kernel before it drains (programmatic stream serialization); the kernel calls
 // after_previous first, which returns once that one has completed and its writes are
 // visible, so nothing is read or written early.  The kernels give no early signal:
-// no block of the next grid takes room from them.  About 2 us a launch: FP64 lid
-// 32^3 7.2 -> 5.7 us a step, FP32 lid 97^3 26.9 -> 24.6, heated 81^3 21.7 -> 19.0.
+// no block of the next grid takes room from them.  About 2 us a launch: FP64 lid 32^3
+// 7.2 -> 5.7 us a step, FP32 lid 97^3 26.9 -> 24.6, heated 81^3 21.7 -> 19.0.
+// Such a kernel does not read through __ldg or const __restrict__: read-only loads are
+// for memory that nothing writes during the kernel's lifetime, and that begins before
+// the wait.
 #pragma once
 #include <cuda_runtime.h>
 

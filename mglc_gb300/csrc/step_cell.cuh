@@ -28,8 +28,11 @@ struct St<double> {
     __device__ static void st_s(double* p, C v) { *p = v; }
     __device__ static void st_sr_s(double* p, C v, unsigned) { *p = v; }
     __device__ static C ld(const double* p, float) { return __ldg(p); }
-    __device__ static double raw(const double* p) { return __ldg(p); }
-    // raw_rw: plain load, for a buffer that the same kernel also writes
+    // raw: a two-buffer step's load, from L2 (coherent, as launch.cuh asks; through L1 FP32
+    // 97^3 took 25.2 us a step against 23.8, eight served solves 23.2 ms against 22.3);
+    // raw_rw: for a buffer that the same kernel also writes (in place FP32 128^3 51.8 us
+    // through L1, 53.1 from L2)
+    __device__ static double raw(const double* p) { return __ldcg(p); }
     __device__ static double raw_rw(const double* p) { return *p; }
     __device__ static void st_sr(double* p, C v, float, unsigned) { *p = v; }
     __device__ static C cvt(double v, float) { return v; }
@@ -44,7 +47,7 @@ struct St<float> {
     __device__ static void st_s(float* p, C v) { *p = v; }
     __device__ static void st_sr_s(float* p, C v, unsigned) { *p = v; }
     __device__ static C ld(const float* p, float) { return __ldg(p); }
-    __device__ static float raw(const float* p) { return __ldg(p); }
+    __device__ static float raw(const float* p) { return __ldcg(p); }
     __device__ static float raw_rw(const float* p) { return *p; }
     __device__ static void st_sr(float* p, C v, float, unsigned) { *p = v; }
     __device__ static C cvt(float v, float) { return v; }
@@ -70,7 +73,7 @@ struct St<__half> {
     }
     __device__ static void st_bits(__half* p, unsigned short v) { *p = __ushort_as_half(v); }
     __device__ static C ld(const __half* p, float inv) { return __half2float(__ldg(p)) * inv; }
-    __device__ static __half raw(const __half* p) { return __ldg(p); }
+    __device__ static __half raw(const __half* p) { return __ldcg(p); }
     __device__ static __half raw_rw(const __half* p) { return *p; }
     // stochastic rounding: 13 uniform bits added below the 10 kept mantissa
     // bits, then truncation (unbiased; rounding errors do not correlate from
@@ -104,7 +107,7 @@ struct St<__nv_bfloat16> {
     __device__ static C ld(const __nv_bfloat16* p, float inv) {
         return __bfloat162float(__ldg(p)) * inv;
     }
-    __device__ static __nv_bfloat16 raw(const __nv_bfloat16* p) { return __ldg(p); }
+    __device__ static __nv_bfloat16 raw(const __nv_bfloat16* p) { return __ldcg(p); }
     __device__ static __nv_bfloat16 raw_rw(const __nv_bfloat16* p) { return *p; }
     __device__ static void st_sr(__nv_bfloat16* p, C v, float sc, unsigned r) {
         *p = __float2bfloat16_rz(__uint_as_float(__float_as_uint(v * sc) + (r >> 16)));
@@ -308,10 +311,10 @@ template <typename S, bool FIRST, typename IDX, bool SR = false, bool SWAP_STORE
 __device__ __forceinline__ void lid_cell_from(int i, int j, int k, const S (&raw)[Q19],
                                               S* __restrict__ fout,
                                               const StepK<typename St<S>::C>& K, IDX P,
-                                              const double* __restrict__ mrho,
-                                              const double* __restrict__ mu,
-                                              const double* __restrict__ mv,
-                                              const double* __restrict__ mw, unsigned seed) {
+                                              const double* mrho,
+                                              const double* mu,
+                                              const double* mv,
+                                              const double* mw, unsigned seed) {
     using C = typename St<S>::C;
     const int nx = K.nx, ny = K.ny, nz = K.nz;
     const IDX cell = (IDX)i + (IDX)nx * ((IDX)j + (IDX)ny * (IDX)k);
@@ -443,7 +446,7 @@ __device__ __forceinline__ void lid_cell_from(int i, int j, int k, const S (&raw
 }
 
 template <typename S, typename IDX>
-__device__ __forceinline__ void lid_load(int i, int j, int k, const S* __restrict__ fin, int nx,
+__device__ __forceinline__ void lid_load(int i, int j, int k, const S* fin, int nx,
                                          int ny, IDX P, S (&raw)[Q19]) {
     const IDX cell = (IDX)i + (IDX)nx * ((IDX)j + (IDX)ny * (IDX)k);
 #pragma unroll
@@ -489,12 +492,12 @@ __device__ __forceinline__ void lid_load_aa(int i, int j, int k, const S* f, int
 }
 
 template <typename S, bool FIRST, typename IDX, bool SR = false>
-__device__ __forceinline__ void lid_cell(int i, int j, int k, const S* __restrict__ fin,
+__device__ __forceinline__ void lid_cell(int i, int j, int k, const S* fin,
                                          S* __restrict__ fout, const StepK<typename St<S>::C>& K,
-                                         IDX P, const double* __restrict__ mrho,
-                                         const double* __restrict__ mu,
-                                         const double* __restrict__ mv,
-                                         const double* __restrict__ mw, unsigned seed) {
+                                         IDX P, const double* mrho,
+                                         const double* mu,
+                                         const double* mv,
+                                         const double* mw, unsigned seed) {
     S raw[Q19];  // every load is issued before the first conversion
     lid_load<S, IDX>(i, j, k, fin, K.nx, K.ny, P, raw);
     lid_cell_from<S, FIRST, IDX, SR>(i, j, k, raw, fout, K, P, mrho, mu, mv, mw, seed);
@@ -529,8 +532,8 @@ __device__ __forceinline__ void thermal_cell_from(
     int i, int j, int k, typename St<S>::C (&f)[Q19], typename St<S>::C (&g)[Q7],
     const typename St<S>::C (&fp)[3], S* __restrict__ fout, typename St<S>::C* __restrict__ gout,
     typename St<S>::C* __restrict__ F, const StepK<typename St<S>::C>& K, IDX P,
-    const double* __restrict__ mrho, const double* __restrict__ mu, const double* __restrict__ mv,
-    const double* __restrict__ mw, const double* __restrict__ mT, IDX fz_off, unsigned seed) {
+    const double* mrho, const double* mu, const double* mv,
+    const double* mw, const double* mT, IDX fz_off, unsigned seed) {
     // F holds F_x, F_y at planes 0 and 1 (rotation only) and F_z at element offset fz_off
     using C = typename St<S>::C;
     const int nx = K.nx, ny = K.ny, nz = K.nz;
@@ -776,11 +779,11 @@ __device__ __forceinline__ void thermal_cell_from(
 
 template <typename S, bool FIRST, bool ROT, typename IDX, bool SR = false>
 __device__ __forceinline__ void thermal_cell(
-    int i, int j, int k, const S* __restrict__ fin, S* __restrict__ fout,
-    const typename St<S>::C* __restrict__ gin, typename St<S>::C* __restrict__ gout,
+    int i, int j, int k, const S* fin, S* __restrict__ fout,
+    const typename St<S>::C* gin, typename St<S>::C* __restrict__ gout,
     typename St<S>::C* __restrict__ F, const StepK<typename St<S>::C>& K, IDX P,
-    const double* __restrict__ mrho, const double* __restrict__ mu, const double* __restrict__ mv,
-    const double* __restrict__ mw, const double* __restrict__ mT, IDX fz_off, unsigned seed) {
+    const double* mrho, const double* mu, const double* mv,
+    const double* mw, const double* mT, IDX fz_off, unsigned seed) {
     using C = typename St<S>::C;
     const IDX cell = (IDX)i + (IDX)K.nx * ((IDX)j + (IDX)K.ny * (IDX)k);
     // every load is issued before the first conversion (as in lid_cell):
