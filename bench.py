@@ -1026,7 +1026,7 @@ def main():
         "metric": METRIC, "value": round(value, 3), "unit": "MLUPS", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(ms_step, 4),
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": {"fp64": "f64", "fx64": "i64 Q61 fixed point (f64 storage)"}.get(args.form, "f32"),
+        "dtype": "f64" if args.form in ("fp64", "fx64") else "f32",
         "data": wl.get("data", "synthetic (analytic cavity initial state, no dataset)"),
         "config": mglc_config(wl, args.form, world, args.in_place),
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",

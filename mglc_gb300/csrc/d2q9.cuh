@@ -5,7 +5,7 @@
 // warp's instruction holds the SM's unit for 16 clocks or more), so the fast
 // path writes the statements with as few FP64 instructions as give the same bits:
 // 108 a node with the quotients of the macro (ncu), where the statements as written
-// took about 210 (2-D cavity, 1024^2: 404 us a step as written, 331 with
+// took about 190 (2-D cavity, 1024^2: 404 us a step as written, 331 with
 // the first three of these, 221 with all; 22 are its bytes):
 //  * products by 2, 4, 1/2 and 1/4 are exact, so a sum with one is a single
 //    fused multiply-add with the same rounding, and a chain of sums of doubled

@@ -52,8 +52,8 @@ __device__ __forceinline__ float to_f(float v) { return v; }
 __device__ __forceinline__ float to_f(__half v) { return __half2float(v); }
 __device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// macro64.cuh: 384^3 FP64 in about 3.5 ms (its traffic is 1.5 ms of HBM), 11 ms
-// with every addition on the FP64 pipe; 256^3 FP16 1.7 ms against 4.0
+// macro64.cuh: 384^3 FP64 in 2.6 ms (its traffic is 1.5 ms of HBM), 11 ms with every
+// addition on the FP64 pipe; 256^3 FP16 0.48 ms against 1.03
 // ORDERED (reduced forms): every addition in FP64 and in the reference's order,
 // for the fields that the first step after a load starts from (another rounding
 // of them, however small, and the 16-bit stores round otherwise from there on)

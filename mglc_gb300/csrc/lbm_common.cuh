@@ -657,8 +657,8 @@ __device__ __forceinline__ void pair_collide_lid(double* f, double rho, double j
 }
 
 // the forced collision (trt_collide_forced): J = rho u = j + Fp/2, F this
-// step's force, dF = F - Fp (DF: not zero); ROT: F_x, F_y are not zero
-template <bool ROT, bool DF>
+// step's force, dF = F - Fp; ROT: F_x, F_y are not zero
+template <bool ROT>
 __device__ __forceinline__ void pair_collide_forced(double* f, double rho, double Jx, double Jy,
                                                     double Jz, double ux, double uy, double uz,
                                                     double fx, double fy, double fz, double dfx,
@@ -681,8 +681,8 @@ __device__ __forceinline__ void pair_collide_forced(double* f, double rho, doubl
         wx = wx + k.kw6 * fx;
         wy = wy + k.kw6 * fy;
     }
-    double wz = Jz * k.lo6 + k.kw6 * fz, az;
-    if (DF && ROT) {
+    double wz = Jz * k.lo6 + k.kw6 * fz;
+    if (ROT) {
         ax = 2.0 * wx + k.lo10 * dfx;
         ay = 2.0 * wy + k.lo10 * dfy;
         wx = wx + k.lo10 * dfx;
@@ -691,12 +691,8 @@ __device__ __forceinline__ void pair_collide_forced(double* f, double rho, doubl
         ax = 2.0 * wx;
         ay = 2.0 * wy;
     }
-    if (DF) {
-        az = 2.0 * wz + k.lo10 * dfz;
-        wz = wz + k.lo10 * dfz;
-    } else {
-        az = 2.0 * wz;
-    }
+    const double az = 2.0 * wz + k.lo10 * dfz;
+    wz = wz + k.lo10 * dfz;
     f[0] = k.om * f[0] + 12.0 * b;
     pair_out(f, 1, 2, k.c1, k.c2, b2 + 2.0 * X, ax);
     pair_out(f, 3, 4, k.c1, k.c2, b2 + 2.0 * Y, ay);

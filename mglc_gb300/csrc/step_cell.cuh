@@ -643,7 +643,7 @@ __device__ __forceinline__ void thermal_cell_from(
                                                  fy + 2.0 * (jy - rho * uy),
                                                  fz + 2.0 * (jz - rho * uz), K.c, rf - rho);
             } else {
-                pair_collide_forced<ROT, true>(f, rho, jx + 0.5 * fxp, jy + 0.5 * fyp,
+                pair_collide_forced<ROT>(f, rho, jx + 0.5 * fxp, jy + 0.5 * fyp,
                                                jz + 0.5 * fzp, ux, uy, uz, fx, fy, fz, fx - fxp,
                                                fy - fyp, fz - fzp, K.pk);
             }
